@@ -610,7 +610,9 @@ using namespace tplr_tc;
 
 constexpr int TC_A_TILE = 128 * 128;          // bytes: 128 rows x 64 bf16
 constexpr int TC_B_TILE = 64 * 128;           // bytes: 64 rows x 64 bf16
-constexpr int TC_ACC_BYTES = 2 * 4096 * 8;    // two chunks: fp32 sums + int counts = 64 KB
+// two chunks: fp32 sums and 16-bit counts (32 peers that name one place 64 times each make 2048) = 48 KB, the size of the
+// three operand tiles that take their place, so that three CTAs fit an SM
+constexpr int TC_ACC_BYTES = 2 * 4096 * 6;
 constexpr int TC_SMEM_AGG = TC_ACC_BYTES + 3 * TC_B_TILE + 1024;
 
 __device__ __forceinline__ void split3(float x, __nv_bfloat16& b1, __nv_bfloat16& b2, __nv_bfloat16& b3) {
@@ -692,7 +694,7 @@ __device__ __forceinline__ void issue_split_gemm(uint32_t tD, uint32_t sA, uint3
   }
 }
 
-__global__ void __launch_bounds__(NT, 2) aggregate_tc_kernel(const AggArgs a) {
+__global__ void __launch_bounds__(NT, 3) aggregate_tc_kernel(const AggArgs a) {
   extern __shared__ uint8_t smem_raw_tc[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw_tc) + 1023) & ~(uintptr_t)1023);
   __shared__ __align__(8) uint64_t bar_mma;
@@ -702,7 +704,8 @@ __global__ void __launch_bounds__(NT, 2) aggregate_tc_kernel(const AggArgs a) {
   __shared__ long long s_gbase[2];                                 // element offset of each chunk of the pair, -1: none
   __shared__ int s_cols[2], s_skip[2];
   float* S = reinterpret_cast<float*>(smem);                       // [2][4096] sums, later the A tiles
-  int* Cnt = reinterpret_cast<int*>(smem + 2 * 4096 * 4);          // [2][4096] contributor counts
+  unsigned int* Cnt = reinterpret_cast<unsigned int*>(smem + 2 * 4096 * 4);        // [2][4096] contributor counts, two to a word
+  const unsigned short* Cnt16 = reinterpret_cast<const unsigned short*>(Cnt);
   const uint32_t sA = smem_u32(smem), sB = sA + TC_ACC_BYTES;
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -729,7 +732,9 @@ __global__ void __launch_bounds__(NT, 2) aggregate_tc_kernel(const AggArgs a) {
   const uint32_t tZ = s_tmem_base, tG = s_tmem_base + 64;
   const int n_pairs = (a.total_chunks + 1) / 2;
   bool ok = true;
-  TplrParamDesc d = a.descs[0];
+  const TplrParamDesc& d = s_desc[ch];                             // in shared memory: 20 registers a thread otherwise
+  if (tid < 2) s_desc[tid] = a.descs[0];
+  __syncthreads();
 
   // One pair ahead: thread t owns scatter task t of a pair (chunk of the pair, peer, index pair) and holds
   // that task's raw bytes for the NEXT pair in registers, so the dependent chain packed index -> value ->
@@ -779,28 +784,24 @@ __global__ void __launch_bounds__(NT, 2) aggregate_tc_kernel(const AggArgs a) {
     // this thread's chunk of the pair
     const int c = 2 * q + ch;
     const bool active = c < a.total_chunks;
-    {
+    __syncthreads();                                   // previous pair's tiles, accumulators and entries are done with
+    if (rin == 0 && hf == 0) {
       // consecutive chunks mostly belong to the same tensor: search the table only when the cached entry misses
       const int cc = active ? c : a.total_chunks - 1;
-      if (!(cc >= d.chunk_begin && cc < d.chunk_begin + d.n_chunks)) d = a.descs[find_desc(a.descs, a.n_desc, cc)];
-    }
-    const int cl = c - d.chunk_begin;
-    const int cy = d.chunk_row0 + cl / d.chunks_x, cx = cl % d.chunks_x;
-    const long long base = d.elem_off + (long long)cy * 64 * d.cols + (long long)cx * 64;
-    const bool skipped = a.skip && a.skip[d.param_id];
-    __syncthreads();                                   // previous pair's tiles and accumulators are free
-    if (rin == 0 && hf == 0) {                         // the scatter and the update below work on both chunks of the pair
-      s_desc[ch] = d;
-      s_gbase[ch] = active ? base : -1;
+      if (!(cc >= d.chunk_begin && cc < d.chunk_begin + d.n_chunks)) s_desc[ch] = a.descs[find_desc(a.descs, a.n_desc, cc)];
+      const int cl = c - d.chunk_begin;
+      s_gbase[ch] = active ? d.elem_off + (long long)(d.chunk_row0 + cl / d.chunks_x) * 64 * d.cols + (long long)(cl % d.chunks_x) * 64 : -1;
       s_cols[ch] = d.cols;
-      s_skip[ch] = skipped ? 1 : 0;
+      s_skip[ch] = a.skip && a.skip[d.param_id] ? 1 : 0;
     }
+    for (int i = tid; i < TC_ACC_BYTES / 16; i += NT) reinterpret_cast<uint4*>(smem)[i] = make_uint4(0, 0, 0, 0);
+    __syncthreads();
     if (d.fh_off != cur_f) {                           // uniform: every 64 x 64 chunk uses the same basis
       load_basis_split(a.basis + d.fh_off, sB);
       cur_f = d.fh_off;
     }
-    for (int i = tid; i < TC_ACC_BYTES / 16; i += NT) reinterpret_cast<uint4*>(smem)[i] = make_uint4(0, 0, 0, 0);
-    __syncthreads();
+    if (active && a.update_mode != 2)                  // this thread's 128 bytes of the snapshot, used after the second product
+      asm volatile("prefetch.global.L2 [%0];" ::"l"(a.theta0 + s_gbase[ch] + (long long)rin * d.cols + hf * 32));
     // ---- pull + unpack + scale + scatter-add, both chunks --------------------------------
     if (ahead) {
       if (pf_valid) {                                  // this thread's task of the pair, fetched one pair ago
@@ -817,8 +818,8 @@ __global__ void __launch_bounds__(NT, 2) aggregate_tc_kernel(const AggArgs a) {
           v0 = qt[min((int)pf_r0, a.n_bins - 1)] + shift; v1 = qt[min((int)pf_r1, a.n_bins - 1)] + shift;
         }
         v0 *= pf_sc; v1 *= pf_sc;
-        atomicAdd(&S[pf_c2 * 4096 + i0], v0); atomicAdd(&Cnt[pf_c2 * 4096 + i0], 1);
-        atomicAdd(&S[pf_c2 * 4096 + i1], v1); atomicAdd(&Cnt[pf_c2 * 4096 + i1], 1);
+        atomicAdd(&S[pf_c2 * 4096 + i0], v0); atomicAdd(&Cnt[pf_c2 * 2048 + (i0 >> 1)], 1u << ((i0 & 1) * 16));
+        atomicAdd(&S[pf_c2 * 4096 + i1], v1); atomicAdd(&Cnt[pf_c2 * 2048 + (i1 >> 1)], 1u << ((i1 & 1) * 16));
       }
       fetch_ahead(q + gridDim.x);
     }
@@ -841,8 +842,8 @@ __global__ void __launch_bounds__(NT, 2) aggregate_tc_kernel(const AggArgs a) {
         const float sc = a.clip ? a.clip[(long long)peer * a.n_params + d2.param_id] : 1.f;
         const float v0 = load_val(a.pp.val[peer], vo, a.val_dtype, qt, a.n_bins) * sc;
         const float v1 = load_val(a.pp.val[peer], vo + 1, a.val_dtype, qt, a.n_bins) * sc;
-        atomicAdd(&S[c2 * 4096 + i0], v0); atomicAdd(&Cnt[c2 * 4096 + i0], 1);   // 12-bit indices: always < 4096
-        atomicAdd(&S[c2 * 4096 + i1], v1); atomicAdd(&Cnt[c2 * 4096 + i1], 1);
+        atomicAdd(&S[c2 * 4096 + i0], v0); atomicAdd(&Cnt[c2 * 2048 + (i0 >> 1)], 1u << ((i0 & 1) * 16));   // 12-bit indices: always < 4096
+        atomicAdd(&S[c2 * 4096 + i1], v1); atomicAdd(&Cnt[c2 * 2048 + (i1 >> 1)], 1u << ((i1 & 1) * 16));
       }
     }
     __syncthreads();
@@ -852,7 +853,7 @@ __global__ void __launch_bounds__(NT, 2) aggregate_tc_kernel(const AggArgs a) {
     for (int e = 0; e < 32; ++e) {
       const int n = hf * 32 + e;
       const float s = S[ch * 4096 + n * 64 + rin];
-      const int cnt = Cnt[ch * 4096 + n * 64 + rin];
+      const int cnt = Cnt16[ch * 4096 + n * 64 + rin];
       v[e] = cnt > 1 ? s / (float)cnt : s;
     }
     __syncthreads();                                   // accumulators are read out: their bytes become the A tiles
@@ -865,7 +866,7 @@ __global__ void __launch_bounds__(NT, 2) aggregate_tc_kernel(const AggArgs a) {
       issue_split_gemm(tZ, sA, sB, /*a_mn=*/false, /*b_mn=*/true);      // Z = S^T F
       umma_commit(smem_u32(&bar_mma));
     }
-    ok = mbar_wait(smem_u32(&bar_mma), phase, abort_flag);
+    ok = warp != 0 || mbar_wait(smem_u32(&bar_mma), phase, abort_flag);      // one warp polls, the barrier releases the others
     phase ^= 1;
     ok = __syncthreads_and(ok);
     if (!ok) break;
@@ -880,18 +881,8 @@ __global__ void __launch_bounds__(NT, 2) aggregate_tc_kernel(const AggArgs a) {
     store_split_row(sA + (uint32_t)ch * 8192u, TC_A_TILE, rin, hf, v);
     // The update runs in a row-contiguous mapping: half a warp per row of the stacked 128 x 64 result, 16 bytes
     // per lane, so that every global access of a warp covers two whole 256-byte rows (the accumulator mapping,
-    // one row per lane, touches 32 lines per instruction).  The snapshot values are requested here and used
-    // after the second product.
+    // one row per lane, touches 32 lines per instruction).
     const int urow = tid >> 4, uc4 = tid & 15;
-    float4 t0r[8];
-    if (a.update_mode != 2) {
-#pragma unroll
-      for (int i = 0; i < 8; ++i) {
-        const int row = i * 16 + urow, c2 = row >> 6;
-        const long long gb = s_gbase[c2];
-        if (gb >= 0) t0r[i] = *reinterpret_cast<const float4*>(a.theta0 + gb + (long long)(row & 63) * s_cols[c2] + uc4 * 4);
-      }
-    }
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     tcgen05_fence_before();
     __syncthreads();
@@ -900,7 +891,7 @@ __global__ void __launch_bounds__(NT, 2) aggregate_tc_kernel(const AggArgs a) {
       issue_split_gemm(tG, sA, sB, /*a_mn=*/true, /*b_mn=*/true);       // g = Z^T F
       umma_commit(smem_u32(&bar_mma));
     }
-    ok = mbar_wait(smem_u32(&bar_mma), phase, abort_flag);
+    ok = warp != 0 || mbar_wait(smem_u32(&bar_mma), phase, abort_flag);      // one warp polls, the barrier releases the others
     phase ^= 1;
     ok = __syncthreads_and(ok);
     if (!ok) break;
@@ -920,8 +911,17 @@ __global__ void __launch_bounds__(NT, 2) aggregate_tc_kernel(const AggArgs a) {
                      "r"(gr[4 * q4 + 1]), "r"(gr[4 * q4 + 2]), "r"(gr[4 * q4 + 3]) : "memory");
     }
     __syncthreads();
+    float4 t0r[4];
 #pragma unroll
     for (int i = 0; i < 8; ++i) {
+      if ((i & 3) == 0 && a.update_mode != 2) {        // the snapshot's rows, asked into L2 at the start of the pair
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+          const int row = (i + u) * 16 + urow;
+          const long long gb = s_gbase[row >> 6];
+          if (gb >= 0) t0r[u] = *reinterpret_cast<const float4*>(a.theta0 + gb + (long long)(row & 63) * s_cols[row >> 6] + uc4 * 4);
+        }
+      }
       const int row = i * 16 + urow, c2 = row >> 6;
       const long long gb = s_gbase[c2];
       if (gb < 0) continue;
@@ -936,7 +936,7 @@ __global__ void __launch_bounds__(NT, 2) aggregate_tc_kernel(const AggArgs a) {
       if (skp) { gv[0] = gv[1] = gv[2] = gv[3] = 0.f; }
       if (a.grad_out) *reinterpret_cast<float4*>(a.grad_out + g0) = make_float4(gv[0], gv[1], gv[2], gv[3]);
       if (a.update_mode != 2) {
-        const float tv[4] = {t0r[i].x, t0r[i].y, t0r[i].z, t0r[i].w};
+        const float tv[4] = {t0r[i & 3].x, t0r[i & 3].y, t0r[i & 3].z, t0r[i & 3].w};
         float o[4];
 #pragma unroll
         for (int e = 0; e < 4; ++e) {
@@ -1396,7 +1396,7 @@ TPLR_API int tplr_aggregate_apply_tc(const void* descs, int n_desc, int total_ch
   for (int i = 0; i < n_peers; ++i) { a.pp.idx[i] = (const uint8_t*)idx_ptrs[i]; a.pp.val[i] = val_ptrs[i]; }
   cudaError_t err = cudaFuncSetAttribute(aggregate_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, TC_SMEM_AGG);
   if (err != cudaSuccess) return (int)err;
-  int grid = tplr_sm_count() * 2;
+  int grid = tplr_sm_count() * 3;
   const int n_pairs = (total_chunks + 1) / 2;
   if (grid > n_pairs) grid = n_pairs;
   aggregate_tc_kernel<<<grid, NT, TC_SMEM_AGG, (cudaStream_t)stream>>>(a);
