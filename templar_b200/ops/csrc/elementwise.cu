@@ -28,138 +28,6 @@ static __device__ __forceinline__ bf16x8 pack8(const float* f) {
 }
 
 // ------------------------------------------------------------------------------------- //
-// RMSNorm: one CTA per row, 8 bf16 per thread per trip, row cached in registers (D <= 8192)
-// ------------------------------------------------------------------------------------- //
-#define RMS_MAXV 4
-__global__ void __launch_bounds__(256) rmsnorm_fwd_kernel(const bf16* __restrict__ x, const bf16* __restrict__ w,
-                                                          bf16* __restrict__ y, float* __restrict__ rstd,
-                                                          int D, float eps) {
-  __shared__ float red[32];
-  const long long row = blockIdx.x;
-  const bf16x8* xr = reinterpret_cast<const bf16x8*>(x + row * D);
-  const bf16x8* wr = reinterpret_cast<const bf16x8*>(w);
-  bf16x8* yr = reinterpret_cast<bf16x8*>(y + row * D);
-  const int nv = D / 8;
-  float xv[RMS_MAXV][8];
-  float ss = 0.f;
-#pragma unroll
-  for (int j = 0; j < RMS_MAXV; ++j) {
-    const int i = threadIdx.x + j * 256;
-    if (i < nv) {
-      unpack8(xr[i], xv[j]);
-#pragma unroll
-      for (int e = 0; e < 8; ++e) ss = fmaf(xv[j][e], xv[j][e], ss);
-    }
-  }
-  for (int i = threadIdx.x + RMS_MAXV * 256; i < nv; i += 256) {
-    float t[8]; unpack8(xr[i], t);
-#pragma unroll
-    for (int e = 0; e < 8; ++e) ss = fmaf(t[e], t[e], ss);
-  }
-  ss = block_sum(ss, red);
-  const float r = rsqrtf(ss / (float)D + eps);
-  if (threadIdx.x == 0 && rstd) rstd[row] = r;
-#pragma unroll
-  for (int j = 0; j < RMS_MAXV; ++j) {
-    const int i = threadIdx.x + j * 256;
-    if (i < nv) {
-      float wv[8], o[8]; unpack8(wr[i], wv);
-#pragma unroll
-      for (int e = 0; e < 8; ++e) o[e] = xv[j][e] * r * wv[e];
-      yr[i] = pack8(o);
-    }
-  }
-  for (int i = threadIdx.x + RMS_MAXV * 256; i < nv; i += 256) {
-    float t[8], wv[8], o[8]; unpack8(xr[i], t); unpack8(wr[i], wv);
-#pragma unroll
-    for (int e = 0; e < 8; ++e) o[e] = t[e] * r * wv[e];
-    yr[i] = pack8(o);
-  }
-}
-
-TPLR_API int tplr_rmsnorm_fwd(const void* x, const void* w, void* y, float* rstd, long long T, int D,
-                              float eps, void* stream) {
-  TPLR_ENTER();
-  if (D % 8) return (int)cudaErrorInvalidValue;
-  if (T <= 0) return 0;
-  rmsnorm_fwd_kernel<<<(unsigned)T, 256, 0, (cudaStream_t)stream>>>((const bf16*)x, (const bf16*)w, (bf16*)y, rstd, D, eps);
-  return (int)cudaGetLastError();
-}
-
-// dx = rstd * (g - xhat * mean(g * xhat)),  g = dy * w, xhat = x * rstd;  dw += sum_rows dy * xhat.
-// Persistent CTAs walk rows with stride gridDim.x; each thread owns fixed columns so the dw
-// partial stays in registers and is flushed once with fp32 atomics. D <= 8192.
-__global__ void __launch_bounds__(256) rmsnorm_bwd_kernel(const bf16* __restrict__ dy, const bf16* __restrict__ x,
-                                                          const bf16* __restrict__ w, const float* __restrict__ rstd,
-                                                          bf16* __restrict__ dx, float* __restrict__ dw,
-                                                          long long T, int D) {
-  __shared__ float red[32];
-  const int nv = D / 8;
-  float wv[RMS_MAXV][8], dwv[RMS_MAXV][8];
-#pragma unroll
-  for (int j = 0; j < RMS_MAXV; ++j) {
-    const int i = threadIdx.x + j * 256;
-#pragma unroll
-    for (int e = 0; e < 8; ++e) { dwv[j][e] = 0.f; wv[j][e] = 0.f; }
-    if (i < nv) unpack8(reinterpret_cast<const bf16x8*>(w)[i], wv[j]);
-  }
-  for (long long row = blockIdx.x; row < T; row += gridDim.x) {
-    const bf16x8* xr = reinterpret_cast<const bf16x8*>(x + row * D);
-    const bf16x8* gr = reinterpret_cast<const bf16x8*>(dy + row * D);
-    bf16x8* dr = reinterpret_cast<bf16x8*>(dx + row * D);
-    const float r = rstd[row];
-    float xh[RMS_MAXV][8], g[RMS_MAXV][8];
-    float dot = 0.f;
-#pragma unroll
-    for (int j = 0; j < RMS_MAXV; ++j) {
-      const int i = threadIdx.x + j * 256;
-      if (i < nv) {
-        float xv[8], dv[8]; unpack8(xr[i], xv); unpack8(gr[i], dv);
-#pragma unroll
-        for (int e = 0; e < 8; ++e) {
-          xh[j][e] = xv[e] * r;
-          g[j][e] = dv[e] * wv[j][e];
-          dwv[j][e] = fmaf(dv[e], xh[j][e], dwv[j][e]);
-          dot = fmaf(g[j][e], xh[j][e], dot);
-        }
-      }
-    }
-    dot = block_sum(dot, red) / (float)D;
-#pragma unroll
-    for (int j = 0; j < RMS_MAXV; ++j) {
-      const int i = threadIdx.x + j * 256;
-      if (i < nv) {
-        float o[8];
-#pragma unroll
-        for (int e = 0; e < 8; ++e) o[e] = r * (g[j][e] - xh[j][e] * dot);
-        dr[i] = pack8(o);
-      }
-    }
-  }
-  if (dw) {
-#pragma unroll
-    for (int j = 0; j < RMS_MAXV; ++j) {
-      const int i = threadIdx.x + j * 256;
-      if (i < nv)
-#pragma unroll
-        for (int e = 0; e < 8; ++e) atomicAdd(dw + i * 8 + e, dwv[j][e]);
-    }
-  }
-}
-
-TPLR_API int tplr_rmsnorm_bwd(const void* dy, const void* x, const void* w, const float* rstd, void* dx,
-                              float* dw, long long T, int D, void* stream) {
-  TPLR_ENTER();
-  if (D % 8 || D > RMS_MAXV * 256 * 8) return (int)cudaErrorInvalidValue;
-  if (T <= 0) return 0;
-  long long grid = tplr_sm_count() * 4;
-  if (grid > T) grid = T;
-  rmsnorm_bwd_kernel<<<(unsigned)grid, 256, 0, (cudaStream_t)stream>>>((const bf16*)dy, (const bf16*)x, (const bf16*)w,
-                                                                      rstd, (bf16*)dx, dw, T, D);
-  return (int)cudaGetLastError();
-}
-
-// ------------------------------------------------------------------------------------- //
 // Residual add fused with RMSNorm, one warp per row (D <= 2048): no block barrier, 8 rows in
 // flight per CTA.
 //   forward   h = res + delta (delta may be null: h = res);  y = h * rstd(h) * w;  h written when delta != null
@@ -295,11 +163,16 @@ __global__ void __launch_bounds__(256) add_rmsnorm_bwd_warp_kernel(const bf16* _
   }
 }
 
-// T rows of D (multiple of 8, <= 2048) bf16.  delta may be null (plain RMSNorm, h_out unused).
+extern "C" int tplr_add_rmsnorm_fwd_wide(const void* res, const void* delta, const void* w, void* h_out, void* y, float* rstd,
+                                         long long T, int D, float eps, void* stream);
+
+// T rows of D (multiple of 8, <= 8192) bf16.  delta may be null (plain RMSNorm, h_out unused).  Rows above 2048 elements
+// do not fit a warp's registers: several warps share one there.
 TPLR_API int tplr_add_rmsnorm_fwd(const void* res, const void* delta, const void* w, void* h_out, void* y, float* rstd,
                                   long long T, int D, float eps, void* stream) {
   TPLR_ENTER();
-  if (D % 8 || D > 2048) return (int)cudaErrorInvalidValue;
+  if (D > 2048) return tplr_add_rmsnorm_fwd_wide(res, delta, w, h_out, y, rstd, T, D, eps, stream);
+  if (D % 8) return (int)cudaErrorInvalidValue;
   if (T <= 0) return 0;
   const int vpl = (D / 8 + 31) / 32;
   const unsigned grid = (unsigned)((T + 7) / 8);

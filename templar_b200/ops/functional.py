@@ -186,14 +186,8 @@ class _RMSNorm(torch.autograd.Function):
             T = xc.numel() // xc.shape[-1]
             y = torch.empty_like(xc)
             rstd = torch.empty(T, dtype=torch.float32, device=x.device)
-            if xc.shape[-1] <= 2048:
-                # rows of up to 2048 elements: the warp-per-row kernel (eight rows in flight per CTA, no block barrier)
-                # with no residual to add; measured 1.6x the CTA-per-row kernel's rate at D = 2048
-                native.check(native.lib().tplr_add_rmsnorm_fwd(xc.data_ptr(), None, w.data_ptr(), None, y.data_ptr(),
-                                                               rstd.data_ptr(), T, xc.shape[-1], eps, native.stream_ptr()),
-                             "rmsnorm_fwd")
-            else:
-                native.check(native.lib().tplr_rmsnorm_fwd(xc.data_ptr(), w.data_ptr(), y.data_ptr(), rstd.data_ptr(),
+            # the residual-add kernel with nothing to add
+            native.check(native.lib().tplr_add_rmsnorm_fwd(xc.data_ptr(), None, w.data_ptr(), None, y.data_ptr(), rstd.data_ptr(),
                                                            T, xc.shape[-1], eps, native.stream_ptr()), "rmsnorm_fwd")
             ctx.native = True
             ctx.save_for_backward(xc, w, rstd)
@@ -213,15 +207,10 @@ class _RMSNorm(torch.autograd.Function):
             T, D = x.numel() // x.shape[-1], x.shape[-1]
             dx = torch.empty_like(x)
             dw_buf = mg if mg is not None else torch.zeros(D, dtype=torch.float32, device=x.device)
-            if D <= 2048:
-                native.check(native.lib().tplr_add_rmsnorm_bwd_v2(dyc.data_ptr(), x.data_ptr(), w.data_ptr(), rstd.data_ptr(), None,
-                                                                  dx.data_ptr(), dw_buf.data_ptr(), T, D,
-                                                                  status_word(x.device).data_ptr(), native.stream_ptr()),
-                             "rmsnorm_bwd")
-            else:
-                native.check(native.lib().tplr_rmsnorm_bwd(dyc.data_ptr(), x.data_ptr(), w.data_ptr(), rstd.data_ptr(),
-                                                           dx.data_ptr(), dw_buf.data_ptr(), T, D, native.stream_ptr()),
-                             "rmsnorm_bwd")
+            native.check(native.lib().tplr_add_rmsnorm_bwd_v2(dyc.data_ptr(), x.data_ptr(), w.data_ptr(), rstd.data_ptr(), None,
+                                                              dx.data_ptr(), dw_buf.data_ptr(), T, D,
+                                                              status_word(x.device).data_ptr(), native.stream_ptr()),
+                         "rmsnorm_bwd")
             return dx, (None if mg is not None else dw_buf.to(w.dtype)), None, None
         xf, g = x.float(), dy.float()
         xh = xf * rstd
@@ -250,30 +239,22 @@ class _AddRMSNorm(torch.autograd.Function):
     def forward(ctx, res, delta, w, eps, main_grad):
         ctx.eps, ctx.main_grad = eps, main_grad
         D = res.shape[-1]
-        if _native_ok(res, delta, w) and D % 8 == 0 and D <= 2048 and res.is_contiguous() and delta.is_contiguous():
-            T = res.numel() // D
-            h = torch.empty_like(res)
-            y = torch.empty_like(res)
-            rstd = torch.empty(T, dtype=torch.float32, device=res.device)
-            native.check(native.lib().tplr_add_rmsnorm_fwd(res.data_ptr(), delta.data_ptr(), w.data_ptr(), h.data_ptr(),
-                                                           y.data_ptr(), rstd.data_ptr(), T, D, eps, native.stream_ptr()),
-                         "add_rmsnorm_fwd")
-            ctx.native = 1
-        elif _native_ok(res, delta, w) and D % 8 == 0 and D <= 8192:
-            # wide rows: eager add, then the one-CTA-per-row norm kernels
-            h = res + delta
+        ctx.native = _native_ok(res, delta, w) and D % 8 == 0 and D <= 8192
+        if ctx.native:
+            fused = res.is_contiguous() and delta.is_contiguous() and res.shape == delta.shape
+            # views and broadcast operands: eager add, then the kernel with nothing to add
+            h = torch.empty_like(res) if fused else (res + delta).contiguous()
             T = h.numel() // D
             y = torch.empty_like(h)
-            rstd = torch.empty(T, dtype=torch.float32, device=res.device)
-            native.check(native.lib().tplr_rmsnorm_fwd(h.data_ptr(), w.data_ptr(), y.data_ptr(), rstd.data_ptr(),
-                                                       T, D, eps, native.stream_ptr()), "rmsnorm_fwd")
-            ctx.native = 2
+            rstd = torch.empty(T, dtype=torch.float32, device=h.device)
+            native.check(native.lib().tplr_add_rmsnorm_fwd(
+                res.data_ptr() if fused else h.data_ptr(), delta.data_ptr() if fused else None, w.data_ptr(),
+                h.data_ptr() if fused else None, y.data_ptr(), rstd.data_ptr(), T, D, eps, native.stream_ptr()), "add_rmsnorm_fwd")
         else:
             h = res + delta
             hf = h.float()
             rstd = torch.rsqrt(hf.pow(2).mean(-1, keepdim=True) + eps)
             y = (hf * rstd * w.float()).to(res.dtype)
-            ctx.native = 0
         ctx.save_for_backward(h, w, rstd)
         return h, y
 
@@ -282,17 +263,6 @@ class _AddRMSNorm(torch.autograd.Function):
         h, w, rstd = ctx.saved_tensors
         mg = ctx.main_grad
         D = h.shape[-1]
-        if ctx.native == 2:
-            T = h.numel() // D
-            dyc = dy.contiguous()
-            dx = torch.empty_like(h)
-            dw_buf = mg if mg is not None else torch.zeros(D, dtype=torch.float32, device=h.device)
-            native.check(native.lib().tplr_rmsnorm_bwd(dyc.data_ptr(), h.data_ptr(), w.data_ptr(), rstd.data_ptr(),
-                                                       dx.data_ptr(), dw_buf.data_ptr(), T, D, native.stream_ptr()),
-                         "rmsnorm_bwd")
-            if dh is not None:
-                dx += dh
-            return dx, dx, (None if mg is not None else dw_buf.to(w.dtype)), None, None
         if ctx.native:
             T = h.numel() // D
             dyc = dy.contiguous()
@@ -642,8 +612,9 @@ class _NormLinear(torch.autograd.Function):
             if ctx.native and x.is_contiguous() and x.shape[-1] <= 8192:
                 xn = torch.empty_like(x)
                 T = x.numel() // x.shape[-1]
-                native.check(native.lib().tplr_rmsnorm_fwd(x.data_ptr(), wn.data_ptr(), xn.data_ptr(), rstd.data_ptr(), T,
-                                                           x.shape[-1], ctx.eps, native.stream_ptr()), "rmsnorm_fwd")
+                native.check(native.lib().tplr_add_rmsnorm_fwd(x.data_ptr(), None, wn.data_ptr(), None, xn.data_ptr(),
+                                                               rstd.data_ptr(), T, x.shape[-1], ctx.eps, native.stream_ptr()),
+                             "rmsnorm_fwd")
             else:
                 xn = (x.float() * rstd.reshape(*x.shape[:-1], 1) * wn.float()).to(x.dtype)
         dw = _weight_grad(ctx.main_grad_w, dy2, xn.reshape(-1, xn.shape[-1]), w, ctx.needs_input_grad[5])

@@ -64,8 +64,6 @@ def _declare(L: ctypes.CDLL) -> None:
         "tplr_requant_residual": [vp, i, i, vp, vp, vp, vp, vp, vp, i, i, i, vp],
         "tplr_compress_chunks_tc": [vp, i, i, vp, vp, vp, vp, vp, vp, vp, f, i, i, i, vp],
         "tplr_aggregate_apply_tc": [vp, i, i, vp, i, vp, vp, i, vp, i, i, vp, vp, vp, vp, vp, vp, f, f, i, vp, vp],
-        "tplr_rmsnorm_fwd": [vp, vp, vp, vp, ll, i, f, vp],
-        "tplr_rmsnorm_bwd": [vp, vp, vp, vp, vp, vp, ll, i, vp],
         "tplr_add_rmsnorm_fwd": [vp, vp, vp, vp, vp, vp, ll, i, f, vp],
         "tplr_add_rmsnorm_bwd": [vp, vp, vp, vp, vp, vp, vp, ll, i, vp],
         "tplr_add_rmsnorm_bwd_v2": [vp, vp, vp, vp, vp, vp, vp, ll, i, vp, vp],

@@ -559,3 +559,32 @@ def test_compress_and_aggregate_are_bitwise_repeatable(quantize):
         runs.append(rec)
     for name in runs[0]:
         assert torch.equal(runs[0][name], runs[1][name]), name
+
+
+@pytest.mark.parametrize("D,T", [(2056, 3), (4096, 1), (4096, 1001), (4104, 2), (6144, 149), (8192, 297)])
+def test_add_rmsnorm_wide_rows(D, T):
+    """Rows above 2048 elements (several warps per row): one and two rows per tile, ragged last tile, ragged last vectors."""
+    torch.manual_seed(D + T)
+    res, delta, dh, dy = (torch.randn(T, D, device=DEV).to(torch.bfloat16) for _ in range(4))
+    w = (1 + 0.1 * torch.randn(D, device=DEV)).to(torch.bfloat16)
+    OF.status_word(DEV).zero_()
+    for fused in (True, False):
+        a, b, ww = (t.clone().requires_grad_() for t in (res, delta, w))
+        rf, wf = (res.float() + delta.float()).to(torch.bfloat16).float().requires_grad_(), w.float().requires_grad_()
+        yr = F.rms_norm(rf, (D,), wf, 1e-5)
+        if fused:
+            h, y = OF.add_rmsnorm(a, b, ww, 1e-5)
+            torch.autograd.backward([h, y], [dh, dy])
+            torch.autograd.backward([rf, yr], [dh.float(), dy.float()])
+            assert torch.equal(h.float(), rf.detach()) and torch.equal(a.grad, b.grad)
+        else:
+            a = rf.detach().to(torch.bfloat16).requires_grad_()
+            y = OF.rmsnorm(a, ww, 1e-5)
+            y.backward(dy)
+            yr.backward(dy.float())
+        # one bf16 rounding (2^-9 relative) of values up to ~6, and of the weight gradient's sum
+        assert torch.allclose(y.float(), yr, atol=1e-3, rtol=2 ** -8)
+        assert torch.allclose(a.grad.float(), rf.grad, atol=2e-3, rtol=2 ** -8)
+        assert torch.allclose(ww.grad.float(), wf.grad, atol=1e-3 * T ** 0.5, rtol=2 ** -8)
+    torch.cuda.synchronize()
+    assert int(OF.status_word(DEV).item()) == 0
