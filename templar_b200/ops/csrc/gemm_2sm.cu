@@ -847,14 +847,36 @@ int dispatch2(Gemm2Params& p, int a_mn, int b_mn, int epi, int n_comm_pairs, int
   return -104;
 }
 
-// Accumulating GEMMs (C += ...) reduce-add their tiles, so K may be cut in two to fill the last wave.
-// Every split costs another M*N*4 bytes of L2 reductions (measured: 4 and 8 splits lose more than the
-// fuller waves win), so K is halved only when that lifts the wave efficiency by more than 10 points.
+// Accumulating GEMMs (C += ...) reduce-add their tiles, so a tile's K range may be cut into several work units that run
+// on different CTA pairs: the one with the fewest "k block times" wins, counting waves of units and 8 k blocks per unit for
+// its pipeline fill and its reduction (fitted on 22 weight-gradient shapes from 768 x 768 to 28672 x 4096, K 333 to 16384).
+// Measured, one split against the chosen number: 768 x 768 x 8192 (9 tiles on 74 pairs) 54.8 -> 21.0 us with 4, 2304 x 768 x
+// 8192 55.4 -> 33.1 with 2, 1536 x 4096 x 4096 62.6 -> 51.5 with 2; where the waves are full already a second split costs
+// 3 to 16 % (8192 x 1536 x 4096 88.3 -> 94.2, 28672 x 4096 x 1024 287 -> 333) and none is made.  A split has to win 5 %.
 int pick_k_splits(int M, int N, int K, int max_pairs) {
   static const int forced = [] { const char* e = getenv("TPLR_GEMM_KSPLITS"); return e ? atoi(e) : 0; }();
-  if (forced > 0) return (K + BK - 1) / BK / forced >= 1 ? forced : 1;   // tuning override
+  const long long kb = (K + BK - 1) / BK;
+  if (forced > 0) return kb / forced >= 1 ? forced : 1;   // tuning override
   int pairs = tplr_sm_count() / 2;
   if (max_pairs > 0 && pairs > max_pairs) pairs = max_pairs;
+  const long long tiles = (long long)((M + TILE_M - 1) / TILE_M) * ((N + TILE_N - 1) / TILE_N);
+  int best = 1;
+  double best_cost = 0.0;
+  for (int ks = 1; ks <= 8 && ks <= kb; ks *= 2) {
+    const long long per = (kb + ks - 1) / ks;
+    if ((ks - 1) * per >= kb) break;                      // every unit has work
+    const double cost = (double)((tiles * ks + pairs - 1) / pairs) * (double)(per + 8);
+    if (ks == 1 || cost < 0.95 * best_cost) { best = ks; best_cost = cost; }
+  }
+  return best;
+}
+
+// The scatter entry's rule: its reductions cross NVLink, so K is only halved, and only where that lifts the wave efficiency
+// by more than 10 points (4 and 8 splits lost more than the fuller waves won).
+int pick_scatter_splits(int M, int N, int K) {
+  static const int forced = [] { const char* e = getenv("TPLR_GEMM_KSPLITS"); return e ? atoi(e) : 0; }();
+  if (forced > 0) return (K + BK - 1) / BK / forced >= 1 ? forced : 1;   // tuning override
+  const int pairs = tplr_sm_count() / 2;
   const long long tiles = (long long)((M + TILE_M - 1) / TILE_M) * ((N + TILE_N - 1) / TILE_N);
   if ((K + BK - 1) / BK < 128) return 1;
   auto eff = [&](long long units) { return (double)units / (double)(((units + pairs - 1) / pairs) * pairs); };
@@ -1089,6 +1111,6 @@ TPLR_API int tplr_gemm2_scatter_v(const void* A, const void* B, int M, int N, in
   const int tiles_m = (M + TILE_M - 1) / TILE_M;
   if (world > 1 && tiles_m % world == 0) p.m_inter = world;
   if (world > 1) p.m_rot = (int)(((long long)rank * tiles_m) / world);
-  p.k_splits = pick_k_splits(M, N, K, 0);
+  p.k_splits = pick_scatter_splits(M, N, K);
   return dispatch2(p, a_mn, b_mn, 1, 0, 0, (cudaStream_t)stream);
 }

@@ -219,3 +219,9 @@ def test_feed_forward_with_both_swiglu_epilogues_matches_fp32_reference(T, D, F,
     errs_s = [rel(ys, ref)] + [rel(g, r.grad) for g, r in zip(gs, (xf, af, bf))]
     assert max(errs_f) < 2e-2, (errs_f, errs_s)
     assert all(a_ < 1.3 * b_ + 1e-3 for a_, b_ in zip(errs_f, errs_s)), (errs_f, errs_s)
+
+
+@pytest.mark.parametrize("M,N,K", [(768, 768, 8192), (264, 520, 4104), (256, 256, 576), (2304, 768, 520)])
+def test_accumulating_gemm_with_k_splits(M, N, K, backend):
+    """Weight-gradient products with few tiles (several work units add into one tile), ragged tiles and a ragged last split."""
+    _check(M, N, K, True, True, "acc")
