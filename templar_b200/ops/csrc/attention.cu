@@ -5,7 +5,9 @@
 //
 // Operands come from the packed projection output [B*S, (H + 2 KV) * 128] (q heads, k heads,
 // v heads; RoPE already applied in place), loaded by TMA with 128-byte swizzle; no copy splits
-// q, k and v.  Head dimension 128, sequence length a multiple of 128, grouped-query heads.
+// q, k and v.  Head dimension 128 or 64 (a template parameter), any sequence length, grouped-query heads.  The maps are
+// three-dimensional (column, position, sequence): the rows of a last block that lie past the end of the sequence read as
+// zeros and are not stored, and no block reads the next sequence.
 //
 // CTA = one 128-row query block of one head: warp 0 TMA producer, warp 1 MMA issuer + TMEM
 // owner, warps 2-5 softmax / correction / epilogue.  256 TMEM columns and 97 KB of shared
@@ -23,15 +25,16 @@
 namespace {
 using namespace tplr_tc;
 
-constexpr int BQ = 128, BKV = 128, DH = 128;
-constexpr int TILE_BYTES = 128 * DH * 2;                 // 32 KB: one 128 x 128 bf16 tile
-constexpr int FWD_SMEM = 3 * TILE_BYTES + 1024;          // Q, K, V
+constexpr int BQ = 128, BKV = 128;
+constexpr int PT_BYTES = 128 * 128 * 2;                  // one 128 x 128 bf16 tile (P, dS)
+template <int DH> constexpr int tile_bytes() { return 128 * DH * 2; }            // one operand tile: 32 KB / 16 KB
+template <int DH> constexpr int fwd_smem() { return 3 * tile_bytes<DH>() + 1024; }   // Q, K, V
 constexpr int FWD_THREADS = 192;
 constexpr float RESCALE_THRESHOLD = 8.0f;                // log2 units
 
 struct AttnFwdParams {
-  CUtensorMap tmQKV;      // [B*S, C] bf16, box 64 x 128, 128-byte swizzle
-  CUtensorMap tmO;        // [B*S, H*128] bf16, box 64 x 32, 128-byte swizzle
+  CUtensorMap tmQKV;      // [B, S, C] bf16, box 64 x 128 x 1, 128-byte swizzle
+  CUtensorMap tmO;        // [B, S, H*DH] bf16, box 64 x 32 x 1, 128-byte swizzle
   float* lse;             // [B, H, S] natural-log sum-exp of the scaled scores
   int B, S, H, KV;
   float scale_log2;       // softmax scale * log2(e)
@@ -61,11 +64,51 @@ __device__ __forceinline__ void tma_store_2d(const CUtensorMap* map, uint32_t sr
   asm volatile("cp.async.bulk.tensor.2d.global.shared::cta.bulk_group [%0, {%2, %3}], [%1];"
                ::"l"(map), "r"(src), "r"(x), "r"(y) : "memory");
 }
+__device__ __forceinline__ void tma_load_3d(uint32_t dst, const CUtensorMap* map, uint32_t bar, int x, int y, int z) {
+  asm volatile(
+      "cp.async.bulk.tensor.3d.shared::cta.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5}], [%2];"
+      ::"r"(dst), "l"(map), "r"(bar), "r"(x), "r"(y), "r"(z) : "memory");
+}
+__device__ __forceinline__ void tma_store_3d(const CUtensorMap* map, uint32_t src, int x, int y, int z) {
+  asm volatile("cp.async.bulk.tensor.3d.global.shared::cta.bulk_group [%0, {%2, %3, %4}], [%1];"
+               ::"l"(map), "r"(src), "r"(x), "r"(y), "r"(z) : "memory");
+}
+// 128 rows x DH columns of one head as DH / 64 boxes of 64 columns
+template <int DH>
+__device__ __forceinline__ void load_tile(uint32_t dst, const CUtensorMap* map, uint32_t bar, int col, int row, int b) {
+#pragma unroll
+  for (int q = 0; q < DH / 64; ++q) tma_load_3d(dst + q * (128 * 128), map, bar, col + 64 * q, row, b);
+}
+// [B, S, inner] tensor map (row stride ld elements, sequence stride S * ld), 128-byte swizzle, box box_inner x box_rows x 1
+inline bool make_map3(CUtensorMap* map, const void* ptr, long long inner, int S, int B, long long ld, int box_inner, int box_rows,
+                      bool fp32 = false) {
+  auto enc = get_encode();
+  if (!enc) return false;
+  const cuuint64_t esz = fp32 ? 4 : 2;
+  cuuint64_t dims[3] = {(cuuint64_t)inner, (cuuint64_t)S, (cuuint64_t)B};
+  cuuint64_t strides[2] = {(cuuint64_t)ld * esz, (cuuint64_t)ld * esz * (cuuint64_t)S};
+  cuuint32_t box[3] = {(cuuint32_t)box_inner, (cuuint32_t)box_rows, 1};
+  cuuint32_t estr[3] = {1, 1, 1};
+  auto call = [&] {
+    return enc(map, fp32 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT32 : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, const_cast<void*>(ptr), dims,
+               strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+               CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  };
+  CUresult r = call();
+  if (r == CUDA_ERROR_INVALID_CONTEXT) {     // a thread that has made no runtime call yet (see make_map)
+    cudaFree(0);
+    r = call();
+  }
+  if (r != CUDA_SUCCESS)
+    fprintf(stderr, "[tplr] cuTensorMapEncodeTiled failed (%d): ptr=%p inner=%lld S=%d B=%d ld=%lld box=%dx%d\n", (int)r, ptr,
+            inner, S, B, ld, box_inner, box_rows);
+  return r == CUDA_SUCCESS;
+}
 
-// instruction descriptor: fp32 accumulate, bf16 A and B, M = 128, N = 128; b_mn selects an N-contiguous B
-__device__ __forceinline__ uint32_t idesc_128x128(bool b_mn) {
-  return (1u << 4) | (1u << 7) | (1u << 10) | ((b_mn ? 1u : 0u) << 16) | ((uint32_t)(128 >> 3) << 17) |
-         ((uint32_t)(128 >> 4) << 24);
+// instruction descriptor: fp32 accumulate, bf16 A and B, M = 128, N = n; a_mn / b_mn select an M- / N-contiguous operand
+__device__ __forceinline__ uint32_t idesc_mn(int n, bool a_mn, bool b_mn) {
+  return (1u << 4) | (1u << 7) | (1u << 10) | ((a_mn ? 1u : 0u) << 15) | ((b_mn ? 1u : 0u) << 16) |
+         ((uint32_t)(n >> 3) << 17) | ((uint32_t)(128 >> 4) << 24);
 }
 
 // Softmax passes over one row of S (128 fp32 columns in tensor memory, lane = query row).  DIAG = the block
@@ -143,8 +186,10 @@ __device__ __forceinline__ float attn_row_exp(uint32_t ts_lane, int r, float sl2
   return s0 + s1;
 }
 
+template <int DH>
 __global__ void __launch_bounds__(FWD_THREADS, 2)
 attn_fwd_kernel(const __grid_constant__ AttnFwdParams p) {
+  constexpr int TILE_BYTES = tile_bytes<DH>();
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
   __shared__ __align__(8) uint64_t bar_q, bar_k_full, bar_k_empty, bar_v_full, bar_v_empty, bar_s_full, bar_p_full, bar_o_full;
@@ -152,14 +197,14 @@ attn_fwd_kernel(const __grid_constant__ AttnFwdParams p) {
   __shared__ int s_abort;
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int nQ = p.S / BQ;
+  const int nQ = (p.S + BQ - 1) / BQ;
   // heavy (late) query blocks first
   const int hb = p.H * p.B;
   const int qi = nQ - 1 - (int)(blockIdx.x / hb);
   const int h = (int)(blockIdx.x % hb) % p.H, b = (int)(blockIdx.x % hb) / p.H;
   const int g = h / (p.H / p.KV);
   const int nb = qi + 1;                                   // causal: kv blocks 0..qi
-  const int row0 = b * p.S + qi * BQ;
+  const int row0 = qi * BQ;                                // position of the first query row; rows past S read as zeros
   const int qcol = h * DH, kcol = (p.H + g) * DH, vcol = (p.H + p.KV + g) * DH;
   volatile int* abort_flag = &s_abort;
 
@@ -187,26 +232,23 @@ attn_fwd_kernel(const __grid_constant__ AttnFwdParams p) {
   if (warp == 0) {
     if (lane == 0) {
       mbar_expect_tx(smem_u32(&bar_q), TILE_BYTES);
-      tma_load_2d(sQ, &p.tmQKV, smem_u32(&bar_q), qcol, row0);
-      tma_load_2d(sQ + TILE_BYTES / 2, &p.tmQKV, smem_u32(&bar_q), qcol + 64, row0);
+      load_tile<DH>(sQ, &p.tmQKV, smem_u32(&bar_q), qcol, row0, b);
       bool ok = true;
       for (int j = 0; j < nb && ok; ++j) {
         const uint32_t ph = j & 1;
-        const int krow = b * p.S + j * BKV;
+        const int krow = j * BKV;
         if (!(ok = mbar_wait(smem_u32(&bar_k_empty), ph ^ 1, abort_flag))) break;
         mbar_expect_tx(smem_u32(&bar_k_full), TILE_BYTES);
-        tma_load_2d(sK, &p.tmQKV, smem_u32(&bar_k_full), kcol, krow);
-        tma_load_2d(sK + TILE_BYTES / 2, &p.tmQKV, smem_u32(&bar_k_full), kcol + 64, krow);
+        load_tile<DH>(sK, &p.tmQKV, smem_u32(&bar_k_full), kcol, krow, b);
         if (!(ok = mbar_wait(smem_u32(&bar_v_empty), ph ^ 1, abort_flag))) break;
         mbar_expect_tx(smem_u32(&bar_v_full), TILE_BYTES);
-        tma_load_2d(sV, &p.tmQKV, smem_u32(&bar_v_full), vcol, krow);
-        tma_load_2d(sV + TILE_BYTES / 2, &p.tmQKV, smem_u32(&bar_v_full), vcol + 64, krow);
+        load_tile<DH>(sV, &p.tmQKV, smem_u32(&bar_v_full), vcol, krow, b);
       }
     }
   } else if (warp == 1) {
     if (lane == 0) {
-      const uint32_t id_qk = idesc_128x128(false), id_pv = idesc_128x128(true);
-      const DescBase bQ = desc_base(sQ, 16, 1024), bK = desc_base(sK, 16, 1024), bV = desc_base(sV, TILE_BYTES / 2, 1024);
+      const uint32_t id_qk = idesc_mn(128, false, false), id_pv = idesc_mn(DH, false, true);
+      const DescBase bQ = desc_base(sQ, 16, 1024), bK = desc_base(sK, 16, 1024), bV = desc_base(sV, 128 * 128, 1024);
       bool ok = mbar_wait(smem_u32(&bar_q), 0, abort_flag);
       for (int j = 0; j < nb && ok; ++j) {
         const uint32_t ph = j & 1;
@@ -214,7 +256,7 @@ attn_fwd_kernel(const __grid_constant__ AttnFwdParams p) {
         tcgen05_fence_after();
 #pragma unroll
         for (int kk = 0; kk < DH / 16; ++kk) {
-          const uint32_t off = (uint32_t)(kk >> 2) * (TILE_BYTES / 32) + (uint32_t)(kk & 3) * 2u;    // 16-byte units
+          const uint32_t off = (uint32_t)(kk >> 2) * (128u * 128u / 16u) + (uint32_t)(kk & 3) * 2u;    // 16-byte units
           umma_bf16_b(tS, bQ, off, bK, off, id_qk, kk > 0 ? 1u : 0u);
         }
         umma_commit(smem_u32(&bar_s_full));
@@ -251,7 +293,7 @@ attn_fwd_kernel(const __grid_constant__ AttnFwdParams p) {
         if (j > 0) {
           // S of block j is complete, so every earlier MMA, PV of block j-1 included, has finished with O
 #pragma unroll 1
-          for (int c = 0; c < 4; ++c) {
+          for (int c = 0; c < DH / 32; ++c) {
             uint32_t v[32];
             tmem_ld32(tO + c * 32 + lane_off, v);
 #pragma unroll
@@ -274,10 +316,11 @@ attn_fwd_kernel(const __grid_constant__ AttnFwdParams p) {
     if (ok) {
       tcgen05_fence_after();
       const float inv_l = 1.f / l;
-      const uint32_t stage = sQ + (uint32_t)quad * 8192u;
+      const uint32_t stage = sQ + (uint32_t)quad * (32u * DH * 2u);
+      const int orow = row0 + quad * 32;
       const uint32_t sw = (uint32_t)(lane & 7);
 #pragma unroll 1
-      for (int c = 0; c < 4; ++c) {
+      for (int c = 0; c < DH / 32; ++c) {
         uint32_t v[32];
         tmem_ld32(tO + c * 32 + lane_off, v);
         const uint32_t rowaddr = stage + (uint32_t)(c >> 1) * 4096u + (uint32_t)lane * 128u;
@@ -297,13 +340,13 @@ attn_fwd_kernel(const __grid_constant__ AttnFwdParams p) {
       }
       asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
       __syncwarp();
-      if (lane == 0) {
-        tma_store_2d(&p.tmO, stage, qcol, row0 + quad * 32);
-        tma_store_2d(&p.tmO, stage + 4096u, qcol + 64, row0 + quad * 32);
+      if (lane == 0 && orow < p.S) {
+#pragma unroll
+        for (int q = 0; q < DH / 64; ++q) tma_store_3d(&p.tmO, stage + 4096u * q, qcol + 64 * q, orow, b);
         asm volatile("cp.async.bulk.commit_group;" ::: "memory");
         asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
       }
-      if (p.lse) p.lse[((long long)b * p.H + h) * p.S + qi * BQ + r] = (m_used + log2f(l)) * 0.6931471805599453f;
+      if (p.lse && row0 + r < p.S) p.lse[((long long)b * p.H + h) * p.S + row0 + r] = (m_used + log2f(l)) * 0.6931471805599453f;
     }
   }
   __syncwarp();
@@ -318,24 +361,34 @@ attn_fwd_kernel(const __grid_constant__ AttnFwdParams p) {
 
 }  // namespace
 
-// qkv: packed [B*S, (H + 2*KV) * 128] bf16 (row stride ld_qkv elements); out: [B*S, H*128] bf16 (row stride ld_o);
-// lse: [B, H, S] fp32 or null.  S must be a multiple of 128 and H a multiple of KV.
-TPLR_API int tplr_attention_fwd(const void* qkv, void* out, float* lse, int B, int S, int H, int KV, long long ld_qkv,
-                                long long ld_o, float scale, unsigned int* status, void* stream) {
-  TPLR_ENTER();
-  if (B <= 0 || S <= 0) return 0;
-  if (S % BQ || H % KV || (ld_qkv % 8) || (ld_o % 8) || ((uintptr_t)qkv & 15) || ((uintptr_t)out & 15)) return -201;
+namespace {
+template <int DH>
+int launch_fwd(const void* qkv, void* out, float* lse, int B, int S, int H, int KV, long long ld_qkv, long long ld_o,
+               float scale, unsigned int* status, cudaStream_t st) {
   AttnFwdParams p = {};
-  if (!make_map(&p.tmQKV, qkv, (long long)(H + 2 * KV) * DH, (long long)B * S, ld_qkv, 64, 128)) return -202;
-  if (!make_map(&p.tmO, out, (long long)H * DH, (long long)B * S, ld_o, 64, 32)) return -203;
+  if (!make_map3(&p.tmQKV, qkv, (long long)(H + 2 * KV) * DH, S, B, ld_qkv, 64, 128)) return -202;
+  if (!make_map3(&p.tmO, out, (long long)H * DH, S, B, ld_o, 64, 32)) return -203;
   p.lse = lse; p.B = B; p.S = S; p.H = H; p.KV = KV;
   p.scale_log2 = scale * 1.4426950408889634f;
   p.status = status;
-  cudaError_t e = cudaFuncSetAttribute(attn_fwd_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, FWD_SMEM);
+  cudaError_t e = cudaFuncSetAttribute(attn_fwd_kernel<DH>, cudaFuncAttributeMaxDynamicSharedMemorySize, fwd_smem<DH>());
   if (e != cudaSuccess) return (int)e;
-  const unsigned grid = (unsigned)((S / BQ) * H * B);
-  attn_fwd_kernel<<<grid, FWD_THREADS, FWD_SMEM, (cudaStream_t)stream>>>(p);
+  const unsigned grid = (unsigned)(((S + BQ - 1) / BQ) * H * B);
+  attn_fwd_kernel<DH><<<grid, FWD_THREADS, fwd_smem<DH>(), st>>>(p);
   return (int)cudaGetLastError();
+}
+}  // namespace
+
+// qkv: packed [B*S, (H + 2*KV) * head_dim] bf16 (row stride ld_qkv elements); out: [B*S, H*head_dim] bf16 (row stride
+// ld_o); lse: [B, H, S] fp32 or null.  head_dim 128 or 64, H a multiple of KV.
+TPLR_API int tplr_attention_fwd(const void* qkv, void* out, float* lse, int B, int S, int H, int KV, int head_dim,
+                                long long ld_qkv, long long ld_o, float scale, unsigned int* status, void* stream) {
+  TPLR_ENTER();
+  if (B <= 0 || S <= 0) return 0;
+  if (H % KV || (ld_qkv % 8) || (ld_o % 8) || ((uintptr_t)qkv & 15) || ((uintptr_t)out & 15)) return -201;
+  if (head_dim == 128) return launch_fwd<128>(qkv, out, lse, B, S, H, KV, ld_qkv, ld_o, scale, status, (cudaStream_t)stream);
+  if (head_dim == 64) return launch_fwd<64>(qkv, out, lse, B, S, H, KV, ld_qkv, ld_o, scale, status, (cudaStream_t)stream);
+  return -201;
 }
 
 // ------------------------------------------------------------------------------------------ //
@@ -351,20 +404,20 @@ TPLR_API int tplr_attention_fwd(const void* qkv, void* out, float* lse, int B, i
 // ------------------------------------------------------------------------------------------ //
 namespace {
 
-constexpr int BWD_SMEM = 6 * TILE_BYTES + 1024;
+template <int DH> constexpr int bwd_smem() { return 4 * tile_bytes<DH>() + 2 * PT_BYTES + 1024; }   // K, V, Q, dO; P, dS
 constexpr int BWD_THREADS = 320;                        // TMA warp, MMA warp, 8 softmax warps (2 per TMEM lane quadrant)
 
 struct AttnBwdParams {
-  CUtensorMap tmQKV;    // [B*S, C] bf16, box 64 x 128
-  CUtensorMap tmDO;     // [B*S, H*128] bf16, box 64 x 128
-  CUtensorMap tmDQ;     // [B*S, H*128] fp32, box 32 x 32 (reduce-add target)
-  CUtensorMap tmDQKV;   // [B*S, C] bf16, box 64 x 32 (dK and dV stores)
+  CUtensorMap tmQKV;    // [B, S, C] bf16, box 64 x 128 x 1
+  CUtensorMap tmDO;     // [B, S, H*DH] bf16, box 64 x 128 x 1
+  CUtensorMap tmDQ;     // [B, S, H*DH] fp32, box 32 x 32 x 1 (reduce-add target)
+  CUtensorMap tmDQKV;   // [B, S, C] bf16, box 64 x 32 x 1 (dK and dV stores)
   const float* lse;
   const float* delta;
   int B, S, H, KV;
   float scale, scale_log2;
   unsigned int* status;
-  // not null: q and k were rotated (rotary embedding, interleaved pairs, tables [S, 64] fp32) by the producer of qkv and
+  // not null: q and k were rotated (rotary embedding, interleaved pairs, tables [S, DH / 2] fp32) by the producer of qkv and
   // the gradient is wanted with respect to the un-rotated projection: dK is rotated back in the epilogue
   const float* rope_cos;
   const float* rope_sin;
@@ -374,13 +427,15 @@ __device__ __forceinline__ void tma_reduce_add_2d(const CUtensorMap* map, uint32
   asm volatile("cp.reduce.async.bulk.tensor.2d.global.shared::cta.add.bulk_group [%0, {%2, %3}], [%1];"
                ::"l"(map), "r"(src), "r"(x), "r"(y) : "memory");
 }
-__device__ __forceinline__ uint32_t idesc_bwd(bool a_mn, bool b_mn) {
-  return (1u << 4) | (1u << 7) | (1u << 10) | ((a_mn ? 1u : 0u) << 15) | ((b_mn ? 1u : 0u) << 16) |
-         ((uint32_t)(128 >> 3) << 17) | ((uint32_t)(128 >> 4) << 24);
+__device__ __forceinline__ void tma_reduce_add_3d(const CUtensorMap* map, uint32_t src, int x, int y, int z) {
+  asm volatile("cp.reduce.async.bulk.tensor.3d.global.shared::cta.add.bulk_group [%0, {%2, %3, %4}], [%1];"
+               ::"l"(map), "r"(src), "r"(x), "r"(y), "r"(z) : "memory");
 }
 
+template <int DH>
 __global__ void __launch_bounds__(BWD_THREADS, 1)
 attn_bwd_kernel(const __grid_constant__ AttnBwdParams p) {
+  constexpr int TILE_BYTES = tile_bytes<DH>();
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
   __shared__ __align__(8) uint64_t bar_kv, bar_q_full, bar_q_empty, bar_do_full, bar_do_empty, bar_sp_full, bar_pds_full, bar_dq_full, bar_s_free;
@@ -388,14 +443,14 @@ attn_bwd_kernel(const __grid_constant__ AttnBwdParams p) {
   __shared__ int s_abort;
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int nQ = p.S / BQ;
+  const int nQ = (p.S + BQ - 1) / BQ;
   const int gb = p.KV * p.B;
   const int j = (int)(blockIdx.x / gb);                    // kv block; small j (long walks) first
   const int g = (int)(blockIdx.x % gb) % p.KV, b = (int)(blockIdx.x % gb) / p.KV;
   const int group = p.H / p.KV;
   const int n_i = nQ - j;                                  // query blocks j..nQ-1
   const int n_it = group * n_i;
-  const int kvrow0 = b * p.S + j * BKV;
+  const int kvrow0 = j * BKV;                              // position of the first key row; rows past S read as zeros
   const int kcol = (p.H + g) * DH, vcol = (p.H + p.KV + g) * DH;
   volatile int* abort_flag = &s_abort;
 
@@ -417,45 +472,42 @@ attn_bwd_kernel(const __grid_constant__ AttnBwdParams p) {
   __syncthreads();
   tcgen05_fence_after();
   const uint32_t tmem_base = s_tmem_base;
-  const uint32_t tS = tmem_base, tdP = tmem_base + 128, tdV = tmem_base + 256, tdK = tmem_base + 384;
+  const uint32_t tS = tmem_base, tdP = tmem_base + 128, tdV = tmem_base + 256, tdK = tmem_base + 256 + DH;
   const uint32_t sK = smem_u32(smem), sV = sK + TILE_BYTES, sQ = sV + TILE_BYTES, sdO = sQ + TILE_BYTES,
-                 sP = sdO + TILE_BYTES, sdS = sP + TILE_BYTES;
+                 sP = sdO + TILE_BYTES, sdS = sP + PT_BYTES;
 
   if (warp == 0) {
     if (lane == 0) {
       mbar_expect_tx(smem_u32(&bar_kv), 2 * TILE_BYTES);
-      tma_load_2d(sK, &p.tmQKV, smem_u32(&bar_kv), kcol, kvrow0);
-      tma_load_2d(sK + TILE_BYTES / 2, &p.tmQKV, smem_u32(&bar_kv), kcol + 64, kvrow0);
-      tma_load_2d(sV, &p.tmQKV, smem_u32(&bar_kv), vcol, kvrow0);
-      tma_load_2d(sV + TILE_BYTES / 2, &p.tmQKV, smem_u32(&bar_kv), vcol + 64, kvrow0);
+      load_tile<DH>(sK, &p.tmQKV, smem_u32(&bar_kv), kcol, kvrow0, b);
+      load_tile<DH>(sV, &p.tmQKV, smem_u32(&bar_kv), vcol, kvrow0, b);
       bool ok = true;
       for (int t = 0; t < n_it && ok; ++t) {
         const int h = g * group + t / n_i, i = j + t % n_i;
-        const int qrow0 = b * p.S + i * BQ, qcol = h * DH;
+        const int qrow0 = i * BQ, qcol = h * DH;
         // Q is released by the dK MMAs and dO by the dV MMAs of the previous step, both before its dQ MMAs and the
         // dQ drain: the next tiles are in flight while those run
         if (!(ok = mbar_wait(smem_u32(&bar_q_empty), (uint32_t)((t & 1) ^ 1), abort_flag))) break;
         const uint32_t fq = smem_u32(&bar_q_full);
         mbar_expect_tx(fq, TILE_BYTES);
-        tma_load_2d(sQ, &p.tmQKV, fq, qcol, qrow0);
-        tma_load_2d(sQ + TILE_BYTES / 2, &p.tmQKV, fq, qcol + 64, qrow0);
+        load_tile<DH>(sQ, &p.tmQKV, fq, qcol, qrow0, b);
         if (!(ok = mbar_wait(smem_u32(&bar_do_empty), (uint32_t)((t & 1) ^ 1), abort_flag))) break;
         const uint32_t fd = smem_u32(&bar_do_full);
         mbar_expect_tx(fd, TILE_BYTES);
-        tma_load_2d(sdO, &p.tmDO, fd, qcol, qrow0);
-        tma_load_2d(sdO + TILE_BYTES / 2, &p.tmDO, fd, qcol + 64, qrow0);
+        load_tile<DH>(sdO, &p.tmDO, fd, qcol, qrow0, b);
       }
     }
   } else if (warp == 1) {
     if (lane == 0) {
-      const uint32_t id_kk = idesc_bwd(false, false), id_mm = idesc_bwd(true, true), id_km = idesc_bwd(false, true);
+      const uint32_t id_kk = idesc_mn(128, false, false), id_mm = idesc_mn(DH, true, true), id_km = idesc_mn(DH, false, true);
       // descriptor bases: "k" = contraction along the 128-byte rows, "m" = contraction along the tile rows
       const DescBase kQ = desc_base(sQ, 16, 1024), kK = desc_base(sK, 16, 1024), kdO = desc_base(sdO, 16, 1024),
                      kV = desc_base(sV, 16, 1024), kdS = desc_base(sdS, 16, 1024);
-      const DescBase mP = desc_base(sP, TILE_BYTES / 2, 1024), mdO = desc_base(sdO, TILE_BYTES / 2, 1024),
-                     mdS = desc_base(sdS, TILE_BYTES / 2, 1024), mQ = desc_base(sQ, TILE_BYTES / 2, 1024),
-                     mK = desc_base(sK, TILE_BYTES / 2, 1024);
-#define TPLR_KOFF(kk) ((uint32_t)((kk) >> 2) * (TILE_BYTES / 32) + (uint32_t)((kk) & 3) * 2u)
+      // (every operand is made of 128-row blocks of 64 columns, 16 KB apart)
+      const DescBase mP = desc_base(sP, 128 * 128, 1024), mdO = desc_base(sdO, 128 * 128, 1024),
+                     mdS = desc_base(sdS, 128 * 128, 1024), mQ = desc_base(sQ, 128 * 128, 1024),
+                     mK = desc_base(sK, 128 * 128, 1024);
+#define TPLR_KOFF(kk) ((uint32_t)((kk) >> 2) * (128u * 128u / 16u) + (uint32_t)((kk) & 3) * 2u)
 #define TPLR_MOFF(kk) ((uint32_t)(kk) * 128u)
       bool ok = mbar_wait(smem_u32(&bar_kv), 0, abort_flag);
       for (int t = 0; t < n_it && ok; ++t) {
@@ -464,10 +516,10 @@ attn_bwd_kernel(const __grid_constant__ AttnBwdParams p) {
         if (t > 0 && !(ok = mbar_wait(smem_u32(&bar_s_free), ph ^ 1, abort_flag))) break;
         tcgen05_fence_after();
 #pragma unroll
-        for (int kk = 0; kk < 8; ++kk) umma_bf16_b(tS, kQ, TPLR_KOFF(kk), kK, TPLR_KOFF(kk), id_kk, kk > 0 ? 1u : 0u);
+        for (int kk = 0; kk < DH / 16; ++kk) umma_bf16_b(tS, kQ, TPLR_KOFF(kk), kK, TPLR_KOFF(kk), id_kk, kk > 0 ? 1u : 0u);
         if (!(ok = mbar_wait(smem_u32(&bar_do_full), ph, abort_flag))) break;
 #pragma unroll
-        for (int kk = 0; kk < 8; ++kk) umma_bf16_b(tdP, kdO, TPLR_KOFF(kk), kV, TPLR_KOFF(kk), id_kk, kk > 0 ? 1u : 0u);
+        for (int kk = 0; kk < DH / 16; ++kk) umma_bf16_b(tdP, kdO, TPLR_KOFF(kk), kV, TPLR_KOFF(kk), id_kk, kk > 0 ? 1u : 0u);
         umma_commit(smem_u32(&bar_sp_full));
         if (!(ok = mbar_wait(smem_u32(&bar_pds_full), ph, abort_flag))) break;
         tcgen05_fence_after();
@@ -492,14 +544,16 @@ attn_bwd_kernel(const __grid_constant__ AttnBwdParams p) {
     const uint32_t lane_off = (uint32_t)(quad * 32) << 16;
     const uint32_t sw = (uint32_t)(lane & 7);
     // two private 4 KB staging buffers: the bytes of this warp's own rows and column half in the P and dS tiles
-    const uint32_t stg0 = sP + (uint32_t)ch * (TILE_BYTES / 2) + (uint32_t)quad * 4096u;
-    const uint32_t stg1 = sdS + (uint32_t)ch * (TILE_BYTES / 2) + (uint32_t)quad * 4096u;
+    const uint32_t stg0 = sP + (uint32_t)ch * (PT_BYTES / 2) + (uint32_t)quad * 4096u;
+    const uint32_t stg1 = sdS + (uint32_t)ch * (PT_BYTES / 2) + (uint32_t)quad * 4096u;
     bool ok = true;
     for (int t = 0; t < n_it && ok; ++t) {
       const int h = g * group + t / n_i, i = j + t % n_i;
       const long long stat = ((long long)b * p.H + h) * p.S + i * BQ + r;
-      const float lse2 = p.lse[stat] * 1.4426950408889634f;
-      const float dl = p.delta[stat];
+      // a query row past the end of the sequence has no weight: lse = +inf makes its P and with it dS zero
+      const bool live = i * BQ + r < p.S;
+      const float lse2 = live ? p.lse[stat] * 1.4426950408889634f : INFINITY;
+      const float dl = live ? p.delta[stat] : 0.f;
       ok = mbar_wait(smem_u32(&bar_sp_full), t & 1, abort_flag);
       ok = __all_sync(0xffffffffu, ok);
       if (!ok) break;
@@ -515,8 +569,8 @@ attn_bwd_kernel(const __grid_constant__ AttnBwdParams p) {
           uint32_t sv[32], dv[32];
           tmem_ld32(tS + c * 32 + lane_off, sv);
           tmem_ld32(tdP + c * 32 + lane_off, dv);
-          const uint32_t prow = sP + (uint32_t)(c >> 1) * (TILE_BYTES / 2) + (uint32_t)r * 128u;
-          const uint32_t drow = sdS + (uint32_t)(c >> 1) * (TILE_BYTES / 2) + (uint32_t)r * 128u;
+          const uint32_t prow = sP + (uint32_t)(c >> 1) * (PT_BYTES / 2) + (uint32_t)r * 128u;
+          const uint32_t drow = sdS + (uint32_t)(c >> 1) * (PT_BYTES / 2) + (uint32_t)r * 128u;
 #pragma unroll
           for (int q4 = 0; q4 < 4; ++q4) {
             uint32_t pw[4], dw[4];
@@ -551,10 +605,10 @@ attn_bwd_kernel(const __grid_constant__ AttnBwdParams p) {
       ok = __all_sync(0xffffffffu, ok);
       if (!ok) break;
       tcgen05_fence_after();
-      const int qrow0 = b * p.S + i * BQ + quad * 32;
+      const int qrow0 = i * BQ + quad * 32;
 #pragma unroll
-      for (int cc = 0; cc < 2; ++cc) {
-        const int c = 2 * ch + cc;
+      for (int cc = 0; cc < DH / 64; ++cc) {
+        const int c = DH / 64 * ch + cc;
         uint32_t v[32];
         tmem_ld32(tS + c * 32 + lane_off, v);
         const uint32_t buf = cc ? stg1 : stg0;
@@ -565,8 +619,8 @@ attn_bwd_kernel(const __grid_constant__ AttnBwdParams p) {
                        "r"(v[4 * q8 + 1]), "r"(v[4 * q8 + 2]), "r"(v[4 * q8 + 3]) : "memory");
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
         __syncwarp();
-        if (lane == 0) {
-          tma_reduce_add_2d(&p.tmDQ, buf, h * DH + c * 32, qrow0);
+        if (lane == 0 && qrow0 < p.S) {
+          tma_reduce_add_3d(&p.tmDQ, buf, h * DH + c * 32, qrow0, b);
           asm volatile("cp.async.bulk.commit_group;" ::: "memory");
         }
       }
@@ -580,16 +634,18 @@ attn_bwd_kernel(const __grid_constant__ AttnBwdParams p) {
       tcgen05_fence_after();
       const int orow0 = kvrow0 + quad * 32;
 #pragma unroll
-      for (int acc = 0; acc < 2; ++acc) {      // 0 = dV, 1 = dK; this warp stores its 64-column half of each
+      for (int acc = 0; acc < 2; ++acc) {      // 0 = dV, 1 = dK; at 128 columns this warp stores its half of each, at 64 one of them
+        if (DH == 64 && acc != ch) continue;
+        const int col = DH == 64 ? 0 : ch * 64;
         const uint32_t tacc = acc ? tdK : tdV;
         const uint32_t buf = acc ? stg1 : stg0;
         const uint32_t rowaddr = buf + (uint32_t)lane * 128u;
 #pragma unroll
         for (int hf = 0; hf < 2; ++hf) {
           uint32_t v[32];
-          tmem_ld32(tacc + ch * 64 + hf * 32 + lane_off, v);
+          tmem_ld32(tacc + col + hf * 32 + lane_off, v);
           if (acc == 1 && p.rope_cos) {          // dK back through the rotation of this key row: the opposite angle
-            const long long tb = (long long)((orow0 + lane) % p.S) * (DH / 2) + (ch * 64 + hf * 32) / 2;
+            const long long tb = (long long)min(orow0 + lane, p.S - 1) * (DH / 2) + (col + hf * 32) / 2;
             const float4* cp = reinterpret_cast<const float4*>(p.rope_cos + tb);
             const float4* sp = reinterpret_cast<const float4*>(p.rope_sin + tb);
 #pragma unroll
@@ -618,8 +674,8 @@ attn_bwd_kernel(const __grid_constant__ AttnBwdParams p) {
         }
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
         __syncwarp();
-        if (lane == 0) {
-          tma_store_2d(&p.tmDQKV, buf, (acc ? kcol : vcol) + ch * 64, orow0);
+        if (lane == 0 && orow0 < p.S) {
+          tma_store_3d(&p.tmDQKV, buf, (acc ? kcol : vcol) + col, orow0, b);
           asm volatile("cp.async.bulk.commit_group;" ::: "memory");
         }
       }
@@ -636,15 +692,17 @@ attn_bwd_kernel(const __grid_constant__ AttnBwdParams p) {
   if (threadIdx.x == 0 && s_abort && p.status) atomicOr(p.status, TPLR_ST_WAIT_TIMEOUT);
 }
 
-// delta[b, h, s] = sum_d dO * O : one warp per (token, head), 4 elements per lane
+// delta[b, h, s] = sum_d dO * O : DH / 4 lanes per (token, head), 4 elements per lane
+template <int DH>
 __global__ void __launch_bounds__(256) attn_delta_kernel(const __nv_bfloat16* __restrict__ o, const __nv_bfloat16* __restrict__ dout,
                                                          float* __restrict__ delta, long long tokens, int S, int H,
                                                          long long ld_o) {
-  const long long w = (long long)blockIdx.x * 8 + (threadIdx.x >> 5);
-  if (w >= tokens * H) return;
-  const int lane = threadIdx.x & 31;
-  const long long tok = w / H;
-  const int h = (int)(w % H);
+  constexpr int LANES = DH / 4;
+  const long long w = (long long)blockIdx.x * (256 / LANES) + threadIdx.x / LANES;
+  const bool live = w < tokens * H;
+  const int lane = threadIdx.x % LANES;
+  const long long tok = live ? w / H : 0;
+  const int h = live ? (int)(w % H) : 0;
   const uint2 a = *reinterpret_cast<const uint2*>(o + tok * ld_o + h * DH + lane * 4);
   const uint2 d = *reinterpret_cast<const uint2*>(dout + tok * (long long)H * DH + h * DH + lane * 4);
   const float2 a0 = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&a.x));
@@ -652,14 +710,15 @@ __global__ void __launch_bounds__(256) attn_delta_kernel(const __nv_bfloat16* __
   const float2 d0 = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&d.x));
   const float2 d1 = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&d.y));
   float s = a0.x * d0.x + a0.y * d0.y + a1.x * d1.x + a1.y * d1.y;
-  s = warp_sum(s);
-  if (lane == 0) delta[((tok / S) * H + h) * S + tok % S] = s;
+#pragma unroll
+  for (int k = LANES / 2; k > 0; k >>= 1) s += __shfl_xor_sync(0xffffffffu, s, k);
+  if (lane == 0 && live) delta[((tok / S) * H + h) * S + tok % S] = s;
 }
 
-// dq32 [tokens, H*128] fp32 -> first H*128 columns of the packed bf16 gradient
+// dq32 [tokens, width] fp32 -> first `width` columns (heads of dh) of the packed bf16 gradient
 // cosb / sinb not null: the two pairs are rotated back by the angles of (token % S, pair index in the head) on the way
 __global__ void __launch_bounds__(256) attn_dq_cast_kernel(const float* __restrict__ dq32, __nv_bfloat16* __restrict__ dqkv,
-                                                           long long tokens, int width, long long ld,
+                                                           long long tokens, int width, int dh, long long ld,
                                                            const float* __restrict__ cosb, const float* __restrict__ sinb, int S) {
   const long long n4 = tokens * (width / 4);
   for (long long v = (long long)blockIdx.x * blockDim.x + threadIdx.x; v < n4; v += (long long)gridDim.x * blockDim.x) {
@@ -667,7 +726,7 @@ __global__ void __launch_bounds__(256) attn_dq_cast_kernel(const float* __restri
     const int c4 = (int)(v % (width / 4));
     float4 f = reinterpret_cast<const float4*>(dq32)[v];
     if (cosb) {
-      const long long tb = (tok % S) * (DH / 2) + ((c4 * 4) % DH) / 2;
+      const long long tb = (tok % S) * (dh / 2) + ((c4 * 4) % dh) / 2;
       const float2 c = *reinterpret_cast<const float2*>(cosb + tb), sn = *reinterpret_cast<const float2*>(sinb + tb);
       f = make_float4(f.x * c.x + f.y * sn.x, f.y * c.x - f.x * sn.x, f.z * c.y + f.w * sn.y, f.w * c.y - f.z * sn.y);
     }
@@ -694,6 +753,7 @@ __global__ void __launch_bounds__(256) attn_dq_cast_kernel(const float* __restri
 // ------------------------------------------------------------------------------------------ //
 namespace {
 
+constexpr int DH = 128, TILE_BYTES = tile_bytes<DH>();     // this variant: head dimension 128, sequences that are multiples of 128
 constexpr int B2_BQ = 64;
 constexpr int B2_QTILE = B2_BQ * DH * 2;                // 16 KB: 64 x 128 bf16 (two blocks of 64 rows x 128 B)
 constexpr int B2_DS_TILE = BKV * B2_BQ * 2;             // 16 KB: 128 kv rows x 64 q
@@ -714,10 +774,6 @@ struct AttnBwd2Params {
   unsigned int* status;
 };
 
-__device__ __forceinline__ uint32_t idesc_mn(int n, bool a_mn, bool b_mn) {
-  return (1u << 4) | (1u << 7) | (1u << 10) | ((a_mn ? 1u : 0u) << 15) | ((b_mn ? 1u : 0u) << 16) |
-         ((uint32_t)(n >> 3) << 17) | ((uint32_t)(128 >> 4) << 24);
-}
 __device__ __forceinline__ void bulk_load_1d(uint32_t dst, const void* src, uint32_t bytes, uint32_t bar) {
   asm volatile("cp.async.bulk.shared::cta.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
                ::"r"(dst), "l"(src), "r"(bytes), "r"(bar) : "memory");
@@ -1029,26 +1085,24 @@ TPLR_API int tplr_attention_set_bwd_variant(int v) {
 }
 
 // Gradient of tplr_attention_fwd.  qkv / dqkv: packed [B*S, C] bf16 with row stride ld_qkv; out: the forward's
-// output (row stride ld_o); dout: contiguous [B*S, H*128]; lse from the forward; delta: [B,H,S] fp32 scratch;
-// dq32: [B*S, H*128] fp32 scratch that the caller has zeroed.  dqkv receives dq | dk | dv.
+// output (row stride ld_o); dout: contiguous [B*S, H*head_dim]; lse from the forward; delta: [B,H,S] fp32 scratch;
+// dq32: [B*S, H*head_dim] fp32 scratch that the caller has zeroed.  dqkv receives dq | dk | dv.
 extern "C" int tplr_rope(void* buf, const float* cosb, const float* sinb, long long tokens, int S, int n_heads, int Dh,
                          long long row_stride, int inverse, void* stream);
 
-static int attention_bwd_impl(const void* qkv, const void* out, const void* dout, const float* lse, float* delta,
-                              float* dq32, void* dqkv, int B, int S, int H, int KV, long long ld_qkv, long long ld_o,
-                              float scale, const float* cosb, const float* sinb, unsigned int* status, void* stream,
-                              bool delta_ready = false) {
-  if (B <= 0 || S <= 0) return 0;
-  if (S % BQ || H % KV || (ld_qkv % 8) || (ld_o % 8) || ((uintptr_t)qkv & 15) || ((uintptr_t)dqkv & 15) ||
-      ((uintptr_t)dout & 15) || ((uintptr_t)out & 7) || ((uintptr_t)dq32 & 15))
-    return -201;
-  cudaStream_t st = (cudaStream_t)stream;
+namespace {
+template <int HD>
+int launch_bwd(const void* qkv, const void* out, const void* dout, const float* lse, float* delta, float* dq32, void* dqkv, int B,
+               int S, int H, int KV, long long ld_qkv, long long ld_o, float scale, const float* cosb, const float* sinb,
+               unsigned int* status, cudaStream_t st, bool delta_ready) {
   const long long tokens = (long long)B * S;
-  const int C = (H + 2 * KV) * DH;
-  if (!delta_ready)
-    attn_delta_kernel<<<(unsigned)((tokens * H + 7) / 8), 256, 0, st>>>((const __nv_bfloat16*)out, (const __nv_bfloat16*)dout,
-                                                                         delta, tokens, S, H, ld_o);
-  if (g_bwd_variant == 2) {
+  const int C = (H + 2 * KV) * HD;
+  if (!delta_ready) {
+    constexpr int per_cta = 256 / (HD / 4);
+    attn_delta_kernel<HD><<<(unsigned)((tokens * H + per_cta - 1) / per_cta), 256, 0, st>>>(
+        (const __nv_bfloat16*)out, (const __nv_bfloat16*)dout, delta, tokens, S, H, ld_o);
+  }
+  if (HD == 128 && S % 128 == 0 && g_bwd_variant == 2) {
     // pipelined kernel: dq32 is used as the transposed scratch [B*H*128, S]
     AttnBwd2Params p = {};
     if (!make_map(&p.tmKV, qkv, C, tokens, ld_qkv, 64, 128)) return -202;
@@ -1063,53 +1117,67 @@ static int attention_bwd_impl(const void* qkv, const void* out, const void* dout
     attn_bwd2_kernel<<<(unsigned)((S / BKV) * KV * B), B2_THREADS, B2_SMEM, st>>>(p);
     attn_dq_transpose_kernel<<<dim3((unsigned)(S / 32), (unsigned)(B * H * DH / 32)), 256, 0, st>>>(
         dq32, (__nv_bfloat16*)dqkv, S, H, ld_qkv);
-    if (cosb) return tplr_rope(dqkv, cosb, sinb, tokens, S, H + KV, DH, ld_qkv, 1, stream);   // this variant rotates back in a pass of its own
+    if (cosb) return tplr_rope(dqkv, cosb, sinb, tokens, S, H + KV, DH, ld_qkv, 1, st);   // this variant rotates back in a pass of its own
     return (int)cudaGetLastError();
   }
   AttnBwdParams p = {};
-  if (!make_map(&p.tmQKV, qkv, C, tokens, ld_qkv, 64, 128)) return -202;
-  if (!make_map(&p.tmDO, dout, (long long)H * DH, tokens, (long long)H * DH, 64, 128)) return -203;
-  if (!make_map(&p.tmDQ, dq32, (long long)H * DH, tokens, (long long)H * DH, 32, 32, CU_TENSOR_MAP_SWIZZLE_128B, true)) return -204;
-  if (!make_map(&p.tmDQKV, dqkv, C, tokens, ld_qkv, 64, 32)) return -205;
+  if (!make_map3(&p.tmQKV, qkv, C, S, B, ld_qkv, 64, 128)) return -202;
+  if (!make_map3(&p.tmDO, dout, (long long)H * HD, S, B, (long long)H * HD, 64, 128)) return -203;
+  if (!make_map3(&p.tmDQ, dq32, (long long)H * HD, S, B, (long long)H * HD, 32, 32, true)) return -204;
+  if (!make_map3(&p.tmDQKV, dqkv, C, S, B, ld_qkv, 64, 32)) return -205;
   p.lse = lse; p.delta = delta; p.B = B; p.S = S; p.H = H; p.KV = KV;
   p.scale = scale; p.scale_log2 = scale * 1.4426950408889634f; p.status = status;
   p.rope_cos = cosb; p.rope_sin = sinb;
-  cudaError_t e = cudaFuncSetAttribute(attn_bwd_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, BWD_SMEM);
+  cudaError_t e = cudaFuncSetAttribute(attn_bwd_kernel<HD>, cudaFuncAttributeMaxDynamicSharedMemorySize, bwd_smem<HD>());
   if (e != cudaSuccess) return (int)e;
-  attn_bwd_kernel<<<(unsigned)((S / BKV) * KV * B), BWD_THREADS, BWD_SMEM, st>>>(p);
-  attn_dq_cast_kernel<<<tplr_sm_count() * 8, 256, 0, st>>>(dq32, (__nv_bfloat16*)dqkv, tokens, H * DH, ld_qkv, cosb, sinb, S);
+  attn_bwd_kernel<HD><<<(unsigned)(((S + BKV - 1) / BKV) * KV * B), BWD_THREADS, bwd_smem<HD>(), st>>>(p);
+  attn_dq_cast_kernel<<<tplr_sm_count() * 8, 256, 0, st>>>(dq32, (__nv_bfloat16*)dqkv, tokens, H * HD, HD, ld_qkv, cosb, sinb, S);
   return (int)cudaGetLastError();
+}
+}  // namespace
+
+static int attention_bwd_impl(const void* qkv, const void* out, const void* dout, const float* lse, float* delta,
+                              float* dq32, void* dqkv, int B, int S, int H, int KV, int head_dim, long long ld_qkv,
+                              long long ld_o, float scale, const float* cosb, const float* sinb, unsigned int* status,
+                              void* stream, bool delta_ready = false) {
+  if (B <= 0 || S <= 0) return 0;
+  if ((head_dim != 128 && head_dim != 64) || H % KV || (ld_qkv % 8) || (ld_o % 8) || ((uintptr_t)qkv & 15) ||
+      ((uintptr_t)dqkv & 15) || ((uintptr_t)dout & 15) || ((uintptr_t)out & 7) || ((uintptr_t)dq32 & 15))
+    return -201;
+  auto run = head_dim == 128 ? launch_bwd<128> : launch_bwd<64>;
+  return run(qkv, out, dout, lse, delta, dq32, dqkv, B, S, H, KV, ld_qkv, ld_o, scale, cosb, sinb, status, (cudaStream_t)stream,
+             delta_ready);
 }
 
 TPLR_API int tplr_attention_bwd(const void* qkv, const void* out, const void* dout, const float* lse, float* delta,
-                                float* dq32, void* dqkv, int B, int S, int H, int KV, long long ld_qkv, long long ld_o,
+                                float* dq32, void* dqkv, int B, int S, int H, int KV, int head_dim, long long ld_qkv, long long ld_o,
                                 float scale, unsigned int* status, void* stream) {
   TPLR_ENTER();
-  return attention_bwd_impl(qkv, out, dout, lse, delta, dq32, dqkv, B, S, H, KV, ld_qkv, ld_o, scale, nullptr, nullptr, status, stream);
+  return attention_bwd_impl(qkv, out, dout, lse, delta, dq32, dqkv, B, S, H, KV, head_dim, ld_qkv, ld_o, scale, nullptr, nullptr, status, stream);
 }
 
 // tplr_attention_bwd for a qkv whose q and k heads were rotated by the producer (tplr_gemm2_rope): dq and dk are
 // returned with respect to the un-rotated projection, i.e. rotated back by the opposite angles where they are written
 // (dq in the fp32 -> bf16 pass, dk in the kernel's epilogue), so that no separate pass over the gradient is needed.
-// cosb / sinb: [S, 64] fp32, 16-byte aligned.
+// cosb / sinb: [S, head_dim / 2] fp32, 16-byte aligned.
 TPLR_API int tplr_attention_bwd_unrope(const void* qkv, const void* out, const void* dout, const float* lse, float* delta,
-                                       float* dq32, void* dqkv, int B, int S, int H, int KV, long long ld_qkv, long long ld_o,
+                                       float* dq32, void* dqkv, int B, int S, int H, int KV, int head_dim, long long ld_qkv, long long ld_o,
                                        float scale, const float* cosb, const float* sinb, unsigned int* status, void* stream) {
   TPLR_ENTER();
   if (!cosb || !sinb || ((uintptr_t)cosb & 15) || ((uintptr_t)sinb & 15)) return -201;
-  return attention_bwd_impl(qkv, out, dout, lse, delta, dq32, dqkv, B, S, H, KV, ld_qkv, ld_o, scale, cosb, sinb, status, stream);
+  return attention_bwd_impl(qkv, out, dout, lse, delta, dq32, dqkv, B, S, H, KV, head_dim, ld_qkv, ld_o, scale, cosb, sinb, status, stream);
 }
 
 // tplr_attention_bwd_unrope for a caller that has already filled `delta` ([B, H, S] fp32, delta[b, h, s] = sum over the
-// head's 128 columns of dout * out): the producer of `dout` (tplr_gemm2_attn_dout, the output projection's data
+// head's columns of dout * out): the producer of `dout` (tplr_gemm2_attn_dout, the output projection's data
 // gradient) forms it in its epilogue, where a row of dout is in registers anyway.
 TPLR_API int tplr_attention_bwd_unrope_delta(const void* qkv, const void* out, const void* dout, const float* lse,
-                                             float* delta, float* dq32, void* dqkv, int B, int S, int H, int KV,
+                                             float* delta, float* dq32, void* dqkv, int B, int S, int H, int KV, int head_dim,
                                              long long ld_qkv, long long ld_o, float scale, const float* cosb,
                                              const float* sinb, unsigned int* status, void* stream) {
   TPLR_ENTER();
   if (!cosb || !sinb || ((uintptr_t)cosb & 15) || ((uintptr_t)sinb & 15)) return -201;
-  return attention_bwd_impl(qkv, out, dout, lse, delta, dq32, dqkv, B, S, H, KV, ld_qkv, ld_o, scale, cosb, sinb, status, stream,
+  return attention_bwd_impl(qkv, out, dout, lse, delta, dq32, dqkv, B, S, H, KV, head_dim, ld_qkv, ld_o, scale, cosb, sinb, status, stream,
                             true);
 }
 

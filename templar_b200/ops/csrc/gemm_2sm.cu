@@ -63,11 +63,11 @@ struct Gemm2Params {
   // the epilogue stores dg | du (bf16) through tmC, a map over the [M, 2 * swiglu_f] gradient of that projection
   const __nv_bfloat16* gu;
   long long ld_gu;
-  // data gradient of the attention output projection (EPI 6): C = dO [M, heads * 128] stored as bf16, and for every row
-  // and head delta = sum over the head's 128 columns of dO * O, with O = gu (leading dimension ld_gu), written to
+  // data gradient of the attention output projection (EPI 6): C = dO [M, heads * attn_dh] stored as bf16, and for every row
+  // and head delta = sum over the head's attn_dh (128 or 64) columns of dO * O, with O = gu (leading dimension ld_gu), written to
   // attn_delta[(row / attn_s * heads + head) * attn_s + row % attn_s]
   float* attn_delta;
-  int attn_s, attn_heads;
+  int attn_s, attn_heads, attn_dh;
   // rotary embedding in the epilogue (EPI 4): the first rope_cols columns of C are heads of rope_dh columns whose
   // interleaved pairs (2i, 2i + 1) are rotated by the angle of (row % rope_s, i); tables [rope_s, rope_dh / 2] fp32
   const float* rope_cos;
@@ -491,8 +491,8 @@ __device__ __forceinline__ void epilogue_swiglu_bwd(const Gemm2Params& p, uint32
   }
 }
 
-// Epilogue of the attention output projection's data gradient (EPI 6): the accumulator row is dO for two heads (256
-// columns).  dO is stored as bf16 like a plain epilogue; on the way every lane multiplies its (bf16-rounded) values
+// Epilogue of the attention output projection's data gradient (EPI 6): the accumulator row is dO for two
+// heads of 128 columns or four of 64.  dO is stored as bf16 like a plain epilogue; on the way every lane multiplies its (bf16-rounded) values
 // with the forward's attention output O of the same row and sums per head, which is the `delta` term of the attention
 // backward (the row sum of dO * O): no separate pass over dO and O.  O is fetched one step of 32 columns ahead.
 __device__ __forceinline__ void epilogue_attn_dout(const Gemm2Params& p, uint32_t tmem_acc, int quad, int lane, int m0, int n0,
@@ -519,7 +519,7 @@ __device__ __forceinline__ void epilogue_attn_dout(const Gemm2Params& p, uint32_
   for (int step = 0; step < TILE_N / 32; ++step) {
     const int c = step >> 1, hh = step & 1;
     const int f0 = n0 + c * 64;
-    if (f0 >= p.N) break;                            // warp-uniform (N is a multiple of 128)
+    if (f0 >= p.N) break;                            // warp-uniform (N is a multiple of 64)
     if (step + 1 < TILE_N / 32) fetch(step + 1, on);
     uint32_t buf = 0;
     if (hh == 0) buf = box_begin(lane, stage_base, n_boxes); else buf = stage_base + (n_boxes & 1u) * 4096u;
@@ -542,8 +542,8 @@ __device__ __forceinline__ void epilogue_attn_dout(const Gemm2Params& p, uint32_
     }
     box_half(buf, lane, hh, v);
     if (hh == 1) box_store(&p.tmC, buf, lane, n_boxes, f0, row0);
-    if ((step & 3) == 3) {                           // a head (128 columns) is complete
-      const int head = (n0 + step * 32) / 128;
+    if (((step + 1) * 32) % p.attn_dh == 0) {        // a head is complete
+      const int head = (n0 + step * 32) / p.attn_dh;
       if (live) p.attn_delta[drow + (long long)head * p.attn_s] = acc;
       acc = 0.f;
     }
@@ -966,19 +966,19 @@ TPLR_API int tplr_gemm2_swiglu_bwd(const void* dY, const void* W2, const void* G
 }
 
 // dO[M, N] = dY Wo (dY [M, K] bf16 K-major, Wo [K, N] bf16 with N contiguous: the attention output projection's weight
-// as stored; N = heads * 128), and delta[b, h, s] = sum over head h's 128 columns of dO * O for row b * S + s, with O
+// as stored; N = heads * head_dim), and delta[b, h, s] = sum over head h's columns of dO * O for row b * S + s, with O
 // [M, N] the forward's attention output (see epilogue_attn_dout).  -111 when this entry does not take the arguments.
 TPLR_API int tplr_gemm2_attn_dout(const void* dY, const void* Wo, const void* O, void* dO, float* delta, int M, int N, int K,
-                                  int S, long long lddy, long long ldwo, long long ldo, long long lddo, unsigned int* status,
-                                  void* stream) {
+                                  int S, int head_dim, long long lddy, long long ldwo, long long ldo, long long lddo,
+                                  unsigned int* status, void* stream) {
   TPLR_ENTER();
   if (M <= 0 || N <= 0 || K <= 0) return 0;
-  if (N % 128 || S <= 0 || M % S || ((uintptr_t)O & 15) || ((uintptr_t)dO & 15) || (ldo % 8) || (lddo % 8) || !delta) return -111;
+  if ((head_dim != 128 && head_dim != 64) || N % head_dim || S <= 0 || M % S || ((uintptr_t)O & 15) || ((uintptr_t)dO & 15) || (ldo % 8) || (lddo % 8) || !delta) return -111;
   Gemm2Params p = {};
   if (int r = fill_common(p, dY, Wo, dO, M, N, K, lddy, ldwo, lddo, 0, 1, 0, status)) return r;
   if (!p.c_tma) return -111;
   p.gu = (const __nv_bfloat16*)O; p.ld_gu = ldo;
-  p.attn_delta = delta; p.attn_s = S; p.attn_heads = N / 128;
+  p.attn_delta = delta; p.attn_s = S; p.attn_heads = N / head_dim; p.attn_dh = head_dim;
   return dispatch2(p, 0, 1, 6, 0, 0, (cudaStream_t)stream);
 }
 

@@ -697,6 +697,7 @@ def attention(q, k, v):
     return o.transpose(1, 2)
 
 
+OWN_HEAD_DIMS = (64, 128)      # head dimensions of the own flash-attention kernels (any sequence length)
 _ATTN_BACKEND = "tcgen05"      # "tcgen05": own flash-attention kernels; "sdpa": torch SDPA (library)
 
 
@@ -719,7 +720,7 @@ def _split_qkv(qkv, n_heads, n_kv, hd):
 
 
 class _AttentionPacked(torch.autograd.Function):
-    """Causal GQA attention on the packed projection output [B, S, (H + 2 KV) * 128]; the backward
+    """Causal GQA attention on the packed projection output [B, S, (H + 2 KV) * hd]; the backward
     returns the gradient in the same packed layout, so nothing splits or concatenates q, k and v."""
 
     @staticmethod
@@ -728,7 +729,7 @@ class _AttentionPacked(torch.autograd.Function):
         out = torch.empty(B, S, n_heads * hd, dtype=qkv.dtype, device=qkv.device)
         lse = torch.empty(B, n_heads, S, dtype=torch.float32, device=qkv.device)
         native.check(native.lib().tplr_attention_fwd(qkv.data_ptr(), out.data_ptr(), lse.data_ptr(), B, S, n_heads, n_kv,
-                                                     qkv.stride(1), out.stride(1), hd ** -0.5,
+                                                     hd, qkv.stride(1), out.stride(1), hd ** -0.5,
                                                      status_word(qkv.device).data_ptr(), native.stream_ptr()),
                      "attention_fwd")
         ctx.save_for_backward(qkv, out, lse)
@@ -746,7 +747,7 @@ class _AttentionPacked(torch.autograd.Function):
         delta = torch.empty(B, n_heads, S, dtype=torch.float32, device=qkv.device)
         native.check(native.lib().tplr_attention_bwd(qkv.data_ptr(), out.data_ptr(), do.data_ptr(), lse.data_ptr(),
                                                      delta.data_ptr(), dq32.data_ptr(), dqkv.data_ptr(), B, S, n_heads, n_kv,
-                                                     qkv.stride(1), out.stride(1), hd ** -0.5,
+                                                     hd, qkv.stride(1), out.stride(1), hd ** -0.5,
                                                      status_word(qkv.device).data_ptr(), native.stream_ptr()),
                      "attention_bwd")
         return dqkv, None, None, None
@@ -772,7 +773,7 @@ class _QKVRopeAttention(torch.autograd.Function):
                                        native.stream_ptr()), "gemm2_rope")
         out = torch.empty(B, S, n_heads * hd, dtype=x.dtype, device=x.device)
         lse = torch.empty(B, n_heads, S, dtype=torch.float32, device=x.device)
-        native.check(L.tplr_attention_fwd(qkv.data_ptr(), out.data_ptr(), lse.data_ptr(), B, S, n_heads, n_kv, qkv.stride(1),
+        native.check(L.tplr_attention_fwd(qkv.data_ptr(), out.data_ptr(), lse.data_ptr(), B, S, n_heads, n_kv, hd, qkv.stride(1),
                                           out.stride(1), hd ** -0.5, st, native.stream_ptr()), "attention_fwd")
         ctx.save_for_backward(x, w, qkv, out, lse, cos, sin)
         ctx.main_grad, ctx.dims = main_grad, (n_heads, n_kv, hd)
@@ -789,7 +790,7 @@ class _QKVRopeAttention(torch.autograd.Function):
         delta = torch.empty(B, n_heads, S, dtype=torch.float32, device=qkv.device)
         native.check(native.lib().tplr_attention_bwd_unrope(
             qkv.data_ptr(), out.data_ptr(), do.data_ptr(), lse.data_ptr(), delta.data_ptr(), dq32.data_ptr(), dqkv.data_ptr(),
-            B, S, n_heads, n_kv, qkv.stride(1), out.stride(1), hd ** -0.5, cos.data_ptr(), sin.data_ptr(),
+            B, S, n_heads, n_kv, hd, qkv.stride(1), out.stride(1), hd ** -0.5, cos.data_ptr(), sin.data_ptr(),
             status_word(qkv.device).data_ptr(), native.stream_ptr()), "attention_bwd_unrope")
         del dq32, delta
         d2 = dqkv.view(-1, C)
@@ -818,7 +819,7 @@ class _AttentionBlock(torch.autograd.Function):
                                        native.stream_ptr()), "gemm2_rope")
         out = torch.empty(B, S, n_heads * hd, dtype=x.dtype, device=x.device)
         lse = torch.empty(B, n_heads, S, dtype=torch.float32, device=x.device)
-        native.check(L.tplr_attention_fwd(qkv.data_ptr(), out.data_ptr(), lse.data_ptr(), B, S, n_heads, n_kv, qkv.stride(1),
+        native.check(L.tplr_attention_fwd(qkv.data_ptr(), out.data_ptr(), lse.data_ptr(), B, S, n_heads, n_kv, hd, qkv.stride(1),
                                           out.stride(1), hd ** -0.5, st, native.stream_ptr()), "attention_fwd")
         y = torch.empty(B, S, wo.shape[0], dtype=x.dtype, device=x.device)
         gemm(out.view(-1, n_heads * hd), wo, out=y.view(-1, wo.shape[0]))
@@ -842,14 +843,14 @@ class _AttentionBlock(torch.autograd.Function):
         do = torch.empty(T, N, dtype=qkv.dtype, device=qkv.device)
         delta = torch.empty(B, n_heads, S, dtype=torch.float32, device=qkv.device)
         native.check(L.tplr_gemm2_attn_dout(dy2.data_ptr(), wo.data_ptr(), out2.data_ptr(), do.data_ptr(), delta.data_ptr(), T, N,
-                                            dy2.shape[1], S, dy2.stride(0), wo.stride(0), out2.stride(0), do.stride(0), st,
+                                            dy2.shape[1], S, hd, dy2.stride(0), wo.stride(0), out2.stride(0), do.stride(0), st,
                                             native.stream_ptr()), "gemm2_attn_dout")
         dwo = _weight_grad(mg_wo, dy2, out2, wo, ctx.needs_input_grad[2])
         dqkv = torch.empty_like(qkv)
         dq32 = torch.zeros(B, S, N, dtype=torch.float32, device=qkv.device)
         native.check(L.tplr_attention_bwd_unrope_delta(
             qkv.data_ptr(), out.data_ptr(), do.data_ptr(), lse.data_ptr(), delta.data_ptr(), dq32.data_ptr(), dqkv.data_ptr(),
-            B, S, n_heads, n_kv, qkv.stride(1), out.stride(1), hd ** -0.5, cos.data_ptr(), sin.data_ptr(), st,
+            B, S, n_heads, n_kv, hd, qkv.stride(1), out.stride(1), hd ** -0.5, cos.data_ptr(), sin.data_ptr(), st,
             native.stream_ptr()), "attention_bwd_unrope_delta")
         del dq32, delta, do
         d2 = dqkv.view(T, C)
@@ -868,7 +869,7 @@ def attention_block(x, wqkv, wo, cos, sin, n_heads: int, n_kv: int, hd: int, mai
         main_grad_wo = getattr(wo, "main_grad", None)
     B, S, K = x.shape
     if (FUSED_PROJECTIONS and _ATTN_BACKEND == "tcgen05" and _GEMM_BACKEND == "tcgen05_2sm" and _native_ok(x, wqkv, wo)
-            and x.dtype == torch.bfloat16 and hd == 128 and S % 128 == 0 and n_heads % n_kv == 0 and x.is_contiguous()
+            and x.dtype == torch.bfloat16 and hd in OWN_HEAD_DIMS and n_heads % n_kv == 0 and x.is_contiguous()
             and wqkv.stride(1) == 1 and wo.stride(1) == 1 and wqkv.stride(0) % 8 == 0 and wo.stride(0) % 8 == 0 and K % 8 == 0
             and wo.shape[0] % 8 == 0 and wo.shape[1] == n_heads * hd and cos.is_cuda and cos.dtype == torch.float32
             and cos.is_contiguous() and sin.is_contiguous() and cos.shape[0] >= S and cos.shape[1] == hd // 2
@@ -885,7 +886,7 @@ def rope_attention_projection(x, w, cos, sin, n_heads: int, n_kv: int, hd: int, 
         main_grad = getattr(w, "main_grad", None)
     B, S, K = x.shape
     if (FUSED_PROJECTIONS and _ATTN_BACKEND == "tcgen05" and _GEMM_BACKEND == "tcgen05_2sm" and _native_ok(x, w) and x.dtype == torch.bfloat16
-            and hd == 128 and S % 128 == 0 and n_heads % n_kv == 0 and x.is_contiguous() and w.stride(1) == 1
+            and hd in OWN_HEAD_DIMS and n_heads % n_kv == 0 and x.is_contiguous() and w.stride(1) == 1
             and w.stride(0) % 8 == 0 and K % 8 == 0 and w.shape[0] % 8 == 0 and cos.is_cuda and cos.dtype == torch.float32
             and cos.is_contiguous() and sin.is_contiguous() and cos.shape[0] >= S and cos.shape[1] == hd // 2
             and cos.data_ptr() % 16 == 0 and sin.data_ptr() % 16 == 0 and x.data_ptr() % 16 == 0 and w.data_ptr() % 16 == 0):
@@ -900,17 +901,17 @@ _attn_fallback_seen: set = set()
 def attention_packed(qkv, n_heads: int, n_kv: int, hd: int):
     """Causal attention of ``qkv`` [B, S, (H + 2 KV) * hd] (q heads, k heads, v heads); returns [B, S, H * hd]."""
     B, S, C = qkv.shape
-    if (_ATTN_BACKEND == "tcgen05" and qkv.is_cuda and qkv.dtype == torch.bfloat16 and hd == 128 and S % 128 == 0
+    if (_ATTN_BACKEND == "tcgen05" and qkv.is_cuda and qkv.dtype == torch.bfloat16 and hd in OWN_HEAD_DIMS
             and n_heads % n_kv == 0 and qkv.stride(2) == 1 and qkv.stride(0) == S * qkv.stride(1)
             and qkv.stride(1) % 8 == 0 and qkv.data_ptr() % 16 == 0):
         return _AttentionPacked.apply(qkv, n_heads, n_kv, hd)
-    if _ATTN_BACKEND == "tcgen05" and qkv.is_cuda and (hd, S % 128) not in _attn_fallback_seen:
+    if _ATTN_BACKEND == "tcgen05" and qkv.is_cuda and (hd, qkv.dtype) not in _attn_fallback_seen:
         # said once per shape class: a GPU run that silently uses the library kernel would misreport what ran
-        _attn_fallback_seen.add((hd, S % 128))
+        _attn_fallback_seen.add((hd, qkv.dtype))
         import warnings
 
         warnings.warn(f"attention_packed: head_dim {hd}, sequence {S}, dtype {qkv.dtype} is outside the own flash-attention "
-                      f"kernels (bf16, head_dim 128, sequence a multiple of 128); using torch SDPA for it", stacklevel=2)
+                      f"kernels (bf16, head_dim 64 or 128); using torch SDPA for it", stacklevel=2)
     q, k, v = _split_qkv(qkv, n_heads, n_kv, hd)
     return attention(q, k, v).reshape(B, S, n_heads * hd)
 

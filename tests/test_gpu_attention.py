@@ -196,3 +196,40 @@ def test_attention_block_with_delta_from_the_output_projection_epilogue(B, S, H,
         e_s = [rel(ys, ref)] + [rel(a, b.grad) for a, b in zip(gs, (xf, wf, of))]
         assert max(e_f) < 3e-2, (e_f, e_s)
         assert all(a < 1.5 * b + 2e-3 for a, b in zip(e_f, e_s)), (e_f, e_s)
+
+
+@pytest.mark.parametrize("B,S,H,KV,hd", [(1, 1, 1, 1, 64), (2, 127, 2, 1, 128), (3, 129, 3, 3, 64), (2, 200, 4, 2, 64),
+                                         (2, 384, 6, 2, 64), (1, 161, 2, 2, 128), (2, 1000, 3, 1, 64)])
+def test_attention_head_dim_64_and_ragged_sequences(B, S, H, KV, hd):
+    """Packed attention and the whole attention block at both head dimensions and at sequence lengths around the tile
+    edges (one row, one short, one over, a quarter of the last block only)."""
+    torch.manual_seed(S + hd)
+    D = H * hd
+    OF.status_word(DEV).zero_()
+    qkv = torch.randn(B, S, (H + 2 * KV) * hd, device=DEV).to(torch.bfloat16).requires_grad_()
+    out = OF.attention_packed(qkv, H, KV, hd)
+    dout = torch.randn_like(out)
+    out.backward(dout)
+    ref_in = qkv.detach().float().requires_grad_()
+    ref = _reference(ref_in, H, KV, hd)
+    ref.backward(dout.float())
+    # P and dS enter the products as bf16 (2^-9 relative), outputs are bf16: the bounds of the tests above
+    assert (out.float() - ref).abs().max().item() < 2e-2
+    assert (qkv.grad.float() - ref_in.grad).abs().max().item() < 2e-2 * max(ref_in.grad.abs().max().item(), 1.0)
+    # the block as one node against the same steps in fp32
+    x = torch.randn(B, S, D, device=DEV).to(torch.bfloat16)
+    wqkv = (torch.randn((H + 2 * KV) * hd, D, device=DEV) / D ** 0.5).to(torch.bfloat16)
+    wo = (torch.randn(D, D, device=DEV) / D ** 0.5).to(torch.bfloat16)
+    cos, sin = OF.rope_tables(S, hd, 10000.0, DEV)
+    dy = torch.randn(B, S, D, device=DEV).to(torch.bfloat16)
+    xs = [t.clone().requires_grad_() for t in (x, wqkv, wo)]
+    y = OF.attention_block(*xs, cos, sin, H, KV, hd)
+    y.backward(dy)
+    fs = [t.float().requires_grad_() for t in (x, wqkv, wo)]
+    rot = OF._rope_torch(fs[0] @ fs[1].t(), cos, sin, (H + KV) * hd, hd, False)
+    yr = _reference(rot, H, KV, hd) @ fs[2].t()
+    yr.backward(dy.float())
+    torch.cuda.synchronize()
+    assert int(OF.status_word(DEV).item()) == 0
+    for got, want in [(y, yr)] + [(a.grad, f.grad) for a, f in zip(xs, fs)]:
+        assert ((got.float() - want).norm() / want.norm()).item() < 2e-2      # five roundings to bf16 on the way, 2^-9 each
