@@ -392,29 +392,36 @@ TPLR_API int tplr_attention_fwd(const void* qkv, void* out, float* lse, int B, i
 }
 
 // ------------------------------------------------------------------------------------------ //
-// Backward.  CTA = one 128-row key/value block of one kv head; it walks the query heads of the
-// group and the query blocks at or below the diagonal.  Per step:
+// Backward.  CTA = one 128-row key/value block of one kv head and the query heads of its group, or a part of them; it
+// walks those heads and the query blocks at or below the diagonal.  Per step:
 //   S = Q K^T, dP = dO V^T            (tensor cores -> TMEM)
 //   P = exp2(S*scale - lse), dS = P * (dP - delta) * scale   (softmax warps, one query row per thread;
 //                                      P and dS go to shared memory as bf16 in 128-byte-swizzled tiles)
 //   dV += P^T dO, dK += dS^T Q        (accumulated in TMEM over the whole walk)
-//   dQ_partial = dS K                 (into the S columns, then TMA reduce-add into the fp32 dQ buffer)
+//   dQ_partial = dS K                 (into the dP columns, then TMA reduce-add into the fp32 dQ buffer)
 // The same swizzled tile serves as a K-major operand of one MMA and an MN-major operand of another,
 // so Q, dO, P and dS are each stored once.  K and V stay resident in shared memory.
+//
+// What bounds it is the chain of a step, not the tensor pipe (five products of 512 cycles each at DH = 128): so the step
+// is split where P is ready.  S of the next step is issued as soon as every warp has read this one's (Q has two buffers
+// for it) and runs, with dV, while the warps form dS; dP of the next step runs while they exponentiate its S.
+// B 8, S 2048, 16 heads of 128: 692 us with the parts of a step one after the other, 620 us here; the
+// shared-memory traffic of the five products and of P, dS and dQ would allow about 350.
 // ------------------------------------------------------------------------------------------ //
 namespace {
 
-template <int DH> constexpr int bwd_smem() { return 4 * tile_bytes<DH>() + 2 * PT_BYTES + 1024; }   // K, V, Q, dO; P, dS
+template <int DH> constexpr int bwd_smem() { return 5 * tile_bytes<DH>() + 2 * PT_BYTES + 1024; }   // K, V, two Q, dO; P, dS
 constexpr int BWD_THREADS = 320;                        // TMA warp, MMA warp, 8 softmax warps (2 per TMEM lane quadrant)
 
 struct AttnBwdParams {
   CUtensorMap tmQKV;    // [B, S, C] bf16, box 64 x 128 x 1
   CUtensorMap tmDO;     // [B, S, H*DH] bf16, box 64 x 128 x 1
-  CUtensorMap tmDQ;     // [B, S, H*DH] fp32, box 32 x 32 x 1 (reduce-add target)
+  CUtensorMap tmDQ;     // [B, S, H*DH] (split: all C columns) fp32, box 32 x 32 x 1 (reduce-add target)
   CUtensorMap tmDQKV;   // [B, S, C] bf16, box 64 x 32 x 1 (dK and dV stores)
   const float* lse;
   const float* delta;
   int B, S, H, KV;
+  int split;            // CTAs that share a group's query heads; > 1: dK and dV are reduce-added into the fp32 buffer too
   float scale, scale_log2;
   unsigned int* status;
   // not null: q and k were rotated (rotary embedding, interleaved pairs, tables [S, DH / 2] fp32) by the producer of qkv and
@@ -438,18 +445,21 @@ attn_bwd_kernel(const __grid_constant__ AttnBwdParams p) {
   constexpr int TILE_BYTES = tile_bytes<DH>();
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
-  __shared__ __align__(8) uint64_t bar_kv, bar_q_full, bar_q_empty, bar_do_full, bar_do_empty, bar_sp_full, bar_pds_full, bar_dq_full, bar_s_free;
+  __shared__ __align__(8) uint64_t bar_kv, bar_q_full[2], bar_q_empty[2], bar_do_full, bar_do_empty, bar_s_full, bar_dp_full,
+      bar_p_ready, bar_ds_ready, bar_dq_full, bar_dq_free;
   __shared__ uint32_t s_tmem_base;
   __shared__ int s_abort;
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int nQ = (p.S + BQ - 1) / BQ;
-  const int gb = p.KV * p.B;
+  const int gb = p.KV * p.B * p.split;
   const int j = (int)(blockIdx.x / gb);                    // kv block; small j (long walks) first
-  const int g = (int)(blockIdx.x % gb) % p.KV, b = (int)(blockIdx.x % gb) / p.KV;
-  const int group = p.H / p.KV;
+  const int sub = (int)(blockIdx.x % gb) % p.split;
+  const int g = (int)(blockIdx.x % gb) / p.split % p.KV, b = (int)(blockIdx.x % gb) / p.split / p.KV;
+  const int heads = p.H / p.KV / p.split;                  // query heads of this CTA
+  const int h0 = (g * p.split + sub) * heads;
   const int n_i = nQ - j;                                  // query blocks j..nQ-1
-  const int n_it = group * n_i;
+  const int n_it = heads * n_i;
   const int kvrow0 = j * BKV;                              // position of the first key row; rows past S read as zeros
   const int kcol = (p.H + g) * DH, vcol = (p.H + p.KV + g) * DH;
   volatile int* abort_flag = &s_abort;
@@ -457,10 +467,11 @@ attn_bwd_kernel(const __grid_constant__ AttnBwdParams p) {
   if (threadIdx.x == 0) {
     s_abort = 0;
     mbar_init(smem_u32(&bar_kv), 1);
-    mbar_init(smem_u32(&bar_q_full), 1); mbar_init(smem_u32(&bar_q_empty), 1);
+    for (int s = 0; s < 2; ++s) { mbar_init(smem_u32(&bar_q_full[s]), 1); mbar_init(smem_u32(&bar_q_empty[s]), 1); }
     mbar_init(smem_u32(&bar_do_full), 1); mbar_init(smem_u32(&bar_do_empty), 1);
-    mbar_init(smem_u32(&bar_sp_full), 1); mbar_init(smem_u32(&bar_pds_full), 8);
-    mbar_init(smem_u32(&bar_dq_full), 1); mbar_init(smem_u32(&bar_s_free), 8);
+    mbar_init(smem_u32(&bar_s_full), 1); mbar_init(smem_u32(&bar_dp_full), 1);
+    mbar_init(smem_u32(&bar_p_ready), 8); mbar_init(smem_u32(&bar_ds_ready), 8);
+    mbar_init(smem_u32(&bar_dq_full), 1); mbar_init(smem_u32(&bar_dq_free), 8);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
   }
@@ -473,7 +484,7 @@ attn_bwd_kernel(const __grid_constant__ AttnBwdParams p) {
   tcgen05_fence_after();
   const uint32_t tmem_base = s_tmem_base;
   const uint32_t tS = tmem_base, tdP = tmem_base + 128, tdV = tmem_base + 256, tdK = tmem_base + 256 + DH;
-  const uint32_t sK = smem_u32(smem), sV = sK + TILE_BYTES, sQ = sV + TILE_BYTES, sdO = sQ + TILE_BYTES,
+  const uint32_t sK = smem_u32(smem), sV = sK + TILE_BYTES, sQ = sV + TILE_BYTES, sdO = sQ + 2 * TILE_BYTES,
                  sP = sdO + TILE_BYTES, sdS = sP + PT_BYTES;
 
   if (warp == 0) {
@@ -483,14 +494,12 @@ attn_bwd_kernel(const __grid_constant__ AttnBwdParams p) {
       load_tile<DH>(sV, &p.tmQKV, smem_u32(&bar_kv), vcol, kvrow0, b);
       bool ok = true;
       for (int t = 0; t < n_it && ok; ++t) {
-        const int h = g * group + t / n_i, i = j + t % n_i;
-        const int qrow0 = i * BQ, qcol = h * DH;
-        // Q is released by the dK MMAs and dO by the dV MMAs of the previous step, both before its dQ MMAs and the
-        // dQ drain: the next tiles are in flight while those run
-        if (!(ok = mbar_wait(smem_u32(&bar_q_empty), (uint32_t)((t & 1) ^ 1), abort_flag))) break;
-        const uint32_t fq = smem_u32(&bar_q_full);
+        const int h = h0 + t / n_i, i = j + t % n_i;
+        const int qrow0 = i * BQ, qcol = h * DH, s = t & 1;
+        if (!(ok = mbar_wait(smem_u32(&bar_q_empty[s]), (uint32_t)(((t >> 1) & 1) ^ 1), abort_flag))) break;
+        const uint32_t fq = smem_u32(&bar_q_full[s]);
         mbar_expect_tx(fq, TILE_BYTES);
-        load_tile<DH>(sQ, &p.tmQKV, fq, qcol, qrow0, b);
+        load_tile<DH>(sQ + s * TILE_BYTES, &p.tmQKV, fq, qcol, qrow0, b);
         if (!(ok = mbar_wait(smem_u32(&bar_do_empty), (uint32_t)((t & 1) ^ 1), abort_flag))) break;
         const uint32_t fd = smem_u32(&bar_do_full);
         mbar_expect_tx(fd, TILE_BYTES);
@@ -501,40 +510,60 @@ attn_bwd_kernel(const __grid_constant__ AttnBwdParams p) {
     if (lane == 0) {
       const uint32_t id_kk = idesc_mn(128, false, false), id_mm = idesc_mn(DH, true, true), id_km = idesc_mn(DH, false, true);
       // descriptor bases: "k" = contraction along the 128-byte rows, "m" = contraction along the tile rows
+      // (every operand is made of 128-row blocks of 64 columns, 16 KB apart)
       const DescBase kQ = desc_base(sQ, 16, 1024), kK = desc_base(sK, 16, 1024), kdO = desc_base(sdO, 16, 1024),
                      kV = desc_base(sV, 16, 1024), kdS = desc_base(sdS, 16, 1024);
-      // (every operand is made of 128-row blocks of 64 columns, 16 KB apart)
       const DescBase mP = desc_base(sP, 128 * 128, 1024), mdO = desc_base(sdO, 128 * 128, 1024),
                      mdS = desc_base(sdS, 128 * 128, 1024), mQ = desc_base(sQ, 128 * 128, 1024),
                      mK = desc_base(sK, 128 * 128, 1024);
 #define TPLR_KOFF(kk) ((uint32_t)((kk) >> 2) * (128u * 128u / 16u) + (uint32_t)((kk) & 3) * 2u)
 #define TPLR_MOFF(kk) ((uint32_t)(kk) * 128u)
-      bool ok = mbar_wait(smem_u32(&bar_kv), 0, abort_flag);
-      for (int t = 0; t < n_it && ok; ++t) {
-        const uint32_t ph = t & 1;
-        if (!(ok = mbar_wait(smem_u32(&bar_q_full), ph, abort_flag))) break;
-        if (t > 0 && !(ok = mbar_wait(smem_u32(&bar_s_free), ph ^ 1, abort_flag))) break;
-        tcgen05_fence_after();
+      auto issue_s = [&](int t) {
+        const uint32_t q = (uint32_t)(t & 1) * (TILE_BYTES / 16);
 #pragma unroll
-        for (int kk = 0; kk < DH / 16; ++kk) umma_bf16_b(tS, kQ, TPLR_KOFF(kk), kK, TPLR_KOFF(kk), id_kk, kk > 0 ? 1u : 0u);
-        if (!(ok = mbar_wait(smem_u32(&bar_do_full), ph, abort_flag))) break;
+        for (int kk = 0; kk < DH / 16; ++kk)
+          umma_bf16_b(tS, kQ, q + TPLR_KOFF(kk), kK, TPLR_KOFF(kk), id_kk, kk > 0 ? 1u : 0u);
+        umma_commit(smem_u32(&bar_s_full));
+      };
+      auto issue_dp = [&] {
 #pragma unroll
         for (int kk = 0; kk < DH / 16; ++kk) umma_bf16_b(tdP, kdO, TPLR_KOFF(kk), kV, TPLR_KOFF(kk), id_kk, kk > 0 ? 1u : 0u);
-        umma_commit(smem_u32(&bar_sp_full));
-        if (!(ok = mbar_wait(smem_u32(&bar_pds_full), ph, abort_flag))) break;
+        umma_commit(smem_u32(&bar_dp_full));
+      };
+      bool ok = mbar_wait(smem_u32(&bar_kv), 0, abort_flag);
+      if (ok) ok = mbar_wait(smem_u32(&bar_q_full[0]), 0, abort_flag);
+      if (ok) { tcgen05_fence_after(); issue_s(0); }
+      if (ok) ok = mbar_wait(smem_u32(&bar_do_full), 0, abort_flag);
+      if (ok) { tcgen05_fence_after(); issue_dp(); }
+      for (int t = 0; t < n_it && ok; ++t) {
+        const uint32_t ph = t & 1;
+        if (!(ok = mbar_wait(smem_u32(&bar_p_ready), ph, abort_flag))) break;      // P stored, S read by every warp
         tcgen05_fence_after();
-#pragma unroll
-        for (int kk = 0; kk < 8; ++kk)      // dK[kv, d] += dS^T[kv, q] Q[q, d]   (first: Q is what the next step needs first)
-          umma_bf16_b(tdK, mdS, TPLR_MOFF(kk), mQ, TPLR_MOFF(kk), id_mm, (t > 0 || kk > 0) ? 1u : 0u);
-        umma_commit(smem_u32(&bar_q_empty));
+        if (t + 1 < n_it) {
+          if (!(ok = mbar_wait(smem_u32(&bar_q_full[(t + 1) & 1]), (uint32_t)(((t + 1) >> 1) & 1), abort_flag))) break;
+          tcgen05_fence_after();
+          issue_s(t + 1);
+        }
 #pragma unroll
         for (int kk = 0; kk < 8; ++kk)      // dV[kv, d] += P^T[kv, q] dO[q, d]
           umma_bf16_b(tdV, mP, TPLR_MOFF(kk), mdO, TPLR_MOFF(kk), id_mm, (t > 0 || kk > 0) ? 1u : 0u);
         umma_commit(smem_u32(&bar_do_empty));
+        if (!(ok = mbar_wait(smem_u32(&bar_ds_ready), ph, abort_flag))) break;     // dS stored, dP read by every warp
+        tcgen05_fence_after();
 #pragma unroll
-        for (int kk = 0; kk < 8; ++kk)      // dQ[q, d] = dS[q, kv] K[kv, d]
-          umma_bf16_b(tS, kdS, TPLR_KOFF(kk), mK, TPLR_MOFF(kk), id_km, kk > 0 ? 1u : 0u);
+        for (int kk = 0; kk < 8; ++kk)      // dK[kv, d] += dS^T[kv, q] Q[q, d]
+          umma_bf16_b(tdK, mdS, TPLR_MOFF(kk), mQ, ph * (TILE_BYTES / 16) + TPLR_MOFF(kk), id_mm, (t > 0 || kk > 0) ? 1u : 0u);
+        umma_commit(smem_u32(&bar_q_empty[ph]));
+#pragma unroll
+        for (int kk = 0; kk < 8; ++kk)      // dQ[q, d] = dS[q, kv] K[kv, d], over dP; its commit covers every product before it
+          umma_bf16_b(tdP, kdS, TPLR_KOFF(kk), mK, TPLR_MOFF(kk), id_km, kk > 0 ? 1u : 0u);
         umma_commit(smem_u32(&bar_dq_full));
+        if (t + 1 < n_it) {
+          if (!(ok = mbar_wait(smem_u32(&bar_do_full), ph ^ 1u, abort_flag))) break;
+          if (!(ok = mbar_wait(smem_u32(&bar_dq_free), ph, abort_flag))) break;    // dQ read by every warp
+          tcgen05_fence_after();
+          issue_dp();
+        }
       }
     }
   } else {
@@ -543,140 +572,202 @@ attn_bwd_kernel(const __grid_constant__ AttnBwdParams p) {
     const int r = quad * 32 + lane;
     const uint32_t lane_off = (uint32_t)(quad * 32) << 16;
     const uint32_t sw = (uint32_t)(lane & 7);
-    // two private 4 KB staging buffers: the bytes of this warp's own rows and column half in the P and dS tiles
+    // two private 4 KB staging buffers: the bytes of this warp's own rows and column half in the P and dS tiles.  Free from
+    // the step's last commit on (it covers the products that read them); the reduce-adds have read them before the warp
+    // writes its next P.
     const uint32_t stg0 = sP + (uint32_t)ch * (PT_BYTES / 2) + (uint32_t)quad * 4096u;
     const uint32_t stg1 = sdS + (uint32_t)ch * (PT_BYTES / 2) + (uint32_t)quad * 4096u;
+    const uint32_t prow = sP + (uint32_t)ch * (PT_BYTES / 2) + (uint32_t)r * 128u;
+    const uint32_t drow = sdS + (uint32_t)ch * (PT_BYTES / 2) + (uint32_t)r * 128u;
+    // the row statistics of step t; a query row past the end of the sequence has no weight: lse = +inf makes its P zero
+    auto stats = [&](int t, float& lse2, float& dl) {
+      const int h = h0 + t / n_i, row = (j + t % n_i) * BQ + r;
+      const long long at = ((long long)b * p.H + h) * p.S + row;
+      const bool live = row < p.S;
+      lse2 = live ? p.lse[at] : INFINITY;
+      dl = live ? p.delta[at] : 0.f;
+    };
+    float lse_n, dl_n;
+    stats(0, lse_n, dl_n);
     bool ok = true;
     for (int t = 0; t < n_it && ok; ++t) {
-      const int h = g * group + t / n_i, i = j + t % n_i;
-      const long long stat = ((long long)b * p.H + h) * p.S + i * BQ + r;
-      // a query row past the end of the sequence has no weight: lse = +inf makes its P and with it dS zero
-      const bool live = i * BQ + r < p.S;
-      const float lse2 = live ? p.lse[stat] * 1.4426950408889634f : INFINITY;
-      const float dl = live ? p.delta[stat] : 0.f;
-      ok = mbar_wait(smem_u32(&bar_sp_full), t & 1, abort_flag);
+      const int h = h0 + t / n_i, i = j + t % n_i;
+      const float lse2 = lse_n * 1.4426950408889634f, dls = dl_n * p.scale;
+      if (t + 1 < n_it) stats(t + 1, lse_n, dl_n);           // in flight during this step
+      ok = mbar_wait(smem_u32(&bar_s_full), t & 1, abort_flag);
       ok = __all_sync(0xffffffffu, ok);
       if (!ok) break;
       tcgen05_fence_after();
-      // P and dS of this warp's two 32-column chunks; the diagonal block runs the variant with the causal mask,
-      // the others the one without the per-element compare (the softmax warps are issue-bound).  dS carries the
-      // softmax scale: d = p * (dp - delta) * scale = p * fma(dp, scale, -delta * scale).
-      const float dls = dl * p.scale;
-      auto chunk_pair = [&](auto DIAG) {
+      // P of this warp's 64 columns, kept in fp32 for dS; the diagonal block runs the variant with the causal mask
+      float pv[64];
+      auto p_part = [&](auto DIAG) {
         constexpr bool kDiag = decltype(DIAG)::value;
-#pragma unroll 1
-        for (int c = 2 * ch; c < 2 * ch + 2; ++c) {
-          uint32_t sv[32], dv[32];
-          tmem_ld32(tS + c * 32 + lane_off, sv);
-          tmem_ld32(tdP + c * 32 + lane_off, dv);
-          const uint32_t prow = sP + (uint32_t)(c >> 1) * (PT_BYTES / 2) + (uint32_t)r * 128u;
-          const uint32_t drow = sdS + (uint32_t)(c >> 1) * (PT_BYTES / 2) + (uint32_t)r * 128u;
 #pragma unroll
-          for (int q4 = 0; q4 < 4; ++q4) {
-            uint32_t pw[4], dw[4];
+        for (int cc = 0; cc < 2; ++cc) {
+          uint32_t sv[32];
+          tmem_ld32(tS + ch * 64 + cc * 32 + lane_off, sv);
 #pragma unroll
-            for (int e = 0; e < 4; ++e) {
-              float p0 = exp2f(fmaf(__uint_as_float(sv[q4 * 8 + 2 * e]), p.scale_log2, -lse2));
-              float p1 = exp2f(fmaf(__uint_as_float(sv[q4 * 8 + 2 * e + 1]), p.scale_log2, -lse2));
-              if (kDiag) {
-                const int col = c * 32 + q4 * 8 + 2 * e;
-                if (col > r) p0 = 0.f;
-                if (col + 1 > r) p1 = 0.f;
-              }
-              const float d0 = p0 * fmaf(__uint_as_float(dv[q4 * 8 + 2 * e]), p.scale, -dls);
-              const float d1 = p1 * fmaf(__uint_as_float(dv[q4 * 8 + 2 * e + 1]), p.scale, -dls);
-              __nv_bfloat162 hp = __floats2bfloat162_rn(p0, p1), hd = __floats2bfloat162_rn(d0, d1);
-              pw[e] = *reinterpret_cast<uint32_t*>(&hp);
-              dw[e] = *reinterpret_cast<uint32_t*>(&hd);
-            }
-            const uint32_t off = (((uint32_t)((c & 1) * 4 + q4)) ^ sw) << 4;
-            asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(prow + off), "r"(pw[0]), "r"(pw[1]), "r"(pw[2]), "r"(pw[3]) : "memory");
-            asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(drow + off), "r"(dw[0]), "r"(dw[1]), "r"(dw[2]), "r"(dw[3]) : "memory");
+          for (int e = 0; e < 32; ++e) {
+            float x = exp2f(fmaf(__uint_as_float(sv[e]), p.scale_log2, -lse2));
+            if (kDiag && ch * 64 + cc * 32 + e > r) x = 0.f;
+            pv[cc * 32 + e] = x;
           }
-        }
-      };
-      if (i == j) chunk_pair(cuda::std::true_type{}); else chunk_pair(cuda::std::false_type{});
-      asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-      tcgen05_fence_before();
-      __syncwarp();
-      if (lane == 0) mbar_arrive(smem_u32(&bar_pds_full));
-      // drain dQ_partial (fp32, in the S columns) into the global fp32 dQ with TMA reduce-add
-      ok = mbar_wait(smem_u32(&bar_dq_full), t & 1, abort_flag);
-      ok = __all_sync(0xffffffffu, ok);
-      if (!ok) break;
-      tcgen05_fence_after();
-      const int qrow0 = i * BQ + quad * 32;
-#pragma unroll
-      for (int cc = 0; cc < DH / 64; ++cc) {
-        const int c = DH / 64 * ch + cc;
-        uint32_t v[32];
-        tmem_ld32(tS + c * 32 + lane_off, v);
-        const uint32_t buf = cc ? stg1 : stg0;
-        const uint32_t rowaddr = buf + (uint32_t)lane * 128u;
-#pragma unroll
-        for (int q8 = 0; q8 < 8; ++q8)
-          asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(rowaddr + (((uint32_t)q8 ^ sw) << 4)), "r"(v[4 * q8]),
-                       "r"(v[4 * q8 + 1]), "r"(v[4 * q8 + 2]), "r"(v[4 * q8 + 3]) : "memory");
-        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-        __syncwarp();
-        if (lane == 0 && qrow0 < p.S) {
-          tma_reduce_add_3d(&p.tmDQ, buf, h * DH + c * 32, qrow0, b);
-          asm volatile("cp.async.bulk.commit_group;" ::: "memory");
-        }
-      }
-      if (lane == 0) asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");   // P rows may be rewritten
-      tcgen05_fence_before();
-      __syncwarp();
-      if (lane == 0) mbar_arrive(smem_u32(&bar_s_free));
-    }
-    // dV and dK of this kv block: TMEM -> bf16 -> staging -> TMA store into the packed gradient
-    if (ok) {
-      tcgen05_fence_after();
-      const int orow0 = kvrow0 + quad * 32;
-#pragma unroll
-      for (int acc = 0; acc < 2; ++acc) {      // 0 = dV, 1 = dK; at 128 columns this warp stores its half of each, at 64 one of them
-        if (DH == 64 && acc != ch) continue;
-        const int col = DH == 64 ? 0 : ch * 64;
-        const uint32_t tacc = acc ? tdK : tdV;
-        const uint32_t buf = acc ? stg1 : stg0;
-        const uint32_t rowaddr = buf + (uint32_t)lane * 128u;
-#pragma unroll
-        for (int hf = 0; hf < 2; ++hf) {
-          uint32_t v[32];
-          tmem_ld32(tacc + col + hf * 32 + lane_off, v);
-          if (acc == 1 && p.rope_cos) {          // dK back through the rotation of this key row: the opposite angle
-            const long long tb = (long long)min(orow0 + lane, p.S - 1) * (DH / 2) + (col + hf * 32) / 2;
-            const float4* cp = reinterpret_cast<const float4*>(p.rope_cos + tb);
-            const float4* sp = reinterpret_cast<const float4*>(p.rope_sin + tb);
-#pragma unroll
-            for (int q = 0; q < 4; ++q) {
-              const float4 cv = cp[q], sv = sp[q];
-              const float cc[4] = {cv.x, cv.y, cv.z, cv.w}, ss[4] = {sv.x, sv.y, sv.z, sv.w};
-#pragma unroll
-              for (int e = 0; e < 4; ++e) {
-                const float a = __uint_as_float(v[8 * q + 2 * e]), b = __uint_as_float(v[8 * q + 2 * e + 1]);
-                v[8 * q + 2 * e] = __float_as_uint(a * cc[e] + b * ss[e]);
-                v[8 * q + 2 * e + 1] = __float_as_uint(b * cc[e] - a * ss[e]);
-              }
-            }
+          if (cc == 0 && t > 0) {                            // the staged dQ of the previous step has left these bytes
+            if (lane == 0) asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
+            __syncwarp();
           }
 #pragma unroll
           for (int q4 = 0; q4 < 4; ++q4) {
             uint32_t pw[4];
 #pragma unroll
             for (int e = 0; e < 4; ++e) {
-              __nv_bfloat162 hh = __floats2bfloat162_rn(__uint_as_float(v[8 * q4 + 2 * e]), __uint_as_float(v[8 * q4 + 2 * e + 1]));
-              pw[e] = *reinterpret_cast<uint32_t*>(&hh);
+              __nv_bfloat162 hp = __floats2bfloat162_rn(pv[cc * 32 + q4 * 8 + 2 * e], pv[cc * 32 + q4 * 8 + 2 * e + 1]);
+              pw[e] = *reinterpret_cast<uint32_t*>(&hp);
             }
-            asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(rowaddr + ((((uint32_t)(hf * 4 + q4)) ^ sw) << 4)),
+            asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(prow + ((((uint32_t)(cc * 4 + q4)) ^ sw) << 4)),
                          "r"(pw[0]), "r"(pw[1]), "r"(pw[2]), "r"(pw[3]) : "memory");
           }
         }
-        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+      };
+      if (i == j) p_part(cuda::std::true_type{}); else p_part(cuda::std::false_type{});
+      asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+      tcgen05_fence_before();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(smem_u32(&bar_p_ready));
+      ok = mbar_wait(smem_u32(&bar_dp_full), t & 1, abort_flag);
+      ok = __all_sync(0xffffffffu, ok);
+      if (!ok) break;
+      tcgen05_fence_after();
+      // dS carries the softmax scale: d = p * (dp - delta) * scale = p * fma(dp, scale, -delta * scale)
+#pragma unroll
+      for (int cc = 0; cc < 2; ++cc) {
+        uint32_t dv[32];
+        tmem_ld32(tdP + ch * 64 + cc * 32 + lane_off, dv);
+#pragma unroll
+        for (int q4 = 0; q4 < 4; ++q4) {
+          uint32_t dw[4];
+#pragma unroll
+          for (int e = 0; e < 4; ++e) {
+            const int k = q4 * 8 + 2 * e;
+            const float d0 = pv[cc * 32 + k] * fmaf(__uint_as_float(dv[k]), p.scale, -dls);
+            const float d1 = pv[cc * 32 + k + 1] * fmaf(__uint_as_float(dv[k + 1]), p.scale, -dls);
+            __nv_bfloat162 hd = __floats2bfloat162_rn(d0, d1);
+            dw[e] = *reinterpret_cast<uint32_t*>(&hd);
+          }
+          asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(drow + ((((uint32_t)(cc * 4 + q4)) ^ sw) << 4)),
+                       "r"(dw[0]), "r"(dw[1]), "r"(dw[2]), "r"(dw[3]) : "memory");
+        }
+      }
+      asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+      tcgen05_fence_before();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(smem_u32(&bar_ds_ready));
+      // drain dQ_partial (fp32, in the dP columns) into the global fp32 dQ with TMA reduce-add
+      ok = mbar_wait(smem_u32(&bar_dq_full), t & 1, abort_flag);
+      ok = __all_sync(0xffffffffu, ok);
+      if (!ok) break;
+      tcgen05_fence_after();
+      uint32_t dq[DH / 64][32];
+#pragma unroll
+      for (int cc = 0; cc < DH / 64; ++cc) tmem_ld32(tdP + (DH / 64 * ch + cc) * 32 + lane_off, dq[cc]);
+      tcgen05_fence_before();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(smem_u32(&bar_dq_free));
+      const int qrow0 = i * BQ + quad * 32;
+#pragma unroll
+      for (int cc = 0; cc < DH / 64; ++cc) {
+        const uint32_t rowaddr = (cc ? stg1 : stg0) + (uint32_t)lane * 128u;
+#pragma unroll
+        for (int q8 = 0; q8 < 8; ++q8)
+          asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(rowaddr + (((uint32_t)q8 ^ sw) << 4)), "r"(dq[cc][4 * q8]),
+                       "r"(dq[cc][4 * q8 + 1]), "r"(dq[cc][4 * q8 + 2]), "r"(dq[cc][4 * q8 + 3]) : "memory");
+      }
+      asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+      __syncwarp();
+      if (lane == 0 && qrow0 < p.S) {
+#pragma unroll
+        for (int cc = 0; cc < DH / 64; ++cc)
+          tma_reduce_add_3d(&p.tmDQ, cc ? stg1 : stg0, h * DH + (DH / 64 * ch + cc) * 32, qrow0, b);
+        asm volatile("cp.async.bulk.commit_group;" ::: "memory");
+      }
+    }
+    // dV and dK of this kv block.  Whole group in this CTA: TMEM -> bf16 -> staging -> TMA store into the packed gradient;
+    // a part of it: reduce-added in fp32 beside dQ, and rotated back and rounded by the pass that does so for dQ.
+    if (ok) {
+      tcgen05_fence_after();
+      const int orow0 = kvrow0 + quad * 32;
+      if (p.split > 1) {
+#pragma unroll 1
+        for (int x = 0; x < DH / 32; ++x) {      // 32-column boxes of dV, then of dK; this warp takes one column half of each
+          const int acc = x / (DH / 64), col = (DH / 64 * ch + x % (DH / 64)) * 32;
+          const uint32_t buf = (x & 1) ? stg1 : stg0;
+          if (lane == 0) {
+            if (x < 2) asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
+            else       asm volatile("cp.async.bulk.wait_group.read 1;" ::: "memory");
+          }
+          __syncwarp();
+          uint32_t v[32];
+          tmem_ld32((acc ? tdK : tdV) + col + lane_off, v);
+          const uint32_t rowaddr = buf + (uint32_t)lane * 128u;
+#pragma unroll
+          for (int q8 = 0; q8 < 8; ++q8)
+            asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(rowaddr + (((uint32_t)q8 ^ sw) << 4)), "r"(v[4 * q8]),
+                         "r"(v[4 * q8 + 1]), "r"(v[4 * q8 + 2]), "r"(v[4 * q8 + 3]) : "memory");
+          asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+          __syncwarp();
+          if (lane == 0) {
+            if (orow0 < p.S) tma_reduce_add_3d(&p.tmDQ, buf, (acc ? kcol : vcol) + col, orow0, b);
+            asm volatile("cp.async.bulk.commit_group;" ::: "memory");
+          }
+        }
+      } else {
+        if (lane == 0) asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
         __syncwarp();
-        if (lane == 0 && orow0 < p.S) {
-          tma_store_3d(&p.tmDQKV, buf, (acc ? kcol : vcol) + col, orow0, b);
-          asm volatile("cp.async.bulk.commit_group;" ::: "memory");
+#pragma unroll
+        for (int acc = 0; acc < 2; ++acc) {      // 0 = dV, 1 = dK; at 128 columns this warp stores its half of each, at 64 one of them
+          if (DH == 64 && acc != ch) continue;
+          const int col = DH == 64 ? 0 : ch * 64;
+          const uint32_t tacc = acc ? tdK : tdV;
+          const uint32_t buf = acc ? stg1 : stg0;
+          const uint32_t rowaddr = buf + (uint32_t)lane * 128u;
+#pragma unroll
+          for (int hf = 0; hf < 2; ++hf) {
+            uint32_t v[32];
+            tmem_ld32(tacc + col + hf * 32 + lane_off, v);
+            if (acc == 1 && p.rope_cos) {          // dK back through the rotation of this key row: the opposite angle
+              const long long tb = (long long)min(orow0 + lane, p.S - 1) * (DH / 2) + (col + hf * 32) / 2;
+              const float4* cp = reinterpret_cast<const float4*>(p.rope_cos + tb);
+              const float4* sp = reinterpret_cast<const float4*>(p.rope_sin + tb);
+#pragma unroll
+              for (int q = 0; q < 4; ++q) {
+                const float4 cv = cp[q], sv = sp[q];
+                const float cc[4] = {cv.x, cv.y, cv.z, cv.w}, ss[4] = {sv.x, sv.y, sv.z, sv.w};
+#pragma unroll
+                for (int e = 0; e < 4; ++e) {
+                  const float a = __uint_as_float(v[8 * q + 2 * e]), b2 = __uint_as_float(v[8 * q + 2 * e + 1]);
+                  v[8 * q + 2 * e] = __float_as_uint(a * cc[e] + b2 * ss[e]);
+                  v[8 * q + 2 * e + 1] = __float_as_uint(b2 * cc[e] - a * ss[e]);
+                }
+              }
+            }
+#pragma unroll
+            for (int q4 = 0; q4 < 4; ++q4) {
+              uint32_t pw[4];
+#pragma unroll
+              for (int e = 0; e < 4; ++e) {
+                __nv_bfloat162 hh = __floats2bfloat162_rn(__uint_as_float(v[8 * q4 + 2 * e]), __uint_as_float(v[8 * q4 + 2 * e + 1]));
+                pw[e] = *reinterpret_cast<uint32_t*>(&hh);
+              }
+              asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(rowaddr + ((((uint32_t)(hf * 4 + q4)) ^ sw) << 4)),
+                           "r"(pw[0]), "r"(pw[1]), "r"(pw[2]), "r"(pw[3]) : "memory");
+            }
+          }
+          asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+          __syncwarp();
+          if (lane == 0 && orow0 < p.S) {
+            tma_store_3d(&p.tmDQKV, buf, (acc ? kcol : vcol) + col, orow0, b);
+            asm volatile("cp.async.bulk.commit_group;" ::: "memory");
+          }
         }
       }
     }
@@ -716,16 +807,16 @@ __global__ void __launch_bounds__(256) attn_delta_kernel(const __nv_bfloat16* __
 }
 
 // dq32 [tokens, width] fp32 -> first `width` columns (heads of dh) of the packed bf16 gradient
-// cosb / sinb not null: the two pairs are rotated back by the angles of (token % S, pair index in the head) on the way
+// cosb / sinb not null: the two pairs are rotated back, in the first rot_cols columns, by the angles of (token % S, pair index in the head) on the way
 __global__ void __launch_bounds__(256) attn_dq_cast_kernel(const float* __restrict__ dq32, __nv_bfloat16* __restrict__ dqkv,
-                                                           long long tokens, int width, int dh, long long ld,
+                                                           long long tokens, int width, int rot_cols, int dh, long long ld,
                                                            const float* __restrict__ cosb, const float* __restrict__ sinb, int S) {
   const long long n4 = tokens * (width / 4);
   for (long long v = (long long)blockIdx.x * blockDim.x + threadIdx.x; v < n4; v += (long long)gridDim.x * blockDim.x) {
     const long long tok = v / (width / 4);
     const int c4 = (int)(v % (width / 4));
     float4 f = reinterpret_cast<const float4*>(dq32)[v];
-    if (cosb) {
+    if (cosb && c4 * 4 < rot_cols) {
       const long long tb = (tok % S) * (dh / 2) + ((c4 * 4) % dh) / 2;
       const float2 c = *reinterpret_cast<const float2*>(cosb + tb), sn = *reinterpret_cast<const float2*>(sinb + tb);
       f = make_float4(f.x * c.x + f.y * sn.x, f.y * c.x - f.x * sn.x, f.z * c.y + f.w * sn.y, f.w * c.y - f.z * sn.y);
@@ -1086,9 +1177,11 @@ TPLR_API int tplr_attention_set_bwd_variant(int v) {
 
 // Gradient of tplr_attention_fwd.  qkv / dqkv: packed [B*S, C] bf16 with row stride ld_qkv; out: the forward's
 // output (row stride ld_o); dout: contiguous [B*S, H*head_dim]; lse from the forward; delta: [B,H,S] fp32 scratch;
-// dq32: [B*S, H*head_dim] fp32 scratch that the caller has zeroed.  dqkv receives dq | dk | dv.
+// dq32: [B*S, tplr_attention_bwd_scratch_cols] fp32 scratch that the caller has zeroed.  dqkv receives dq | dk | dv.
 extern "C" int tplr_rope(void* buf, const float* cosb, const float* sinb, long long tokens, int S, int n_heads, int Dh,
                          long long row_stride, int inverse, void* stream);
+
+static int bwd_split(int B, int S, int H, int KV, int head_dim);
 
 namespace {
 template <int HD>
@@ -1123,18 +1216,39 @@ int launch_bwd(const void* qkv, const void* out, const void* dout, const float* 
   AttnBwdParams p = {};
   if (!make_map3(&p.tmQKV, qkv, C, S, B, ld_qkv, 64, 128)) return -202;
   if (!make_map3(&p.tmDO, dout, (long long)H * HD, S, B, (long long)H * HD, 64, 128)) return -203;
-  if (!make_map3(&p.tmDQ, dq32, (long long)H * HD, S, B, (long long)H * HD, 32, 32, true)) return -204;
+  p.split = bwd_split(B, S, H, KV, HD);
+  const int width = p.split > 1 ? C : H * HD;                  // what goes through the fp32 scratch
+  if (!make_map3(&p.tmDQ, dq32, width, S, B, width, 32, 32, true)) return -204;
   if (!make_map3(&p.tmDQKV, dqkv, C, S, B, ld_qkv, 64, 32)) return -205;
   p.lse = lse; p.delta = delta; p.B = B; p.S = S; p.H = H; p.KV = KV;
   p.scale = scale; p.scale_log2 = scale * 1.4426950408889634f; p.status = status;
   p.rope_cos = cosb; p.rope_sin = sinb;
   cudaError_t e = cudaFuncSetAttribute(attn_bwd_kernel<HD>, cudaFuncAttributeMaxDynamicSharedMemorySize, bwd_smem<HD>());
   if (e != cudaSuccess) return (int)e;
-  attn_bwd_kernel<HD><<<(unsigned)(((S + BKV - 1) / BKV) * KV * B), BWD_THREADS, bwd_smem<HD>(), st>>>(p);
-  attn_dq_cast_kernel<<<tplr_sm_count() * 8, 256, 0, st>>>(dq32, (__nv_bfloat16*)dqkv, tokens, H * HD, HD, ld_qkv, cosb, sinb, S);
+  attn_bwd_kernel<HD><<<(unsigned)(((S + BKV - 1) / BKV) * KV * B * p.split), BWD_THREADS, bwd_smem<HD>(), st>>>(p);
+  attn_dq_cast_kernel<<<tplr_sm_count() * 8, 256, 0, st>>>(dq32, (__nv_bfloat16*)dqkv, tokens, width, (H + KV) * HD, HD, ld_qkv, cosb, sinb, S);
   return (int)cudaGetLastError();
 }
 }  // namespace
+
+// CTAs that share a group's query heads.  One CTA per (key block, kv head, sequence) leaves SMs idle where heads are
+// grouped and the batch is small; each part then adds its dK and dV into the fp32 buffer, which costs a pass over 2 KV
+// heads more, so the group is only cut until there are two CTAs per SM.  B 1, S 1024, H 32, KV 8, head_dim 128: 155 us whole
+// (64 CTAs), 49 us in four parts (256 CTAs).
+static int bwd_split(int B, int S, int H, int KV, int head_dim) {
+  if (KV <= 0 || H % KV || (head_dim == 128 && S % 128 == 0 && g_bwd_variant == 2)) return 1;
+  const int group = H / KV;
+  const long long ctas = (long long)((S + BKV - 1) / BKV) * KV * B;
+  int split = 1;
+  for (int s = 1; s <= group && ctas * split < 2LL * tplr_sm_count(); ++s)
+    if (group % s == 0) split = s;
+  return split;
+}
+
+// Columns of the fp32 scratch that the backward needs for these sizes: [B*S, columns], zeroed by the caller.
+TPLR_API int tplr_attention_bwd_scratch_cols(int B, int S, int H, int KV, int head_dim) {
+  return (bwd_split(B, S, H, KV, head_dim) > 1 ? H + 2 * KV : H) * head_dim;
+}
 
 static int attention_bwd_impl(const void* qkv, const void* out, const void* dout, const float* lse, float* delta,
                               float* dq32, void* dqkv, int B, int S, int H, int KV, int head_dim, long long ld_qkv,

@@ -719,6 +719,12 @@ def _split_qkv(qkv, n_heads, n_kv, hd):
             qkv[..., nq + nk:].view(B, S, n_kv, hd))
 
 
+def _attention_scratch(B, S, n_heads, n_kv, hd, device):
+    """Zeroed fp32 buffer that the attention backward accumulates dq (and dk, dv where heads are split) into."""
+    cols = native.lib().tplr_attention_bwd_scratch_cols(B, S, n_heads, n_kv, hd)
+    return torch.zeros(B, S, cols, dtype=torch.float32, device=device)
+
+
 class _AttentionPacked(torch.autograd.Function):
     """Causal GQA attention on the packed projection output [B, S, (H + 2 KV) * hd]; the backward
     returns the gradient in the same packed layout, so nothing splits or concatenates q, k and v."""
@@ -743,7 +749,7 @@ class _AttentionPacked(torch.autograd.Function):
         B, S, C = qkv.shape
         do = dout.contiguous()
         dqkv = torch.empty_like(qkv)
-        dq32 = torch.zeros(B, S, n_heads * hd, dtype=torch.float32, device=qkv.device)
+        dq32 = _attention_scratch(B, S, n_heads, n_kv, hd, qkv.device)
         delta = torch.empty(B, n_heads, S, dtype=torch.float32, device=qkv.device)
         native.check(native.lib().tplr_attention_bwd(qkv.data_ptr(), out.data_ptr(), do.data_ptr(), lse.data_ptr(),
                                                      delta.data_ptr(), dq32.data_ptr(), dqkv.data_ptr(), B, S, n_heads, n_kv,
@@ -786,7 +792,7 @@ class _QKVRopeAttention(torch.autograd.Function):
         B, S, C = qkv.shape
         do = dout.contiguous()
         dqkv = torch.empty_like(qkv)
-        dq32 = torch.zeros(B, S, n_heads * hd, dtype=torch.float32, device=qkv.device)
+        dq32 = _attention_scratch(B, S, n_heads, n_kv, hd, qkv.device)
         delta = torch.empty(B, n_heads, S, dtype=torch.float32, device=qkv.device)
         native.check(native.lib().tplr_attention_bwd_unrope(
             qkv.data_ptr(), out.data_ptr(), do.data_ptr(), lse.data_ptr(), delta.data_ptr(), dq32.data_ptr(), dqkv.data_ptr(),
@@ -847,7 +853,7 @@ class _AttentionBlock(torch.autograd.Function):
                                             native.stream_ptr()), "gemm2_attn_dout")
         dwo = _weight_grad(mg_wo, dy2, out2, wo, ctx.needs_input_grad[2])
         dqkv = torch.empty_like(qkv)
-        dq32 = torch.zeros(B, S, N, dtype=torch.float32, device=qkv.device)
+        dq32 = _attention_scratch(B, S, n_heads, n_kv, hd, qkv.device)
         native.check(L.tplr_attention_bwd_unrope_delta(
             qkv.data_ptr(), out.data_ptr(), do.data_ptr(), lse.data_ptr(), delta.data_ptr(), dq32.data_ptr(), dqkv.data_ptr(),
             B, S, n_heads, n_kv, hd, qkv.stride(1), out.stride(1), hd ** -0.5, cos.data_ptr(), sin.data_ptr(), st,

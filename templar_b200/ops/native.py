@@ -86,6 +86,7 @@ def _declare(L: ctypes.CDLL) -> None:
         "tplr_gemm2_attn_dout": [vp, vp, vp, vp, vp, i, i, i, i, i, ll, ll, ll, ll, vp, vp],
         "tplr_attention_bwd_unrope_delta": [vp, vp, vp, vp, vp, vp, vp, i, i, i, i, i, ll, ll, f, vp, vp, vp, vp],
         "tplr_attention_bwd_unrope": [vp, vp, vp, vp, vp, vp, vp, i, i, i, i, i, ll, ll, f, vp, vp, vp, vp],
+        "tplr_attention_bwd_scratch_cols": [i, i, i, i, i],
         "tplr_attention_fwd": [vp, vp, vp, i, i, i, i, i, ll, ll, f, vp, vp],
         "tplr_attention_bwd": [vp, vp, vp, vp, vp, vp, vp, i, i, i, i, i, ll, ll, f, vp, vp],
         "tplr_gemm_bf16": [vp, vp, vp, i, i, i, ll, ll, ll, i, i, i, vp, i, vp],
