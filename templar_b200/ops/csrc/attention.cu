@@ -111,9 +111,11 @@ __device__ __forceinline__ uint32_t idesc_mn(int n, bool a_mn, bool b_mn) {
          ((uint32_t)(n >> 3) << 17) | ((uint32_t)(128 >> 4) << 24);
 }
 
-// Softmax passes over one row of S (128 fp32 columns in tensor memory, lane = query row).  DIAG = the block
-// on the diagonal (columns above the row are masked); the other blocks run the variant without the per-element
-// compare and select, which is a third of the instructions of the issue-bound softmax warps.
+// Softmax over one row of S (128 fp32 columns in tensor memory, lane = query row).  DIAG = the block on the diagonal
+// (columns above the row are masked); the other blocks run the variant without the per-element compare and select.
+// The row is read from tensor memory once: two passes of four loads, each with its own wait, made the softmax the longer
+// part of a step.  B 8, S 2048: neutral at
+// 16 heads of 128 (193 us), 125 -> 118 us at 12 heads of 64, where it lets the next S be computed ahead.
 // packed fp32 pairs (sm_100): one instruction for two lanes of fma / add, and the three-input max
 __device__ __forceinline__ unsigned long long pack_f32x2(uint32_t lo, uint32_t hi) {
   unsigned long long r;
@@ -139,47 +141,65 @@ __device__ __forceinline__ float max3(float a, float b, float c) {
   return d;
 }
 
+// One row of S (128 fp32 columns): four loads in flight and one wait.  The empty statements make every register an output
+// of something behind the wait, so that no use of it can be scheduled before.
+__device__ __forceinline__ void tmem_ld32_nowait(uint32_t taddr, uint32_t* r) {
+  asm volatile(
+      "tcgen05.ld.sync.aligned.32x32b.x32.b32 "
+      "{%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,"
+      "%16,%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31}, [%32];"
+      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
+        "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15]),
+        "=r"(r[16]), "=r"(r[17]), "=r"(r[18]), "=r"(r[19]), "=r"(r[20]), "=r"(r[21]), "=r"(r[22]), "=r"(r[23]),
+        "=r"(r[24]), "=r"(r[25]), "=r"(r[26]), "=r"(r[27]), "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31])
+      : "r"(taddr) : "memory");
+}
+__device__ __forceinline__ void behind_wait32(uint32_t* r) {
+  asm volatile("" : "+r"(r[0]), "+r"(r[1]), "+r"(r[2]), "+r"(r[3]), "+r"(r[4]), "+r"(r[5]), "+r"(r[6]), "+r"(r[7]),
+        "+r"(r[8]), "+r"(r[9]), "+r"(r[10]), "+r"(r[11]), "+r"(r[12]), "+r"(r[13]), "+r"(r[14]), "+r"(r[15]),
+        "+r"(r[16]), "+r"(r[17]), "+r"(r[18]), "+r"(r[19]), "+r"(r[20]), "+r"(r[21]), "+r"(r[22]), "+r"(r[23]),
+        "+r"(r[24]), "+r"(r[25]), "+r"(r[26]), "+r"(r[27]), "+r"(r[28]), "+r"(r[29]), "+r"(r[30]), "+r"(r[31]));
+}
+__device__ __forceinline__ void tmem_ld128(uint32_t taddr, uint32_t (&v)[128]) {
+#pragma unroll
+  for (int c = 0; c < 4; ++c) tmem_ld32_nowait(taddr + c * 32, v + c * 32);
+  asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+  for (int c = 0; c < 4; ++c) behind_wait32(v + c * 32);
+}
+
 template <bool DIAG>
-__device__ __forceinline__ float attn_row_max(uint32_t ts_lane, int r) {
-  float mx = -INFINITY;
-#pragma unroll 1
-  for (int c = 0; c < 4; ++c) {
-    uint32_t v[32];
-    tmem_ld32(ts_lane + c * 32, v);
+__device__ __forceinline__ float attn_row_max(uint32_t (&v)[128], int r) {
+  float mx = -INFINITY, mx2 = -INFINITY;
+#pragma unroll
+  for (int e = 0; e < 128; e += 4) {
     if (DIAG) {
 #pragma unroll
-      for (int e = 0; e < 32; ++e) mx = fmaxf(mx, (c * 32 + e > r) ? -INFINITY : __uint_as_float(v[e]));
-    } else {
-#pragma unroll
-      for (int e = 0; e < 16; ++e) mx = max3(mx, __uint_as_float(v[2 * e]), __uint_as_float(v[2 * e + 1]));
+      for (int k = 0; k < 4; ++k) if (e + k > r) v[e + k] = 0xff800000u;           // -inf: exp2 makes it zero
     }
+    mx = max3(mx, __uint_as_float(v[e]), __uint_as_float(v[e + 1]));
+    mx2 = max3(mx2, __uint_as_float(v[e + 2]), __uint_as_float(v[e + 3]));
   }
-  return mx;
+  return fmaxf(mx, mx2);
 }
-// P = exp2(S * scale - m) written as packed bf16 over the first 64 columns of S; returns the row sum of P.
-template <bool DIAG>
-__device__ __forceinline__ float attn_row_exp(uint32_t ts_lane, int r, float sl2, float m_used) {
+// P = exp2(S * scale - m) written as packed bf16 to 64 columns; returns the row sum of P.
+__device__ __forceinline__ float attn_row_exp(const uint32_t (&v)[128], uint32_t tp_lane, float sl2, float m_used) {
   const unsigned long long sl2x2 = pack_f32x2(__float_as_uint(sl2), __float_as_uint(sl2));
   const unsigned long long negm = pack_f32x2(__float_as_uint(-m_used), __float_as_uint(-m_used));
   unsigned long long sum = 0ull;                         // (0.f, 0.f)
-#pragma unroll 1
+#pragma unroll
   for (int c = 0; c < 4; ++c) {
-    uint32_t v[32], pk[16];
-    tmem_ld32(ts_lane + c * 32, v);
+    uint32_t pk[16];
 #pragma unroll
     for (int e = 0; e < 16; ++e) {
       float a0, a1;
-      unpack_f32x2(fma_f32x2(pack_f32x2(v[2 * e], v[2 * e + 1]), sl2x2, negm), a0, a1);
-      float p0 = exp2f(a0), p1 = exp2f(a1);
-      if (DIAG) {
-        if (c * 32 + 2 * e > r) p0 = 0.f;
-        if (c * 32 + 2 * e + 1 > r) p1 = 0.f;
-      }
+      unpack_f32x2(fma_f32x2(pack_f32x2(v[c * 32 + 2 * e], v[c * 32 + 2 * e + 1]), sl2x2, negm), a0, a1);
+      const float p0 = exp2f(a0), p1 = exp2f(a1);
       sum = add_f32x2(sum, pack_f32x2(__float_as_uint(p0), __float_as_uint(p1)));
       __nv_bfloat162 hh = __floats2bfloat162_rn(p0, p1);
       pk[e] = *reinterpret_cast<uint32_t*>(&hh);
     }
-    tmem_st16(ts_lane + c * 16, pk);
+    tmem_st16(tp_lane + c * 16, pk);
   }
   float s0, s1;
   unpack_f32x2(sum, s0, s1);
@@ -192,7 +212,7 @@ attn_fwd_kernel(const __grid_constant__ AttnFwdParams p) {
   constexpr int TILE_BYTES = tile_bytes<DH>();
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
-  __shared__ __align__(8) uint64_t bar_q, bar_k_full, bar_k_empty, bar_v_full, bar_v_empty, bar_s_full, bar_p_full, bar_o_full;
+  __shared__ __align__(8) uint64_t bar_q, bar_k_full, bar_k_empty, bar_v_full, bar_v_empty, bar_s_full, bar_s_read, bar_p_full, bar_o_full;
   __shared__ uint32_t s_tmem_base;
   __shared__ int s_abort;
 
@@ -213,7 +233,7 @@ attn_fwd_kernel(const __grid_constant__ AttnFwdParams p) {
     mbar_init(smem_u32(&bar_q), 1);
     mbar_init(smem_u32(&bar_k_full), 1); mbar_init(smem_u32(&bar_k_empty), 1);
     mbar_init(smem_u32(&bar_v_full), 1); mbar_init(smem_u32(&bar_v_empty), 1);
-    mbar_init(smem_u32(&bar_s_full), 1); mbar_init(smem_u32(&bar_p_full), 4);
+    mbar_init(smem_u32(&bar_s_full), 1); mbar_init(smem_u32(&bar_s_read), 4); mbar_init(smem_u32(&bar_p_full), 4);
     mbar_init(smem_u32(&bar_o_full), 1);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
@@ -226,7 +246,10 @@ attn_fwd_kernel(const __grid_constant__ AttnFwdParams p) {
   __syncthreads();
   tcgen05_fence_after();
   const uint32_t tmem_base = s_tmem_base;
-  const uint32_t tS = tmem_base, tO = tmem_base + 128;     // S / P columns 0..127, O columns 128..255
+  // S columns 0..127, O from column 128.  P lies over S at DH = 128; at 64 it has the 64 columns that O leaves, so that the
+  // next block's S is computed as soon as the softmax warps hold this one's in registers (AHEAD).
+  constexpr bool AHEAD = DH == 64;
+  const uint32_t tS = tmem_base, tO = tmem_base + 128, tP = AHEAD ? tmem_base + 192 : tmem_base;
   const uint32_t sQ = smem_u32(smem), sK = sQ + TILE_BYTES, sV = sK + TILE_BYTES;
 
   if (warp == 0) {
@@ -249,10 +272,8 @@ attn_fwd_kernel(const __grid_constant__ AttnFwdParams p) {
     if (lane == 0) {
       const uint32_t id_qk = idesc_mn(128, false, false), id_pv = idesc_mn(DH, false, true);
       const DescBase bQ = desc_base(sQ, 16, 1024), bK = desc_base(sK, 16, 1024), bV = desc_base(sV, 128 * 128, 1024);
-      bool ok = mbar_wait(smem_u32(&bar_q), 0, abort_flag);
-      for (int j = 0; j < nb && ok; ++j) {
-        const uint32_t ph = j & 1;
-        if (!(ok = mbar_wait(smem_u32(&bar_k_full), ph, abort_flag))) break;
+      auto issue_s = [&](int j) -> bool {                  // S(j) = Q K(j)^T
+        if (!mbar_wait(smem_u32(&bar_k_full), (uint32_t)(j & 1), abort_flag)) return false;
         tcgen05_fence_after();
 #pragma unroll
         for (int kk = 0; kk < DH / 16; ++kk) {
@@ -261,12 +282,24 @@ attn_fwd_kernel(const __grid_constant__ AttnFwdParams p) {
         }
         umma_commit(smem_u32(&bar_s_full));
         umma_commit(smem_u32(&bar_k_empty));
+        return true;
+      };
+      bool ok = mbar_wait(smem_u32(&bar_q), 0, abort_flag);
+      if (AHEAD && ok) ok = issue_s(0);
+      for (int j = 0; j < nb && ok; ++j) {
+        const uint32_t ph = j & 1;
+        if (!AHEAD) {
+          if (!(ok = issue_s(j))) break;
+        } else if (j + 1 < nb) {
+          if (!(ok = mbar_wait(smem_u32(&bar_s_read), ph, abort_flag))) break;
+          if (!(ok = issue_s(j + 1))) break;
+        }
         if (!(ok = mbar_wait(smem_u32(&bar_p_full), ph, abort_flag))) break;
         if (!(ok = mbar_wait(smem_u32(&bar_v_full), ph, abort_flag))) break;
         tcgen05_fence_after();
 #pragma unroll
         for (int kk = 0; kk < BKV / 16; ++kk)
-          umma_ts_bf16_b(tO, tS + 8 * kk, bV, (uint32_t)kk * 128u, id_pv, (j > 0 || kk > 0) ? 1u : 0u);
+          umma_ts_bf16_b(tO, tP + 8 * kk, bV, (uint32_t)kk * 128u, id_pv, (j > 0 || kk > 0) ? 1u : 0u);
         umma_commit(smem_u32(&bar_v_empty));
         if (j == nb - 1) umma_commit(smem_u32(&bar_o_full));
       }
@@ -283,15 +316,28 @@ attn_fwd_kernel(const __grid_constant__ AttnFwdParams p) {
       if (!ok) break;
       tcgen05_fence_after();
       const bool diag = j == qi;
-      // pass 1: row maximum of the scores
-      const float mx = diag ? attn_row_max<true>(tS + lane_off, r) : attn_row_max<false>(tS + lane_off, r);
+      // the row is loaded once and stays in registers: maximum, then exponentials
+      uint32_t sv[128];
+      tmem_ld128(tS + lane_off, sv);
+      if (AHEAD) {
+        tcgen05_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(smem_u32(&bar_s_read));
+      }
+      const float mx = diag ? attn_row_max<true>(sv, r) : attn_row_max<false>(sv, r);
+      if (AHEAD && j > 0) {                // O and the P columns: the product of block j-1 has finished with them
+        ok = mbar_wait(smem_u32(&bar_v_empty), (uint32_t)((j - 1) & 1), abort_flag);
+        ok = __all_sync(0xffffffffu, ok);
+        if (!ok) break;
+        tcgen05_fence_after();
+      }
       const float m_new = fmaxf(m_used, mx * p.scale_log2);
       const bool need = m_new > m_used + RESCALE_THRESHOLD;       // true for the first block (m_used = -inf)
       if (__any_sync(0xffffffffu, need)) {
         const float alpha = need ? exp2f(m_used - m_new) : 1.f;   // 0 for the first block
         if (need) { m_used = m_new; l *= alpha; }
         if (j > 0) {
-          // S of block j is complete, so every earlier MMA, PV of block j-1 included, has finished with O
+          // PV of block j-1 has finished with O: waited for above, or (not AHEAD) S of block j was issued behind it
 #pragma unroll 1
           for (int c = 0; c < DH / 32; ++c) {
             uint32_t v[32];
@@ -302,9 +348,7 @@ attn_fwd_kernel(const __grid_constant__ AttnFwdParams p) {
           }
         }
       }
-      // pass 2: P as packed bf16 over the first 64 columns of S
-      l += diag ? attn_row_exp<true>(tS + lane_off, r, p.scale_log2, m_used)
-                : attn_row_exp<false>(tS + lane_off, r, p.scale_log2, m_used);
+      l += attn_row_exp(sv, tP + lane_off, p.scale_log2, m_used);
       tmem_wait_st();
       tcgen05_fence_before();
       __syncwarp();
