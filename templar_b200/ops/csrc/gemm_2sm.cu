@@ -250,6 +250,36 @@ __device__ __forceinline__ void tma_reduce_add_2d(const CUtensorMap* map, uint32
                ::"l"(map), "r"(src), "r"(x), "r"(y) : "memory");
 }
 
+// Rotary angles of one output row for a whole tile (EPI 4): the tile's heads share them, so a lane loads the head's DH / 2
+// cosines and sines once into registers.  Loaded again for every 32 columns they cost 32 cache lines per instruction (each
+// lane has a row of its own), which made the epilogue longer than a short main loop.  16384 x 768 -> 2304, heads of 64:
+// 81 us then, 59 us here.
+template <int DH>
+struct RopeRow {
+  float c[DH / 2], s[DH / 2];
+  __device__ __forceinline__ void load(const Gemm2Params& p, int row) {
+    const long long tb = (long long)(row % p.rope_s) * (DH / 2);
+    const float4* cp = reinterpret_cast<const float4*>(p.rope_cos + tb);
+    const float4* sp = reinterpret_cast<const float4*>(p.rope_sin + tb);
+#pragma unroll
+    for (int q = 0; q < DH / 8; ++q) {
+      const float4 a = cp[q], b = sp[q];
+      c[4 * q] = a.x; c[4 * q + 1] = a.y; c[4 * q + 2] = a.z; c[4 * q + 3] = a.w;
+      s[4 * q] = b.x; s[4 * q + 1] = b.y; s[4 * q + 2] = b.z; s[4 * q + 3] = b.w;
+    }
+  }
+  // 32 columns from column OFF of a head on
+  template <int OFF>
+  __device__ __forceinline__ void turn(uint32_t* r) const {
+#pragma unroll
+    for (int e = 0; e < 16; ++e) {
+      const float a = __uint_as_float(r[2 * e]), b = __uint_as_float(r[2 * e + 1]);
+      r[2 * e] = __float_as_uint(a * c[OFF / 2 + e] - b * s[OFF / 2 + e]);
+      r[2 * e + 1] = __float_as_uint(a * s[OFF / 2 + e] + b * c[OFF / 2 + e]);
+    }
+  }
+};
+
 // Epilogue through shared memory and TMA: a warp stages 32 rows x 128 bytes (64 bf16 or 32 fp32
 // columns) in 128-byte-swizzled order, then one lane stores (EPI 0, 2) or reduce-adds (EPI 1) the
 // box.  Two staging buffers per warp; `n_boxes` counts the boxes this warp has issued so far.
@@ -364,6 +394,44 @@ __device__ __forceinline__ void box_store(const CUtensorMap* map, uint32_t buf, 
     bulk_commit();
   }
   ++n_boxes;
+}
+
+// The plain bf16 epilogue with the rotation, for heads of DH columns (tiles and heads start at multiples of DH).
+template <int DH>
+__device__ __forceinline__ void epilogue_rope(const Gemm2Params& p, uint32_t tmem_acc, int quad, int lane, int m0, int n0,
+                                              uint32_t stage_base, uint32_t& n_boxes) {
+  const int row0 = m0 + quad * 32;
+  if (row0 >= p.M) return;                           // warp-uniform
+  const uint32_t lane_sel = (uint32_t)(quad * 32) << 16;
+  RopeRow<DH> rr;
+  if (n0 < p.rope_cols) rr.load(p, min(row0 + lane, p.M - 1));
+#pragma unroll 1
+  for (int h = 0; h < TILE_N / DH; ++h) {
+    if (n0 + h * DH >= p.N) break;
+    const bool rot = n0 + h * DH < p.rope_cols;      // whole heads (rope_cols is a multiple of DH)
+#pragma unroll
+    for (int q = 0; q < DH / 64; ++q) {
+      const int col = h * DH + q * 64;
+      if (n0 + col >= p.N) break;
+      const uint32_t buf = box_begin(lane, stage_base, n_boxes);
+#pragma unroll
+      for (int hh = 0; hh < 2; ++hh) {
+        uint32_t r[32];
+        float v[32];
+        tmem_ld32(tmem_acc + col + hh * 32 + lane_sel, r);
+        if (rot) {
+          if (q == 0 && hh == 0) rr.template turn<0>(r);
+          if (q == 0 && hh == 1) rr.template turn<32>(r);
+          if (q == 1 && hh == 0) rr.template turn<DH / 2>(r);
+          if (q == 1 && hh == 1) rr.template turn<DH - 32>(r);
+        }
+#pragma unroll
+        for (int e = 0; e < 32; ++e) v[e] = __uint_as_float(r[e]);
+        box_half(buf, lane, hh, v);
+      }
+      box_store(&p.tmC, buf, lane, n_boxes, n0 + col, row0);
+    }
+  }
 }
 
 // Epilogue of the fused [w1; w3] projection (EPI 3): accumulator columns 0..127 of a row are the gate values g of features
@@ -722,6 +790,10 @@ gemm2_kernel(const __grid_constant__ Gemm2Params p) {
         if (EPI == 3)      epilogue_swiglu(p, tmem_acc, quad, lane, m0, tn, sEpi + (uint32_t)quad * 8192u, n_boxes);
         else if (EPI == 5) epilogue_swiglu_bwd(p, tmem_acc, quad, lane, m0, n0, sEpi + (uint32_t)quad * 8192u, n_boxes);
         else if (EPI == 6) epilogue_attn_dout(p, tmem_acc, quad, lane, m0, n0, sEpi + (uint32_t)quad * 8192u, n_boxes);
+        else if (EPI == 4 && p.rope_dh == 128 && p.rope_cols % 128 == 0)
+          epilogue_rope<128>(p, tmem_acc, quad, lane, m0, n0, sEpi + (uint32_t)quad * 8192u, n_boxes);
+        else if (EPI == 4 && p.rope_dh == 64 && p.rope_cols % 64 == 0)
+          epilogue_rope<64>(p, tmem_acc, quad, lane, m0, n0, sEpi + (uint32_t)quad * 8192u, n_boxes);
         else if (p.c_tma)  epilogue_tma<EPI>(p, tmem_acc, quad, lane, m0, n0, sEpi + (uint32_t)quad * 8192u, n_boxes);
         else               epilogue_direct<EPI>(p, tmem_acc, quad, lane, m0, n0);
         tcgen05_fence_before();
