@@ -492,6 +492,14 @@ def feed_forward(x, w13, w2, main_grad13=None, main_grad2=None):
             and Fd % 128 == 0 and x2.is_contiguous() and w13.stride(1) == 1 and w2.stride(1) == 1 and w13.stride(0) % 8 == 0
             and w2.stride(0) % 8 == 0 and x2.shape[1] % 8 == 0 and w2.shape[0] % 8 == 0
             and all(t.data_ptr() % 16 == 0 for t in (x2, w13, w2))):
+        if not torch.is_grad_enabled():          # nothing will ask for the packed projection: it is not stored
+            h = torch.empty(x2.shape[0], Fd, dtype=x.dtype, device=x.device)
+            native.check(native.lib().tplr_gemm2_swiglu(x2.data_ptr(), w13.data_ptr(), None, h.data_ptr(), x2.shape[0], Fd,
+                                                        x2.shape[1], x2.stride(0), w13.stride(0), 2 * Fd, Fd,
+                                                        status_word(x.device).data_ptr(), native.stream_ptr()), "gemm2_swiglu")
+            y = torch.empty(*x.shape[:-1], w2.shape[0], dtype=x.dtype, device=x.device)
+            gemm(h, w2, out=y.view(-1, w2.shape[0]))
+            return y
         return _FeedForward.apply(x, w13, w2, main_grad13, main_grad2)
     return _Linear.apply(linear_swiglu(x, w13, main_grad13), w2, main_grad2)
 

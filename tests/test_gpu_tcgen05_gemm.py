@@ -225,3 +225,16 @@ def test_feed_forward_with_both_swiglu_epilogues_matches_fp32_reference(T, D, F,
 def test_accumulating_gemm_with_k_splits(M, N, K, backend):
     """Weight-gradient products with few tiles (several work units add into one tile), ragged tiles and a ragged last split."""
     _check(M, N, K, True, True, "acc")
+
+
+@pytest.mark.parametrize("T,D,F", [(300, 192, 384), (1000, 64, 128)])
+def test_feed_forward_without_grad_gives_the_same_output(T, D, F, backend):
+    """Without a backward pass the packed projection is not stored; the activation and the output are the same bits."""
+    if backend != "tcgen05_2sm":
+        pytest.skip("the fused epilogue is a mode of the CTA-pair kernel")
+    torch.manual_seed(T)
+    x, w13, w2 = (torch.randn(*s, device=DEV).to(torch.bfloat16).requires_grad_() for s in ((T, D), (2 * F, D), (D, F)))
+    want = OF.feed_forward(x, w13, w2).detach()
+    with torch.no_grad():
+        assert torch.equal(OF.feed_forward(x, w13, w2), want)
+    assert int(OF.status_word(DEV).item()) == 0
