@@ -34,6 +34,8 @@ constexpr int B_STAGE = CTA_N * BK * 2;            // 16 KB
 constexpr int STAGE_BYTES = A_STAGE + B_STAGE;     // 32 KB
 constexpr int EPI_STAGE_BYTES = 4 * 2 * 4096;      // 4 epilogue warps x 2 buffers x (32 rows x 128 B)
 constexpr int SMEM_BYTES = STAGES * STAGE_BYTES + EPI_STAGE_BYTES + 1024;
+constexpr int EPI5_STAGES = STAGES - 1;            // the SwiGLU backward has a second pair of staging buffers per warp instead
+static_assert(4 * 8192 <= STAGE_BYTES, "the freed stage holds four warps' second pair");
 constexpr int NUM_THREADS = 192;
 constexpr int MAX_RANKS = 8;
 constexpr int CHUNK_ROWS = 128;                    // gather / scatter flag granularity (rows)
@@ -59,8 +61,9 @@ struct Gemm2Params {
                                      // (odd CTA), so every accumulator row holds g and u of the same 128 features; the epilogue
                                      // stores both into C [M, 2 * swiglu_f] and silu(g) * u into tmCr[0]'s tensor [M, swiglu_f]
   // backward of the SwiGLU in the epilogue of the down projection's data gradient (EPI 5): the accumulator tile is
-  // dh[M, swiglu_f] = dY W2; gu is the forward's packed [M, 2 * swiglu_f] projection (gate | up), leading dimension ld_gu;
+  // dh[M, swiglu_f] = dY W2; tmGU is the forward's packed [M, 2 * swiglu_f] projection (gate | up);
   // the epilogue stores dg | du (bf16) through tmC, a map over the [M, 2 * swiglu_f] gradient of that projection
+  CUtensorMap tmGU;                  // EPI 5: the packed projection, box 64 x 32, 128-byte swizzle
   const __nv_bfloat16* gu;
   long long ld_gu;
   // data gradient of the attention output projection (EPI 6): C = dO [M, heads * attn_dh] stored as bf16, and for every row
@@ -487,76 +490,82 @@ __device__ __forceinline__ void epilogue_swiglu(const Gemm2Params& p, uint32_t t
 //   s = sigmoid(g),  du = dh * g * s,  dg = dh * u * s * (1 + g * (1 - s)),
 // and dg / du are stored (bf16) at columns f and swiglu_f + f of the packed gradient.  This replaces a pass that writes
 // dh, reads it back with g and u and writes dg | du (the backward of the reference's F.silu(w1(x)) * w3(x)).
-// Both staging buffers of the warp are in use at once (one box of dg, one of du), so a step waits until the two stores
-// of the previous step have read them.
-__device__ __forceinline__ void epilogue_swiglu_bwd(const Gemm2Params& p, uint32_t tmem_acc, int quad, int lane, int m0, int n0,
-                                                    uint32_t stage_base, uint32_t& n_boxes) {
+// g and u come as TMA boxes of 32 rows x 64 columns into the staging buffers that dg and du leave from, in place: a lane
+// reading its own row from global memory touches 32 lines per instruction, which made the epilogue longer than the main loop
+// (2048 x 768 -> 3072: 67 -> 41 us in one run of all its products; 16384 x 2048 -> 8192: 651 -> 542 us).  Two pairs of buffers per warp (the operand ring has one stage less for them): the next
+// pair is in flight while this one is computed, the first of a tile while its main loop runs.
+struct GuLoads {
+  uint32_t bar;                      // two mbarriers of this warp
+  uint32_t base;                     // two pairs of 4 KB buffers
+  uint32_t issued, used;             // box pairs asked for and consumed so far
+};
+__device__ __forceinline__ void gu_issue(const Gemm2Params& p, GuLoads& L, int lane, int f0, int row0) {
+  if (lane == 0) {
+    const uint32_t s = L.issued & 1u, bar = L.bar + 8u * s, buf = L.base + s * 8192u;
+    asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");      // the stores that leave from this pair have read it
+    mbar_expect_tx(bar, 8192);
+    tma_load_2d(buf, &p.tmGU, bar, f0, row0);
+    tma_load_2d(buf + 4096u, &p.tmGU, bar, p.swiglu_f + f0, row0);
+  }
+  ++L.issued;
+}
+__device__ __forceinline__ bool epilogue_swiglu_bwd(const Gemm2Params& p, uint32_t tmem_acc, int quad, int lane, int m0, int n0,
+                                                    GuLoads& L, volatile int* abort_flag) {
   const int row0 = m0 + quad * 32;
-  if (row0 >= p.M) return;                           // warp-uniform
+  if (row0 >= p.M || n0 >= p.swiglu_f) return true;  // warp-uniform; nothing was asked for
   const uint32_t lane_sel = (uint32_t)(quad * 32) << 16;
-  const int row = min(row0 + lane, p.M - 1);
-  const __nv_bfloat16* grow = p.gu + (long long)row * p.ld_gu;
-  const uint32_t buf_g = stage_base, buf_u = stage_base + 4096u;
-  // g and u of this lane's row for one step of 32 features: 64 bytes each (row base and feature offset are multiples
-  // of 8 elements).  The loads of step i + 1 are issued before step i is computed: a step's loads come from L2 or
-  // DRAM, and eight such latencies in a row would make the epilogue as long as the tile's main loop.
-  uint4 gq[4], uq[4], gn[4], un[4];
-  auto fetch = [&](int step, uint4* g4, uint4* u4) {
-    const int f = n0 + step * 32;
-    if (f < p.swiglu_f) {
-      const uint4* gp = reinterpret_cast<const uint4*>(grow + f);
-      const uint4* up = reinterpret_cast<const uint4*>(grow + p.swiglu_f + f);
-#pragma unroll
-      for (int q = 0; q < 4; ++q) { g4[q] = gp[q]; u4[q] = up[q]; }
-    }
-  };
-  fetch(0, gq, uq);
-#pragma unroll
-  for (int step = 0; step < TILE_N / 32; ++step) {
-    const int c = step >> 1, hh = step & 1;
+  const uint32_t sw = (uint32_t)(lane & 7);
+#pragma unroll 1
+  for (int c = 0; c < TILE_N / 64; ++c) {
     const int f0 = n0 + c * 64;
     if (f0 >= p.swiglu_f) break;                     // warp-uniform (swiglu_f is a multiple of 64)
-    if (step + 1 < TILE_N / 32) fetch(step + 1, gn, un);
-    if (hh == 0 && n_boxes > 0) {                    // both buffers free: the previous step's stores have read them
-      if (lane == 0) asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
-      __syncwarp();
-    }
-    uint32_t r[32];
-    tmem_ld32(tmem_acc + c * 64 + hh * 32 + lane_sel, r);
-    float dg[32], du[32];
+    if (c + 1 < TILE_N / 64 && f0 + 64 < p.swiglu_f) gu_issue(p, L, lane, f0 + 64, row0);
+    const uint32_t s = L.used & 1u;
+    const bool ok = mbar_wait(L.bar + 8u * s, (L.used >> 1) & 1u, abort_flag);
+    if (!__all_sync(0xffffffffu, ok)) return false;
+    ++L.used;
+    const uint32_t grow = L.base + s * 8192u + (uint32_t)lane * 128u, urow = grow + 4096u;
 #pragma unroll
-    for (int q = 0; q < 4; ++q) {
-      const uint32_t gw[4] = {gq[q].x, gq[q].y, gq[q].z, gq[q].w}, uw[4] = {uq[q].x, uq[q].y, uq[q].z, uq[q].w};
+    for (int hh = 0; hh < 2; ++hh) {
+      uint32_t r[32];
+      tmem_ld32(tmem_acc + c * 64 + hh * 32 + lane_sel, r);
 #pragma unroll
-      for (int e = 0; e < 4; ++e) {
-        const float2 g2 = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&gw[e]));
-        const float2 u2 = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&uw[e]));
-        const float gg[2] = {g2.x, g2.y}, uu[2] = {u2.x, u2.y};
+      for (int q = 0; q < 4; ++q) {
+        const uint32_t off = ((uint32_t)(hh * 4 + q) ^ sw) << 4;
+        uint32_t gw[4], uw[4];
+        asm volatile("ld.shared.v4.b32 {%0, %1, %2, %3}, [%4];" : "=r"(gw[0]), "=r"(gw[1]), "=r"(gw[2]), "=r"(gw[3]) : "r"(grow + off) : "memory");
+        asm volatile("ld.shared.v4.b32 {%0, %1, %2, %3}, [%4];" : "=r"(uw[0]), "=r"(uw[1]), "=r"(uw[2]), "=r"(uw[3]) : "r"(urow + off) : "memory");
 #pragma unroll
-        for (int k = 0; k < 2; ++k) {
-          const float dh = __uint_as_float(r[8 * q + 2 * e + k]);
-          const float sg = __fdividef(1.f, 1.f + __expf(-gg[k]));
-          const float silu = gg[k] * sg;
-          du[8 * q + 2 * e + k] = dh * silu;
-          dg[8 * q + 2 * e + k] = dh * uu[k] * (sg + silu * (1.f - sg));
+        for (int e = 0; e < 4; ++e) {
+          const float2 g2 = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&gw[e]));
+          const float2 u2 = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&uw[e]));
+          const float gg[2] = {g2.x, g2.y}, uu[2] = {u2.x, u2.y};
+          float dg[2], du[2];
+#pragma unroll
+          for (int k = 0; k < 2; ++k) {
+            const float dh = __uint_as_float(r[8 * q + 2 * e + k]);
+            const float sg = __fdividef(1.f, 1.f + __expf(-gg[k]));
+            const float silu = gg[k] * sg;
+            du[k] = dh * silu;
+            dg[k] = dh * uu[k] * (sg + silu * (1.f - sg));
+          }
+          const __nv_bfloat162 hg = __floats2bfloat162_rn(dg[0], dg[1]), hu = __floats2bfloat162_rn(du[0], du[1]);
+          gw[e] = *reinterpret_cast<const uint32_t*>(&hg);
+          uw[e] = *reinterpret_cast<const uint32_t*>(&hu);
         }
+        asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(grow + off), "r"(gw[0]), "r"(gw[1]), "r"(gw[2]), "r"(gw[3]) : "memory");
+        asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(urow + off), "r"(uw[0]), "r"(uw[1]), "r"(uw[2]), "r"(uw[3]) : "memory");
       }
     }
-    box_half(buf_g, lane, hh, dg);
-    box_half(buf_u, lane, hh, du);
-    if (hh == 1) {
-      asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-      __syncwarp();
-      if (lane == 0) {
-        tma_store_2d(&p.tmC, buf_g, f0, row0);
-        tma_store_2d(&p.tmC, buf_u, p.swiglu_f + f0, row0);
-        bulk_commit();
-      }
-      n_boxes += 2;
+    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+    __syncwarp();
+    if (lane == 0) {
+      tma_store_2d(&p.tmC, L.base + s * 8192u, f0, row0);
+      tma_store_2d(&p.tmC, L.base + s * 8192u + 4096u, p.swiglu_f + f0, row0);
+      bulk_commit();
     }
-#pragma unroll
-    for (int q = 0; q < 4; ++q) { gq[q] = gn[q]; uq[q] = un[q]; }
   }
+  return true;
 }
 
 // Epilogue of the attention output projection's data gradient (EPI 6): the accumulator row is dO for two
@@ -626,11 +635,13 @@ __device__ __forceinline__ void epilogue_attn_dout(const Gemm2Params& p, uint32_
 template <bool A_MN, bool B_MN, int EPI>
 __global__ void __launch_bounds__(NUM_THREADS, 1)
 gemm2_kernel(const __grid_constant__ Gemm2Params p) {
+  constexpr int STAGES = EPI == 5 ? EPI5_STAGES : ::STAGES;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
   __shared__ __align__(8) uint64_t bar_full[STAGES], bar_empty[STAGES], bar_tfull[2], bar_tempty[2];
   __shared__ uint32_t s_tmem_base;
   __shared__ int s_abort;
+  __shared__ __align__(8) uint64_t bar_gu[EPI == 5 ? 8 : 1];      // EPI 5: two per epilogue warp
   __shared__ uint32_t s_ready[32];   // gather: bit c set once chunk c was seen ready (1024 chunks)
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -650,6 +661,8 @@ gemm2_kernel(const __grid_constant__ Gemm2Params p) {
       mbar_init(smem_u32(&bar_empty[s]), 1);
     }
     for (int s = 0; s < 2; ++s) { mbar_init(smem_u32(&bar_tfull[s]), 1); mbar_init(smem_u32(&bar_tempty[s]), 8); }
+    if (EPI == 5)
+      for (int s = 0; s < 8; ++s) mbar_init(smem_u32(&bar_gu[s]), 1);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
   }
@@ -774,6 +787,8 @@ gemm2_kernel(const __grid_constant__ Gemm2Params p) {
       // ----------------------------- epilogue (warps 2..5 of both CTAs) --------------
       const int quad = warp & 3;
       uint32_t tile_i = 0, n_boxes = 0;
+      GuLoads gl = {};
+      if (EPI == 5) gl = {smem_u32(&bar_gu[EPI == 5 ? 2 * quad : 0]), sEpi + (uint32_t)quad * 16384u, 0u, 0u};
       bool ok = true;
       Work w;
       work_init(p, w, pair);
@@ -782,13 +797,14 @@ gemm2_kernel(const __grid_constant__ Gemm2Params p) {
         tile_coords(p, w.tile, tiles_m, tiles_n, tm, tn);
         const int m0 = tm * TILE_M + (int)cr * CTA_M, n0 = tn * TILE_N;
         const uint32_t acc = tile_i & 1, acc_ph = (tile_i >> 1) & 1;
+        if (EPI == 5 && m0 + quad * 32 < p.M && n0 < p.swiglu_f) gu_issue(p, gl, lane, n0, m0 + quad * 32);   // while the main loop runs
         ok = mbar_wait(smem_u32(&bar_tfull[acc]), acc_ph, abort_flag);
         ok = __all_sync(0xffffffffu, ok);
         if (!ok) break;
         tcgen05_fence_after();
         const uint32_t tmem_acc = tmem_base + acc * TILE_N;
         if (EPI == 3)      epilogue_swiglu(p, tmem_acc, quad, lane, m0, tn, sEpi + (uint32_t)quad * 8192u, n_boxes);
-        else if (EPI == 5) epilogue_swiglu_bwd(p, tmem_acc, quad, lane, m0, n0, sEpi + (uint32_t)quad * 8192u, n_boxes);
+        else if (EPI == 5) { if (!(ok = epilogue_swiglu_bwd(p, tmem_acc, quad, lane, m0, n0, gl, abort_flag))) break; }
         else if (EPI == 6) epilogue_attn_dout(p, tmem_acc, quad, lane, m0, n0, sEpi + (uint32_t)quad * 8192u, n_boxes);
         else if (EPI == 4 && p.rope_dh == 128 && p.rope_cols % 128 == 0)
           epilogue_rope<128>(p, tmem_acc, quad, lane, m0, n0, sEpi + (uint32_t)quad * 8192u, n_boxes);
@@ -800,6 +816,8 @@ gemm2_kernel(const __grid_constant__ Gemm2Params p) {
         __syncwarp();
         if (lane == 0) mbar_arrive_cluster(mapa(smem_u32(&bar_tempty[acc]), 0));
       }
+      // a role that gave up leaves no load in flight into the shared memory that it returns
+      for (; EPI == 5 && gl.used < gl.issued; ++gl.used) mbar_wait(gl.bar + 8u * (gl.used & 1u), (gl.used >> 1) & 1u, abort_flag);
       if (lane == 0) {
         bulk_wait0();                // staging buffers are read out and the stores / reductions are performed
         if (p.rs_on) __threadfence_system();
@@ -1033,8 +1051,8 @@ TPLR_API int tplr_gemm2_swiglu_bwd(const void* dY, const void* W2, const void* G
   if (int r = fill_common(p, dY, W2, dGU, M, F, K, lddy, ldw2, lddgu, 0, 1, 0, status)) return r;
   if (!p.c_tma) return -111;
   if (!make_map(&p.tmC, dGU, 2LL * F, M, lddgu, 64, 32, CU_TENSOR_MAP_SWIZZLE_128B, false)) return -110;
+  if (!make_map(&p.tmGU, GU, 2LL * F, M, ldgu, 64, 32, CU_TENSOR_MAP_SWIZZLE_128B, false)) return -110;
   p.swiglu_f = F;
-  p.gu = (const __nv_bfloat16*)GU; p.ld_gu = ldgu;
   return dispatch2(p, 0, 1, 5, 0, 0, (cudaStream_t)stream);
 }
 
