@@ -24,9 +24,9 @@ NS_CONSTS = [(4.0848, -6.8946, 2.9270), (3.9505, -6.3029, 2.6377), (3.7418, -5.5
              (2.8769, -3.1427, 1.2046), (2.8366, -3.0525, 1.2012)]
 
 
-def _one_triangle_ok(X: torch.Tensor) -> bool:
-    return (X.is_cuda and X.dtype == torch.bfloat16 and OF.gemm_backend() == "tcgen05_2sm" and X.shape[0] >= 512
-            and X.shape[0] % 8 == 0 and X.shape[1] % 8 == 0 and SYMMETRIC_PRODUCTS)
+def _one_triangle_ok(G: torch.Tensor) -> bool:
+    return (G.is_cuda and OF.gemm_backend() == "tcgen05_2sm" and min(G.shape) >= 512 and G.shape[0] % 8 == 0
+            and G.shape[1] % 8 == 0 and SYMMETRIC_PRODUCTS)
 
 
 SYMMETRIC_PRODUCTS = True        # lines 1 and 2 as one-triangle products (module switch, for the comparison benchmark)
@@ -34,13 +34,17 @@ SYMMETRIC_PRODUCTS = True        # lines 1 and 2 as one-triangle products (modul
 
 class _SymmetricChain:
     """The five iterations for one matrix shape on static buffers, captured once in a CUDA graph and replayed:
-    25 launches (per iteration: one-triangle X X^T, mirror, one-triangle A A, mirror with the line's scalars and the
-    identity term, full product) with no host work between them.
+    24 launches (per iteration: one-triangle X X^T, mirror, one-triangle A A, mirror with the line's scalars and the
+    identity term, full product) with no host work between them.  Before the graph ``tplr_ns_prepare`` writes the
+    scaled operand into the chain's buffer; after it the last product writes the caller's new tensor, so nothing is
+    copied in or out.
 
     Lines 1 and 2 compute only the 256 x 256 tiles on or above the diagonal of their symmetric results
     (``tplr_gemm2_syrk``: half the tensor-core work) and ``tplr_sym_axpby`` mirrors the triangle while it applies
-    the line's scalars.  Line 3, ``a X + B X``, is one product ``(B + a I) X``: the mirror kernel of line 2 adds
-    ``a`` on the diagonal, so no element-wise pass over X remains."""
+    the line's scalars.  Where those tiles are too few for the chip, K is split and the triangle accumulates in fp32
+    (``tplr_gemm2_syrk_acc``; ``tplr_sym_axpby_acc`` leaves it zeroed for the next product).  Line 3, ``a X + B X``, is
+    one product ``(B + a I) X``: the mirror kernel of line 2 adds ``a`` on the diagonal, so no element-wise pass over X
+    remains."""
 
     def __init__(self, M: int, K: int, device):
         from ..ops import native
@@ -49,6 +53,9 @@ class _SymmetricChain:
         z = lambda *shape: torch.empty(*shape, dtype=torch.bfloat16, device=device)       # noqa: E731
         self.x = [z(M, K), z(M, K)]
         self.U, self.A, self.B = z(M, M), z(M, M), z(M, M)
+        self.split = {k: native.lib().tplr_gemm2_syrk_splits(M, k) > 1 for k in (M, K)}
+        self.acc = torch.zeros(M, M, dtype=torch.float32, device=device) if any(self.split.values()) else None
+        self.scratch = torch.empty(native.lib().tplr_sumsq_blocks(), dtype=torch.float32, device=device)
         self.status = OF.status_word(device)
         self.graph = None
         self._run()                                    # warm-up outside the capture (first-use set-up of the kernels)
@@ -62,45 +69,63 @@ class _SymmetricChain:
         native, L, M, K = self.native, self.native.lib(), self.M, self.K
         st = self.status.data_ptr()
         src, dst = self.x
-        for a, b, c in NS_CONSTS:
-            s = native.stream_ptr()
-            native.check(L.tplr_gemm2_syrk(src.data_ptr(), self.U.data_ptr(), M, K, K, M, st, s), "syrk")
-            native.check(L.tplr_sym_axpby(self.U.data_ptr(), M, M, 1.0, None, 0, 0.0, 0.0, self.A.data_ptr(), M, s), "sym_axpby")
-            native.check(L.tplr_gemm2_syrk(self.A.data_ptr(), self.U.data_ptr(), M, M, M, M, st, s), "syrk")   # A A = A A^T
-            native.check(L.tplr_sym_axpby(self.U.data_ptr(), M, M, c, self.A.data_ptr(), M, b, a, self.B.data_ptr(), M, s),
-                         "sym_axpby")
-            OF.gemm(self.B, src, b_mn=True, out=dst)                                      # (B + a I) X
-            src, dst = dst, src
-        self.result = src
 
-    def __call__(self, X: torch.Tensor) -> torch.Tensor:
-        self.x[0].copy_(X)
+        def product(x, k, alpha, aux, beta, diag, out):
+            """out = alpha x x^T + beta aux + diag I for x [M, k]."""
+            s = native.stream_ptr()
+            aux = None if aux is None else aux.data_ptr()
+            if self.split[k]:
+                native.check(L.tplr_gemm2_syrk_acc(x.data_ptr(), self.acc.data_ptr(), M, k, k, M, st, s), "syrk_acc")
+                native.check(L.tplr_sym_axpby_acc(self.acc.data_ptr(), M, alpha, aux, beta, diag, out.data_ptr(), s), "sym_axpby_acc")
+            else:
+                native.check(L.tplr_gemm2_syrk(x.data_ptr(), self.U.data_ptr(), M, k, k, M, st, s), "syrk")
+                native.check(L.tplr_sym_axpby(self.U.data_ptr(), M, M, alpha, aux, M, beta, diag, out.data_ptr(), M, s), "sym_axpby")
+
+        for n, (a, b, c) in enumerate(NS_CONSTS):
+            product(src, K, 1.0, None, 0.0, 0.0, self.A)
+            product(self.A, M, c, self.A, b, a, self.B)                                   # A A = A A^T
+            if n + 1 < len(NS_CONSTS):                                                    # the last one: __call__
+                OF.gemm(self.B, src, b_mn=True, out=dst)                                  # (B + a I) X
+                src, dst = dst, src
+        self.last = src
+
+    def __call__(self, G: torch.Tensor, epsilon: float) -> torch.Tensor:
+        """G: contiguous bf16 or fp32; the result is [M, K] (G's transpose when G is taller than wide)."""
+        rows, cols = G.shape
+        self.native.check(self.native.lib().tplr_ns_prepare(
+            G.data_ptr(), int(G.dtype == torch.float32), rows, cols, int(rows > cols), epsilon, self.scratch.data_ptr(),
+            self.x[0].data_ptr(), self.native.stream_ptr()), "ns_prepare")
         self.graph.replay()
-        return self.result.clone()
+        return OF.gemm(self.B, self.last, b_mn=True)
 
 
 _chains: dict = {}
 
 
-def _ns_2d_symmetric(X: torch.Tensor) -> torch.Tensor:
-    key = (X.shape[0], X.shape[1], X.device.index, torch.cuda.current_stream(X.device).cuda_stream)
+def _ns_2d_symmetric(G: torch.Tensor, epsilon: float) -> torch.Tensor:
+    M, K = min(G.shape), max(G.shape)
+    key = (M, K, G.device.index, torch.cuda.current_stream(G.device).cuda_stream)
     chain = _chains.get(key)
     if chain is None:
         if len(_chains) >= 32:                          # a model has a handful of matrix shapes; bound the cache anyway
             _chains.clear()
-        chain = _chains[key] = _SymmetricChain(X.shape[0], X.shape[1], X.device)
-    return chain(X)
+        chain = _chains[key] = _SymmetricChain(M, K, G.device)
+    X = chain(G, epsilon)
+    return X.mT if G.shape[0] > G.shape[1] else X
 
 
 def _ns_2d(G: torch.Tensor, epsilon: float) -> torch.Tensor:
+    if _one_triangle_ok(G):
+        if G.dtype not in (torch.bfloat16, torch.float32):
+            G = G.to(torch.bfloat16)
+        if not G.is_contiguous() or G.data_ptr() % 16:
+            G = G.clone(memory_format=torch.contiguous_format)
+        return _ns_2d_symmetric(G, epsilon)
     X = G.to(torch.bfloat16)
     transposed = G.size(-2) > G.size(-1)
     if transposed:
         X = X.mT
     X = (X / (X.float().norm() + epsilon).to(X.dtype)).contiguous()
-    if _one_triangle_ok(X):
-        X = _ns_2d_symmetric(X)
-        return X.mT if transposed else X
     for a, b, c in NS_CONSTS:
         A = OF.gemm(X, X)                       # X X^T
         AA = OF.gemm(A, A)                      # A A^T = A A

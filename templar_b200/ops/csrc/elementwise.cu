@@ -490,6 +490,97 @@ __global__ void __launch_bounds__(512) sumsq_partial_kernel(const float* __restr
 }
 
 // partial must hold tplr_sumsq_blocks() floats; out[0] = sum(x^2). x must be 16-byte aligned.
+// ------------------------------------------------------------------------------------- //
+// Entry of the Newton-Schulz chain: out = X / bf16(|X| + eps) with X = bf16(G), transposed on the way when G is taller
+// than wide, so that the chain's operand is written once in the layout that its products read.  Bound by DRAM (one read
+// for the norm, one read from L2 and one write here); as eager ops the conversions, the norm, the division and the
+// copies into the transposed layout were nine passes.  8192 x 2048 bf16: 190 us eager, 34 us here.
+// ------------------------------------------------------------------------------------- //
+template <typename T>
+static __device__ __forceinline__ void ns_load8(const T* p, float* f);
+template <>
+__device__ __forceinline__ void ns_load8<bf16>(const bf16* p, float* f) { unpack8(*reinterpret_cast<const bf16x8*>(p), f); }
+template <>
+__device__ __forceinline__ void ns_load8<float>(const float* p, float* f) {      // rounded to bf16 as X is
+  const float4 a = reinterpret_cast<const float4*>(p)[0], b = reinterpret_cast<const float4*>(p)[1];
+  const float t[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
+  unpack8(pack8(t), f);
+}
+
+template <typename T>
+__global__ void __launch_bounds__(256) ns_sumsq_kernel(const T* __restrict__ g, long long n8, float* __restrict__ partial) {
+  __shared__ float red[32];
+  float s = 0.f;
+  for (long long i = blockIdx.x * 256LL + threadIdx.x; i < n8; i += gridDim.x * 256LL) {
+    float f[8]; ns_load8(g + i * 8, f);
+#pragma unroll
+    for (int e = 0; e < 8; ++e) s = fmaf(f[e], f[e], s);
+  }
+  s = block_sum(s, red);
+  if (threadIdx.x == 0) partial[blockIdx.x] = s;
+}
+
+// one 64 x 64 tile of G per CTA; rows and cols multiples of 8
+template <typename T>
+__global__ void __launch_bounds__(256) ns_scale_kernel(const T* __restrict__ g, int rows, int cols, const float* __restrict__ partial,
+                                                       int n_partial, float eps, int transpose, bf16* __restrict__ out) {
+  __shared__ float red[32];
+  __shared__ float tile[64][65];
+  float s = 0.f;
+  for (int i = threadIdx.x; i < n_partial; i += 256) s += partial[i];
+  s = block_sum(s, red);
+  const float den = __bfloat162float(__float2bfloat16(sqrtf(s) + eps));
+  const int i0 = blockIdx.y * 64, j0 = blockIdx.x * 64;
+  const int vx = threadIdx.x & 7, vy = threadIdx.x >> 3;
+#pragma unroll
+  for (int r = 0; r < 2; ++r) {
+    const int li = vy + 32 * r, i = i0 + li, j = j0 + vx * 8;
+    if (i < rows && j < cols) {
+      float f[8]; ns_load8(g + (long long)i * cols + j, f);
+#pragma unroll
+      for (int e = 0; e < 8; ++e) f[e] = f[e] / den;
+      if (!transpose) *reinterpret_cast<bf16x8*>(out + (long long)i * cols + j) = pack8(f);
+      else {
+#pragma unroll
+        for (int e = 0; e < 8; ++e) tile[li][vx * 8 + e] = f[e];
+      }
+    }
+  }
+  if (!transpose) return;
+  __syncthreads();
+#pragma unroll
+  for (int r = 0; r < 2; ++r) {
+    const int lj = vy + 32 * r, j = j0 + lj, i = i0 + vx * 8;
+    if (j < cols && i < rows) {
+      float f[8];
+#pragma unroll
+      for (int e = 0; e < 8; ++e) f[e] = tile[vx * 8 + e][lj];
+      *reinterpret_cast<bf16x8*>(out + (long long)j * rows + i) = pack8(f);
+    }
+  }
+}
+
+// g: contiguous [rows, cols] bf16 or fp32 (16-byte aligned, both sizes multiples of 8); out: [rows, cols], or [cols, rows]
+// when transpose; scratch: tplr_sumsq_blocks() floats.
+TPLR_API int tplr_ns_prepare(const void* g, int is_fp32, int rows, int cols, int transpose, float eps, float* scratch, void* out,
+                             void* stream) {
+  TPLR_ENTER();
+  if (rows % 8 || cols % 8 || (((uintptr_t)g | (uintptr_t)out) & 15)) return (int)cudaErrorInvalidValue;
+  if (rows <= 0 || cols <= 0) return 0;
+  cudaStream_t st = (cudaStream_t)stream;
+  const long long n8 = (long long)rows * cols / 8;
+  const int blocks = tplr_sm_count() * 4;
+  const dim3 grid((cols + 63) / 64, (rows + 63) / 64);
+  if (is_fp32) {
+    ns_sumsq_kernel<float><<<blocks, 256, 0, st>>>((const float*)g, n8, scratch);
+    ns_scale_kernel<float><<<grid, 256, 0, st>>>((const float*)g, rows, cols, scratch, blocks, eps, transpose, (bf16*)out);
+  } else {
+    ns_sumsq_kernel<bf16><<<blocks, 256, 0, st>>>((const bf16*)g, n8, scratch);
+    ns_scale_kernel<bf16><<<grid, 256, 0, st>>>((const bf16*)g, rows, cols, scratch, blocks, eps, transpose, (bf16*)out);
+  }
+  return (int)cudaGetLastError();
+}
+
 TPLR_API int tplr_sumsq_blocks() { return tplr_sm_count() * 4; }
 TPLR_API int tplr_sumsq(const float* x, long long n, float* partial, float* out, void* stream) {
   TPLR_ENTER();
@@ -620,6 +711,66 @@ __global__ void __launch_bounds__(256) sym_axpby_kernel(const bf16* __restrict__
     out[(long long)i * ldo + j] = __float2bfloat16(v);
   }
 }
+// The same from an fp32 U whose products were accumulated by several CTA pairs per tile (tplr_gemm2_syrk_acc), which wants
+// zeros to add into: every tile is set back to zero as it is read.  M a multiple of 8, dense matrices, 16-byte aligned.  One
+// CTA per 64 x 64 tile; those below the diagonal only clear what the product wrote there (the 256-wide diagonal tiles).
+__global__ void __launch_bounds__(256) sym_axpby_acc_kernel(float* __restrict__ U, int M, float alpha, const bf16* __restrict__ aux,
+                                                            float beta, float diag, bf16* __restrict__ out) {
+  __shared__ float tile[64][65];
+  const int ti = blockIdx.y, tj = blockIdx.x;
+  if (tj / 4 < ti / 4) return;
+  const int vx = threadIdx.x & 7, vy = threadIdx.x >> 3;      // 8 vectors of 8 columns, 32 rows per trip
+#pragma unroll
+  for (int r = 0; r < 2; ++r) {
+    const int li = vy + 32 * r, i = ti * 64 + li, j = tj * 64 + vx * 8;
+    if (i < M && j < M) {
+      float4* u = reinterpret_cast<float4*>(U + (long long)i * M + j);
+      if (tj >= ti) {
+        const float4 a = u[0], b = u[1];
+        const float f[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
+#pragma unroll
+        for (int e = 0; e < 8; ++e) tile[li][vx * 8 + e] = alpha * f[e];
+      }
+      u[0] = u[1] = make_float4(0.f, 0.f, 0.f, 0.f);
+    }
+  }
+  if (tj < ti) return;
+  __syncthreads();
+#pragma unroll
+  for (int half = 0; half < 2; ++half) {                      // 0: the tile, 1: its mirror image
+    if (half == 1 && ti == tj) break;
+    const int bi = half ? tj : ti, bj = half ? ti : tj;
+#pragma unroll
+    for (int r = 0; r < 2; ++r) {
+      const int li = vy + 32 * r, i = bi * 64 + li, j = bj * 64 + vx * 8;
+      if (i >= M || j >= M) continue;
+      float v[8];
+#pragma unroll
+      for (int e = 0; e < 8; ++e) {
+        const int lj = vx * 8 + e;
+        v[e] = half || (ti == tj && lj < li) ? tile[lj][li] : tile[li][lj];     // a diagonal tile is its own mirror image
+      }
+      if (aux) {
+        float x[8]; unpack8(*reinterpret_cast<const bf16x8*>(aux + (long long)i * M + j), x);
+#pragma unroll
+        for (int e = 0; e < 8; ++e) v[e] += beta * x[e];
+      }
+#pragma unroll
+      for (int e = 0; e < 8; ++e) if (i == j + e) v[e] += diag;
+      *reinterpret_cast<bf16x8*>(out + (long long)i * M + j) = pack8(v);
+    }
+  }
+}
+
+TPLR_API int tplr_sym_axpby_acc(float* U, int M, float alpha, const void* aux, float beta, float diag, void* out, void* stream) {
+  TPLR_ENTER();
+  if (M <= 0) return 0;
+  if (M % 8 || (((uintptr_t)U | (uintptr_t)aux | (uintptr_t)out) & 15)) return (int)cudaErrorInvalidValue;
+  const unsigned n = (unsigned)((M + 63) / 64);
+  sym_axpby_acc_kernel<<<dim3(n, n), 256, 0, (cudaStream_t)stream>>>(U, M, alpha, (const bf16*)aux, beta, diag, (bf16*)out);
+  return (int)cudaGetLastError();
+}
+
 TPLR_API int tplr_sym_axpby(const void* U, long long ldu, int M, float alpha, const void* aux, long long ldaux, float beta,
                             float diag, void* out, long long ldo, void* stream) {
   TPLR_ENTER();

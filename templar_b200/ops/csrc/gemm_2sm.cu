@@ -943,13 +943,12 @@ int dispatch2(Gemm2Params& p, int a_mn, int b_mn, int epi, int n_comm_pairs, int
 // Measured, one split against the chosen number: 768 x 768 x 8192 (9 tiles on 74 pairs) 54.8 -> 21.0 us with 4, 2304 x 768 x
 // 8192 55.4 -> 33.1 with 2, 1536 x 4096 x 4096 62.6 -> 51.5 with 2; where the waves are full already a second split costs
 // 3 to 16 % (8192 x 1536 x 4096 88.3 -> 94.2, 28672 x 4096 x 1024 287 -> 333) and none is made.  A split has to win 5 %.
-int pick_k_splits(int M, int N, int K, int max_pairs) {
+int pick_k_splits(long long tiles, int K, int max_pairs) {
   static const int forced = [] { const char* e = getenv("TPLR_GEMM_KSPLITS"); return e ? atoi(e) : 0; }();
   const long long kb = (K + BK - 1) / BK;
   if (forced > 0) return kb / forced >= 1 ? forced : 1;   // tuning override
   int pairs = tplr_sm_count() / 2;
   if (max_pairs > 0 && pairs > max_pairs) pairs = max_pairs;
-  const long long tiles = (long long)((M + TILE_M - 1) / TILE_M) * ((N + TILE_N - 1) / TILE_N);
   int best = 1;
   double best_cost = 0.0;
   for (int ks = 1; ks <= 8 && ks <= kb; ks *= 2) {
@@ -1006,6 +1005,28 @@ TPLR_API int tplr_gemm2_syrk(const void* A, void* C, int M, int K, long long lda
   return dispatch2(p, 0, 0, 0, 0, 0, (cudaStream_t)stream);
 }
 
+static long long syrk_tiles(int M) {
+  const long long t = (M + TILE_M - 1) / TILE_M;
+  return t * (t + 1) / 2;
+}
+// K splits that tplr_gemm2_syrk_acc makes for this size (1: tplr_gemm2_syrk is the better call).
+TPLR_API int tplr_gemm2_syrk_splits(int M, int K) { return pick_k_splits(syrk_tiles(M), K, 0); }
+
+// tplr_gemm2_syrk adding into an fp32 C (ldc a multiple of 4, zeroed by the caller) with K cut into several work units per
+// tile: the triangle of a small matrix has fewer tiles than the chip has CTA pairs.  2048 x 8192 (36 tiles on 74 pairs):
+// 49 us in one pass; an iteration's two products (K = 8192 and 2048) 64 us in one pass each, 44 us split.
+TPLR_API int tplr_gemm2_syrk_acc(const void* A, float* C, int M, int K, long long lda, long long ldc, unsigned int* status,
+                                 void* stream) {
+  TPLR_ENTER();
+  if (M <= 0 || K <= 0) return 0;
+  if ((ldc % 4) || ((uintptr_t)C & 15)) return -101;
+  Gemm2Params p = {};
+  if (int r = fill_common(p, A, A, C, M, M, K, lda, lda, ldc, 0, 0, 1, status)) return r;
+  p.tri = 1;
+  p.k_splits = pick_k_splits(syrk_tiles(M), K, 0);
+  return dispatch2(p, 0, 0, 1, 0, 0, (cudaStream_t)stream);
+}
+
 // Same contract as tplr_gemm_bf16; max_pairs <= 0 uses every SM pair.
 TPLR_API int tplr_gemm2_bf16(const void* A, const void* B, void* C, int M, int N, int K, long long lda,
                              long long ldb, long long ldc, int a_mn, int b_mn, int epi, unsigned int* status,
@@ -1014,7 +1035,7 @@ TPLR_API int tplr_gemm2_bf16(const void* A, const void* B, void* C, int M, int N
   if (M <= 0 || N <= 0 || K <= 0) return 0;
   Gemm2Params p = {};
   if (int r = fill_common(p, A, B, C, M, N, K, lda, ldb, ldc, a_mn, b_mn, epi, status)) return r;
-  if (epi == 1 && p.c_tma) p.k_splits = pick_k_splits(M, N, K, max_pairs);
+  if (epi == 1 && p.c_tma) p.k_splits = pick_k_splits((long long)((M + TILE_M - 1) / TILE_M) * ((N + TILE_N - 1) / TILE_N), K, max_pairs);
   return dispatch2(p, a_mn, b_mn, epi, 0, max_pairs, (cudaStream_t)stream);
 }
 

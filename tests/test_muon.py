@@ -244,3 +244,48 @@ def test_trainer_maps_muon_hparams_to_the_engine():
     assert kw["inner_optimizer"] == "muon" and kw["inner_lr"] == 0.03 and kw["muon_momentum"] == 0.9
     assert dict(kw["muon_aux_lr_scale"]) == {"head": 0.4, "embed": 0.5, "scalar": 0.2} and kw["weight_decay"] == 0.05
     assert t._muon_engine_args("adamw", {}) == {}
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("M,K", [(512, 512), (520, 264), (776, 2048), (1024, 2816)])
+def test_split_triangle_products_match_fp32(M, K):
+    """The triangle product accumulated in fp32 by several units per tile, its mirror with scalars, and the zeroed
+    accumulator that the next product finds: twice in a row, against fp32 of the bf16 operands."""
+    from templar_b200.ops import functional as OF
+    from templar_b200.ops import native
+
+    torch.manual_seed(M)
+    L, st = native.lib(), OF.status_word(torch.device("cuda")).data_ptr()
+    assert L.tplr_gemm2_syrk_splits(M, K) > 1 and L.tplr_gemm2_syrk_splits(8192, 8192) == 1
+    acc = torch.zeros(M, M, device="cuda")
+    out = torch.empty(M, M, dtype=torch.bfloat16, device="cuda")
+    aux = torch.randn(M, M, device="cuda")
+    aux = (aux + aux.t()).to(torch.bfloat16)
+    for _ in range(2):
+        x = (torch.randn(M, K, device="cuda") / K ** 0.5).to(torch.bfloat16)
+        native.check(L.tplr_gemm2_syrk_acc(x.data_ptr(), acc.data_ptr(), M, K, K, M, st, native.stream_ptr()), "syrk_acc")
+        native.check(L.tplr_sym_axpby_acc(acc.data_ptr(), M, 0.5, aux.data_ptr(), -2.0, 3.0, out.data_ptr(), native.stream_ptr()),
+                     "sym_axpby_acc")
+        want = 0.5 * (x.float() @ x.float().t()) - 2.0 * aux.float() + 3.0 * torch.eye(M, device="cuda")
+        assert torch.allclose(out.float(), want, atol=1e-3, rtol=2 ** -8)            # one rounding to bf16; K fp32 products
+        assert torch.equal(out, out.t()) and not acc.any()
+    assert int(OF.status_word(torch.device("cuda")).item()) == 0
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("shape,dtype", [((520, 1032), torch.float32), ((1032, 520), torch.bfloat16), ((512, 512), torch.float32)])
+def test_chain_operand_matches_eager(shape, dtype):
+    """tplr_ns_prepare against the eager conversion, norm, division and transpose."""
+    from templar_b200.ops import native
+
+    torch.manual_seed(5)
+    G = (torch.randn(*shape, device="cuda") * 1e-3).to(dtype)
+    X = G.to(torch.bfloat16)
+    X = X.mT if shape[0] > shape[1] else X
+    want = X / (X.float().norm() + 1e-7).to(X.dtype)
+    got = torch.empty(want.shape, dtype=torch.bfloat16, device="cuda")
+    scratch = torch.empty(native.lib().tplr_sumsq_blocks(), device="cuda")
+    native.check(native.lib().tplr_ns_prepare(G.data_ptr(), int(dtype == torch.float32), *shape, int(shape[0] > shape[1]), 1e-7,
+                                              scratch.data_ptr(), got.data_ptr(), native.stream_ptr()), "ns_prepare")
+    # the norm is summed in another order: at most one bf16 step of the divisor, 2^-8 relative
+    assert torch.allclose(got.float(), want.float(), rtol=2 ** -7, atol=0)
