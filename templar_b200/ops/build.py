@@ -1,4 +1,5 @@
-"""Builds the native library (``libtplr_b200.so``) in-tree with nvcc for sm_100a.
+"""Builds the native library (``libtplr_b200.so``) in-tree with nvcc for sm_100a, and the autograd nodes
+(``csrc_host/*.cpp`` -> ``tplr_host.so``) with the host compiler against PyTorch's headers.
 
 ``python -m templar_b200.ops.build`` (or :func:`build`) compiles every ``csrc/*.cu``
 translation unit with ``-gencode arch=compute_100a,code=sm_100a -lineinfo`` and links
@@ -19,6 +20,8 @@ HERE = Path(__file__).resolve().parent
 CSRC = HERE / "csrc"
 LIBDIR = HERE / "_lib"
 LIBNAME = "libtplr_b200.so"
+HOST_SRC = HERE / "csrc_host"
+HOSTNAME = "tplr_host.so"
 
 NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a",
@@ -42,6 +45,28 @@ def _nvcc() -> str:
 
 def lib_path() -> Path:
     return LIBDIR / LIBNAME
+
+
+def host_path() -> Path:
+    return LIBDIR / HOSTNAME
+
+
+def _build_host(run) -> None:
+    """The extension module of the autograd nodes: plain C++, no CUDA compiler involved."""
+    import sysconfig
+
+    import torch
+    from torch.utils.cpp_extension import include_paths
+
+    srcs = sorted(HOST_SRC.glob("*.cpp"))
+    out = host_path()
+    if out.exists() and all(s.stat().st_mtime <= out.stat().st_mtime for s in srcs):
+        return
+    inc = [x for p in [*include_paths("cuda"), sysconfig.get_paths()["include"]] for x in ("-isystem", p)]
+    tmp = out.with_suffix(".so.tmp")
+    run([os.environ.get("CXX", "g++"), "-O2", "-std=c++17", "-fPIC", "-shared", "-fvisibility=hidden", *inc, *map(str, srcs), "-o",
+         str(tmp), "-L" + str(Path(torch.__file__).parent / "lib"), "-lc10", "-ltorch_cpu", "-ltorch", "-ltorch_python", "-lc10_cuda"])
+    os.replace(tmp, out)
 
 
 def sources() -> list[Path]:
@@ -74,7 +99,7 @@ def build(verbose: bool = False, force: bool = False) -> Path:
     def run(cmd):
         r = subprocess.run(cmd, capture_output=True, text=True)
         if r.returncode != 0:
-            raise RuntimeError("nvcc failed: " + " ".join(cmd) + "\n" + r.stdout + r.stderr)
+            raise RuntimeError("compiler failed: " + " ".join(cmd) + "\n" + r.stdout + r.stderr)
         return r.stderr
 
     if jobs:
@@ -82,6 +107,7 @@ def build(verbose: bool = False, force: bool = False) -> Path:
             for out in ex.map(run, jobs):
                 if verbose and out:
                     print(out, file=sys.stderr)
+    _build_host(run)
     lib = lib_path()
     if jobs or not lib.exists():
         tmp = lib.with_suffix(".so.tmp")          # link beside the target, then rename: readers never see a partial file

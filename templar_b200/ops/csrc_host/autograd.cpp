@@ -1,0 +1,310 @@
+// Autograd nodes of the decoder block's operators, host side.
+//
+// The same sequences of kernel launches as the Python nodes in functional.py (_RMSNorm, _AddRMSNorm, _Linear, _FeedForward,
+// _AttentionBlock), for bf16 CUDA operands that those nodes would hand to the own kernels.  A Python node costs its
+// interpreter time twice (the backward half on the autograd thread, behind the interpreter lock): for one residual add and
+// norm of a small batch that was 115 us around 9 us of kernels.  Here it is 80 us, most of it the engine's own.
+//
+// functional.py decides which calls come here (operand types, strides and alignment) and keeps its nodes for all others.
+// Tensors are saved as saved variables only; the gradient buffers of the flat store are held by reference as there.
+#include <c10/cuda/CUDAStream.h>
+#include <dlfcn.h>
+#include <torch/extension.h>
+
+#include <atomic>
+
+namespace {
+
+using torch::Tensor;
+using torch::autograd::AutogradContext;
+using torch::autograd::Function;
+using torch::autograd::variable_list;
+typedef long long ll;
+
+std::atomic<ll> g_launches{0};
+
+// C entry points of the kernel library
+struct Entries {
+  int (*add_rmsnorm_fwd)(const void*, const void*, const void*, void*, void*, float*, ll, int, float, void*);
+  int (*add_rmsnorm_bwd)(const void*, const void*, const void*, const float*, const void*, void*, float*, ll, int, unsigned*, void*);
+  int (*gemm)(const void*, const void*, void*, int, int, int, ll, ll, ll, int, int, int, unsigned*, int, void*);
+  int (*swiglu)(const void*, const void*, void*, void*, int, int, int, ll, ll, ll, ll, unsigned*, void*);
+  int (*swiglu_bwd)(const void*, const void*, const void*, void*, int, int, int, ll, ll, ll, ll, unsigned*, void*);
+  int (*gemm_rope)(const void*, const void*, void*, int, int, int, ll, ll, ll, const float*, const float*, int, int, int, unsigned*, void*);
+  int (*attention_fwd)(const void*, void*, float*, int, int, int, int, int, ll, ll, float, unsigned*, void*);
+  int (*attn_dout)(const void*, const void*, const void*, void*, float*, int, int, int, int, int, ll, ll, ll, ll, unsigned*, void*);
+  int (*bwd_scratch_cols)(int, int, int, int, int);
+  int (*attention_bwd)(const void*, const void*, const void*, const float*, float*, float*, void*, int, int, int, int, int, ll, ll,
+                       float, const float*, const float*, unsigned*, void*);
+} E;
+
+void bind(const std::string& path) {
+  void* so = dlopen(path.c_str(), RTLD_NOW | RTLD_LOCAL);
+  TORCH_CHECK(so, "cannot open ", path, ": ", dlerror());
+  auto get = [&](auto& fn, const char* name) {
+    void* p = dlsym(so, name);
+    TORCH_CHECK(p, name, " is missing in ", path);
+    fn = reinterpret_cast<std::decay_t<decltype(fn)>>(p);
+  };
+  get(E.add_rmsnorm_fwd, "tplr_add_rmsnorm_fwd");
+  get(E.add_rmsnorm_bwd, "tplr_add_rmsnorm_bwd_v2");
+  get(E.gemm, "tplr_gemm2_bf16");
+  get(E.swiglu, "tplr_gemm2_swiglu");
+  get(E.swiglu_bwd, "tplr_gemm2_swiglu_bwd");
+  get(E.gemm_rope, "tplr_gemm2_rope");
+  get(E.attention_fwd, "tplr_attention_fwd");
+  get(E.attn_dout, "tplr_gemm2_attn_dout");
+  get(E.bwd_scratch_cols, "tplr_attention_bwd_scratch_cols");
+  get(E.attention_bwd, "tplr_attention_bwd_unrope_delta");
+}
+
+void check(int err, const char* what) {
+  g_launches.fetch_add(1, std::memory_order_relaxed);
+  TORCH_CHECK(err == 0, what, " failed with CUDA error ", err);
+}
+void* stream() { return c10::cuda::getCurrentCUDAStream().stream(); }
+unsigned* word(int64_t status) { return reinterpret_cast<unsigned*>(status); }
+
+// A gradient as the kernels read it: dense, on a 16-byte boundary.
+Tensor dense(const Tensor& t) {
+  Tensor c = t.contiguous();
+  return reinterpret_cast<uintptr_t>(c.data_ptr()) % 16 ? c.clone() : c;
+}
+Tensor f32(at::IntArrayRef shape, const Tensor& like) { return at::empty(shape, like.options().dtype(at::kFloat)); }
+Tensor bf16(at::IntArrayRef shape, const Tensor& like) { return at::empty(shape, like.options()); }
+
+// a tensor that takes no part in differentiation (a gradient buffer, the rotary tables); may be undefined
+struct Aside { Tensor t; };
+Tensor aside(AutogradContext* ctx, const char* key) {
+  auto it = ctx->saved_data.find(key);
+  return it == ctx->saved_data.end() ? Tensor() : it->second.toTensor();
+}
+void keep(AutogradContext* ctx, const char* key, const Aside& a) {
+  if (a.t.defined()) ctx->saved_data[key] = a.t;
+}
+
+// out = op(a) op(b)^T as functional.gemm; epi 0: store bf16, 1: add into fp32
+void gemm(const Tensor& a, const Tensor& b, const Tensor& out, bool a_mn, bool b_mn, int epi, int64_t status) {
+  const ll M = a_mn ? a.size(1) : a.size(0), K = a_mn ? a.size(0) : a.size(1), N = b_mn ? b.size(1) : b.size(0);
+  check(E.gemm(a.data_ptr(), b.data_ptr(), out.data_ptr(), (int)M, (int)N, (int)K, a.stride(0), b.stride(0), out.stride(0), a_mn,
+               b_mn, epi, word(status), 0, stream()),
+        "tplr_gemm_bf16");
+}
+// dW of y = x W^T: added into the gradient buffer when there is one, else returned when wanted
+Tensor weight_grad(const Tensor& buffer, const Tensor& dy2, const Tensor& x2, const Tensor& w, bool wanted, int64_t status) {
+  if (buffer.defined()) {
+    gemm(dy2, x2, buffer, true, true, 1, status);
+    return Tensor();
+  }
+  if (!wanted) return Tensor();
+  Tensor dw = bf16(w.sizes(), w);
+  gemm(dy2, x2, dw, true, true, 0, status);
+  return dw;
+}
+Tensor rows(const Tensor& t) { return t.reshape({-1, t.size(-1)}); }
+
+// ------------------------------------------------------------------------------------------ norms
+// inputs: x (or res, delta), w, buffer, eps, status
+variable_list norm_backward(AutogradContext* ctx, const Tensor& dh, const Tensor& dy_in, const Tensor& h, const Tensor& w,
+                            const Tensor& rstd, int w_index) {
+  const int64_t status = ctx->saved_data["status"].toInt();
+  const Tensor buffer = aside(ctx, "buffer");
+  const ll D = h.size(-1), T = h.numel() / D;
+  const Tensor dy = dy_in.defined() ? dense(dy_in) : at::zeros_like(h);
+  const Tensor dres = dh.defined() ? dense(dh) : Tensor();
+  Tensor dx = at::empty_like(h);
+  Tensor dw = buffer.defined() ? buffer : at::zeros({D}, h.options().dtype(at::kFloat));
+  check(E.add_rmsnorm_bwd(dy.data_ptr(), h.data_ptr(), w.data_ptr(), rstd.data_ptr<float>(), dres.defined() ? dres.data_ptr() : nullptr,
+                          dx.data_ptr(), dw.data_ptr<float>(), T, (int)D, word(status), stream()),
+        "add_rmsnorm_bwd");
+  return {dx, buffer.defined() || !ctx->needs_input_grad(w_index) ? Tensor() : dw.to(w.scalar_type())};
+}
+
+struct RMSNorm : Function<RMSNorm> {
+  static Tensor forward(AutogradContext* ctx, const Tensor& x, const Tensor& w, Aside buffer, double eps, int64_t status) {
+    const ll D = x.size(-1), T = x.numel() / D;
+    Tensor y = at::empty_like(x), rstd = f32({T}, x);
+    check(E.add_rmsnorm_fwd(x.data_ptr(), nullptr, w.data_ptr(), nullptr, y.data_ptr(), rstd.data_ptr<float>(), T, (int)D, (float)eps,
+                            stream()),
+          "rmsnorm_fwd");
+    ctx->save_for_backward({x, w, rstd});
+    keep(ctx, "buffer", buffer);
+    ctx->saved_data["status"] = status;
+    return y;
+  }
+  static variable_list backward(AutogradContext* ctx, variable_list g) {
+    auto s = ctx->get_saved_variables();
+    auto r = norm_backward(ctx, Tensor(), g[0], s[0], s[1], s[2], 1);
+    return {r[0], r[1], Tensor(), Tensor(), Tensor()};
+  }
+};
+
+struct AddRMSNorm : Function<AddRMSNorm> {
+  static variable_list forward(AutogradContext* ctx, const Tensor& res, const Tensor& delta, const Tensor& w, Aside buffer, double eps,
+                               int64_t status) {
+    const ll D = res.size(-1), T = res.numel() / D;
+    Tensor h = at::empty_like(res), y = at::empty_like(res), rstd = f32({T}, res);
+    check(E.add_rmsnorm_fwd(res.data_ptr(), delta.data_ptr(), w.data_ptr(), h.data_ptr(), y.data_ptr(), rstd.data_ptr<float>(), T,
+                            (int)D, (float)eps, stream()),
+          "add_rmsnorm_fwd");
+    ctx->save_for_backward({h, w, rstd});
+    keep(ctx, "buffer", buffer);
+    ctx->saved_data["status"] = status;
+    return {h, y};
+  }
+  static variable_list backward(AutogradContext* ctx, variable_list g) {
+    auto s = ctx->get_saved_variables();
+    auto r = norm_backward(ctx, g[0], g[1], s[0], s[1], s[2], 2);
+    return {r[0], r[0], r[1], Tensor(), Tensor(), Tensor()};
+  }
+};
+
+// ------------------------------------------------------------------------------------------ projections
+struct Linear : Function<Linear> {
+  static Tensor forward(AutogradContext* ctx, const Tensor& x, const Tensor& w, Aside buffer, int64_t status) {
+    auto shape = x.sizes().vec();
+    shape.back() = w.size(0);
+    Tensor y = bf16(shape, x);
+    gemm(rows(x), w, y.view({-1, w.size(0)}), false, false, 0, status);
+    ctx->save_for_backward({x, w});
+    keep(ctx, "buffer", buffer);
+    ctx->saved_data["status"] = status;
+    return y;
+  }
+  static variable_list backward(AutogradContext* ctx, variable_list g) {
+    auto s = ctx->get_saved_variables();
+    const int64_t status = ctx->saved_data["status"].toInt();
+    const Tensor dy2 = dense(rows(g[0])), x2 = rows(s[0]);
+    Tensor dx;
+    if (ctx->needs_input_grad(0)) {
+      dx = bf16(s[0].sizes(), s[0]);
+      gemm(dy2, s[1], dx.view({-1, s[1].size(1)}), false, true, 0, status);
+    }
+    return {dx, weight_grad(aside(ctx, "buffer"), dy2, x2, s[1], ctx->needs_input_grad(1), status), Tensor(), Tensor()};
+  }
+};
+
+struct FeedForward : Function<FeedForward> {
+  static Tensor forward(AutogradContext* ctx, const Tensor& x, const Tensor& w13, const Tensor& w2, Aside buffer13, Aside buffer2,
+                        int64_t status) {
+    const Tensor x2 = rows(x);
+    const ll T = x2.size(0), F2 = w13.size(0), F = F2 / 2;
+    Tensor gu = bf16({T, F2}, x), h = bf16({T, F}, x);
+    check(E.swiglu(x2.data_ptr(), w13.data_ptr(), gu.data_ptr(), h.data_ptr(), (int)T, (int)F, (int)x2.size(1), x2.stride(0),
+                   w13.stride(0), F2, F, word(status), stream()),
+          "gemm2_swiglu");
+    auto shape = x.sizes().vec();
+    shape.back() = w2.size(0);
+    Tensor y = bf16(shape, x);
+    gemm(h, w2, y.view({-1, w2.size(0)}), false, false, 0, status);
+    ctx->save_for_backward({x, w13, w2, gu, h});
+    keep(ctx, "buffer13", buffer13);
+    keep(ctx, "buffer2", buffer2);
+    ctx->saved_data["status"] = status;
+    return y;
+  }
+  static variable_list backward(AutogradContext* ctx, variable_list g) {
+    auto s = ctx->get_saved_variables();
+    const Tensor &x = s[0], &w13 = s[1], &w2 = s[2], &gu = s[3], &h = s[4];
+    const int64_t status = ctx->saved_data["status"].toInt();
+    const Tensor dy2 = dense(rows(g[0])), x2 = rows(x);
+    const ll T = gu.size(0), F = gu.size(1) / 2;
+    Tensor dgu = at::empty_like(gu);
+    check(E.swiglu_bwd(dy2.data_ptr(), w2.data_ptr(), gu.data_ptr(), dgu.data_ptr(), (int)T, (int)F, (int)dy2.size(1), dy2.stride(0),
+                       w2.stride(0), gu.stride(0), dgu.stride(0), word(status), stream()),
+          "gemm2_swiglu_bwd");
+    Tensor dw2 = weight_grad(aside(ctx, "buffer2"), dy2, h, w2, ctx->needs_input_grad(2), status);
+    Tensor dx;
+    if (ctx->needs_input_grad(0)) {
+      dx = bf16(x.sizes(), x);
+      gemm(dgu, w13, dx.view({-1, w13.size(1)}), false, true, 0, status);
+    }
+    Tensor dw13 = weight_grad(aside(ctx, "buffer13"), dgu, x2, w13, ctx->needs_input_grad(1), status);
+    return {dx, dw13, dw2, Tensor(), Tensor(), Tensor()};
+  }
+};
+
+struct AttentionBlock : Function<AttentionBlock> {
+  static Tensor forward(AutogradContext* ctx, const Tensor& x, const Tensor& wqkv, const Tensor& wo, Aside buffer_qkv, Aside buffer_o,
+                        Aside cos, Aside sin, int64_t heads, int64_t kv, int64_t hd, int64_t status) {
+    const ll B = x.size(0), S = x.size(1), C = wqkv.size(0), N = heads * hd;
+    const Tensor x2 = rows(x);
+    Tensor qkv = bf16({B, S, C}, x);
+    check(E.gemm_rope(x2.data_ptr(), wqkv.data_ptr(), qkv.data_ptr(), (int)x2.size(0), (int)C, (int)x2.size(1), x2.stride(0),
+                      wqkv.stride(0), C, cos.t.data_ptr<float>(), sin.t.data_ptr<float>(), (int)S, (int)((heads + kv) * hd), (int)hd,
+                      word(status), stream()),
+          "gemm2_rope");
+    Tensor out = bf16({B, S, N}, x), lse = f32({B, heads, S}, x);
+    check(E.attention_fwd(qkv.data_ptr(), out.data_ptr(), lse.data_ptr<float>(), (int)B, (int)S, (int)heads, (int)kv, (int)hd, C, N,
+                          (float)std::pow((double)hd, -0.5), word(status), stream()),
+          "attention_fwd");
+    Tensor y = bf16({B, S, wo.size(0)}, x);
+    gemm(out.view({-1, N}), wo, y.view({-1, wo.size(0)}), false, false, 0, status);
+    ctx->save_for_backward({x, wqkv, wo, qkv, out, lse, cos.t, sin.t});
+    keep(ctx, "buffer_qkv", buffer_qkv);
+    keep(ctx, "buffer_o", buffer_o);
+    ctx->saved_data["dims"] = std::vector<int64_t>{heads, kv, hd, status};
+    return y;
+  }
+  static variable_list backward(AutogradContext* ctx, variable_list g) {
+    auto s = ctx->get_saved_variables();
+    const Tensor &x = s[0], &wqkv = s[1], &wo = s[2], &qkv = s[3], &out = s[4], &lse = s[5], &cos = s[6], &sin = s[7];
+    const auto dims = ctx->saved_data["dims"].toIntVector();
+    const int64_t heads = dims[0], kv = dims[1], hd = dims[2], status = dims[3];
+    const ll B = qkv.size(0), S = qkv.size(1), C = qkv.size(2), T = B * S, N = heads * hd;
+    const Tensor dy2 = dense(rows(g[0])), out2 = out.view({T, N});
+    Tensor dO = bf16({T, N}, qkv), delta = f32({B, heads, S}, qkv);
+    check(E.attn_dout(dy2.data_ptr(), wo.data_ptr(), out2.data_ptr(), dO.data_ptr(), delta.data_ptr<float>(), (int)T, (int)N,
+                      (int)dy2.size(1), (int)S, (int)hd, dy2.stride(0), wo.stride(0), out2.stride(0), dO.stride(0), word(status),
+                      stream()),
+          "gemm2_attn_dout");
+    Tensor dwo = weight_grad(aside(ctx, "buffer_o"), dy2, out2, wo, ctx->needs_input_grad(2), status);
+    Tensor dqkv = at::empty_like(qkv);
+    {
+      Tensor scratch = at::zeros({B, S, E.bwd_scratch_cols((int)B, (int)S, (int)heads, (int)kv, (int)hd)},
+                                 qkv.options().dtype(at::kFloat));
+      check(E.attention_bwd(qkv.data_ptr(), out.data_ptr(), dO.data_ptr(), lse.data_ptr<float>(), delta.data_ptr<float>(),
+                            scratch.data_ptr<float>(), dqkv.data_ptr(), (int)B, (int)S, (int)heads, (int)kv, (int)hd, C, N,
+                            (float)std::pow((double)hd, -0.5), cos.data_ptr<float>(), sin.data_ptr<float>(), word(status), stream()),
+            "attention_bwd_unrope_delta");
+    }
+    const Tensor d2 = dqkv.view({T, C}), x2 = rows(x);
+    Tensor dx;
+    if (ctx->needs_input_grad(0)) {
+      dx = bf16(x.sizes(), x);
+      gemm(d2, wqkv, dx.view({-1, wqkv.size(1)}), false, true, 0, status);
+    }
+    Tensor dwqkv = weight_grad(aside(ctx, "buffer_qkv"), d2, x2, wqkv, ctx->needs_input_grad(1), status);
+    return {dx, dwqkv, dwo, Tensor(), Tensor(), Tensor(), Tensor(), Tensor(), Tensor(), Tensor(), Tensor()};
+  }
+};
+
+Aside opt(const std::optional<Tensor>& t) { return Aside{t ? *t : Tensor()}; }
+
+}  // namespace
+
+PYBIND11_MODULE(tplr_host, m) {
+  typedef py::call_guard<py::gil_scoped_release> nogil;
+  m.def("bind", &bind);
+  m.def("launches", [] { return g_launches.load(std::memory_order_relaxed); });
+  m.def("rmsnorm", [](const Tensor& x, const Tensor& w, const std::optional<Tensor>& buffer, double eps, int64_t status) {
+    return RMSNorm::apply(x, w, opt(buffer), eps, status);
+  }, nogil());
+  m.def("add_rmsnorm", [](const Tensor& res, const Tensor& delta, const Tensor& w, const std::optional<Tensor>& buffer, double eps,
+                          int64_t status) {
+    auto r = AddRMSNorm::apply(res, delta, w, opt(buffer), eps, status);
+    return std::make_tuple(r[0], r[1]);
+  }, nogil());
+  m.def("linear", [](const Tensor& x, const Tensor& w, const std::optional<Tensor>& buffer, int64_t status) {
+    return Linear::apply(x, w, opt(buffer), status);
+  }, nogil());
+  m.def("feed_forward", [](const Tensor& x, const Tensor& w13, const Tensor& w2, const std::optional<Tensor>& b13,
+                           const std::optional<Tensor>& b2, int64_t status) {
+    return FeedForward::apply(x, w13, w2, opt(b13), opt(b2), status);
+  }, nogil());
+  m.def("attention_block", [](const Tensor& x, const Tensor& wqkv, const Tensor& wo, const std::optional<Tensor>& bq,
+                              const std::optional<Tensor>& bo, const Tensor& cos, const Tensor& sin, int64_t heads, int64_t kv,
+                              int64_t hd, int64_t status) {
+    return AttentionBlock::apply(x, wqkv, wo, opt(bq), opt(bo), Aside{cos}, Aside{sin}, heads, kv, hd, status);
+  }, nogil());
+}

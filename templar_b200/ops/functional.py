@@ -56,6 +56,17 @@ def _native_ok(*ts) -> bool:
     return all(t.is_cuda for t in ts) and all(t.dtype == torch.bfloat16 for t in ts if t.is_floating_point())
 
 
+def _buffers_ok(*pairs) -> bool:
+    """Gradient targets that the autograd nodes in C++ (``native.host()``) can add into: none, or a dense fp32 buffer of
+    the weight's shape.  A target with a method of its own (sharded parameters) stays with the Python nodes."""
+    return all(g is None or (torch.is_tensor(g) and g.dtype == torch.float32 and g.shape == w.shape and g.is_contiguous())
+               for g, w in pairs)
+
+
+def _aligned(*ts) -> bool:
+    return all(t.data_ptr() % 16 == 0 for t in ts)
+
+
 # --------------------------------------------------------------------------- #
 # GEMM
 # --------------------------------------------------------------------------- #
@@ -170,6 +181,9 @@ class _Linear(torch.autograd.Function):
 def linear(x: torch.Tensor, w: torch.Tensor, main_grad: torch.Tensor | None = None) -> torch.Tensor:
     if main_grad is None:
         main_grad = getattr(w, "main_grad", None)
+    if (_GEMM_BACKEND == "tcgen05_2sm" and _native_ok(x, w) and x.is_contiguous() and w.is_contiguous() and w.shape[0] % 8 == 0
+            and w.shape[1] % 8 == 0 and x.shape[-1] == w.shape[1] and _buffers_ok((main_grad, w)) and _aligned(x, w)):
+        return native.host().linear(x, w, main_grad, status_word(x.device).data_ptr())
     return _Linear.apply(x, w, main_grad)
 
 
@@ -228,6 +242,10 @@ class _RMSNorm(torch.autograd.Function):
 def rmsnorm(x, w, eps: float = 1e-5, main_grad=None):
     if main_grad is None:
         main_grad = getattr(w, "main_grad", None)
+    D = x.shape[-1]
+    if (_native_ok(x, w) and D % 8 == 0 and D <= 8192 and x.is_contiguous() and w.is_contiguous() and w.numel() == D
+            and _buffers_ok((main_grad, w)) and _aligned(x, w)):
+        return native.host().rmsnorm(x, w, main_grad, eps, status_word(x.device).data_ptr())
     return _RMSNorm.apply(x, w, eps, main_grad)
 
 
@@ -294,6 +312,11 @@ def add_rmsnorm(res, delta, w, eps: float = 1e-5, main_grad=None):
     """Returns ``(res + delta, rmsnorm(res + delta) * w)``."""
     if main_grad is None:
         main_grad = getattr(w, "main_grad", None)
+    D = res.shape[-1]
+    if (_native_ok(res, delta, w) and D % 8 == 0 and D <= 8192 and res.shape == delta.shape and res.is_contiguous()
+            and delta.is_contiguous() and w.is_contiguous() and w.numel() == D and _buffers_ok((main_grad, w))
+            and _aligned(res, delta, w)):
+        return native.host().add_rmsnorm(res, delta, w, main_grad, eps, status_word(res.device).data_ptr())
     return _AddRMSNorm.apply(res, delta, w, eps, main_grad)
 
 
@@ -500,6 +523,8 @@ def feed_forward(x, w13, w2, main_grad13=None, main_grad2=None):
             y = torch.empty(*x.shape[:-1], w2.shape[0], dtype=x.dtype, device=x.device)
             gemm(h, w2, out=y.view(-1, w2.shape[0]))
             return y
+        if _buffers_ok((main_grad13, w13), (main_grad2, w2)) and w13.shape[1] == x2.shape[1] and w2.shape[1] == Fd:
+            return native.host().feed_forward(x, w13, w2, main_grad13, main_grad2, status_word(x.device).data_ptr())
         return _FeedForward.apply(x, w13, w2, main_grad13, main_grad2)
     return _Linear.apply(linear_swiglu(x, w13, main_grad13), w2, main_grad2)
 
@@ -888,6 +913,10 @@ def attention_block(x, wqkv, wo, cos, sin, n_heads: int, n_kv: int, hd: int, mai
             and wo.shape[0] % 8 == 0 and wo.shape[1] == n_heads * hd and cos.is_cuda and cos.dtype == torch.float32
             and cos.is_contiguous() and sin.is_contiguous() and cos.shape[0] >= S and cos.shape[1] == hd // 2
             and all(t.data_ptr() % 16 == 0 for t in (x, wqkv, wo, cos, sin))):
+        if (_buffers_ok((main_grad_qkv, wqkv), (main_grad_wo, wo)) and sin.dtype == torch.float32 and sin.shape == cos.shape
+                and wqkv.shape == ((n_heads + 2 * n_kv) * hd, K)):
+            return native.host().attention_block(x, wqkv, wo, main_grad_qkv, main_grad_wo, cos, sin, n_heads, n_kv, hd,
+                                                 status_word(x.device).data_ptr())
         return _AttentionBlock.apply(x, wqkv, wo, main_grad_qkv, main_grad_wo, cos, sin, n_heads, n_kv, hd)
     return _Linear.apply(rope_attention_projection(x, wqkv, cos, sin, n_heads, n_kv, hd, main_grad_qkv), wo, main_grad_wo)
 

@@ -11,7 +11,9 @@ not the one running.
 from __future__ import annotations
 
 import ctypes
+import sys
 import threading
+import types
 from ctypes import c_float, c_int, c_longlong, c_void_p
 
 import torch
@@ -20,7 +22,8 @@ from . import build as _build
 
 _lock = threading.Lock()
 _lib = None
-launch_count = 0          # number of kernel-launching native calls made by this process
+_host = None
+_launches = 0             # kernel-launching native calls made through check(); see launch_count below
 
 
 class NativeError(RuntimeError):
@@ -48,6 +51,28 @@ def lib() -> ctypes.CDLL:
             _lib = ctypes.CDLL(str(path))
             _declare(_lib)
     return _lib
+
+
+def host():
+    """The extension module with the autograd nodes of the block's operators (``csrc_host/autograd.cpp``)."""
+    global _host
+    if _host is not None:
+        return _host
+    lib()
+    with _lock:
+        if _host is None:
+            import importlib.machinery
+            import importlib.util
+
+            path = _build.host_path()
+            if not path.exists():
+                _build.build()
+            loader = importlib.machinery.ExtensionFileLoader("tplr_host", str(path))
+            mod = importlib.util.module_from_spec(importlib.util.spec_from_loader("tplr_host", loader))
+            loader.exec_module(mod)
+            mod.bind(str(_build.lib_path()))
+            _host = mod
+    return _host
 
 
 def _declare(L: ctypes.CDLL) -> None:
@@ -122,12 +147,28 @@ def _declare(L: ctypes.CDLL) -> None:
 
 
 def stream_ptr() -> int:
-    return torch.cuda.current_stream().cuda_stream
+    # the raw handle: building a torch.cuda.Stream object for it costs 3 us a launch
+    return torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice())
+
+
+class _Module(types.ModuleType):
+    @property
+    def launch_count(self) -> int:
+        """Kernel-launching native calls made by this process, from here and from the autograd nodes in C++."""
+        return _launches + (_host.launches() if _host is not None else 0)
+
+    @launch_count.setter
+    def launch_count(self, n: int) -> None:
+        global _launches
+        _launches = n - (_host.launches() if _host is not None else 0)
+
+
+sys.modules[__name__].__class__ = _Module
 
 
 def check(err: int, what: str) -> None:
-    global launch_count
-    launch_count += 1
+    global _launches
+    _launches += 1
     if err != 0:
         raise NativeError(f"{what} failed with CUDA error {err}")
 
