@@ -87,6 +87,7 @@ def _declare(L: ctypes.CDLL) -> None:
         "tplr_quantize_values": [vp, i, vp, vp, vp, vp, i, i, f, vp],
         "tplr_dequantize_values": [vp, i, vp, vp, vp, i, vp],
         "tplr_requant_residual": [vp, i, i, vp, vp, vp, vp, vp, vp, i, i, i, vp],
+        "tplr_requant_residual_64": [vp, i, i, vp, vp, vp, vp, vp, vp, i, vp],
         "tplr_compress_chunks_tc": [vp, i, i, vp, vp, vp, vp, vp, vp, vp, f, i, i, i, vp],
         "tplr_aggregate_apply_tc": [vp, i, i, vp, i, vp, vp, i, vp, i, i, vp, vp, vp, vp, vp, vp, f, f, i, vp, vp],
         "tplr_add_rmsnorm_fwd": [vp, vp, vp, vp, vp, vp, ll, i, f, vp],

@@ -724,6 +724,12 @@ class WindowEngine:
             desc, n_desc, n_chunks = self._desc[square]
             if n_chunks == 0:
                 continue
+            if square and cfg.use_dct and self._dct_on_tensor_cores:       # every chunk of this table is 64 x 64
+                native.check(L.tplr_requant_residual_64(desc.data_ptr(), n_desc, n_chunks, self.basis.data_ptr(),
+                                                        self.ef.data_ptr() - bias, at0(self.own_idx), at0(self.own_val),
+                                                        at0(codes), at0(table), cfg.quant_bins, native.stream_ptr()),
+                             "requant_residual_64")
+                continue
             native.check(L.tplr_requant_residual(desc.data_ptr(), n_desc, n_chunks, self.basis.data_ptr(),
                                                  self.ef.data_ptr() - bias, at0(self.own_idx), at0(self.own_val),
                                                  at0(codes), at0(table), cfg.quant_bins, int(cfg.use_dct),

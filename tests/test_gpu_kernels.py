@@ -588,3 +588,38 @@ def test_add_rmsnorm_wide_rows(D, T):
         assert torch.allclose(ww.grad.float(), wf.grad, atol=1e-3 * T ** 0.5, rtol=2 ** -8)
     torch.cuda.synchronize()
     assert int(OF.status_word(DEV).item()) == 0
+
+
+@pytest.mark.parametrize("use_dct", [True, False])
+@pytest.mark.parametrize("shapes,topk,null_round", [
+    ([(64, 64)], 32, False),                                  # half a chunk pair
+    ([(192, 64), (64, 128)], 64, False),                      # pairs that span two tensors, an odd chunk at the end
+    ([(320, 192), (96, 40), (130,)], 2, False),               # chunks of other shapes beside the 64 x 64 ones
+    ([(128, 192), (48,)], 16, True),
+])
+def test_quantised_residual_is_taken_against_the_decoded_values(shapes, topk, null_round, use_dct):
+    """With 8-bit codes e <- gamma*e + delta - decode(dequantised values), against float64 with the engine's own payload.
+    Bound: fp32 sums of at most 64 products of values below 4 (2^-24 * 64 * 4 = 1.5e-5 worst case, 5e-6 as in the other
+    residual tests here)."""
+    torch.manual_seed(4)
+    model = _Bag(shapes).to(DEV)
+    eng = WindowEngine(model, EngineConfig(topk=topk, use_dct=use_dct, momentum_decay=0.9, quantize=True), device=DEV,
+                       compute_dtype=torch.float32)
+    eng.snapshot()
+    ef0 = torch.randn_like(eng.ef) * 0.01
+    eng.ef.copy_(ef0)
+    eng.store.master_shard.add_(torch.randn_like(eng.store.master_shard) * 0.02)
+    eng.compress(null_round=null_round)
+    torch.cuda.synchronize()
+    assert eng.check_status() == 0
+    comp = C.TopKCompressor()
+    for s in eng.layout.specs:
+        sl = slice(s.offset, s.offset + s.numel)
+        x = 0.9 * ef0[sl].cpu().double() + (eng.theta0[sl] - eng.store.master_shard[sl]).cpu().double()
+        x = torch.zeros_like(x) if null_round else x
+        idx, val = eng.layout.payload_views(eng.own_idx, eng.own_val, s.name)
+        tr = C.ChunkingTransformer(None, 64)
+        tr.register_shape(s.shape, dtype=torch.float64)
+        ref = torch.empty(s.shape, dtype=torch.float64)
+        sent = tr.decode(comp.decompress(ref, idx.cpu(), val.cpu().double(), eng.layout.xshape(s.name), s.totalk), use_dct=use_dct)
+        assert torch.allclose(eng.ef[sl].cpu().double(), x - sent.reshape(-1), atol=5e-6, rtol=1e-4), s.name
