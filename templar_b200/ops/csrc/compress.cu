@@ -622,6 +622,17 @@ __device__ __forceinline__ void split3(float x, __nv_bfloat16& b1, __nv_bfloat16
   b3 = __float2bfloat16_rn(r1 - __bfloat162float(b2));
 }
 
+// The same for two values, each term packed as the tiles store it: one conversion instruction per term and pair.
+__device__ __forceinline__ void split3_pair(float x, float y, uint32_t& w1, uint32_t& w2, uint32_t& w3) {
+  const __nv_bfloat162 h1 = __floats2bfloat162_rn(x, y);
+  w1 = *reinterpret_cast<const uint32_t*>(&h1);
+  const float rx = x - __uint_as_float(w1 << 16), ry = y - __uint_as_float(w1 & 0xffff0000u);
+  const __nv_bfloat162 h2 = __floats2bfloat162_rn(rx, ry);
+  w2 = *reinterpret_cast<const uint32_t*>(&h2);
+  const __nv_bfloat162 h3 = __floats2bfloat162_rn(rx - __uint_as_float(w2 << 16), ry - __uint_as_float(w2 & 0xffff0000u));
+  w3 = *reinterpret_cast<const uint32_t*>(&h3);
+}
+
 // Writes 32 consecutive fp32 values of one tile row (columns 32*hf .. 32*hf+31) as three bf16 split tiles.
 // row: 128-byte row index inside the tile whose three term copies start at base, base + stride, base + 2*stride.
 __device__ __forceinline__ void store_split_row(uint32_t base, uint32_t stride, int row, int hf, const float* v) {
@@ -631,15 +642,7 @@ __device__ __forceinline__ void store_split_row(uint32_t base, uint32_t stride, 
   for (int q = 0; q < 4; ++q) {
     uint32_t w1[4], w2[4], w3[4];
 #pragma unroll
-    for (int e = 0; e < 4; ++e) {
-      __nv_bfloat16 a1, a2, a3, c1, c2, c3;
-      split3(v[8 * q + 2 * e], a1, a2, a3);
-      split3(v[8 * q + 2 * e + 1], c1, c2, c3);
-      __nv_bfloat162 h1 = __halves2bfloat162(a1, c1), h2 = __halves2bfloat162(a2, c2), h3 = __halves2bfloat162(a3, c3);
-      w1[e] = *reinterpret_cast<uint32_t*>(&h1);
-      w2[e] = *reinterpret_cast<uint32_t*>(&h2);
-      w3[e] = *reinterpret_cast<uint32_t*>(&h3);
-    }
+    for (int e = 0; e < 4; ++e) split3_pair(v[8 * q + 2 * e], v[8 * q + 2 * e + 1], w1[e], w2[e], w3[e]);
     const uint32_t off = (((uint32_t)(hf * 4 + q)) ^ sw) << 4;
     asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(rowaddr + off), "r"(w1[0]), "r"(w1[1]), "r"(w1[2]), "r"(w1[3]) : "memory");
     asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(rowaddr + stride + off), "r"(w2[0]), "r"(w2[1]), "r"(w2[2]), "r"(w2[3]) : "memory");
@@ -972,25 +975,31 @@ __global__ void __launch_bounds__(NT, 3) aggregate_tc_kernel(const AggArgs a) {
 // second GEMM, the coefficients Y[32*hf .. 32*hf+31][rin] (the GEMM pair leaves Y transposed).
 // ------------------------------------------------------------------------------------- //
 constexpr int TC_NCAND = 256;                // candidates of the threshold search per chunk (the histogram's storage)
-constexpr int TC_X_BYTES = 128 * 64 * 4;     // fp32 copy of the two chunks (each thread re-reads only its own part)
-constexpr int TC_SMEM_CMP = 3 * TC_A_TILE + 3 * TC_B_TILE + TC_X_BYTES + 1024;
+// Three CTAs per SM (73 KB and 80 registers): a pair is a chain of loads, four products, a selection and a dozen barriers, and
+// what it waits for is covered by the other CTAs.  For that the fp32 copy of the pair is not kept in shared memory but written
+// to e and read back (from L2) at the end, the table entries and the search's scratch share memory that is there anyway,
+// and only one warp polls for a product.  402 M parameters, k = 32: 3744 us with two
+// CTAs and the copy in shared memory, 3193 us here, the same bits.
+constexpr int TC_SMEM_CMP = 3 * TC_A_TILE + 3 * TC_B_TILE + 1024;
 
-__global__ void __launch_bounds__(NT, 2) compress_tc_kernel(const CompressArgs a) {
+__global__ void __launch_bounds__(NT, 3) compress_tc_kernel(const CompressArgs a) {
   extern __shared__ uint8_t smem_raw_tc[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw_tc) + 1023) & ~(uintptr_t)1023);
   __shared__ __align__(8) uint64_t bar_mma;
   __shared__ uint32_t s_tmem_base;
   __shared__ int s_abort;
-  __shared__ int s_hist[2][256];
   __shared__ int s_wsum[8];
   __shared__ int s_bin[2], s_krem[2];
-  __shared__ __align__(16) unsigned int s_tmax[2][128];
-  __shared__ unsigned int s_thr[2];
+  // scratch of the threshold search: in the operand tiles, which are free between the second product and the next
+  // writes to them (both behind a barrier)
+  int (*s_hist)[256] = reinterpret_cast<int (*)[256]>(smem);
+  __shared__ unsigned int s_thr[8];                      // per warp
   __shared__ long long s_gbase[2];                       // element offset of each chunk of the pair, -1: none
   __shared__ int s_cols[2];
+  __shared__ TplrParamDesc s_d[2];                       // the chunks' table entries (20 registers a thread otherwise)
   __shared__ int s_sel_idx[2][TPLR_TILE];
   __shared__ float s_sel_val[2][TPLR_TILE];
-  const uint32_t sA = smem_u32(smem), sB = sA + 3 * TC_A_TILE, sX = sB + 3 * TC_B_TILE;
+  const uint32_t sA = smem_u32(smem), sB = sA + 3 * TC_A_TILE;
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int qd = warp & 3, hf = warp >> 2;
@@ -998,8 +1007,6 @@ __global__ void __launch_bounds__(NT, 2) compress_tc_kernel(const CompressArgs a
   const int trow = ch * 64 + rin;
   const int lt = rin + hf * 64;                          // thread index inside the chunk's group of 128
   const uint32_t lane_off = (uint32_t)(qd * 32) << 16;
-  const uint32_t xaddr = sX + (uint32_t)trow * 256u + (uint32_t)hf * 128u;
-  const uint32_t xsw = (uint32_t)(lane & 7);
   volatile int* abort_flag = &s_abort;
   int cur_f = -1;
   uint32_t phase = 0;
@@ -1020,7 +1027,8 @@ __global__ void __launch_bounds__(NT, 2) compress_tc_kernel(const CompressArgs a
   const int n_pairs = (a.total_chunks + 1) / 2;
   bool ok = true;
 
-  TplrParamDesc d = a.descs[0];
+  const TplrParamDesc& d = s_d[ch];
+  if (tid < 2) s_d[tid] = a.descs[0];
   auto run_gemm = [&](uint32_t tD, bool a_mn, bool b_mn) -> bool {
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     tcgen05_fence_before();
@@ -1030,7 +1038,7 @@ __global__ void __launch_bounds__(NT, 2) compress_tc_kernel(const CompressArgs a
       issue_split_gemm(tD, sA, sB, a_mn, b_mn);
       umma_commit(smem_u32(&bar_mma));
     }
-    bool o = mbar_wait(smem_u32(&bar_mma), phase, abort_flag);
+    bool o = warp != 0 || mbar_wait(smem_u32(&bar_mma), phase, abort_flag);     // one warp polls, the barrier releases the others
     phase ^= 1;
     o = __syncthreads_and(o);
     tcgen05_fence_after();
@@ -1040,26 +1048,25 @@ __global__ void __launch_bounds__(NT, 2) compress_tc_kernel(const CompressArgs a
   for (int q = blockIdx.x; q < n_pairs && ok; q += gridDim.x) {
     const int c = 2 * q + ch;
     const bool active = c < a.total_chunks;
-    {
+    __syncthreads();                                     // the previous pair's tiles, payload and entries are done with
+    if (rin == 0 && hf == 0) {
       const int cc = active ? c : a.total_chunks - 1;
-      if (!(cc >= d.chunk_begin && cc < d.chunk_begin + d.n_chunks)) d = a.descs[find_desc(a.descs, a.n_desc, cc)];
+      if (!(cc >= d.chunk_begin && cc < d.chunk_begin + d.n_chunks)) s_d[ch] = a.descs[find_desc(a.descs, a.n_desc, cc)];
+      const int cl = c - d.chunk_begin;
+      s_gbase[ch] = active ? d.elem_off + (long long)(d.chunk_row0 + cl / d.chunks_x) * 64 * d.cols + (long long)(cl % d.chunks_x) * 64 : -1;
+      s_cols[ch] = d.cols;
     }
-    const int k = d.k;
-    const int cl = c - d.chunk_begin;
-    const int cy = d.chunk_row0 + cl / d.chunks_x, cx = cl % d.chunks_x;
-    const long long gbase = d.elem_off + (long long)cy * 64 * d.cols + (long long)cx * 64;
     __syncthreads();
-    if (rin == 0 && hf == 0) { s_gbase[ch] = active ? gbase : -1; s_cols[ch] = d.cols; }
-    if (d.fh_off != cur_f) {
+    const int k = d.k;
+    if (d.fh_off != cur_f) {                             // read behind the first product's barrier
       load_basis_split(a.basis + d.fh_off, sB);
       cur_f = d.fh_off;
     }
-    __syncthreads();
-    // ---- X = gamma*e + delta into the fp32 copy in shared memory ------------------------------------
+    // ---- X = gamma*e + delta into the operand tiles and, in fp32, into e ------------------------------
     // Row-contiguous mapping: half a warp per row of the stacked 128 x 64 tile, 16 bytes per lane, so that every
-    // global access of a warp covers two whole 256-byte rows (one row per lane would touch 32 lines per
-    // instruction).  Slot (row, 16-byte column c4) of the copy: row * 256 + (c4 / 8) * 128 + ((c4 % 8) ^ (row % 8)) * 16.
+    // global access of a warp covers two whole 256-byte rows (one row per lane would touch 32 lines per instruction).
     const int urow = tid >> 4, uc4 = tid & 15;
+    float4 xs[8];                                        // stored behind the loop: a store to e would hold back the next rows' loads
 #pragma unroll
     for (int i = 0; i < 8; ++i) {
       const int row = i * 16 + urow, c2 = row >> 6;
@@ -1076,17 +1083,23 @@ __global__ void __launch_bounds__(NT, 2) compress_tc_kernel(const CompressArgs a
         x.x = fmaf(a.gamma, e.x, dl.x); x.y = fmaf(a.gamma, e.y, dl.y);
         x.z = fmaf(a.gamma, e.z, dl.z); x.w = fmaf(a.gamma, e.w, dl.w);
       }
-      asm volatile("st.shared.v4.f32 [%0], {%1, %2, %3, %4};" ::"r"(sX + (uint32_t)row * 256u + (uint32_t)(uc4 >> 3) * 128u +
-                   ((((uint32_t)uc4 & 7u) ^ (uint32_t)(row & 7)) << 4)), "f"(x.x), "f"(x.y), "f"(x.z), "f"(x.w) : "memory");
+      xs[i] = x;
+      uint32_t w1[2], w2[2], w3[2];
+      split3_pair(x.x, x.y, w1[0], w2[0], w3[0]);
+      split3_pair(x.z, x.w, w1[1], w2[1], w3[1]);
+      // no memory clobber: the next rows' loads may move above these stores (the barrier before the product orders them)
+      const uint32_t ad = sA + (uint32_t)row * 128u + ((((uint32_t)uc4 >> 1) ^ (uint32_t)(row & 7)) << 4) + ((uint32_t)uc4 & 1u) * 8u;
+      asm volatile("st.shared.v2.b32 [%0], {%1, %2};" ::"r"(ad), "r"(w1[0]), "r"(w1[1]));
+      asm volatile("st.shared.v2.b32 [%0], {%1, %2};" ::"r"(ad + TC_A_TILE), "r"(w2[0]), "r"(w2[1]));
+      asm volatile("st.shared.v2.b32 [%0], {%1, %2};" ::"r"(ad + 2 * TC_A_TILE), "r"(w3[0]), "r"(w3[1]));
     }
-    __syncthreads();
-    // this thread's 32 values (row trow, columns 32*hf ..) for the operand tile
-    float v[32];
 #pragma unroll
-    for (int q4 = 0; q4 < 8; ++q4)
-      asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v[4 * q4]), "=f"(v[4 * q4 + 1]), "=f"(v[4 * q4 + 2]),
-                   "=f"(v[4 * q4 + 3]) : "r"(xaddr + (((uint32_t)q4 ^ xsw) << 4)) : "memory");
-    store_split_row(sA, TC_A_TILE, trow, hf, v);
+    for (int i = 0; i < 8; ++i) {
+      const int row = i * 16 + urow;
+      const long long gb = s_gbase[row >> 6];
+      if (gb >= 0) *reinterpret_cast<float4*>(a.ef + gb + (long long)(row & 63) * s_cols[row >> 6] + uc4 * 4) = xs[i];
+    }
+    float v[32];
     if ((a.variant & 2) && !a.null_round) {
       // the next pair's 128 bytes of this thread in the three dense tensors, asked into L2 now
       const int cn = c + 2 * (int)gridDim.x;
@@ -1117,9 +1130,10 @@ __global__ void __launch_bounds__(NT, 2) compress_tc_kernel(const CompressArgs a
     tcgen05_fence_before();
     // ---- threshold of the k largest |Y| of each chunk (its 128 threads, 32 keys each) ---------
     // Result: prefix = the k-th largest key, krem = how many keys equal to it belong to the selection.
-    // Fast path: the k-th largest of the 128 per-thread maxima is a lower bound of the k-th largest key
-    // (k distinct keys are at least that large), so only the keys at or above it (a few dozen for k = 32)
-    // are candidates; they are compacted into shared memory and the exact threshold is found by counting
+    // Fast path: every warp finds the ceil(k / 4)-th largest of its 32 per-thread maxima; the smallest of the four
+    // is a lower bound of the k-th largest key (k distinct keys are at least that large), so only the keys at or
+    // above it (a few dozen for k = 32) are candidates (the k-th of all 128 maxima is a little closer, for 350
+    // instructions a thread more and a barrier); they are compacted into shared memory and the exact threshold is found by counting
     // among them.  No shared-memory atomics: the histogram of the radix select below serialises on the
     // few exponent values that the keys share.  More candidates than fit (many equal keys) or
     // k > 128 take the radix select.
@@ -1130,27 +1144,20 @@ __global__ void __launch_bounds__(NT, 2) compress_tc_kernel(const CompressArgs a
       unsigned int m = 0u;
 #pragma unroll
       for (int i = 0; i < 32; ++i) m = max(m, __float_as_uint(v[i]) & 0x7fffffffu);
-      s_tmax[ch][lt] = m;
-      __syncthreads();
-      {
-        int rank = 0;
-        const uint4* row = reinterpret_cast<const uint4*>(s_tmax[ch]);
-#pragma unroll 8
-        for (int j4 = 0; j4 < 32; ++j4) {
-          const uint4 o = row[j4];
-          const int j = 4 * j4;
-          rank += (o.x > m) || (o.x == m && j < lt);
-          rank += (o.y > m) || (o.y == m && j + 1 < lt);
-          rank += (o.z > m) || (o.z == m && j + 2 < lt);
-          rank += (o.w > m) || (o.w == m && j + 3 < lt);
-        }
-        if (rank == k - 1) s_thr[ch] = m;
+      int rank = 0;
+#pragma unroll
+      for (int j = 0; j < 32; ++j) {
+        const unsigned int o = __shfl_sync(0xffffffffu, m, j);
+        rank += (o > m) || (o == m && j < lane);
       }
+      if (rank == (k + 3) / 4 - 1) s_thr[warp] = m;
       __syncthreads();
+      // warps of chunk ch: 2ch, 2ch+1, 2ch+4, 2ch+5
+      const unsigned int low = min(min(s_thr[2 * ch], s_thr[2 * ch + 1]), min(s_thr[2 * ch + 4], s_thr[2 * ch + 5]));
       // zero keys never are candidates: a chunk with fewer than k non-zero coefficients (rows of the embedding that
-      // no token touched, a null round) has t0 == 0 and is resolved without any search: all non-zero keys and the
-      // first k - n_cand zeros in order
-      const unsigned int t0 = s_thr[ch] ? s_thr[ch] : 1u;
+      // no token touched, a null round) is resolved without any search: all non-zero keys and the first k - n_cand
+      // zeros in order
+      const unsigned int t0 = low ? low : 1u;
       int cnt = 0;
 #pragma unroll
       for (int i = 0; i < 32; ++i) cnt += (__float_as_uint(v[i]) & 0x7fffffffu) >= t0;
@@ -1275,6 +1282,7 @@ __global__ void __launch_bounds__(NT, 2) compress_tc_kernel(const CompressArgs a
     __syncthreads();
     // ---- payload ------------------------------------------------------------------------------
     if (active) {
+      const int cl = c - d.chunk_begin;
       uint8_t* ip = a.idx_out + d.idx_off + (long long)cl * (k / 2) * 3;
       float* vp = a.val_out + d.val_off + (long long)cl * k;
       if (lt < k / 2) {
@@ -1286,59 +1294,60 @@ __global__ void __launch_bounds__(NT, 2) compress_tc_kernel(const CompressArgs a
       if (lt >= 64 && lt < 64 + k) vp[lt - 64] = s_sel_val[ch][lt - 64];
     }
     // ---- residual e <- X - F^T S F with S the selected coefficients ------------------------------
-    float t32[32];
-    if (a.write_residual) {
-      for (int i = tid; i < 3 * TC_A_TILE / 16; i += NT) reinterpret_cast<uint4*>(smem)[i] = make_uint4(0, 0, 0, 0);
-      __syncthreads();
-      if (lt < k) {
-        const int e = s_sel_idx[ch][lt];
-        const int n = e >> 6, jx = e & 63;                 // S[n][jx] goes to row jx, column n of the S^T tile
-        const int row = ch * 64 + jx;
-        const uint32_t addr = (uint32_t)row * 128u + ((((uint32_t)(n >> 3)) ^ (uint32_t)(row & 7)) << 4) + (uint32_t)(n & 7) * 2u;
-        __nv_bfloat16 b1, b2, b3;
-        split3(s_sel_val[ch][lt], b1, b2, b3);
-        *reinterpret_cast<__nv_bfloat16*>(smem + addr) = b1;
-        *reinterpret_cast<__nv_bfloat16*>(smem + TC_A_TILE + addr) = b2;
-        *reinterpret_cast<__nv_bfloat16*>(smem + 2 * TC_A_TILE + addr) = b3;
-      }
-      if (!(ok = run_gemm(tZ, /*a_mn=*/false, /*b_mn=*/true))) break;        // Z' = S^T F
-      {
-        uint32_t r[32];
-        tmem_ld32(tZ + hf * 32 + lane_off, r);
+    if (!a.write_residual) continue;
+    for (int i = tid; i < 3 * TC_A_TILE / 16; i += NT) reinterpret_cast<uint4*>(smem)[i] = make_uint4(0, 0, 0, 0);
+    __syncthreads();
+    if (lt < k) {
+      const int e = s_sel_idx[ch][lt];
+      const int n = e >> 6, jx = e & 63;                 // S[n][jx] goes to row jx, column n of the S^T tile
+      const int row = ch * 64 + jx;
+      const uint32_t addr = (uint32_t)row * 128u + ((((uint32_t)(n >> 3)) ^ (uint32_t)(row & 7)) << 4) + (uint32_t)(n & 7) * 2u;
+      __nv_bfloat16 b1, b2, b3;
+      split3(s_sel_val[ch][lt], b1, b2, b3);
+      *reinterpret_cast<__nv_bfloat16*>(smem + addr) = b1;
+      *reinterpret_cast<__nv_bfloat16*>(smem + TC_A_TILE + addr) = b2;
+      *reinterpret_cast<__nv_bfloat16*>(smem + 2 * TC_A_TILE + addr) = b3;
+    }
+    if (!(ok = run_gemm(tZ, /*a_mn=*/false, /*b_mn=*/true))) break;          // Z' = S^T F
+    {
+      uint32_t r[32];
+      tmem_ld32(tZ + hf * 32 + lane_off, r);
 #pragma unroll
-        for (int e = 0; e < 32; ++e) t32[e] = __uint_as_float(r[e]);
-      }
-      store_split_row(sA + (uint32_t)ch * 8192u, TC_A_TILE, rin, hf, t32);
-      if (!(ok = run_gemm(tY, /*a_mn=*/true, /*b_mn=*/true))) break;         // transmit = Z'^T F
+      for (int e = 0; e < 32; ++e) v[e] = __uint_as_float(r[e]);
+    }
+    store_split_row(sA + (uint32_t)ch * 8192u, TC_A_TILE, rin, hf, v);
+    if (!(ok = run_gemm(tY, /*a_mn=*/true, /*b_mn=*/true))) break;           // transmit = Z'^T F
+    {
+      // into shared memory (the tiles are free again) and out in the row-contiguous mapping, subtracted from the X that this
+      // thread stored above.  Slot (row, 16-byte column c4): row * 256 + (c4 / 8) * 128 + ((c4 % 8) ^ (row % 8)) * 16.
       uint32_t r[32];
       tmem_ld32(tY + hf * 32 + lane_off, r);
       tcgen05_fence_before();
+      const uint32_t ad = sA + (uint32_t)trow * 256u + (uint32_t)hf * 128u;
 #pragma unroll
-      for (int e = 0; e < 32; ++e) t32[e] = __uint_as_float(r[e]);
-    } else {
-#pragma unroll
-      for (int e = 0; e < 32; ++e) t32[e] = 0.f;
-    }
-    // e <- X - transmit: subtracted in place in the shared copy (own slots), written out in the row-contiguous mapping
-#pragma unroll
-    for (int q4 = 0; q4 < 8; ++q4) {
-      float4 x;
-      const uint32_t ad = xaddr + (((uint32_t)q4 ^ xsw) << 4);
-      asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(x.x), "=f"(x.y), "=f"(x.z), "=f"(x.w) : "r"(ad) : "memory");
-      asm volatile("st.shared.v4.f32 [%0], {%1, %2, %3, %4};" ::"r"(ad), "f"(x.x - t32[4 * q4]), "f"(x.y - t32[4 * q4 + 1]),
-                   "f"(x.z - t32[4 * q4 + 2]), "f"(x.w - t32[4 * q4 + 3]) : "memory");
+      for (int q4 = 0; q4 < 8; ++q4)
+        asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(ad + (((uint32_t)q4 ^ (uint32_t)(lane & 7)) << 4)), "r"(r[4 * q4]),
+                     "r"(r[4 * q4 + 1]), "r"(r[4 * q4 + 2]), "r"(r[4 * q4 + 3]) : "memory");
     }
     __syncthreads();
-#pragma unroll
-    for (int i = 0; i < 8; ++i) {
-      const int row = i * 16 + urow, c2 = row >> 6;
-      const long long gb = s_gbase[c2];
+#pragma unroll 1
+    for (int half = 0; half < 2; ++half) {               // half = chunk of the pair
+      const long long gb = s_gbase[half];
       if (gb < 0) continue;
-      float4 x;
-      asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(x.x), "=f"(x.y), "=f"(x.z), "=f"(x.w)
-                   : "r"(sX + (uint32_t)row * 256u + (uint32_t)(uc4 >> 3) * 128u + ((((uint32_t)uc4 & 7u) ^ (uint32_t)(row & 7)) << 4))
-                   : "memory");
-      *reinterpret_cast<float4*>(a.ef + gb + (long long)(row & 63) * s_cols[c2] + uc4 * 4) = x;
+      float4 xr[4];
+#pragma unroll
+      for (int i = 0; i < 4; ++i)
+        xr[i] = *reinterpret_cast<const float4*>(a.ef + gb + (long long)(i * 16 + urow) * s_cols[half] + uc4 * 4);
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const int row = half * 64 + i * 16 + urow;
+        float4 t;
+        asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(t.x), "=f"(t.y), "=f"(t.z), "=f"(t.w)
+                     : "r"(sA + (uint32_t)row * 256u + (uint32_t)(uc4 >> 3) * 128u + ((((uint32_t)uc4 & 7u) ^ (uint32_t)(row & 7)) << 4))
+                     : "memory");
+        *reinterpret_cast<float4*>(a.ef + gb + (long long)(row & 63) * s_cols[half] + uc4 * 4) =
+            make_float4(xr[i].x - t.x, xr[i].y - t.y, xr[i].z - t.z, xr[i].w - t.w);
+      }
     }
   }
   tcgen05_fence_before();
@@ -1368,7 +1377,7 @@ TPLR_API int tplr_compress_chunks_tc(const void* descs, int n_desc, int total_ch
   a.variant = g_tc_variant.load(std::memory_order_relaxed);
   cudaError_t err = cudaFuncSetAttribute(compress_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, TC_SMEM_CMP);
   if (err != cudaSuccess) return (int)err;
-  int grid = tplr_sm_count() * 2;
+  int grid = tplr_sm_count() * 3;
   const int n_pairs = (total_chunks + 1) / 2;
   if (grid > n_pairs) grid = n_pairs;
   compress_tc_kernel<<<grid, NT, TC_SMEM_CMP, (cudaStream_t)stream>>>(a);
