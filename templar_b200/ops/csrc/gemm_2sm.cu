@@ -54,7 +54,8 @@ struct Gemm2Params {
   int m_rot;                         // rotation of the tile-row order (in 256-row tiles)
   int n_rot;                         // rotation of the tile-column order (in 256-column tiles)
   int m_inter;                       // > 1: logical tile row l is row (l % m_inter) * (tiles_m / m_inter) + l / m_inter
-  int k_splits;                      // > 1 (reduce-add epilogues only): a tile's K range is cut into this many work units
+  int k_splits;                      // > 1 (reduce-add epilogues, or with plane_rows): a tile's K range is cut into this many work units
+  int plane_rows;                    // EPI 2: part s of a tile's K range is stored s * plane_rows rows further down
   int tri;                           // 1: C is symmetric (B is A): only tiles on or above the diagonal are computed
   int swiglu_f;                      // > 0 (EPI 3): B is the packed [w1; w3] weight of 2 * swiglu_f rows.  Tile column j pairs
                                      // gate rows [128 j, 128 j + 128) (staged by the even CTA) with up rows swiglu_f + the same
@@ -288,13 +289,13 @@ struct RopeRow {
 // box.  Two staging buffers per warp; `n_boxes` counts the boxes this warp has issued so far.
 template <int EPI>
 __device__ __forceinline__ void epilogue_tma(const Gemm2Params& p, uint32_t tmem_acc, int quad, int lane, int m0, int n0,
-                                             uint32_t stage_base, uint32_t& n_boxes) {
+                                             uint32_t stage_base, uint32_t& n_boxes, int part) {
   constexpr bool BF16_OUT = EPI == 0 || EPI == 4;
   constexpr int COLS = BF16_OUT ? 64 : 32;
   const int row0 = m0 + quad * 32;
   const uint32_t sw = (uint32_t)(lane & 7);
   const CUtensorMap* map = &p.tmC;
-  int y = row0;
+  int y = EPI == 2 ? row0 + part * p.plane_rows : row0;
   if (p.rs_on && row0 < p.M) {                       // the 32 rows of a warp have one owner (32 | every bound)
     int owner = 0;
     while (owner + 1 < p.world && row0 >= p.rs_bound[owner + 1]) ++owner;
@@ -810,7 +811,7 @@ gemm2_kernel(const __grid_constant__ Gemm2Params p) {
           epilogue_rope<128>(p, tmem_acc, quad, lane, m0, n0, sEpi + (uint32_t)quad * 8192u, n_boxes);
         else if (EPI == 4 && p.rope_dh == 64 && p.rope_cols % 64 == 0)
           epilogue_rope<64>(p, tmem_acc, quad, lane, m0, n0, sEpi + (uint32_t)quad * 8192u, n_boxes);
-        else if (p.c_tma)  epilogue_tma<EPI>(p, tmem_acc, quad, lane, m0, n0, sEpi + (uint32_t)quad * 8192u, n_boxes);
+        else if (p.c_tma)  epilogue_tma<EPI>(p, tmem_acc, quad, lane, m0, n0, sEpi + (uint32_t)quad * 8192u, n_boxes, w.t % p.k_splits);
         else               epilogue_direct<EPI>(p, tmem_acc, quad, lane, m0, n0);
         tcgen05_fence_before();
         __syncwarp();
@@ -972,6 +973,48 @@ int pick_scatter_splits(int M, int N, int K) {
   return eff(2 * tiles) > eff(tiles) + 0.10 ? 2 : 1;
 }
 
+// Parts of a product with a bf16 result: for long K on few tiles, where most CTA pairs would idle, each part of K stores an
+// fp32 plane of its own and one kernel adds the planes in order and rounds once (the same bits on every run, which
+// reductions into one plane would not give).  In k block times (a third of a microsecond each): 10 for the second launch and
+// M * N * (8 * parts + 2) bytes for what moves, and the cut has to win 15 %.  One pass against the chosen number of parts:
+// 2048 x 768 x 6144 (24 tiles on 74 pairs) 39 -> 25 us, 777 x 1024 x 32000 (16 tiles) 166 -> 56 us.
+int pick_out_splits(int M, int N, int K) {
+  const int pairs = tplr_sm_count() / 2;
+  const long long tiles = (long long)((M + TILE_M - 1) / TILE_M) * ((N + TILE_N - 1) / TILE_N), kb = (K + BK - 1) / BK;
+  if (2 * tiles > pairs || kb < 64 || (N % 8)) return 1;      // a short K: not worth another launch
+  const double whole = (double)(kb + 8);
+  int best = 1;
+  double best_cost = 0.85 * whole;
+  for (int ks = 2; ks <= 8 && ks <= kb; ++ks) {
+    const long long per = (kb + ks - 1) / ks;
+    if ((ks - 1) * per >= kb) continue;                   // every unit has work
+    const double cost = (double)((tiles * ks + pairs - 1) / pairs) * (double)(per + 8) + 10.0 +
+                        (double)M * N * (8 * ks + 2) / 5e12 / 0.33e-6;
+    if (cost < best_cost) { best = ks; best_cost = cost; }
+  }
+  return best;
+}
+
+// The parts' planes ([parts][plane] fp32, rows of N elements) added in order -> bf16 rows of ldc elements; N, plane and ldc
+// multiples of 8, 16-byte aligned.
+__global__ void __launch_bounds__(256) round_rows_kernel(const float* __restrict__ x, __nv_bfloat16* __restrict__ y, long long M, int n8,
+                                                         long long ldc, int parts, long long plane) {
+  const long long total = M * n8;
+  for (long long i = blockIdx.x * 256LL + threadIdx.x; i < total; i += gridDim.x * 256LL) {
+    float4 a = reinterpret_cast<const float4*>(x)[2 * i], b = reinterpret_cast<const float4*>(x)[2 * i + 1];
+    for (int s = 1; s < parts; ++s) {
+      const float4* q = reinterpret_cast<const float4*>(x + s * plane) + 2 * i;
+      const float4 c = q[0], d = q[1];
+      a.x += c.x; a.y += c.y; a.z += c.z; a.w += c.w;
+      b.x += d.x; b.y += d.y; b.z += d.z; b.w += d.w;
+    }
+    const __nv_bfloat162 h[4] = {__floats2bfloat162_rn(a.x, a.y), __floats2bfloat162_rn(a.z, a.w), __floats2bfloat162_rn(b.x, b.y),
+                                 __floats2bfloat162_rn(b.z, b.w)};
+    const long long row = i / n8;
+    *reinterpret_cast<uint4*>(y + row * ldc + (i - row * n8) * 8) = *reinterpret_cast<const uint4*>(h);
+  }
+}
+
 // Fills the operand maps and the plain fields; returns 0 or a negative argument error.
 int fill_common(Gemm2Params& p, const void* A, const void* B, void* C, int M, int N, int K, long long lda,
                 long long ldb, long long ldc, int a_mn, int b_mn, int epi, unsigned int* status) {
@@ -1037,6 +1080,29 @@ TPLR_API int tplr_gemm2_bf16(const void* A, const void* B, void* C, int M, int N
   if (int r = fill_common(p, A, B, C, M, N, K, lda, ldb, ldc, a_mn, b_mn, epi, status)) return r;
   if (epi == 1 && p.c_tma) p.k_splits = pick_k_splits((long long)((M + TILE_M - 1) / TILE_M) * ((N + TILE_N - 1) / TILE_N), K, max_pairs);
   return dispatch2(p, a_mn, b_mn, epi, 0, max_pairs, (cudaStream_t)stream);
+}
+
+// Parts that tplr_gemm2_bf16_split would cut K into for a bf16 result of this size; 1: no workspace, call tplr_gemm2_bf16.
+TPLR_API int tplr_gemm2_out_splits(int M, int N, int K) { return pick_out_splits(M, N, K); }
+
+// tplr_gemm2_bf16 with a bf16 result (epi 0) through an fp32 workspace `ws` of parts * (M rounded up to 32) * N elements
+// (16-byte aligned, contents irrelevant); C 16-byte aligned with ldc a multiple of 8, N a multiple of 8.
+TPLR_API int tplr_gemm2_bf16_split(const void* A, const void* B, void* C, float* ws, int M, int N, int K, long long lda,
+                                   long long ldb, long long ldc, int a_mn, int b_mn, unsigned int* status, void* stream) {
+  TPLR_ENTER();
+  if (M <= 0 || N <= 0 || K <= 0) return 0;
+  if ((N % 8) || (ldc % 8) || (((uintptr_t)C | (uintptr_t)ws) & 15)) return -101;
+  Gemm2Params p = {};
+  if (int r = fill_common(p, A, B, ws, M, N, K, lda, ldb, N, a_mn, b_mn, 2, status)) return r;
+  p.k_splits = pick_out_splits(M, N, K);
+  p.plane_rows = (M + 31) / 32 * 32;                    // a warp's box of 32 rows stays inside its plane
+  if (!make_map(&p.tmC, ws, N, (long long)p.k_splits * p.plane_rows, N, 32, 32, CU_TENSOR_MAP_SWIZZLE_128B, true)) return -110;
+  if (int r = dispatch2(p, a_mn, b_mn, 2, 0, 0, (cudaStream_t)stream)) return r;
+  const long long n = (long long)M * (N / 8);
+  const unsigned grid = (unsigned)((n + 255) / 256 < 8LL * tplr_sm_count() ? (n + 255) / 256 : 8LL * tplr_sm_count());
+  round_rows_kernel<<<grid, 256, 0, (cudaStream_t)stream>>>(ws, (__nv_bfloat16*)C, M, N / 8, ldc, p.k_splits,
+                                                            (long long)p.plane_rows * N);
+  return (int)cudaGetLastError();
 }
 
 // GU[M, 2F] = X W^T for the packed weight W = [w1; w3] ([2F, K] bf16, K-major) and H[M, F] = silu(GU[:, :F]) * GU[:, F:]

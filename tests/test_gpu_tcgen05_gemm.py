@@ -238,3 +238,22 @@ def test_feed_forward_without_grad_gives_the_same_output(T, D, F, backend):
     with torch.no_grad():
         assert torch.equal(OF.feed_forward(x, w13, w2), want)
     assert int(OF.status_word(DEV).item()) == 0
+
+
+@pytest.mark.parametrize("M,N,K,b_mn", [(256, 256, 4096, False), (777, 264, 6152, True), (8, 8, 8192, False), (300, 1024, 5000, True)])
+def test_bf16_gemm_through_split_workspace(M, N, K, b_mn, backend):
+    """Few tiles and a long K: partial products summed in fp32 and rounded once; ragged tiles, a ragged last split, a
+    result that is a view with a leading dimension of its own, and the same bits on a second run."""
+    from templar_b200.ops import native
+
+    if backend == "tcgen05_2sm":
+        assert native.lib().tplr_gemm2_out_splits(M, N, K) > 1
+    _check(M, N, K, False, b_mn, "bf16")
+    A = (torch.randn(M, K, device=DEV) / K ** 0.5).to(torch.bfloat16)
+    B = torch.randn((K, N) if b_mn else (N, K), device=DEV).to(torch.bfloat16)
+    wide = torch.full((M, N + 16), 7.0, device=DEV, dtype=torch.bfloat16)
+    OF.gemm(A, B, b_mn=b_mn, out=wide[:, 8:-8])
+    ref = A.float() @ (B if b_mn else B.t()).float()
+    assert torch.allclose(wide[:, 8:-8].float(), ref, rtol=2 ** -8, atol=1e-3)        # one rounding; fp32 sums of K products
+    assert (wide[:, :8] == 7).all() and (wide[:, -8:] == 7).all()
+    assert torch.equal(OF.gemm(A, B, b_mn=b_mn), wide[:, 8:-8])
