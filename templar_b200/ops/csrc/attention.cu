@@ -1275,16 +1275,18 @@ int launch_bwd(const void* qkv, const void* out, const void* dout, const float* 
 }
 }  // namespace
 
-// CTAs that share a group's query heads.  One CTA per (key block, kv head, sequence) leaves SMs idle where heads are
-// grouped and the batch is small; each part then adds its dK and dV into the fp32 buffer, which costs a pass over 2 KV
-// heads more, so the group is only cut until there are two CTAs per SM.  B 1, S 1024, H 32, KV 8, head_dim 128: 155 us whole
-// (64 CTAs), 49 us in four parts (256 CTAs).
+// CTAs that share a group's query heads.  One CTA per (key block, kv head, sequence), one CTA per SM: with few of them the
+// longest walk (key block 0 over all n query blocks) takes longer than an even share of the work, (n + 1) / 2 blocks a CTA on
+// average, does.  A cut shortens the walk, but each part adds its dK and dV into the fp32 buffer, a pass over 2 KV heads
+// more, so the group is only cut until the walk is within a tenth of the even share.  32 query heads on 8 of 128: B 1, S 1024
+// 155 us whole (64 CTAs), 49 us in four parts (256 CTAs); B 6, S 640 (240 CTAs) 103 us whole, 113 us in two parts
+// and 14 us more for the buffer; B 4, S 1024 (256 CTAs) 151 us whole, 163 and 15 us more in two.
 static int bwd_split(int B, int S, int H, int KV, int head_dim) {
   if (KV <= 0 || H % KV || (head_dim == 128 && S % 128 == 0 && g_bwd_variant == 2)) return 1;
   const int group = H / KV;
-  const long long ctas = (long long)((S + BKV - 1) / BKV) * KV * B;
+  const long long n = (S + BKV - 1) / BKV, ctas = n * KV * B;
   int split = 1;
-  for (int s = 1; s <= group && ctas * split < 2LL * tplr_sm_count(); ++s)
+  for (int s = 1; s <= group && 10 * ctas * split * (n + 1) < 18 * n * tplr_sm_count(); ++s)
     if (group % s == 0) split = s;
   return split;
 }
