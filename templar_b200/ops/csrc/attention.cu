@@ -850,25 +850,35 @@ __global__ void __launch_bounds__(256) attn_delta_kernel(const __nv_bfloat16* __
   if (lane == 0 && live) delta[((tok / S) * H + h) * S + tok % S] = s;
 }
 
-// dq32 [tokens, width] fp32 -> first `width` columns (heads of dh) of the packed bf16 gradient
-// cosb / sinb not null: the two pairs are rotated back, in the first rot_cols columns, by the angles of (token % S, pair index in the head) on the way
+// dq32 [tokens, width] fp32 -> first `width` columns (heads of HD) of the packed bf16 gradient, eight values a thread
+// cosb / sinb not null: the pairs are rotated back, in the first rot_cols columns, by the angles of (token % S, pair index in the
+// head) on the way.  A pass over memory (4 bytes in and 2 out a value): one 32-bit division for eight values, because with
+// four values, 64-bit divisions and a head size of run time it was bound by them (5120 x 4096: 31 us, 19 us here).
+template <int HD>
 __global__ void __launch_bounds__(256) attn_dq_cast_kernel(const float* __restrict__ dq32, __nv_bfloat16* __restrict__ dqkv,
-                                                           long long tokens, int width, int rot_cols, int dh, long long ld,
+                                                           long long tokens, int width, int rot_cols, long long ld,
                                                            const float* __restrict__ cosb, const float* __restrict__ sinb, int S) {
-  const long long n4 = tokens * (width / 4);
-  for (long long v = (long long)blockIdx.x * blockDim.x + threadIdx.x; v < n4; v += (long long)gridDim.x * blockDim.x) {
-    const long long tok = v / (width / 4);
-    const int c4 = (int)(v % (width / 4));
-    float4 f = reinterpret_cast<const float4*>(dq32)[v];
-    if (cosb && c4 * 4 < rot_cols) {
-      const long long tb = (tok % S) * (dh / 2) + ((c4 * 4) % dh) / 2;
-      const float2 c = *reinterpret_cast<const float2*>(cosb + tb), sn = *reinterpret_cast<const float2*>(sinb + tb);
-      f = make_float4(f.x * c.x + f.y * sn.x, f.y * c.x - f.x * sn.x, f.z * c.y + f.w * sn.y, f.w * c.y - f.z * sn.y);
+  const unsigned w8 = (unsigned)width / 8;
+  const long long n8 = tokens * w8;                     // below 2^32: the scratch would be 137 GB there
+  for (long long v = (long long)blockIdx.x * blockDim.x + threadIdx.x; v < n8; v += (long long)gridDim.x * blockDim.x) {
+    const unsigned tok = (unsigned)v / w8, col = ((unsigned)v - tok * w8) * 8u;
+    const float4 f0 = reinterpret_cast<const float4*>(dq32)[2 * v], f1 = reinterpret_cast<const float4*>(dq32)[2 * v + 1];
+    float f[8] = {f0.x, f0.y, f0.z, f0.w, f1.x, f1.y, f1.z, f1.w};
+    if (cosb && (int)col < rot_cols) {
+      const long long tb = (long long)(tok % (unsigned)S) * (HD / 2) + (col % HD) / 2;
+      const float2 c0 = *reinterpret_cast<const float2*>(cosb + tb), c1 = *reinterpret_cast<const float2*>(cosb + tb + 2);
+      const float2 s0 = *reinterpret_cast<const float2*>(sinb + tb), s1 = *reinterpret_cast<const float2*>(sinb + tb + 2);
+      const float c[4] = {c0.x, c0.y, c1.x, c1.y}, s[4] = {s0.x, s0.y, s1.x, s1.y};
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        const float x = f[2 * e], y = f[2 * e + 1];
+        f[2 * e] = x * c[e] + y * s[e];
+        f[2 * e + 1] = y * c[e] - x * s[e];
+      }
     }
-    __nv_bfloat162 lo = __floats2bfloat162_rn(f.x, f.y), hi = __floats2bfloat162_rn(f.z, f.w);
-    uint2 o;
-    o.x = *reinterpret_cast<uint32_t*>(&lo); o.y = *reinterpret_cast<uint32_t*>(&hi);
-    *reinterpret_cast<uint2*>(dqkv + tok * ld + c4 * 4) = o;
+    const __nv_bfloat162 h[4] = {__floats2bfloat162_rn(f[0], f[1]), __floats2bfloat162_rn(f[2], f[3]), __floats2bfloat162_rn(f[4], f[5]),
+                                 __floats2bfloat162_rn(f[6], f[7])};
+    *reinterpret_cast<uint4*>(dqkv + (long long)tok * ld + col) = *reinterpret_cast<const uint4*>(h);
   }
 }
 
@@ -1270,7 +1280,7 @@ int launch_bwd(const void* qkv, const void* out, const void* dout, const float* 
   cudaError_t e = cudaFuncSetAttribute(attn_bwd_kernel<HD>, cudaFuncAttributeMaxDynamicSharedMemorySize, bwd_smem<HD>());
   if (e != cudaSuccess) return (int)e;
   attn_bwd_kernel<HD><<<(unsigned)(((S + BKV - 1) / BKV) * KV * B * p.split), BWD_THREADS, bwd_smem<HD>(), st>>>(p);
-  attn_dq_cast_kernel<<<tplr_sm_count() * 8, 256, 0, st>>>(dq32, (__nv_bfloat16*)dqkv, tokens, width, (H + KV) * HD, HD, ld_qkv, cosb, sinb, S);
+  attn_dq_cast_kernel<HD><<<tplr_sm_count() * 8, 256, 0, st>>>(dq32, (__nv_bfloat16*)dqkv, tokens, width, (H + KV) * HD, ld_qkv, cosb, sinb, S);
   return (int)cudaGetLastError();
 }
 }  // namespace
