@@ -41,8 +41,9 @@ class _SymmetricChain:
 
     Lines 1 and 2 compute only the 256 x 256 tiles on or above the diagonal of their symmetric results
     (``tplr_gemm2_syrk``: half the tensor-core work) and ``tplr_sym_axpby`` mirrors the triangle while it applies
-    the line's scalars.  Where those tiles are too few for the chip, K is split and the triangle accumulates in fp32
-    (``tplr_gemm2_syrk_acc``; ``tplr_sym_axpby_acc`` leaves it zeroed for the next product).  Line 3, ``a X + B X``, is
+    the line's scalars.  Where those tiles are too few for the chip, K is cut in two and the triangle accumulates in fp32
+    (``tplr_gemm2_syrk_acc``; ``tplr_sym_axpby_acc`` leaves it zeroed for the next product); the result is the same bits on
+    every call and rank, which replicas that orthogonalise for themselves rely on.  Line 3, ``a X + B X``, is
     one product ``(B + a I) X``: the mirror kernel of line 2 adds ``a`` on the diagonal, so no element-wise pass over X
     remains."""
 

@@ -711,7 +711,7 @@ __global__ void __launch_bounds__(256) sym_axpby_kernel(const bf16* __restrict__
     out[(long long)i * ldo + j] = __float2bfloat16(v);
   }
 }
-// The same from an fp32 U whose products were accumulated by several CTA pairs per tile (tplr_gemm2_syrk_acc), which wants
+// The same from an fp32 U whose products were accumulated by two CTA pairs per tile (tplr_gemm2_syrk_acc), which wants
 // zeros to add into: every tile is set back to zero as it is read.  M a multiple of 8, dense matrices, 16-byte aligned.  One
 // CTA per 64 x 64 tile; those below the diagonal only clear what the product wrote there (the 256-wide diagonal tiles).
 __global__ void __launch_bounds__(256) sym_axpby_acc_kernel(float* __restrict__ U, int M, float alpha, const bf16* __restrict__ aux,

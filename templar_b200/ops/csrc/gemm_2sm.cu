@@ -944,15 +944,15 @@ int dispatch2(Gemm2Params& p, int a_mn, int b_mn, int epi, int n_comm_pairs, int
 // Measured, one split against the chosen number: 768 x 768 x 8192 (9 tiles on 74 pairs) 54.8 -> 21.0 us with 4, 2304 x 768 x
 // 8192 55.4 -> 33.1 with 2, 1536 x 4096 x 4096 62.6 -> 51.5 with 2; where the waves are full already a second split costs
 // 3 to 16 % (8192 x 1536 x 4096 88.3 -> 94.2, 28672 x 4096 x 1024 287 -> 333) and none is made.  A split has to win 5 %.
-int pick_k_splits(long long tiles, int K, int max_pairs) {
+int pick_k_splits(long long tiles, int K, int max_pairs, int most = 8) {
   static const int forced = [] { const char* e = getenv("TPLR_GEMM_KSPLITS"); return e ? atoi(e) : 0; }();
   const long long kb = (K + BK - 1) / BK;
-  if (forced > 0) return kb / forced >= 1 ? forced : 1;   // tuning override
+  if (forced > 0 && forced <= most) return kb / forced >= 1 ? forced : 1;   // tuning override
   int pairs = tplr_sm_count() / 2;
   if (max_pairs > 0 && pairs > max_pairs) pairs = max_pairs;
   int best = 1;
   double best_cost = 0.0;
-  for (int ks = 1; ks <= 8 && ks <= kb; ks *= 2) {
+  for (int ks = 1; ks <= most && ks <= kb; ks *= 2) {
     const long long per = (kb + ks - 1) / ks;
     if ((ks - 1) * per >= kb) break;                      // every unit has work
     const double cost = (double)((tiles * ks + pairs - 1) / pairs) * (double)(per + 8);
@@ -1052,10 +1052,12 @@ static long long syrk_tiles(int M) {
   const long long t = (M + TILE_M - 1) / TILE_M;
   return t * (t + 1) / 2;
 }
-// K splits that tplr_gemm2_syrk_acc makes for this size (1: tplr_gemm2_syrk is the better call).
-TPLR_API int tplr_gemm2_syrk_splits(int M, int K) { return pick_k_splits(syrk_tiles(M), K, 0); }
+// K splits that tplr_gemm2_syrk_acc makes for this size (1: tplr_gemm2_syrk is the better call).  Two at most: replicas
+// orthogonalise the same matrix each for itself, so the result must not depend on the order in which the parts arrive, and
+// two parts added into zeros give the same sum in either order.
+TPLR_API int tplr_gemm2_syrk_splits(int M, int K) { return pick_k_splits(syrk_tiles(M), K, 0, 2); }
 
-// tplr_gemm2_syrk adding into an fp32 C (ldc a multiple of 4, zeroed by the caller) with K cut into several work units per
+// tplr_gemm2_syrk adding into an fp32 C (ldc a multiple of 4, zeroed by the caller) with K cut into two work units per
 // tile: the triangle of a small matrix has fewer tiles than the chip has CTA pairs.  2048 x 8192 (36 tiles on 74 pairs):
 // 49 us in one pass; an iteration's two products (K = 8192 and 2048) 64 us in one pass each, 44 us split.
 TPLR_API int tplr_gemm2_syrk_acc(const void* A, float* C, int M, int K, long long lda, long long ldc, unsigned int* status,
@@ -1066,7 +1068,7 @@ TPLR_API int tplr_gemm2_syrk_acc(const void* A, float* C, int M, int K, long lon
   Gemm2Params p = {};
   if (int r = fill_common(p, A, A, C, M, M, K, lda, lda, ldc, 0, 0, 1, status)) return r;
   p.tri = 1;
-  p.k_splits = pick_k_splits(syrk_tiles(M), K, 0);
+  p.k_splits = tplr_gemm2_syrk_splits(M, K);
   return dispatch2(p, 0, 0, 1, 0, 0, (cudaStream_t)stream);
 }
 

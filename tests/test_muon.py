@@ -289,3 +289,15 @@ def test_chain_operand_matches_eager(shape, dtype):
                                               scratch.data_ptr(), got.data_ptr(), native.stream_ptr()), "ns_prepare")
     # the norm is summed in another order: at most one bf16 step of the divisor, 2^-8 relative
     assert torch.allclose(got.float(), want.float(), rtol=2 ** -7, atol=0)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("shape", [(512, 512), (768, 768), (3072, 768), (1024, 2816)])
+def test_newton_schulz_repeats_its_bits(shape):
+    """Replicas orthogonalise the same gradient each for itself and ranks apply slices of one result: equal bits on every
+    call, also where the triangle has few tiles and K is cut into parts."""
+    torch.manual_seed(shape[1])
+    G = torch.randn(*shape, device="cuda") * 1e-3
+    first = newton_schulz(G)
+    for _ in range(30):
+        assert torch.equal(newton_schulz(G), first)
