@@ -460,12 +460,13 @@ constexpr int BWD_THREADS = 320;                        // TMA warp, MMA warp, 8
 struct AttnBwdParams {
   CUtensorMap tmQKV;    // [B, S, C] bf16, box 64 x 128 x 1
   CUtensorMap tmDO;     // [B, S, H*DH] bf16, box 64 x 128 x 1
-  CUtensorMap tmDQ;     // [B, S, H*DH] (split: all C columns) fp32, box 32 x 32 x 1 (reduce-add target)
+  CUtensorMap tmDQ;     // [B, S, H*DH] fp32, box 32 x 32 x 1 (reduce-add target)
+  CUtensorMap tmPart;   // split: [B, S, split*2*KV*DH] fp32, box 32 x 32 x 1 (dK | dV of every part)
   CUtensorMap tmDQKV;   // [B, S, C] bf16, box 64 x 32 x 1 (dK and dV stores)
   const float* lse;
   const float* delta;
   int B, S, H, KV;
-  int split;            // CTAs that share a group's query heads; > 1: dK and dV are reduce-added into the fp32 buffer too
+  int split;            // CTAs that share a group's query heads; > 1: each stores its part of dK and dV in fp32
   float scale, scale_log2;
   unsigned int* status;
   // not null: q and k were rotated (rotary embedding, interleaved pairs, tables [S, DH / 2] fp32) by the producer of qkv and
@@ -736,7 +737,7 @@ attn_bwd_kernel(const __grid_constant__ AttnBwdParams p) {
       }
     }
     // dV and dK of this kv block.  Whole group in this CTA: TMEM -> bf16 -> staging -> TMA store into the packed gradient;
-    // a part of it: reduce-added in fp32 beside dQ, and rotated back and rounded by the pass that does so for dQ.
+    // a part of it: stored in fp32 in columns of its own; the pass that rotates dQ back and rounds it adds the parts in order.
     if (ok) {
       tcgen05_fence_after();
       const int orow0 = kvrow0 + quad * 32;
@@ -760,7 +761,7 @@ attn_bwd_kernel(const __grid_constant__ AttnBwdParams p) {
           asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
           __syncwarp();
           if (lane == 0) {
-            if (orow0 < p.S) tma_reduce_add_3d(&p.tmDQ, buf, (acc ? kcol : vcol) + col, orow0, b);
+            if (orow0 < p.S) tma_store_3d(&p.tmPart, buf, (sub * 2 * p.KV + (acc ? g : p.KV + g)) * DH + col, orow0, b);
             asm volatile("cp.async.bulk.commit_group;" ::: "memory");
           }
         }
@@ -850,20 +851,33 @@ __global__ void __launch_bounds__(256) attn_delta_kernel(const __nv_bfloat16* __
   if (lane == 0 && live) delta[((tok / S) * H + h) * S + tok % S] = s;
 }
 
-// dq32 [tokens, width] fp32 -> first `width` columns (heads of HD) of the packed bf16 gradient, eight values a thread
+// dq32 [tokens, q_cols] fp32 -> first q_cols columns (heads of HD) of the packed bf16 gradient, eight values a thread; PARTS: the
+// next kv_cols columns (dK | dV of a split walk) are the sums, in order, of `split` parts in part [tokens, split, kv_cols].
 // cosb / sinb not null: the pairs are rotated back, in the first rot_cols columns, by the angles of (token % S, pair index in the
 // head) on the way.  A pass over memory (4 bytes in and 2 out a value): one 32-bit division for eight values, because with
 // four values, 64-bit divisions and a head size of run time it was bound by them (5120 x 4096: 31 us, 19 us here).
-template <int HD>
-__global__ void __launch_bounds__(256) attn_dq_cast_kernel(const float* __restrict__ dq32, __nv_bfloat16* __restrict__ dqkv,
-                                                           long long tokens, int width, int rot_cols, long long ld,
-                                                           const float* __restrict__ cosb, const float* __restrict__ sinb, int S) {
-  const unsigned w8 = (unsigned)width / 8;
+template <int HD, bool PARTS>
+__global__ void __launch_bounds__(256) attn_dq_cast_kernel(const float* __restrict__ dq32, const float* __restrict__ part, int split,
+                                                           __nv_bfloat16* __restrict__ dqkv, long long tokens, int q_cols, int kv_cols,
+                                                           int rot_cols, long long ld, const float* __restrict__ cosb,
+                                                           const float* __restrict__ sinb, int S) {
+  const unsigned w8 = (unsigned)(PARTS ? q_cols + kv_cols : q_cols) / 8;
   const long long n8 = tokens * w8;                     // below 2^32: the scratch would be 137 GB there
   for (long long v = (long long)blockIdx.x * blockDim.x + threadIdx.x; v < n8; v += (long long)gridDim.x * blockDim.x) {
     const unsigned tok = (unsigned)v / w8, col = ((unsigned)v - tok * w8) * 8u;
-    const float4 f0 = reinterpret_cast<const float4*>(dq32)[2 * v], f1 = reinterpret_cast<const float4*>(dq32)[2 * v + 1];
+    const bool summed = PARTS && (int)col >= q_cols;
+    const float* src = dq32 + 8 * v;                    // without parts the rows lie one behind the other
+    if (PARTS) src = summed ? part + (long long)tok * split * kv_cols + (col - q_cols) : dq32 + (long long)tok * q_cols + col;
+    const float4 f0 = reinterpret_cast<const float4*>(src)[0], f1 = reinterpret_cast<const float4*>(src)[1];
     float f[8] = {f0.x, f0.y, f0.z, f0.w, f1.x, f1.y, f1.z, f1.w};
+    if (summed) {
+      for (int s = 1; s < split; ++s) {
+        const float4* more = reinterpret_cast<const float4*>(src + (long long)s * kv_cols);
+        const float4 g0 = more[0], g1 = more[1];
+        f[0] += g0.x; f[1] += g0.y; f[2] += g0.z; f[3] += g0.w;
+        f[4] += g1.x; f[5] += g1.y; f[6] += g1.z; f[7] += g1.w;
+      }
+    }
     if (cosb && (int)col < rot_cols) {
       const long long tb = (long long)(tok % (unsigned)S) * (HD / 2) + (col % HD) / 2;
       const float2 c0 = *reinterpret_cast<const float2*>(cosb + tb), c1 = *reinterpret_cast<const float2*>(cosb + tb + 2);
@@ -1231,7 +1245,8 @@ TPLR_API int tplr_attention_set_bwd_variant(int v) {
 
 // Gradient of tplr_attention_fwd.  qkv / dqkv: packed [B*S, C] bf16 with row stride ld_qkv; out: the forward's
 // output (row stride ld_o); dout: contiguous [B*S, H*head_dim]; lse from the forward; delta: [B,H,S] fp32 scratch;
-// dq32: [B*S, tplr_attention_bwd_scratch_cols] fp32 scratch that the caller has zeroed.  dqkv receives dq | dk | dv.
+// dq32: B*S*tplr_attention_bwd_scratch_cols fp32 elements of scratch, of which the caller has zeroed the first
+// B*S*H*head_dim.  dqkv receives dq | dk | dv.
 extern "C" int tplr_rope(void* buf, const float* cosb, const float* sinb, long long tokens, int S, int n_heads, int Dh,
                          long long row_stride, int inverse, void* stream);
 
@@ -1271,8 +1286,10 @@ int launch_bwd(const void* qkv, const void* out, const void* dout, const float* 
   if (!make_map3(&p.tmQKV, qkv, C, S, B, ld_qkv, 64, 128)) return -202;
   if (!make_map3(&p.tmDO, dout, (long long)H * HD, S, B, (long long)H * HD, 64, 128)) return -203;
   p.split = bwd_split(B, S, H, KV, HD);
-  const int width = p.split > 1 ? C : H * HD;                  // what goes through the fp32 scratch
-  if (!make_map3(&p.tmDQ, dq32, width, S, B, width, 32, 32, true)) return -204;
+  float* part = dq32 + tokens * H * HD;                        // the parts of dK and dV lie behind dQ
+  const int kv_cols = p.split > 1 ? 2 * KV * HD : 0;
+  if (!make_map3(&p.tmDQ, dq32, (long long)H * HD, S, B, (long long)H * HD, 32, 32, true)) return -204;
+  if (kv_cols && !make_map3(&p.tmPart, part, (long long)p.split * kv_cols, S, B, (long long)p.split * kv_cols, 32, 32, true)) return -204;
   if (!make_map3(&p.tmDQKV, dqkv, C, S, B, ld_qkv, 64, 32)) return -205;
   p.lse = lse; p.delta = delta; p.B = B; p.S = S; p.H = H; p.KV = KV;
   p.scale = scale; p.scale_log2 = scale * 1.4426950408889634f; p.status = status;
@@ -1280,17 +1297,19 @@ int launch_bwd(const void* qkv, const void* out, const void* dout, const float* 
   cudaError_t e = cudaFuncSetAttribute(attn_bwd_kernel<HD>, cudaFuncAttributeMaxDynamicSharedMemorySize, bwd_smem<HD>());
   if (e != cudaSuccess) return (int)e;
   attn_bwd_kernel<HD><<<(unsigned)(((S + BKV - 1) / BKV) * KV * B * p.split), BWD_THREADS, bwd_smem<HD>(), st>>>(p);
-  attn_dq_cast_kernel<HD><<<tplr_sm_count() * 8, 256, 0, st>>>(dq32, (__nv_bfloat16*)dqkv, tokens, width, (H + KV) * HD, ld_qkv, cosb, sinb, S);
+  auto cast = kv_cols ? attn_dq_cast_kernel<HD, true> : attn_dq_cast_kernel<HD, false>;
+  cast<<<tplr_sm_count() * 8, 256, 0, st>>>(dq32, part, p.split, (__nv_bfloat16*)dqkv, tokens, H * HD, kv_cols, (H + KV) * HD, ld_qkv,
+                                            cosb, sinb, S);
   return (int)cudaGetLastError();
 }
 }  // namespace
 
 // CTAs that share a group's query heads.  One CTA per (key block, kv head, sequence), one CTA per SM: with few of them the
 // longest walk (key block 0 over all n query blocks) takes longer than an even share of the work, (n + 1) / 2 blocks a CTA on
-// average, does.  A cut shortens the walk, but each part adds its dK and dV into the fp32 buffer, a pass over 2 KV heads
-// more, so the group is only cut until the walk is within a tenth of the even share.  32 query heads on 8 of 128: B 1, S 1024
-// 155 us whole (64 CTAs), 49 us in four parts (256 CTAs); B 6, S 640 (240 CTAs) 103 us whole, 113 us in two parts
-// and 14 us more for the buffer; B 4, S 1024 (256 CTAs) 151 us whole, 163 and 15 us more in two.
+// average, does.  A cut shortens the walk, but each part stores its dK and dV in fp32, a pass over 2 KV heads more, so the
+// group is only cut until the walk is within a tenth of the even share.  32 query heads on 8 of 128: B 1, S 1024 155 us whole
+// (64 CTAs), 46 us in four parts (256 CTAs; the pass that adds them 2 us more); B 6, S 640 (240 CTAs) 103 us whole, 113 us in
+// two parts; B 4, S 1024 (256 CTAs) 151 us whole, 163 us in two.
 static int bwd_split(int B, int S, int H, int KV, int head_dim) {
   if (KV <= 0 || H % KV || (head_dim == 128 && S % 128 == 0 && g_bwd_variant == 2)) return 1;
   const int group = H / KV;
@@ -1301,9 +1320,11 @@ static int bwd_split(int B, int S, int H, int KV, int head_dim) {
   return split;
 }
 
-// Columns of the fp32 scratch that the backward needs for these sizes: [B*S, columns], zeroed by the caller.
+// Fp32 elements per token of the scratch that the backward needs for these sizes: the first B*S*H*head_dim hold dQ (zeroed by
+// the caller), what is beyond them the parts of dK and dV.
 TPLR_API int tplr_attention_bwd_scratch_cols(int B, int S, int H, int KV, int head_dim) {
-  return (bwd_split(B, S, H, KV, head_dim) > 1 ? H + 2 * KV : H) * head_dim;
+  const int split = bwd_split(B, S, H, KV, head_dim);
+  return (H + (split > 1 ? 2 * KV * split : 0)) * head_dim;
 }
 
 static int attention_bwd_impl(const void* qkv, const void* out, const void* dout, const float* lse, float* delta,

@@ -273,8 +273,8 @@ struct AttentionBlock : Function<AttentionBlock> {
     Tensor dwo = weight_grad(aside(ctx, "buffer_o"), dy2, out2, wo, ctx->needs_input_grad(2), status);
     Tensor dqkv = at::empty_like(qkv);
     {
-      Tensor scratch = at::zeros({B, S, E.bwd_scratch_cols((int)B, (int)S, (int)heads, (int)kv, (int)hd)},
-                                 qkv.options().dtype(at::kFloat));
+      Tensor scratch = f32({T * E.bwd_scratch_cols((int)B, (int)S, (int)heads, (int)kv, (int)hd)}, qkv);
+      scratch.narrow(0, 0, T * N).zero_();                   // dQ accumulates; the parts behind it are written whole
       check(E.attention_bwd(qkv.data_ptr(), out.data_ptr(), dO.data_ptr(), lse.data_ptr<float>(), delta.data_ptr<float>(),
                             scratch.data_ptr<float>(), dqkv.data_ptr(), (int)B, (int)S, (int)heads, (int)kv, (int)hd, C, N,
                             (float)std::pow((double)hd, -0.5), cos.data_ptr<float>(), sin.data_ptr<float>(), word(status), stream()),

@@ -765,9 +765,12 @@ def _split_qkv(qkv, n_heads, n_kv, hd):
 
 
 def _attention_scratch(B, S, n_heads, n_kv, hd, device):
-    """Zeroed fp32 buffer that the attention backward accumulates dq (and dk, dv where heads are split) into."""
+    """fp32 buffer of the attention backward: zeros that dq accumulates into, then the parts of dk and dv where the query
+    heads of a group are split (written whole)."""
     cols = native.lib().tplr_attention_bwd_scratch_cols(B, S, n_heads, n_kv, hd)
-    return torch.zeros(B, S, cols, dtype=torch.float32, device=device)
+    buf = torch.empty(B * S * cols, dtype=torch.float32, device=device)
+    buf[:B * S * n_heads * hd].zero_()
+    return buf
 
 
 class _AttentionPacked(torch.autograd.Function):

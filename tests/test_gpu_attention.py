@@ -233,3 +233,18 @@ def test_attention_head_dim_64_and_ragged_sequences(B, S, H, KV, hd):
     assert int(OF.status_word(DEV).item()) == 0
     for got, want in [(y, yr)] + [(a.grad, f.grad) for a, f in zip(xs, fs)]:
         assert ((got.float() - want).norm() / want.norm()).item() < 2e-2      # five roundings to bf16 on the way, 2^-9 each
+
+
+@pytest.mark.parametrize("B,S,H,KV,hd", [(1, 1024, 32, 8, 128), (1, 300, 8, 1, 64), (2, 520, 12, 2, 128)])
+def test_key_and_value_gradients_repeat_their_bits(B, S, H, KV, hd):
+    """Few key blocks: the query heads of a group are shared by several CTAs, whose parts of dK and dV are added in order.
+    (dQ is a sum over key blocks in order of arrival, as it is without the cut.)"""
+    from templar_b200.ops import native
+
+    assert native.lib().tplr_attention_bwd_scratch_cols(B, S, H, KV, hd) > H * hd
+    torch.manual_seed(S)
+    qkv = torch.randn(B, S, (H + 2 * KV) * hd, device=DEV).to(torch.bfloat16).requires_grad_()
+    dout = torch.randn(B, S, H * hd, device=DEV).to(torch.bfloat16)
+    grads = [torch.autograd.grad(OF.attention_packed(qkv, H, KV, hd), qkv, dout)[0][..., H * hd:] for _ in range(30)]
+    for g in grads[1:]:
+        assert torch.equal(g, grads[0])
