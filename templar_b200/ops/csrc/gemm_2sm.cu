@@ -55,7 +55,8 @@ struct Gemm2Params {
   int n_rot;                         // rotation of the tile-column order (in 256-column tiles)
   int m_inter;                       // > 1: logical tile row l is row (l % m_inter) * (tiles_m / m_inter) + l / m_inter
   int k_splits;                      // > 1 (reduce-add epilogues, or with plane_rows): a tile's K range is cut into this many work units
-  int plane_rows;                    // EPI 2: part s of a tile's K range is stored s * plane_rows rows further down
+  int plane_rows;                    // > 0: the parts of a tile's K range go to planes of plane_rows rows, part s to plane s of tmC
+                                     // (EPI 2), or part 0 into tmC and part s to plane s - 1 of tmCr[0] (EPI 1)
   int tri;                           // 1: C is symmetric (B is A): only tiles on or above the diagonal are computed
   int swiglu_f;                      // > 0 (EPI 3): B is the packed [w1; w3] weight of 2 * swiglu_f rows.  Tile column j pairs
                                      // gate rows [128 j, 128 j + 128) (staged by the even CTA) with up rows swiglu_f + the same
@@ -296,6 +297,8 @@ __device__ __forceinline__ void epilogue_tma(const Gemm2Params& p, uint32_t tmem
   const uint32_t sw = (uint32_t)(lane & 7);
   const CUtensorMap* map = &p.tmC;
   int y = EPI == 2 ? row0 + part * p.plane_rows : row0;
+  const bool plane = EPI == 1 && p.plane_rows > 0 && part > 0;
+  if (plane) { map = &p.tmCr[0]; y = row0 + (part - 1) * p.plane_rows; }
   if (p.rs_on && row0 < p.M) {                       // the 32 rows of a warp have one owner (32 | every bound)
     int owner = 0;
     while (owner + 1 < p.world && row0 >= p.rs_bound[owner + 1]) ++owner;
@@ -359,7 +362,7 @@ __device__ __forceinline__ void epilogue_tma(const Gemm2Params& p, uint32_t tmem
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     __syncwarp();
     if (lane == 0) {
-      if (EPI == 1 || p.rs_on) tma_reduce_add_2d(map, buf, col0, y);
+      if ((EPI == 1 && !plane) || p.rs_on) tma_reduce_add_2d(map, buf, col0, y);
       else                     tma_store_2d(map, buf, col0, y);
       bulk_commit();
     }
@@ -938,34 +941,52 @@ int dispatch2(Gemm2Params& p, int a_mn, int b_mn, int epi, int n_comm_pairs, int
   return -104;
 }
 
-// Accumulating GEMMs (C += ...) reduce-add their tiles, so a tile's K range may be cut into several work units that run
-// on different CTA pairs: the one with the fewest "k block times" wins, counting waves of units and 8 k blocks per unit for
-// its pipeline fill and its reduction (fitted on 22 weight-gradient shapes from 768 x 768 to 28672 x 4096, K 333 to 16384).
-// Measured, one split against the chosen number: 768 x 768 x 8192 (9 tiles on 74 pairs) 54.8 -> 21.0 us with 4, 2304 x 768 x
-// 8192 55.4 -> 33.1 with 2, 1536 x 4096 x 4096 62.6 -> 51.5 with 2; where the waves are full already a second split costs
-// 3 to 16 % (8192 x 1536 x 4096 88.3 -> 94.2, 28672 x 4096 x 1024 287 -> 333) and none is made.  A split has to win 5 %.
-int pick_k_splits(long long tiles, int K, int max_pairs, int most = 8) {
+int forced_splits() {                                     // tuning override
   static const int forced = [] { const char* e = getenv("TPLR_GEMM_KSPLITS"); return e ? atoi(e) : 0; }();
-  const long long kb = (K + BK - 1) / BK;
-  if (forced > 0 && forced <= most) return kb / forced >= 1 ? forced : 1;   // tuning override
-  int pairs = tplr_sm_count() / 2;
-  if (max_pairs > 0 && pairs > max_pairs) pairs = max_pairs;
+  return forced;
+}
+
+// Parts of K of an accumulating GEMM (C += ...): where its tiles fill the chip's CTA pairs badly, a tile's K range is cut into
+// several work units that run on different pairs.  Part 0 adds into C, the others store fp32 planes, and a second kernel adds
+// those to C in order: the same bits on every run, which parts added into C as they arrive do not give.  The number with the
+// fewest k block times (0.37 us each) wins, fitted on 33 weight-gradient shapes from 768 x 768 to 32000 x 2048, K 333 to
+// 16384: waves of units, 8 k blocks per unit for its pipeline fill and its reduction, and for the planes 6 for the launch and
+// 2 + 1.2 * parts per million elements of C.  A cut has to win 5 %.  One part against the chosen number: 768 x 768 x 8192
+// (9 tiles on 74 pairs) 53.0 -> 17.7 us with 8, 2304 x 768 x 8192 53.2 -> 35.1 with 2, 1536 x 1536 x 4096 31.5 -> 25.1 with 2;
+// beyond that the planes cost what the fuller waves win: 768 x 3072 x 2048 19.4 in one part and 19.3 in two,
+// 1536 x 4096 x 4096 65.4 and 66.6, and where the waves are full already a cut loses (8192 x 1536 x 4096 87.5 and 116.9).
+int pick_acc_splits(int M, int N, int K) {
+  const long long kb = (K + BK - 1) / BK, tiles = (long long)((M + TILE_M - 1) / TILE_M) * ((N + TILE_N - 1) / TILE_N);
+  if (N % 8) return 1;
+  if (forced_splits() > 0) return kb / forced_splits() >= 1 ? forced_splits() : 1;
+  const int pairs = tplr_sm_count() / 2;
   int best = 1;
   double best_cost = 0.0;
-  for (int ks = 1; ks <= most && ks <= kb; ks *= 2) {
+  for (int ks = 1; ks <= 8 && ks <= kb; ks *= 2) {
     const long long per = (kb + ks - 1) / ks;
     if ((ks - 1) * per >= kb) break;                      // every unit has work
-    const double cost = (double)((tiles * ks + pairs - 1) / pairs) * (double)(per + 8);
+    const double planes = ks == 1 ? 0.0 : 6.0 + (double)M * N * 1e-6 * (2.0 + 1.2 * ks);
+    const double cost = (double)((tiles * ks + pairs - 1) / pairs) * (double)(per + 8) + planes;
     if (ks == 1 || cost < 0.95 * best_cost) { best = ks; best_cost = cost; }
   }
   return best;
 }
 
+// Parts of K of the triangle product for Newton-Schulz, by the same count of waves.  Two at most: replicas orthogonalise the
+// same matrix each for itself, so the result must not depend on the order in which the parts arrive, and two parts added into
+// zeros give the same sum in either order.
+int pick_syrk_splits(int M, int K) {
+  const long long t = (M + TILE_M - 1) / TILE_M, tiles = t * (t + 1) / 2, kb = (K + BK - 1) / BK, per = (kb + 1) / 2;
+  const int pairs = tplr_sm_count() / 2;
+  if (per >= kb) return 1;
+  auto waves = [&](long long units) { return (double)((units + pairs - 1) / pairs); };
+  return waves(2 * tiles) * (double)(per + 8) < 0.95 * waves(tiles) * (double)(kb + 8) ? 2 : 1;
+}
+
 // The scatter entry's rule: its reductions cross NVLink, so K is only halved, and only where that lifts the wave efficiency
 // by more than 10 points (4 and 8 splits lost more than the fuller waves won).
 int pick_scatter_splits(int M, int N, int K) {
-  static const int forced = [] { const char* e = getenv("TPLR_GEMM_KSPLITS"); return e ? atoi(e) : 0; }();
-  if (forced > 0) return (K + BK - 1) / BK / forced >= 1 ? forced : 1;   // tuning override
+  if (forced_splits() > 0) return (K + BK - 1) / BK / forced_splits() >= 1 ? forced_splits() : 1;
   const int pairs = tplr_sm_count() / 2;
   const long long tiles = (long long)((M + TILE_M - 1) / TILE_M) * ((N + TILE_N - 1) / TILE_N);
   if ((K + BK - 1) / BK < 128) return 1;
@@ -993,6 +1014,23 @@ int pick_out_splits(int M, int N, int K) {
     if (cost < best_cost) { best = ks; best_cost = cost; }
   }
   return best;
+}
+
+// C += the planes ([n_planes][plane] fp32, rows of N elements), in order; C: rows of ldc elements, all multiples of 4 and 16-byte
+// aligned.
+__global__ void __launch_bounds__(256) add_planes_kernel(const float* __restrict__ x, float* __restrict__ c, long long M, int n4, long long ldc,
+                                                         int n_planes, long long plane) {
+  const long long total = M * n4;
+  for (long long i = blockIdx.x * 256LL + threadIdx.x; i < total; i += gridDim.x * 256LL) {
+    const long long row = i / n4;
+    float4* p = reinterpret_cast<float4*>(c + row * ldc) + (i - row * n4);
+    float4 a = *p;
+    for (int s = 0; s < n_planes; ++s) {
+      const float4 q = reinterpret_cast<const float4*>(x + s * plane)[i];
+      a.x += q.x; a.y += q.y; a.z += q.z; a.w += q.w;
+    }
+    *p = a;
+  }
 }
 
 // The parts' planes ([parts][plane] fp32, rows of N elements) added in order -> bf16 rows of ldc elements; N, plane and ldc
@@ -1048,14 +1086,8 @@ TPLR_API int tplr_gemm2_syrk(const void* A, void* C, int M, int K, long long lda
   return dispatch2(p, 0, 0, 0, 0, 0, (cudaStream_t)stream);
 }
 
-static long long syrk_tiles(int M) {
-  const long long t = (M + TILE_M - 1) / TILE_M;
-  return t * (t + 1) / 2;
-}
-// K splits that tplr_gemm2_syrk_acc makes for this size (1: tplr_gemm2_syrk is the better call).  Two at most: replicas
-// orthogonalise the same matrix each for itself, so the result must not depend on the order in which the parts arrive, and
-// two parts added into zeros give the same sum in either order.
-TPLR_API int tplr_gemm2_syrk_splits(int M, int K) { return pick_k_splits(syrk_tiles(M), K, 0, 2); }
+// K splits that tplr_gemm2_syrk_acc makes for this size (1: tplr_gemm2_syrk is the better call).
+TPLR_API int tplr_gemm2_syrk_splits(int M, int K) { return pick_syrk_splits(M, K); }
 
 // tplr_gemm2_syrk adding into an fp32 C (ldc a multiple of 4, zeroed by the caller) with K cut into two work units per
 // tile: the triangle of a small matrix has fewer tiles than the chip has CTA pairs.  2048 x 8192 (36 tiles on 74 pairs):
@@ -1068,7 +1100,7 @@ TPLR_API int tplr_gemm2_syrk_acc(const void* A, float* C, int M, int K, long lon
   Gemm2Params p = {};
   if (int r = fill_common(p, A, A, C, M, M, K, lda, lda, ldc, 0, 0, 1, status)) return r;
   p.tri = 1;
-  p.k_splits = tplr_gemm2_syrk_splits(M, K);
+  p.k_splits = pick_syrk_splits(M, K);
   return dispatch2(p, 0, 0, 1, 0, 0, (cudaStream_t)stream);
 }
 
@@ -1080,8 +1112,32 @@ TPLR_API int tplr_gemm2_bf16(const void* A, const void* B, void* C, int M, int N
   if (M <= 0 || N <= 0 || K <= 0) return 0;
   Gemm2Params p = {};
   if (int r = fill_common(p, A, B, C, M, N, K, lda, ldb, ldc, a_mn, b_mn, epi, status)) return r;
-  if (epi == 1 && p.c_tma) p.k_splits = pick_k_splits((long long)((M + TILE_M - 1) / TILE_M) * ((N + TILE_N - 1) / TILE_N), K, max_pairs);
   return dispatch2(p, a_mn, b_mn, epi, 0, max_pairs, (cudaStream_t)stream);
+}
+
+// Parts that tplr_gemm2_acc_split cuts K into for this size; 1: no workspace, call tplr_gemm2_bf16 with epi 1.
+TPLR_API int tplr_gemm2_acc_splits(int M, int N, int K) { return pick_acc_splits(M, N, K); }
+
+// tplr_gemm2_bf16 with epi 1 (C fp32, C += ...) with K cut into parts: the workspace `ws` holds (parts - 1) * (M rounded up to
+// 32) * N fp32 elements (contents irrelevant).  C and ws 16-byte aligned, ldc a multiple of 4, N a multiple of 8.
+TPLR_API int tplr_gemm2_acc_split(const void* A, const void* B, float* C, float* ws, int M, int N, int K, long long lda, long long ldb,
+                                  long long ldc, int a_mn, int b_mn, unsigned int* status, void* stream) {
+  TPLR_ENTER();
+  if (M <= 0 || N <= 0 || K <= 0) return 0;
+  if ((N % 8) || (ldc % 4) || (((uintptr_t)C | (uintptr_t)ws) & 15)) return -101;
+  Gemm2Params p = {};
+  if (int r = fill_common(p, A, B, C, M, N, K, lda, ldb, ldc, a_mn, b_mn, 1, status)) return r;
+  p.k_splits = pick_acc_splits(M, N, K);
+  p.plane_rows = (M + 31) / 32 * 32;                    // a warp's box of 32 rows stays inside its plane
+  const int n_planes = p.k_splits - 1;
+  if (n_planes && !make_map(&p.tmCr[0], ws, N, (long long)n_planes * p.plane_rows, N, 32, 32, CU_TENSOR_MAP_SWIZZLE_128B, true)) return -110;
+  if (int r = dispatch2(p, a_mn, b_mn, 1, 0, 0, (cudaStream_t)stream)) return r;
+  if (n_planes) {
+    const long long n = ((long long)M * (N / 4) + 255) / 256;
+    const unsigned grid = (unsigned)(n < 8LL * tplr_sm_count() ? n : 8LL * tplr_sm_count());
+    add_planes_kernel<<<grid, 256, 0, (cudaStream_t)stream>>>(ws, C, M, N / 4, ldc, n_planes, (long long)p.plane_rows * N);
+  }
+  return (int)cudaGetLastError();
 }
 
 // Parts that tplr_gemm2_bf16_split would cut K into for a bf16 result of this size; 1: no workspace, call tplr_gemm2_bf16.

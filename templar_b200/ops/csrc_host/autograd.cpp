@@ -28,6 +28,8 @@ struct Entries {
   int (*add_rmsnorm_fwd)(const void*, const void*, const void*, void*, void*, float*, ll, int, float, void*);
   int (*add_rmsnorm_bwd)(const void*, const void*, const void*, const float*, const void*, void*, float*, ll, int, unsigned*, void*);
   int (*gemm)(const void*, const void*, void*, int, int, int, ll, ll, ll, int, int, int, unsigned*, int, void*);
+  int (*acc_splits)(int, int, int);
+  int (*acc_split)(const void*, const void*, float*, float*, int, int, int, ll, ll, ll, int, int, unsigned*, void*);
   int (*out_splits)(int, int, int);
   int (*gemm_split)(const void*, const void*, void*, float*, int, int, int, ll, ll, ll, int, int, unsigned*, void*);
   int (*swiglu)(const void*, const void*, void*, void*, int, int, int, ll, ll, ll, ll, unsigned*, void*);
@@ -51,6 +53,8 @@ void bind(const std::string& path) {
   get(E.add_rmsnorm_fwd, "tplr_add_rmsnorm_fwd");
   get(E.add_rmsnorm_bwd, "tplr_add_rmsnorm_bwd_v2");
   get(E.gemm, "tplr_gemm2_bf16");
+  get(E.acc_splits, "tplr_gemm2_acc_splits");
+  get(E.acc_split, "tplr_gemm2_acc_split");
   get(E.out_splits, "tplr_gemm2_out_splits");
   get(E.gemm_split, "tplr_gemm2_bf16_split");
   get(E.swiglu, "tplr_gemm2_swiglu");
@@ -90,13 +94,23 @@ void keep(AutogradContext* ctx, const char* key, const Aside& a) {
 // out = op(a) op(b)^T as functional.gemm; epi 0: store bf16, 1: add into fp32
 void gemm(const Tensor& a, const Tensor& b, const Tensor& out, bool a_mn, bool b_mn, int epi, int64_t status) {
   const ll M = a_mn ? a.size(1) : a.size(0), K = a_mn ? a.size(0) : a.size(1), N = b_mn ? b.size(1) : b.size(0);
-  const ll parts = epi == 0 ? E.out_splits((int)M, (int)N, (int)K) : 1;
-  if (parts > 1) {
-    Tensor ws = f32({parts * ((M + 31) / 32 * 32) * N}, a);
-    check(E.gemm_split(a.data_ptr(), b.data_ptr(), out.data_ptr(), ws.data_ptr<float>(), (int)M, (int)N, (int)K, a.stride(0),
-                       b.stride(0), out.stride(0), a_mn, b_mn, word(status), stream()),
-          "tplr_gemm2_bf16_split");
-    return;
+  const ll plane = (M + 31) / 32 * 32 * N;             // workspace of one part of K, where K is cut
+  if (epi == 0) {
+    if (const ll parts = E.out_splits((int)M, (int)N, (int)K); parts > 1) {
+      Tensor ws = f32({parts * plane}, a);
+      check(E.gemm_split(a.data_ptr(), b.data_ptr(), out.data_ptr(), ws.data_ptr<float>(), (int)M, (int)N, (int)K, a.stride(0),
+                         b.stride(0), out.stride(0), a_mn, b_mn, word(status), stream()),
+            "tplr_gemm2_bf16_split");
+      return;
+    }
+  } else if (reinterpret_cast<uintptr_t>(out.data_ptr()) % 16 == 0) {
+    if (const ll parts = E.acc_splits((int)M, (int)N, (int)K); parts > 1) {
+      Tensor ws = f32({(parts - 1) * plane}, a);
+      check(E.acc_split(a.data_ptr(), b.data_ptr(), out.data_ptr<float>(), ws.data_ptr<float>(), (int)M, (int)N, (int)K, a.stride(0),
+                        b.stride(0), out.stride(0), a_mn, b_mn, word(status), stream()),
+            "tplr_gemm2_acc_split");
+      return;
+    }
   }
   check(E.gemm(a.data_ptr(), b.data_ptr(), out.data_ptr(), (int)M, (int)N, (int)K, a.stride(0), b.stride(0), out.stride(0), a_mn,
                b_mn, epi, word(status), 0, stream()),

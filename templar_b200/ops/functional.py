@@ -100,17 +100,20 @@ def gemm(a: torch.Tensor, b: torch.Tensor, *, a_mn: bool = False, b_mn: bool = F
             raise ValueError("gemm: accumulate needs an fp32 out")
         epi = 0 if out.dtype == torch.bfloat16 else (1 if accumulate else 2)
         L = native.lib()
-        # few tiles and a long K: cut K and sum the parts from an fp32 workspace (the rule is the library's; most products
-        # have more tiles than half the chip's CTA pairs and do not ask it)
-        parts = 1
-        if (epi == 0 and _GEMM_BACKEND == "tcgen05_2sm" and K >= 4096 and -(-M // 256) * -(-N // 256) <= 64 and out.data_ptr() % 16 == 0
-                and out.stride(0) % 8 == 0):
-            parts = L.tplr_gemm2_out_splits(M, N, K)
-        if parts > 1:
-            ws = torch.empty(parts * (-(-M // 32) * 32) * N, dtype=torch.float32, device=a.device)
-            native.check(L.tplr_gemm2_bf16_split(a.data_ptr(), b.data_ptr(), out.data_ptr(), ws.data_ptr(), M, N, K, a.stride(0),
-                                                 b.stride(0), out.stride(0), int(a_mn), int(b_mn), status_word(a.device).data_ptr(),
-                                                 native.stream_ptr()), "tplr_gemm2_bf16_split")
+        # few tiles and a long K: cut K and sum the parts from an fp32 workspace (the rules are the library's; most bf16
+        # products have more tiles than half the chip's CTA pairs and do not ask)
+        planes, split = 0, None
+        if _GEMM_BACKEND == "tcgen05_2sm" and out.data_ptr() % 16 == 0:
+            if epi == 0 and K >= 4096 and -(-M // 256) * -(-N // 256) <= 64 and out.stride(0) % 8 == 0:
+                planes, split = L.tplr_gemm2_out_splits(M, N, K), L.tplr_gemm2_bf16_split
+                planes = 0 if planes == 1 else planes
+            elif epi == 1 and out.stride(0) % 4 == 0:
+                planes, split = L.tplr_gemm2_acc_splits(M, N, K) - 1, L.tplr_gemm2_acc_split
+        if planes > 0:
+            ws = torch.empty(planes * (-(-M // 32) * 32) * N, dtype=torch.float32, device=a.device)
+            native.check(split(a.data_ptr(), b.data_ptr(), out.data_ptr(), ws.data_ptr(), M, N, K, a.stride(0), b.stride(0),
+                               out.stride(0), int(a_mn), int(b_mn), status_word(a.device).data_ptr(), native.stream_ptr()),
+                         "tplr_gemm2_split")
             return out
         fn = L.tplr_gemm2_bf16 if _GEMM_BACKEND == "tcgen05_2sm" else L.tplr_gemm_bf16
         err = fn(a.data_ptr(), b.data_ptr(), out.data_ptr(), M, N, K,

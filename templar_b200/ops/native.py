@@ -117,6 +117,8 @@ def _declare(L: ctypes.CDLL) -> None:
         "tplr_attention_bwd": [vp, vp, vp, vp, vp, vp, vp, i, i, i, i, i, ll, ll, f, vp, vp],
         "tplr_gemm_bf16": [vp, vp, vp, i, i, i, ll, ll, ll, i, i, i, vp, i, vp],
         "tplr_gemm2_bf16": [vp, vp, vp, i, i, i, ll, ll, ll, i, i, i, vp, i, vp],
+        "tplr_gemm2_acc_splits": [i, i, i],
+        "tplr_gemm2_acc_split": [vp, vp, vp, vp, i, i, i, ll, ll, ll, i, i, vp, vp],
         "tplr_gemm2_out_splits": [i, i, i],
         "tplr_gemm2_bf16_split": [vp, vp, vp, vp, i, i, i, ll, ll, ll, i, i, vp, vp],
         "tplr_gemm2_gather": [vp, vp, vp, i, i, i, ll, ll, ll, i, i, i, i, i, i, i, vp, vp, ctypes.c_uint, i, vp, vp],

@@ -257,3 +257,16 @@ def test_bf16_gemm_through_split_workspace(M, N, K, b_mn, backend):
     assert torch.allclose(wide[:, 8:-8].float(), ref, rtol=2 ** -8, atol=1e-3)        # one rounding; fp32 sums of K products
     assert (wide[:, :8] == 7).all() and (wide[:, -8:] == 7).all()
     assert torch.equal(OF.gemm(A, B, b_mn=b_mn), wide[:, 8:-8])
+
+
+@pytest.mark.parametrize("M,N,K", [(768, 768, 8192), (264, 520, 4104), (2304, 768, 8192), (1536, 4096, 4096)])
+def test_accumulating_gemm_repeats_its_bits(M, N, K, backend):
+    """A weight gradient added into a buffer that holds an earlier one: the parts of K are added in order, not as they arrive."""
+    if backend != "tcgen05_2sm":
+        pytest.skip("only the CTA-pair kernel cuts K")
+    torch.manual_seed(M + N)
+    A, B = (torch.randn(K, n, device=DEV).to(torch.bfloat16) for n in (M, N))
+    before = torch.randn(M, N, device=DEV)
+    first = OF.gemm(A, B, a_mn=True, b_mn=True, out=before.clone(), accumulate=True)
+    for _ in range(30):
+        assert torch.equal(OF.gemm(A, B, a_mn=True, b_mn=True, out=before.clone(), accumulate=True), first)
