@@ -67,6 +67,12 @@ def _aligned(*ts) -> bool:
     return all(t.data_ptr() % 16 == 0 for t in ts)
 
 
+def _dense(t: torch.Tensor) -> torch.Tensor:
+    """``t`` as the kernels read it: contiguous, on a 16-byte boundary."""
+    c = t.contiguous()
+    return c if c.data_ptr() % 16 == 0 else c.clone()
+
+
 # --------------------------------------------------------------------------- #
 # GEMM
 # --------------------------------------------------------------------------- #
@@ -205,21 +211,36 @@ def linear(x: torch.Tensor, w: torch.Tensor, main_grad: torch.Tensor | None = No
 # --------------------------------------------------------------------------- #
 # RMSNorm
 # --------------------------------------------------------------------------- #
+def _norm_native(D: int, w: torch.Tensor, *rows: torch.Tensor) -> bool:
+    """Rows and a weight that the norm kernels take: the nodes hand them over dense and aligned (copied where they are not)."""
+    return _native_ok(*rows, w) and D % 8 == 0 and D <= 8192 and w.numel() == D
+
+
+def _norm_weight_grad(mg, D: int, device):
+    """(buffer the kernel adds dw into, what to call with it afterwards): the gradient buffer itself where it is dense fp32."""
+    if mg is not None and mg.dtype == torch.float32 and mg.is_contiguous() and mg.numel() == D:
+        return mg, lambda w: None
+    buf = torch.zeros(D, dtype=torch.float32, device=device)
+    if mg is None:
+        return buf, lambda w: buf.to(w.dtype)
+    return buf, lambda w: (mg.add_(buf.view(mg.shape).to(mg.dtype)), None)[1]
+
+
 class _RMSNorm(torch.autograd.Function):
     @staticmethod
     def forward(ctx, x, w, eps, main_grad):
         ctx.eps = eps
         ctx.main_grad = main_grad
-        if _native_ok(x, w) and x.shape[-1] % 8 == 0 and x.shape[-1] <= 8192:
-            xc = x.contiguous()
+        if _norm_native(x.shape[-1], w, x):
+            xc, wc = _dense(x), _dense(w)
             T = xc.numel() // xc.shape[-1]
             y = torch.empty_like(xc)
             rstd = torch.empty(T, dtype=torch.float32, device=x.device)
             # the residual-add kernel with nothing to add
-            native.check(native.lib().tplr_add_rmsnorm_fwd(xc.data_ptr(), None, w.data_ptr(), None, y.data_ptr(), rstd.data_ptr(),
+            native.check(native.lib().tplr_add_rmsnorm_fwd(xc.data_ptr(), None, wc.data_ptr(), None, y.data_ptr(), rstd.data_ptr(),
                                                            T, xc.shape[-1], eps, native.stream_ptr()), "rmsnorm_fwd")
             ctx.native = True
-            ctx.save_for_backward(xc, w, rstd)
+            ctx.save_for_backward(xc, wc, rstd)
             return y
         ctx.native = False
         xf = x.float()
@@ -232,15 +253,15 @@ class _RMSNorm(torch.autograd.Function):
         x, w, rstd = ctx.saved_tensors
         mg = ctx.main_grad
         if ctx.native:
-            dyc = dy.contiguous()
+            dyc = _dense(dy)
             T, D = x.numel() // x.shape[-1], x.shape[-1]
             dx = torch.empty_like(x)
-            dw_buf = mg if mg is not None else torch.zeros(D, dtype=torch.float32, device=x.device)
+            dw_buf, done = _norm_weight_grad(mg, D, x.device)
             native.check(native.lib().tplr_add_rmsnorm_bwd_v2(dyc.data_ptr(), x.data_ptr(), w.data_ptr(), rstd.data_ptr(), None,
                                                               dx.data_ptr(), dw_buf.data_ptr(), T, D,
                                                               status_word(x.device).data_ptr(), native.stream_ptr()),
                          "rmsnorm_bwd")
-            return dx, (None if mg is not None else dw_buf.to(w.dtype)), None, None
+            return dx, done(w), None, None
         xf, g = x.float(), dy.float()
         xh = xf * rstd
         gw = g * w.float()
@@ -258,8 +279,7 @@ def rmsnorm(x, w, eps: float = 1e-5, main_grad=None):
     if main_grad is None:
         main_grad = getattr(w, "main_grad", None)
     D = x.shape[-1]
-    if (_native_ok(x, w) and D % 8 == 0 and D <= 8192 and x.is_contiguous() and w.is_contiguous() and w.numel() == D
-            and _buffers_ok((main_grad, w)) and _aligned(x, w)):
+    if (_norm_native(D, w, x) and x.is_contiguous() and w.is_contiguous() and _buffers_ok((main_grad, w)) and _aligned(x, w)):
         return native.host().rmsnorm(x, w, main_grad, eps, status_word(x.device).data_ptr())
     return _RMSNorm.apply(x, w, eps, main_grad)
 
@@ -272,10 +292,13 @@ class _AddRMSNorm(torch.autograd.Function):
     def forward(ctx, res, delta, w, eps, main_grad):
         ctx.eps, ctx.main_grad = eps, main_grad
         D = res.shape[-1]
-        ctx.native = _native_ok(res, delta, w) and D % 8 == 0 and D <= 8192
+        ctx.native = _norm_native(D, w, res, delta)
         if ctx.native:
             fused = res.is_contiguous() and delta.is_contiguous() and res.shape == delta.shape
             # views and broadcast operands: eager add, then the kernel with nothing to add
+            if fused:
+                res, delta = _dense(res), _dense(delta)
+            w = _dense(w)
             h = torch.empty_like(res) if fused else (res + delta).contiguous()
             T = h.numel() // D
             y = torch.empty_like(h)
@@ -298,15 +321,15 @@ class _AddRMSNorm(torch.autograd.Function):
         D = h.shape[-1]
         if ctx.native:
             T = h.numel() // D
-            dyc = dy.contiguous()
-            dhc = dh.contiguous() if dh is not None else None
+            dyc = _dense(dy)
+            dhc = _dense(dh) if dh is not None else None
             dx = torch.empty_like(h)
-            dw_buf = mg if mg is not None else torch.zeros(D, dtype=torch.float32, device=h.device)
+            dw_buf, done = _norm_weight_grad(mg, D, h.device)
             native.check(native.lib().tplr_add_rmsnorm_bwd_v2(dyc.data_ptr(), h.data_ptr(), w.data_ptr(), rstd.data_ptr(),
                                                               dhc.data_ptr() if dhc is not None else None, dx.data_ptr(),
                                                               dw_buf.data_ptr(), T, D, status_word(h.device).data_ptr(),
                                                               native.stream_ptr()), "add_rmsnorm_bwd")
-            return dx, dx, (None if mg is not None else dw_buf.to(w.dtype)), None, None
+            return dx, dx, done(w), None, None
         hf, g = h.float(), dy.float()
         xh = hf * rstd
         gw = g * w.float()
@@ -328,9 +351,8 @@ def add_rmsnorm(res, delta, w, eps: float = 1e-5, main_grad=None):
     if main_grad is None:
         main_grad = getattr(w, "main_grad", None)
     D = res.shape[-1]
-    if (_native_ok(res, delta, w) and D % 8 == 0 and D <= 8192 and res.shape == delta.shape and res.is_contiguous()
-            and delta.is_contiguous() and w.is_contiguous() and w.numel() == D and _buffers_ok((main_grad, w))
-            and _aligned(res, delta, w)):
+    if (_norm_native(D, w, res, delta) and res.shape == delta.shape and res.is_contiguous() and delta.is_contiguous()
+            and w.is_contiguous() and _buffers_ok((main_grad, w)) and _aligned(res, delta, w)):
         return native.host().add_rmsnorm(res, delta, w, main_grad, eps, status_word(res.device).data_ptr())
     return _AddRMSNorm.apply(res, delta, w, eps, main_grad)
 

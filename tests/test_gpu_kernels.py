@@ -623,3 +623,48 @@ def test_quantised_residual_is_taken_against_the_decoded_values(shapes, topk, nu
         ref = torch.empty(s.shape, dtype=torch.float64)
         sent = tr.decode(comp.decompress(ref, idx.cpu(), val.cpu().double(), eng.layout.xshape(s.name), s.totalk), use_dct=use_dct)
         assert torch.allclose(eng.ef[sl].cpu().double(), x - sent.reshape(-1), atol=5e-6, rtol=1e-4), s.name
+
+
+@pytest.mark.parametrize("D", [64, 768, 2048, 4096])
+@pytest.mark.parametrize("layout", ["offset", "strided weight", "strided target", "offset gradient"])
+def test_norms_of_operands_that_are_not_dense(D, layout):
+    """Views off a 16-byte boundary, a strided weight or gradient target, and an incoming gradient off its boundary give what
+    dense operands give (the kernels read 16 bytes at a time, so the nodes copy such operands first)."""
+    torch.manual_seed(D)
+    T = 37
+
+    def off(t):
+        """The same values one element off the boundary."""
+        base = torch.empty(t.numel() + 8, dtype=t.dtype, device=DEV)
+        return base[1:1 + t.numel()].view(t.shape).copy_(t)
+
+    res, delta, dh, dy = (torch.randn(T, D, device=DEV).to(torch.bfloat16) for _ in range(4))
+    w = (1 + 0.1 * torch.randn(D, device=DEV)).to(torch.bfloat16)
+    view = off if layout == "offset" else (lambda t: t)
+    grad = off if layout == "offset gradient" else (lambda t: t)
+
+    def run(fn, view, grad, weight, target):
+        a, b = view(res.clone()).requires_grad_(), view(delta.clone()).requires_grad_()
+        out = fn(a, b, weight, target)
+        g = torch.autograd.grad(out, (a, b) if len(out) == 2 else (a,), [grad(t) for t in (dh, dy)[-len(out):]])
+        return [*out, *g, target.clone()]
+
+    for fn in (lambda a, b, w_, t: (OF.rmsnorm(a, w_, 1e-5, t),), lambda a, b, w_, t: OF.add_rmsnorm(a, b, w_, 1e-5, t)):
+        weight = w.repeat_interleave(2)[::2] if layout == "strided weight" else view(w)
+        target = torch.ones(2 * D, device=DEV)[::2] if layout == "strided target" else torch.ones(D, device=DEV)
+        got = run(fn, view, grad, weight.requires_grad_(), target)
+        want = run(fn, lambda t: t, lambda t: t, w.clone().requires_grad_(), torch.ones(D, device=DEV))
+        for x, y in zip(got[:-1], want[:-1]):
+            assert torch.equal(x, y)
+        # fp32 sums of T products below 30 in another order
+        assert torch.allclose(got[-1], want[-1], atol=30 * T * 2 ** -23, rtol=0)
+
+
+def test_norms_refuse_a_weight_of_another_length():
+    x = torch.randn(4, 768, device=DEV).to(torch.bfloat16)
+    for n in (760, 384):
+        w = torch.ones(n, device=DEV, dtype=torch.bfloat16)
+        with pytest.raises(RuntimeError):
+            OF.rmsnorm(x, w)
+        with pytest.raises(RuntimeError):
+            OF.add_rmsnorm(x, x, w)
