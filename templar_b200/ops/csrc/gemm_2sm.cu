@@ -745,9 +745,10 @@ gemm2_kernel(const __grid_constant__ Gemm2Params p) {
         }
         // drain (leader): every armed stage has landed in both CTAs before the pair may retire
         if (cr == 0) {
+          Drain drain;
           for (uint32_t back = 0; back < STAGES && back < it; ++back) {
             const uint32_t j = it - 1 - back;
-            mbar_wait(smem_u32(&bar_full[j % STAGES]), (j / STAGES) & 1, abort_flag);
+            drain.wait(smem_u32(&bar_full[j % STAGES]), (j / STAGES) & 1);
           }
         }
       }
@@ -821,7 +822,10 @@ gemm2_kernel(const __grid_constant__ Gemm2Params p) {
         if (lane == 0) mbar_arrive_cluster(mapa(smem_u32(&bar_tempty[acc]), 0));
       }
       // a role that gave up leaves no load in flight into the shared memory that it returns
-      for (; EPI == 5 && gl.used < gl.issued; ++gl.used) mbar_wait(gl.bar + 8u * (gl.used & 1u), (gl.used >> 1) & 1u, abort_flag);
+      if (EPI == 5) {
+        Drain drain;
+        for (; gl.used < gl.issued; ++gl.used) drain.wait(gl.bar + 8u * (gl.used & 1u), (gl.used >> 1) & 1u);
+      }
       if (lane == 0) {
         bulk_wait0();                // staging buffers are read out and the stores / reductions are performed
         if (p.rs_on) __threadfence_system();
@@ -877,8 +881,8 @@ gemm2_kernel(const __grid_constant__ Gemm2Params p) {
       }
       bulk_wait0();
       // loads that were issued but never stored (abort path) must land before the CTA retires
-      for (long long g = stored; g < issued; ++g)
-        mbar_wait(smem_u32(&bar_full[g % STAGES]), (uint32_t)((g / STAGES) & 1), abort_flag);
+      Drain drain;
+      for (long long g = stored; g < issued; ++g) drain.wait(smem_u32(&bar_full[g % STAGES]), (uint32_t)((g / STAGES) & 1));
     }
   }
   __syncwarp();

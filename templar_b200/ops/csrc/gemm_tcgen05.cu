@@ -92,9 +92,10 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
         }
       }
       // drain: every armed stage must have landed before the CTA may retire
+      Drain drain;
       for (uint32_t back = 0; back < STAGES && back < it; ++back) {
         const uint32_t j = it - 1 - back;
-        mbar_wait(smem_u32(&bar_full[j % STAGES]), (j / STAGES) & 1, abort_flag);
+        drain.wait(smem_u32(&bar_full[j % STAGES]), (j / STAGES) & 1);
       }
     }
   } else if (warp == 1) {

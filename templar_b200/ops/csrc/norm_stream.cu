@@ -91,11 +91,14 @@ add_rmsnorm_bwd_stream_kernel(const bf16* __restrict__ dy, const bf16* __restric
         if (dres) bulk_g2s(base + 2u * arr_bytes, dres + r0 * D, bytes, fb);
       }
       // every copy that was issued has landed before this CTA may retire (the consumers may have given up)
+      Drain drain;
       for (uint32_t back = 0; back < NS_STAGES && back < it; ++back) {
         const uint32_t j = it - 1u - back;
-        mbar_wait(smem_u32(&bar_full[j % NS_STAGES]), (j / NS_STAGES) & 1u, abort_flag);
+        drain.wait(smem_u32(&bar_full[j % NS_STAGES]), (j / NS_STAGES) & 1u);
       }
     }
+    __syncwarp();
+    __syncthreads();                                         // the consumers' flush below
   } else {
     // ------------------------------ consumers: warp r of the CTA owns row r of every tile ----------
     float dwv[VPL][8];
@@ -154,8 +157,10 @@ add_rmsnorm_bwd_stream_kernel(const bf16* __restrict__ dy, const bf16* __restric
       __syncwarp();
       if (lane == 0) mbar_arrive(smem_u32(&bar_empty[s]));
     }
-    // the eight warps' partial dw through the (now unused) first stage, one slab of 32 vectors at a time
-    if (dw) {
+    // the eight warps' partial dw through the (now unused) first stage, one slab of 32 vectors at a time.  The producer reaches
+    // the barrier after waiting for its copies; nothing is flushed when a role has given up (no one raises the flag any more).
+    __syncthreads();
+    if (dw && !*abort_flag) {
       float* s_dw = reinterpret_cast<float*>(smem);          // [8][256 + 1]
 #pragma unroll
       for (int v = 0; v < VPL; ++v) {
@@ -309,9 +314,10 @@ add_rmsnorm_bwd_wide_kernel(const bf16* __restrict__ dy, const bf16* __restrict_
         if (dres) bulk_g2s(base + 2u * arr_bytes, dres + r0 * D, bytes, fb);
       }
       // every copy that was issued has landed before this CTA may retire (the consumers may have given up)
+      Drain drain;
       for (uint32_t back = 0; back < NW_STAGES && back < it; ++back) {
         const uint32_t j = it - 1u - back;
-        mbar_wait(smem_u32(&bar_full[j % NW_STAGES]), (j / NW_STAGES) & 1u, abort_flag);
+        drain.wait(smem_u32(&bar_full[j % NW_STAGES]), (j / NW_STAGES) & 1u);
       }
     }
     __syncwarp();
@@ -387,9 +393,10 @@ add_rmsnorm_bwd_wide_kernel(const bf16* __restrict__ dy, const bf16* __restrict_
       if (lane == 0) mbar_arrive(smem_u32(&bar_empty[s]));
     }
     // weight-gradient partials: the rows of a tile are added through the (now unused) stages, then one atomic per column
-    // and CTA.  All copies have landed before the first write: the producer reaches the barrier after waiting for them.
+    // and CTA.  All copies have landed before the first write: the producer reaches the barrier after waiting for them.  Nothing
+    // is flushed when a role has given up (no one raises the flag any more).
     __syncthreads();
-    if (dw) {
+    if (dw && !*abort_flag) {
       float* s_dw = reinterpret_cast<float*>(smem);           // [R - 1][D]
       if (grp > 0) {
 #pragma unroll

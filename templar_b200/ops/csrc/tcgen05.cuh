@@ -50,6 +50,14 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatil
   return false;
 }
 
+// Waits for copies in flight before a role returns.  A role also gets there when another one has given up, and mbar_wait
+// returns at once then, because the CTA's flag is up: a drain has a flag of its own, so that only its own time limit (one for
+// all its waits) ends it.
+struct Drain {
+  volatile int gave_up = 0;
+  __device__ __forceinline__ void wait(uint32_t bar, uint32_t parity) { (void)mbar_wait(bar, parity, &gave_up); }
+};
+
 __device__ __forceinline__ void tma_load_2d(uint32_t dst, const CUtensorMap* map, uint32_t bar, int x, int y) {
   asm volatile(
       "cp.async.bulk.tensor.2d.shared::cta.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];"
