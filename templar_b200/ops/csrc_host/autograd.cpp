@@ -128,6 +128,11 @@ Tensor weight_grad(const Tensor& buffer, const Tensor& dy2, const Tensor& x2, co
   return dw;
 }
 Tensor rows(const Tensor& t) { return t.reshape({-1, t.size(-1)}); }
+// rows of a tensor whose last dimension is D; an integer division by zero would end the process
+ll count_rows(const Tensor& t, ll D) {
+  TORCH_CHECK(D > 0, "rows of no elements");
+  return t.numel() / D;
+}
 
 // ------------------------------------------------------------------------------------------ norms
 // inputs: x (or res, delta), w, buffer, eps, status
@@ -135,7 +140,7 @@ variable_list norm_backward(AutogradContext* ctx, const Tensor& dh, const Tensor
                             const Tensor& rstd, int w_index) {
   const int64_t status = ctx->saved_data["status"].toInt();
   const Tensor buffer = aside(ctx, "buffer");
-  const ll D = h.size(-1), T = h.numel() / D;
+  const ll D = h.size(-1), T = count_rows(h, D);
   const Tensor dy = dy_in.defined() ? dense(dy_in) : at::zeros_like(h);
   const Tensor dres = dh.defined() ? dense(dh) : Tensor();
   Tensor dx = at::empty_like(h);
@@ -148,7 +153,7 @@ variable_list norm_backward(AutogradContext* ctx, const Tensor& dh, const Tensor
 
 struct RMSNorm : Function<RMSNorm> {
   static Tensor forward(AutogradContext* ctx, const Tensor& x, const Tensor& w, Aside buffer, double eps, int64_t status) {
-    const ll D = x.size(-1), T = x.numel() / D;
+    const ll D = x.size(-1), T = count_rows(x, D);
     Tensor y = at::empty_like(x), rstd = f32({T}, x);
     check(E.add_rmsnorm_fwd(x.data_ptr(), nullptr, w.data_ptr(), nullptr, y.data_ptr(), rstd.data_ptr<float>(), T, (int)D, (float)eps,
                             stream()),
@@ -168,7 +173,7 @@ struct RMSNorm : Function<RMSNorm> {
 struct AddRMSNorm : Function<AddRMSNorm> {
   static variable_list forward(AutogradContext* ctx, const Tensor& res, const Tensor& delta, const Tensor& w, Aside buffer, double eps,
                                int64_t status) {
-    const ll D = res.size(-1), T = res.numel() / D;
+    const ll D = res.size(-1), T = count_rows(res, D);
     Tensor h = at::empty_like(res), y = at::empty_like(res), rstd = f32({T}, res);
     check(E.add_rmsnorm_fwd(res.data_ptr(), delta.data_ptr(), w.data_ptr(), h.data_ptr(), y.data_ptr(), rstd.data_ptr<float>(), T,
                             (int)D, (float)eps, stream()),

@@ -279,7 +279,7 @@ def rmsnorm(x, w, eps: float = 1e-5, main_grad=None):
     if main_grad is None:
         main_grad = getattr(w, "main_grad", None)
     D = x.shape[-1]
-    if (_norm_native(D, w, x) and x.is_contiguous() and w.is_contiguous() and _buffers_ok((main_grad, w)) and _aligned(x, w)):
+    if (_norm_native(D, w, x) and D > 0 and x.is_contiguous() and w.is_contiguous() and _buffers_ok((main_grad, w)) and _aligned(x, w)):
         return native.host().rmsnorm(x, w, main_grad, eps, status_word(x.device).data_ptr())
     return _RMSNorm.apply(x, w, eps, main_grad)
 
@@ -351,7 +351,7 @@ def add_rmsnorm(res, delta, w, eps: float = 1e-5, main_grad=None):
     if main_grad is None:
         main_grad = getattr(w, "main_grad", None)
     D = res.shape[-1]
-    if (_norm_native(D, w, res, delta) and res.shape == delta.shape and res.is_contiguous() and delta.is_contiguous()
+    if (_norm_native(D, w, res, delta) and D > 0 and res.shape == delta.shape and res.is_contiguous() and delta.is_contiguous()
             and w.is_contiguous() and _buffers_ok((main_grad, w)) and _aligned(res, delta, w)):
         return native.host().add_rmsnorm(res, delta, w, main_grad, eps, status_word(res.device).data_ptr())
     return _AddRMSNorm.apply(res, delta, w, eps, main_grad)

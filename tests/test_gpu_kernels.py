@@ -668,3 +668,14 @@ def test_norms_refuse_a_weight_of_another_length():
             OF.rmsnorm(x, w)
         with pytest.raises(RuntimeError):
             OF.add_rmsnorm(x, x, w)
+
+
+def test_norms_refuse_rows_of_no_elements():
+    """As an exception: in C++ the division by the row's length would end the process."""
+    x, w = torch.empty(4, 0, device=DEV, dtype=torch.bfloat16), torch.empty(0, device=DEV, dtype=torch.bfloat16)
+    with pytest.raises(ZeroDivisionError):
+        OF.rmsnorm(x, w)
+    with pytest.raises(ZeroDivisionError):
+        OF.add_rmsnorm(x, x, w)
+    with pytest.raises(RuntimeError):
+        native.host().rmsnorm(x, w, None, 1e-5, 0)
