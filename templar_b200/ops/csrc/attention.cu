@@ -257,16 +257,23 @@ attn_fwd_kernel(const __grid_constant__ AttnFwdParams p) {
       mbar_expect_tx(smem_u32(&bar_q), TILE_BYTES);
       load_tile<DH>(sQ, &p.tmQKV, smem_u32(&bar_q), qcol, row0, b);
       bool ok = true;
+      int n_k = 0, n_v = 0;                                // tiles asked for
       for (int j = 0; j < nb && ok; ++j) {
         const uint32_t ph = j & 1;
         const int krow = j * BKV;
         if (!(ok = mbar_wait(smem_u32(&bar_k_empty), ph ^ 1, abort_flag))) break;
         mbar_expect_tx(smem_u32(&bar_k_full), TILE_BYTES);
         load_tile<DH>(sK, &p.tmQKV, smem_u32(&bar_k_full), kcol, krow, b);
+        ++n_k;
         if (!(ok = mbar_wait(smem_u32(&bar_v_empty), ph ^ 1, abort_flag))) break;
         mbar_expect_tx(smem_u32(&bar_v_full), TILE_BYTES);
         load_tile<DH>(sV, &p.tmQKV, smem_u32(&bar_v_full), vcol, krow, b);
+        ++n_v;
       }
+      Drain drain;                                         // no load may land after the CTA has retired: a role may have given up
+      drain.wait(smem_u32(&bar_q), 0);
+      if (n_k) drain.wait(smem_u32(&bar_k_full), (uint32_t)((n_k - 1) & 1));
+      if (n_v) drain.wait(smem_u32(&bar_v_full), (uint32_t)((n_v - 1) & 1));
     }
   } else if (warp == 1) {
     if (lane == 0) {
@@ -538,6 +545,7 @@ attn_bwd_kernel(const __grid_constant__ AttnBwdParams p) {
       load_tile<DH>(sK, &p.tmQKV, smem_u32(&bar_kv), kcol, kvrow0, b);
       load_tile<DH>(sV, &p.tmQKV, smem_u32(&bar_kv), vcol, kvrow0, b);
       bool ok = true;
+      int n_q = 0, n_do = 0;                                 // tiles asked for
       for (int t = 0; t < n_it && ok; ++t) {
         const int h = h0 + t / n_i, i = j + t % n_i;
         const int qrow0 = i * BQ, qcol = h * DH, s = t & 1;
@@ -545,11 +553,17 @@ attn_bwd_kernel(const __grid_constant__ AttnBwdParams p) {
         const uint32_t fq = smem_u32(&bar_q_full[s]);
         mbar_expect_tx(fq, TILE_BYTES);
         load_tile<DH>(sQ + s * TILE_BYTES, &p.tmQKV, fq, qcol, qrow0, b);
+        ++n_q;
         if (!(ok = mbar_wait(smem_u32(&bar_do_empty), (uint32_t)((t & 1) ^ 1), abort_flag))) break;
         const uint32_t fd = smem_u32(&bar_do_full);
         mbar_expect_tx(fd, TILE_BYTES);
         load_tile<DH>(sdO, &p.tmDO, fd, qcol, qrow0, b);
+        ++n_do;
       }
+      Drain drain;                                           // no load may land after the CTA has retired: a role may have given up
+      drain.wait(smem_u32(&bar_kv), 0);
+      for (int t = n_q > 2 ? n_q - 2 : 0; t < n_q; ++t) drain.wait(smem_u32(&bar_q_full[t & 1]), (uint32_t)((t >> 1) & 1));
+      if (n_do) drain.wait(smem_u32(&bar_do_full), (uint32_t)((n_do - 1) & 1));
     }
   } else if (warp == 1) {
     if (lane == 0) {
@@ -991,6 +1005,7 @@ attn_bwd2_kernel(const __grid_constant__ AttnBwd2Params p) {
       tma_load_2d(sV, &p.tmKV, smem_u32(&bar_kv), vcol, kvrow0);
       tma_load_2d(sV + TILE_BYTES / 2, &p.tmKV, smem_u32(&bar_kv), vcol + 64, kvrow0);
       bool ok = true;
+      int n_q = 0;                                           // steps asked for
       for (int t = 0; t < n_it && ok; ++t) {
         const int s = t & 1, k = t >> 1;
         const int h = g * group + t / n_i, iq = iq0 + t % n_i;
@@ -1006,7 +1021,11 @@ attn_bwd2_kernel(const __grid_constant__ AttnBwd2Params p) {
         const long long so = ((long long)b * p.H + h) * p.S + (long long)iq * B2_BQ;
         bulk_load_1d(sStat + s * 512, p.lse + so, 256, fb);
         bulk_load_1d(sStat + s * 512 + 256, p.delta + so, 256, fb);
+        ++n_q;
       }
+      Drain drain;                                           // as in the kernel above
+      drain.wait(smem_u32(&bar_kv), 0);
+      for (int t = n_q > 2 ? n_q - 2 : 0; t < n_q; ++t) drain.wait(smem_u32(&bar_q_full[t & 1]), (uint32_t)((t >> 1) & 1));
     }
   } else if (warp == 1) {
     if (lane == 0) {

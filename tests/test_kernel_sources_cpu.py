@@ -17,3 +17,14 @@ def test_drains_do_not_wait_on_the_shared_flag(src):
     # a statement that starts with the call: after a brace, a semicolon or a loop head
     ignored = re.findall(r"(?:[;{}]|\bfor \([^{}]*\))\s*(mbar_wait\([^;]*);", text)
     assert not ignored, ignored
+
+
+@pytest.mark.parametrize("src", sorted(p.name for p in CSRC.glob("*.cu") if "mbar_expect_tx(" in p.read_text()))
+def test_every_kernel_that_asks_for_copies_drains_them(src):
+    """Each kernel that arms a barrier for bulk copies waits for them before its CTA retires."""
+    text = re.sub(r"//[^\n]*", "", (CSRC / src).read_text())
+    kernels = re.split(r"__global__", text)[1:]
+    arming = [k for k in kernels if "mbar_expect_tx(" in k.split("<<<")[0]]
+    assert arming
+    for k in arming:
+        assert "Drain drain" in k, k[:200]
