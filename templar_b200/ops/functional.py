@@ -820,8 +820,8 @@ class _AttentionPacked(torch.autograd.Function):
         qkv, out, lse = ctx.saved_tensors
         n_heads, n_kv, hd = ctx.dims
         B, S, C = qkv.shape
-        do = dout.contiguous()
-        dqkv = torch.empty_like(qkv)
+        do = _dense(dout)
+        dqkv = torch.empty(B, S, qkv.stride(1), dtype=qkv.dtype, device=qkv.device)[..., :C]        # rows as far apart as qkv's
         dq32 = _attention_scratch(B, S, n_heads, n_kv, hd, qkv.device)
         delta = torch.empty(B, n_heads, S, dtype=torch.float32, device=qkv.device)
         native.check(native.lib().tplr_attention_bwd(qkv.data_ptr(), out.data_ptr(), do.data_ptr(), lse.data_ptr(),
@@ -863,7 +863,7 @@ class _QKVRopeAttention(torch.autograd.Function):
         x, w, qkv, out, lse, cos, sin = ctx.saved_tensors
         n_heads, n_kv, hd = ctx.dims
         B, S, C = qkv.shape
-        do = dout.contiguous()
+        do = _dense(dout)
         dqkv = torch.empty_like(qkv)
         dq32 = _attention_scratch(B, S, n_heads, n_kv, hd, qkv.device)
         delta = torch.empty(B, n_heads, S, dtype=torch.float32, device=qkv.device)
@@ -915,9 +915,7 @@ class _AttentionBlock(torch.autograd.Function):
         T, N = B * S, n_heads * hd
         L = native.lib()
         st = status_word(qkv.device).data_ptr()
-        dy2 = dy.reshape(T, dy.shape[-1])
-        if not dy2.is_contiguous():
-            dy2 = dy2.contiguous()
+        dy2 = _dense(dy.reshape(T, dy.shape[-1]))
         out2 = out.view(T, N)
         do = torch.empty(T, N, dtype=qkv.dtype, device=qkv.device)
         delta = torch.empty(B, n_heads, S, dtype=torch.float32, device=qkv.device)
@@ -985,7 +983,7 @@ def attention_packed(qkv, n_heads: int, n_kv: int, hd: int):
     """Causal attention of ``qkv`` [B, S, (H + 2 KV) * hd] (q heads, k heads, v heads); returns [B, S, H * hd]."""
     B, S, C = qkv.shape
     if (_ATTN_BACKEND == "tcgen05" and qkv.is_cuda and qkv.dtype == torch.bfloat16 and hd in OWN_HEAD_DIMS
-            and n_heads % n_kv == 0 and qkv.stride(2) == 1 and qkv.stride(0) == S * qkv.stride(1)
+            and n_heads % n_kv == 0 and qkv.stride(2) == 1 and qkv.stride(0) == S * qkv.stride(1) and qkv.stride(1) >= C
             and qkv.stride(1) % 8 == 0 and qkv.data_ptr() % 16 == 0):
         return _AttentionPacked.apply(qkv, n_heads, n_kv, hd)
     if _ATTN_BACKEND == "tcgen05" and qkv.is_cuda and (hd, qkv.dtype) not in _attn_fallback_seen:

@@ -248,3 +248,23 @@ def test_key_and_value_gradients_repeat_their_bits(B, S, H, KV, hd):
     grads = [torch.autograd.grad(OF.attention_packed(qkv, H, KV, hd), qkv, dout)[0][..., H * hd:] for _ in range(30)]
     for g in grads[1:]:
         assert torch.equal(g, grads[0])
+
+
+@pytest.mark.parametrize("B,S,H,KV,hd", [(2, 200, 4, 2, 64), (2, 256, 2, 1, 128)])
+def test_attention_of_rows_with_a_pitch(B, S, H, KV, hd):
+    """A packed projection whose rows lie further apart than its width (the gradient has rows of the same pitch), with an
+    incoming gradient off its 16-byte boundary."""
+    torch.manual_seed(S)
+    C = (H + 2 * KV) * hd
+    wide = torch.randn(B, S, C + 72, device=DEV).to(torch.bfloat16)
+    dout = torch.randn(B, S, H * hd, device=DEV).to(torch.bfloat16)
+    off = torch.empty(dout.numel() + 8, device=DEV, dtype=torch.bfloat16)[1:-7].view(dout.shape).copy_(dout)
+    outs = []
+    for qkv, do in ((wide[..., :C], off), (wide[..., :C].contiguous(), dout)):
+        qkv = qkv.detach().requires_grad_()
+        out = OF.attention_packed(qkv, H, KV, hd)
+        outs.append((out.detach(), torch.autograd.grad(out, qkv, do)[0]))
+    (a, ga), (b, gb) = outs
+    assert torch.equal(a, b)
+    # dQ is summed over two key blocks in order of arrival: the last bit of a bf16 value may differ
+    assert torch.equal(ga[..., H * hd:], gb[..., H * hd:]) and torch.allclose(ga.float(), gb.float(), rtol=2 ** -7, atol=1e-6)
