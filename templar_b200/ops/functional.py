@@ -937,6 +937,17 @@ class _AttentionBlock(torch.autograd.Function):
         return dx, dwqkv, dwo, None, None, None, None, None, None, None
 
 
+def _own_heads(width: int, n_heads: int, n_kv: int, hd: int) -> bool:
+    """Heads that the own attention kernels take, filling the packed projection's ``width`` exactly: the kernels address the
+    heads by their number and do not look at the width."""
+    return hd in OWN_HEAD_DIMS and n_heads % n_kv == 0 and width == (n_heads + 2 * n_kv) * hd
+
+
+def _rope_tables_ok(cos, sin, S: int, hd: int) -> bool:
+    return all(t.is_cuda and t.dtype == torch.float32 and t.is_contiguous() and t.dim() == 2 and t.shape[0] >= S
+               and t.shape[1] == hd // 2 and t.data_ptr() % 16 == 0 for t in (cos, sin))
+
+
 def attention_block(x, wqkv, wo, cos, sin, n_heads: int, n_kv: int, hd: int, main_grad_qkv=None, main_grad_wo=None):
     """Causal attention block without its norm and residual: ``attention(rope(x @ wqkv.T)) @ wo.T`` for the packed
     ``wqkv = [wq; wk; wv]``.  One autograd node on the own kernels, three elsewhere."""
@@ -946,13 +957,11 @@ def attention_block(x, wqkv, wo, cos, sin, n_heads: int, n_kv: int, hd: int, mai
         main_grad_wo = getattr(wo, "main_grad", None)
     B, S, K = x.shape
     if (FUSED_PROJECTIONS and _ATTN_BACKEND == "tcgen05" and _GEMM_BACKEND == "tcgen05_2sm" and _native_ok(x, wqkv, wo)
-            and x.dtype == torch.bfloat16 and hd in OWN_HEAD_DIMS and n_heads % n_kv == 0 and x.is_contiguous()
+            and x.dtype == torch.bfloat16 and _own_heads(wqkv.shape[0], n_heads, n_kv, hd) and x.is_contiguous()
             and wqkv.stride(1) == 1 and wo.stride(1) == 1 and wqkv.stride(0) % 8 == 0 and wo.stride(0) % 8 == 0 and K % 8 == 0
-            and wo.shape[0] % 8 == 0 and wo.shape[1] == n_heads * hd and cos.is_cuda and cos.dtype == torch.float32
-            and cos.is_contiguous() and sin.is_contiguous() and cos.shape[0] >= S and cos.shape[1] == hd // 2
-            and all(t.data_ptr() % 16 == 0 for t in (x, wqkv, wo, cos, sin))):
-        if (_buffers_ok((main_grad_qkv, wqkv), (main_grad_wo, wo)) and sin.dtype == torch.float32 and sin.shape == cos.shape
-                and wqkv.shape == ((n_heads + 2 * n_kv) * hd, K)):
+            and wqkv.shape[1] == K and wo.shape[0] % 8 == 0 and wo.shape[1] == n_heads * hd and _aligned(x, wqkv, wo)
+            and _rope_tables_ok(cos, sin, S, hd)):
+        if _buffers_ok((main_grad_qkv, wqkv), (main_grad_wo, wo)):
             return native.host().attention_block(x, wqkv, wo, main_grad_qkv, main_grad_wo, cos, sin, n_heads, n_kv, hd,
                                                  status_word(x.device).data_ptr())
         return _AttentionBlock.apply(x, wqkv, wo, main_grad_qkv, main_grad_wo, cos, sin, n_heads, n_kv, hd)
@@ -967,10 +976,8 @@ def rope_attention_projection(x, w, cos, sin, n_heads: int, n_kv: int, hd: int, 
         main_grad = getattr(w, "main_grad", None)
     B, S, K = x.shape
     if (FUSED_PROJECTIONS and _ATTN_BACKEND == "tcgen05" and _GEMM_BACKEND == "tcgen05_2sm" and _native_ok(x, w) and x.dtype == torch.bfloat16
-            and hd in OWN_HEAD_DIMS and n_heads % n_kv == 0 and x.is_contiguous() and w.stride(1) == 1
-            and w.stride(0) % 8 == 0 and K % 8 == 0 and w.shape[0] % 8 == 0 and cos.is_cuda and cos.dtype == torch.float32
-            and cos.is_contiguous() and sin.is_contiguous() and cos.shape[0] >= S and cos.shape[1] == hd // 2
-            and cos.data_ptr() % 16 == 0 and sin.data_ptr() % 16 == 0 and x.data_ptr() % 16 == 0 and w.data_ptr() % 16 == 0):
+            and _own_heads(w.shape[0], n_heads, n_kv, hd) and x.is_contiguous() and w.stride(1) == 1 and w.stride(0) % 8 == 0
+            and K % 8 == 0 and w.shape[1] == K and _aligned(x, w) and _rope_tables_ok(cos, sin, S, hd)):
         return _QKVRopeAttention.apply(x, w, main_grad, cos, sin, n_heads, n_kv, hd)
     qkv = rope(_Linear.apply(x, w, main_grad), cos, sin, n_heads + n_kv, hd)
     return attention_packed(qkv, n_heads, n_kv, hd)
@@ -982,9 +989,9 @@ _attn_fallback_seen: set = set()
 def attention_packed(qkv, n_heads: int, n_kv: int, hd: int):
     """Causal attention of ``qkv`` [B, S, (H + 2 KV) * hd] (q heads, k heads, v heads); returns [B, S, H * hd]."""
     B, S, C = qkv.shape
-    if (_ATTN_BACKEND == "tcgen05" and qkv.is_cuda and qkv.dtype == torch.bfloat16 and hd in OWN_HEAD_DIMS
-            and n_heads % n_kv == 0 and qkv.stride(2) == 1 and qkv.stride(0) == S * qkv.stride(1) and qkv.stride(1) >= C
-            and qkv.stride(1) % 8 == 0 and qkv.data_ptr() % 16 == 0):
+    if (_ATTN_BACKEND == "tcgen05" and qkv.is_cuda and qkv.dtype == torch.bfloat16 and _own_heads(C, n_heads, n_kv, hd)
+            and qkv.stride(2) == 1 and qkv.stride(0) == S * qkv.stride(1) and qkv.stride(1) >= C and qkv.stride(1) % 8 == 0
+            and qkv.data_ptr() % 16 == 0):
         return _AttentionPacked.apply(qkv, n_heads, n_kv, hd)
     if _ATTN_BACKEND == "tcgen05" and qkv.is_cuda and (hd, qkv.dtype) not in _attn_fallback_seen:
         # said once per shape class: a GPU run that silently uses the library kernel would misreport what ran
@@ -992,7 +999,7 @@ def attention_packed(qkv, n_heads: int, n_kv: int, hd: int):
         import warnings
 
         warnings.warn(f"attention_packed: head_dim {hd}, sequence {S}, dtype {qkv.dtype} is outside the own flash-attention "
-                      f"kernels (bf16, head_dim 64 or 128); using torch SDPA for it", stacklevel=2)
+                      f"kernels (bf16, head_dim 64 or 128, rows of whole heads); using torch SDPA for it", stacklevel=2)
     q, k, v = _split_qkv(qkv, n_heads, n_kv, hd)
     return attention(q, k, v).reshape(B, S, n_heads * hd)
 

@@ -268,3 +268,22 @@ def test_attention_of_rows_with_a_pitch(B, S, H, KV, hd):
     assert torch.equal(a, b)
     # dQ is summed over two key blocks in order of arrival: the last bit of a bf16 value may differ
     assert torch.equal(ga[..., H * hd:], gb[..., H * hd:]) and torch.allclose(ga.float(), gb.float(), rtol=2 ** -7, atol=1e-6)
+
+
+@pytest.mark.parametrize("S,hd", [(100, 64), (128, 64), (100, 128), (128, 128)])
+def test_attention_refuses_widths_that_do_not_fit_the_heads(S, hd):
+    H, KV, D = 4, 2, 256
+    C = (H + 2 * KV) * hd
+    bf = lambda *shape: torch.zeros(*shape, device=DEV, dtype=torch.bfloat16)      # noqa: E731
+    cos, sin = OF.rope_tables(S, hd, 10000.0, DEV)
+    for width in (C - hd, C + hd):
+        with pytest.raises(RuntimeError):
+            OF.attention_packed(bf(1, S, width), H, KV, hd)
+        with pytest.raises(RuntimeError):
+            OF.rope_attention_projection(bf(1, S, D), bf(width, D), cos, sin, H, KV, hd)
+        with pytest.raises(RuntimeError):
+            OF.attention_block(bf(1, S, D), bf(width, D), bf(D, H * hd), cos, sin, H, KV, hd)
+    with pytest.raises(ValueError):
+        OF.attention_block(bf(1, S, D), bf(C, D - 8), bf(D, H * hd), cos, sin, H, KV, hd)
+    with pytest.raises(ValueError):
+        OF.rope_attention_projection(bf(1, S, D), bf(C, D + 8), cos, sin, H, KV, hd)
