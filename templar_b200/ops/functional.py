@@ -467,7 +467,8 @@ class _LinearSwiGLU(torch.autograd.Function):
         gu = torch.empty(*x.shape[:-1], F2, dtype=x.dtype, device=x.device)
         h = None
         if (FUSED_PROJECTIONS and _native_ok(x2, w) and _GEMM_BACKEND == "tcgen05_2sm" and x.dtype == torch.bfloat16 and Fd % 128 == 0
-                and x2.is_contiguous() and w.stride(1) == 1 and w.stride(0) % 8 == 0 and x2.shape[1] % 8 == 0):
+                and x2.is_contiguous() and w.stride(1) == 1 and w.stride(0) % 8 == 0 and x2.shape[1] % 8 == 0
+                and w.shape[1] == x2.shape[1]):
             h = torch.empty(*x.shape[:-1], Fd, dtype=x.dtype, device=x.device)
             rc = native.lib().tplr_gemm2_swiglu(x2.data_ptr(), w.data_ptr(), gu.data_ptr(), h.data_ptr(), x2.shape[0], Fd,
                                                 x2.shape[1], x2.stride(0), w.stride(0), F2, Fd, status_word(x.device).data_ptr(),
@@ -550,8 +551,8 @@ def feed_forward(x, w13, w2, main_grad13=None, main_grad2=None):
     x2 = x.reshape(-1, x.shape[-1])
     if (FUSED_PROJECTIONS and _GEMM_BACKEND == "tcgen05_2sm" and _native_ok(x2, w13, w2) and x.dtype == torch.bfloat16
             and Fd % 128 == 0 and x2.is_contiguous() and w13.stride(1) == 1 and w2.stride(1) == 1 and w13.stride(0) % 8 == 0
-            and w2.stride(0) % 8 == 0 and x2.shape[1] % 8 == 0 and w2.shape[0] % 8 == 0
-            and all(t.data_ptr() % 16 == 0 for t in (x2, w13, w2))):
+            and w2.stride(0) % 8 == 0 and x2.shape[1] % 8 == 0 and w2.shape[0] % 8 == 0 and w13.shape[1] == x2.shape[1]
+            and w2.shape[1] == Fd and _aligned(x2, w13, w2)):
         if not torch.is_grad_enabled():          # nothing will ask for the packed projection: it is not stored
             h = torch.empty(x2.shape[0], Fd, dtype=x.dtype, device=x.device)
             native.check(native.lib().tplr_gemm2_swiglu(x2.data_ptr(), w13.data_ptr(), None, h.data_ptr(), x2.shape[0], Fd,
@@ -560,7 +561,7 @@ def feed_forward(x, w13, w2, main_grad13=None, main_grad2=None):
             y = torch.empty(*x.shape[:-1], w2.shape[0], dtype=x.dtype, device=x.device)
             gemm(h, w2, out=y.view(-1, w2.shape[0]))
             return y
-        if _buffers_ok((main_grad13, w13), (main_grad2, w2)) and w13.shape[1] == x2.shape[1] and w2.shape[1] == Fd:
+        if _buffers_ok((main_grad13, w13), (main_grad2, w2)):
             return native.host().feed_forward(x, w13, w2, main_grad13, main_grad2, status_word(x.device).data_ptr())
         return _FeedForward.apply(x, w13, w2, main_grad13, main_grad2)
     return _Linear.apply(linear_swiglu(x, w13, main_grad13), w2, main_grad2)

@@ -270,3 +270,14 @@ def test_accumulating_gemm_repeats_its_bits(M, N, K, backend):
     first = OF.gemm(A, B, a_mn=True, b_mn=True, out=before.clone(), accumulate=True)
     for _ in range(30):
         assert torch.equal(OF.gemm(A, B, a_mn=True, b_mn=True, out=before.clone(), accumulate=True), first)
+
+
+@pytest.mark.parametrize("grad", [True, False])
+def test_feed_forward_refuses_weights_of_other_widths(grad, backend):
+    """The fused projection takes its inner dimension from the input: a weight of another one would be read out of range."""
+    bf = lambda *shape: torch.zeros(*shape, device=DEV, dtype=torch.bfloat16)      # noqa: E731
+    x, w13, w2 = bf(64, 256), bf(512, 256), bf(256, 256)
+    with torch.set_grad_enabled(grad):
+        for a, b in ((bf(512, 248), w2), (bf(512, 264), w2), (w13, bf(256, 264)), (w13, bf(256, 248))):
+            with pytest.raises(ValueError):
+                OF.feed_forward(x, a, b)
