@@ -530,7 +530,8 @@ __global__ void __launch_bounds__(256) ns_scale_kernel(const T* __restrict__ g, 
   for (int i = threadIdx.x; i < n_partial; i += 256) s += partial[i];
   s = block_sum(s, red);
   const float den = __bfloat162float(__float2bfloat16(sqrtf(s) + eps));
-  const int i0 = blockIdx.y * 64, j0 = blockIdx.x * 64;
+  const unsigned across = (unsigned)(cols + 63) / 64;             // one grid dimension: either side may be the long one
+  const int i0 = (int)(blockIdx.x / across) * 64, j0 = (int)(blockIdx.x % across) * 64;
   const int vx = threadIdx.x & 7, vy = threadIdx.x >> 3;
 #pragma unroll
   for (int r = 0; r < 2; ++r) {
@@ -570,7 +571,7 @@ TPLR_API int tplr_ns_prepare(const void* g, int is_fp32, int rows, int cols, int
   cudaStream_t st = (cudaStream_t)stream;
   const long long n8 = (long long)rows * cols / 8;
   const int blocks = tplr_sm_count() * 4;
-  const dim3 grid((cols + 63) / 64, (rows + 63) / 64);
+  const unsigned grid = (unsigned)((cols + 63) / 64) * (unsigned)((rows + 63) / 64);
   if (is_fp32) {
     ns_sumsq_kernel<float><<<blocks, 256, 0, st>>>((const float*)g, n8, scratch);
     ns_scale_kernel<float><<<grid, 256, 0, st>>>((const float*)g, rows, cols, scratch, blocks, eps, transpose, (bf16*)out);

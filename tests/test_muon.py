@@ -301,3 +301,18 @@ def test_newton_schulz_repeats_its_bits(shape):
     first = newton_schulz(G)
     for _ in range(30):
         assert torch.equal(newton_schulz(G), first)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("rows,cols", [(65536 * 64 + 8, 8), (8, 65536 * 64 + 8)])
+def test_chain_operand_of_a_very_long_matrix(rows, cols):
+    """More 64-row (or 64-column) tiles than a grid's second dimension holds."""
+    from templar_b200.ops import native
+
+    G = torch.zeros(rows, cols, dtype=torch.bfloat16, device="cuda")
+    G.view(-1)[-9:] = 2.0
+    got = torch.full((cols, rows) if rows > cols else (rows, cols), 7.0, dtype=torch.bfloat16, device="cuda")
+    scratch = torch.empty(native.lib().tplr_sumsq_blocks(), device="cuda")
+    native.check(native.lib().tplr_ns_prepare(G.data_ptr(), 0, rows, cols, int(rows > cols), 1e-7, scratch.data_ptr(), got.data_ptr(),
+                                              native.stream_ptr()), "ns_prepare")
+    assert torch.equal(got, (G.t() if rows > cols else G) / 6.0)          # |G| = 6 exactly
