@@ -58,7 +58,9 @@ def _build_host(run) -> None:
     import torch
     from torch.utils.cpp_extension import include_paths
 
-    srcs = sorted(HOST_SRC.glob("*.cpp"))
+    srcs = host_sources()
+    if not srcs:
+        raise RuntimeError(f"no sources of the autograd nodes in {HOST_SRC}: the installed package is incomplete")
     out = host_path()
     if out.exists() and all(s.stat().st_mtime <= out.stat().st_mtime for s in srcs):
         return
@@ -73,23 +75,30 @@ def sources() -> list[Path]:
     return sorted(CSRC.glob("*.cu"))
 
 
-def _stale(obj: Path, src: Path, headers: list[Path]) -> bool:
+def host_sources() -> list[Path]:
+    return sorted(HOST_SRC.glob("*.cpp"))
+
+
+def headers() -> list[Path]:
+    return sorted([*CSRC.glob("*.cuh"), *CSRC.glob("*.h")])
+
+
+def _stale(obj: Path, src: Path) -> bool:
     if not obj.exists():
         return True
     t = obj.stat().st_mtime
-    return any(p.stat().st_mtime > t for p in [src, *headers])
+    return any(p.stat().st_mtime > t for p in [src, *headers()])
 
 
 def build(verbose: bool = False, force: bool = False) -> Path:
     """Compile and link the library; returns its path."""
     nvcc = _nvcc()
     LIBDIR.mkdir(exist_ok=True)
-    headers = sorted(CSRC.glob("*.cuh")) + sorted(CSRC.glob("*.h"))
     objs, jobs = [], []
     for src in sources():
         obj = LIBDIR / (src.stem + ".o")
         objs.append(obj)
-        if force or _stale(obj, src, headers):
+        if force or _stale(obj, src):
             extra = ["--use_fast_math"] if src.name in FAST_MATH_SOURCES else []
             cmd = [nvcc, *NVCC_FLAGS, *extra, "-I", str(CSRC), "-c", str(src), "-o", str(obj)]
             if verbose:
