@@ -4,7 +4,8 @@
 ``python -m templar_b200.ops.build`` (or :func:`build`) compiles every ``csrc/*.cu``
 translation unit with ``-gencode arch=compute_100a,code=sm_100a -lineinfo`` and links
 them into ``templar_b200/ops/_lib/libtplr_b200.so``.  nvcc cross-compiles without a GPU.
-Objects are rebuilt only when a source or header is newer than the object.
+Objects are rebuilt only when a source or header is newer than the object, the library when an object is newer, the
+extension module when its sources, its compiler call or PyTorch have changed.
 """
 
 from __future__ import annotations
@@ -29,6 +30,7 @@ NVCC_FLAGS = [
     "-Xcompiler", "-fPIC,-fvisibility=hidden",
     "--expt-relaxed-constexpr",
 ]
+HOST_FLAGS = ["-O2", "-std=c++17", "-fPIC", "-shared", "-fvisibility=hidden"]
 # Approximate intrinsics and flush-to-zero only where the arithmetic is a softmax in base 2 (the flash
 # attention kernels).  The loss, the norms, the optimizer, the quantiser and the compression kernels are
 # compiled with IEEE division / square root and keep denormals; where they want a fast exponential they
@@ -51,26 +53,6 @@ def host_path() -> Path:
     return LIBDIR / HOSTNAME
 
 
-def _build_host(run) -> None:
-    """The extension module of the autograd nodes: plain C++, no CUDA compiler involved."""
-    import sysconfig
-
-    import torch
-    from torch.utils.cpp_extension import include_paths
-
-    srcs = host_sources()
-    if not srcs:
-        raise RuntimeError(f"no sources of the autograd nodes in {HOST_SRC}: the installed package is incomplete")
-    out = host_path()
-    if out.exists() and all(s.stat().st_mtime <= out.stat().st_mtime for s in srcs):
-        return
-    inc = [x for p in [*include_paths("cuda"), sysconfig.get_paths()["include"]] for x in ("-isystem", p)]
-    tmp = out.with_suffix(".so.tmp")
-    run([os.environ.get("CXX", "g++"), "-O2", "-std=c++17", "-fPIC", "-shared", "-fvisibility=hidden", *inc, *map(str, srcs), "-o",
-         str(tmp), "-L" + str(Path(torch.__file__).parent / "lib"), "-lc10", "-ltorch_cpu", "-ltorch", "-ltorch_python", "-lc10_cuda"])
-    os.replace(tmp, out)
-
-
 def sources() -> list[Path]:
     return sorted(CSRC.glob("*.cu"))
 
@@ -90,8 +72,56 @@ def _stale(obj: Path, src: Path) -> bool:
     return any(p.stat().st_mtime > t for p in [src, *headers()])
 
 
-def build(verbose: bool = False, force: bool = False) -> Path:
-    """Compile and link the library; returns its path."""
+def _run(cmd: list[str]) -> str:
+    r = subprocess.run(cmd, capture_output=True, text=True)
+    if r.returncode != 0:
+        raise RuntimeError("compiler failed: " + " ".join(cmd) + "\n" + r.stdout + r.stderr)
+    return r.stderr
+
+
+def _host_key() -> str:
+    """What the extension module depends on beside its sources: a module of another PyTorch must not be loaded."""
+    import torch
+
+    return "\n".join([torch.__version__, sys.version, *HOST_FLAGS])
+
+
+def _host_key_path() -> Path:
+    return host_path().with_suffix(".key")
+
+
+def host_usable() -> bool:
+    """The extension module is there and not known to be of another PyTorch or Python."""
+    key = _host_key_path()
+    return host_path().exists() and (not key.exists() or key.read_text() == _host_key())
+
+
+def build_host(force: bool = False) -> Path:
+    """Compile the extension module of the autograd nodes (plain C++, no CUDA compiler involved); returns its path."""
+    import sysconfig
+
+    import torch
+
+    srcs = host_sources()
+    if not srcs:
+        raise RuntimeError(f"no sources of the autograd nodes in {HOST_SRC}: the installed package is incomplete")
+    out = host_path()
+    if not force and host_usable() and _host_key_path().exists() and not any(_stale(out, s) for s in srcs):
+        return out
+    from torch.utils.cpp_extension import include_paths
+
+    LIBDIR.mkdir(exist_ok=True)
+    inc = [x for p in [*include_paths("cuda"), sysconfig.get_paths()["include"]] for x in ("-isystem", p)]
+    tmp = out.with_suffix(".so.tmp")
+    _run([os.environ.get("CXX", "g++"), *HOST_FLAGS, *inc, *map(str, srcs), "-o", str(tmp),
+          "-L" + str(Path(torch.__file__).parent / "lib"), "-lc10", "-ltorch_cpu", "-ltorch", "-ltorch_python", "-lc10_cuda"])
+    os.replace(tmp, out)
+    _host_key_path().write_text(_host_key())
+    return out
+
+
+def build_library(verbose: bool = False, force: bool = False) -> Path:
+    """Compile and link the kernel library; returns its path."""
     nvcc = _nvcc()
     LIBDIR.mkdir(exist_ok=True)
     objs, jobs = [], []
@@ -104,24 +134,27 @@ def build(verbose: bool = False, force: bool = False) -> Path:
             if verbose:
                 cmd.insert(1, "-Xptxas=-v")
             jobs.append(cmd)
-
-    def run(cmd):
-        r = subprocess.run(cmd, capture_output=True, text=True)
-        if r.returncode != 0:
-            raise RuntimeError("compiler failed: " + " ".join(cmd) + "\n" + r.stdout + r.stderr)
-        return r.stderr
-
     if jobs:
         with ThreadPoolExecutor(max_workers=min(8, len(jobs))) as ex:
-            for out in ex.map(run, jobs):
+            for out in ex.map(_run, jobs):
                 if verbose and out:
                     print(out, file=sys.stderr)
-    _build_host(run)
     lib = lib_path()
-    if jobs or not lib.exists():
+    # an object may be newer than the library without having been compiled here: a build that failed later leaves it
+    if not lib.exists() or any(o.stat().st_mtime > lib.stat().st_mtime for o in objs):
         tmp = lib.with_suffix(".so.tmp")          # link beside the target, then rename: readers never see a partial file
-        run([nvcc, "-shared", "-o", str(tmp), *map(str, objs), "-lcudart"])
+        _run([nvcc, "-shared", "-o", str(tmp), *map(str, objs), "-lcudart"])
         os.replace(tmp, lib)
+    return lib
+
+
+def build(verbose: bool = False, force: bool = False) -> Path:
+    """Build both, one beside the other; returns the kernel library's path.  The library is linked whether or not the
+    extension module could be compiled."""
+    with ThreadPoolExecutor(max_workers=1) as ex:
+        host = ex.submit(build_host, force)
+        lib = build_library(verbose, force)
+        host.result()
     return lib
 
 

@@ -47,7 +47,7 @@ def lib() -> ctypes.CDLL:
         if _lib is None:
             path = _build.lib_path()
             if not path.exists():
-                _build.build()
+                _build.build_library()
             _lib = ctypes.CDLL(str(path))
             _declare(_lib)
     return _lib
@@ -65,8 +65,8 @@ def host():
             import importlib.util
 
             path = _build.host_path()
-            if not path.exists():
-                _build.build()
+            if not _build.host_usable():
+                _build.build_host()
             loader = importlib.machinery.ExtensionFileLoader("tplr_host", str(path))
             mod = importlib.util.module_from_spec(importlib.util.spec_from_loader("tplr_host", loader))
             loader.exec_module(mod)
