@@ -14,6 +14,7 @@ import os
 import shutil
 import subprocess
 import sys
+import zlib
 from concurrent.futures import ThreadPoolExecutor
 from pathlib import Path
 
@@ -65,11 +66,13 @@ def headers() -> list[Path]:
     return sorted([*CSRC.glob("*.cuh"), *CSRC.glob("*.h")])
 
 
-def _stale(obj: Path, src: Path) -> bool:
-    if not obj.exists():
-        return True
-    t = obj.stat().st_mtime
-    return any(p.stat().st_mtime > t for p in [src, *headers()])
+def _stale(out: Path, *made_from: Path) -> bool:
+    return not out.exists() or any(p.stat().st_mtime > out.stat().st_mtime for p in made_from)
+
+
+def _abi_flag() -> str:
+    """The number that the library and the extension module must agree on: made from the declarations they share."""
+    return f"-DTPLR_ABI={zlib.crc32((CSRC / 'entries.h').read_bytes()) & 0x7FFFFFFF}"
 
 
 def _run(cmd: list[str]) -> str:
@@ -83,7 +86,7 @@ def _host_key() -> str:
     """What the extension module depends on beside its sources: a module of another PyTorch must not be loaded."""
     import torch
 
-    return "\n".join([torch.__version__, sys.version, *HOST_FLAGS])
+    return "\n".join([torch.__version__, sys.version, *HOST_FLAGS, _abi_flag()])
 
 
 def _host_key_path() -> Path:
@@ -106,14 +109,14 @@ def build_host(force: bool = False) -> Path:
     if not srcs:
         raise RuntimeError(f"no sources of the autograd nodes in {HOST_SRC}: the installed package is incomplete")
     out = host_path()
-    if not force and host_usable() and _host_key_path().exists() and not any(_stale(out, s) for s in srcs):
+    if not force and host_usable() and _host_key_path().exists() and not _stale(out, *srcs):
         return out
     from torch.utils.cpp_extension import include_paths
 
     LIBDIR.mkdir(exist_ok=True)
     inc = [x for p in [*include_paths("cuda"), sysconfig.get_paths()["include"]] for x in ("-isystem", p)]
     tmp = out.with_suffix(".so.tmp")
-    _run([os.environ.get("CXX", "g++"), *HOST_FLAGS, *inc, *map(str, srcs), "-o", str(tmp),
+    _run([os.environ.get("CXX", "g++"), *HOST_FLAGS, _abi_flag(), *inc, *map(str, srcs), "-o", str(tmp),
           "-L" + str(Path(torch.__file__).parent / "lib"), "-lc10", "-ltorch_cpu", "-ltorch", "-ltorch_python", "-lc10_cuda"])
     os.replace(tmp, out)
     _host_key_path().write_text(_host_key())
@@ -128,9 +131,9 @@ def build_library(verbose: bool = False, force: bool = False) -> Path:
     for src in sources():
         obj = LIBDIR / (src.stem + ".o")
         objs.append(obj)
-        if force or _stale(obj, src):
+        if force or _stale(obj, src, *headers()):
             extra = ["--use_fast_math"] if src.name in FAST_MATH_SOURCES else []
-            cmd = [nvcc, *NVCC_FLAGS, *extra, "-I", str(CSRC), "-c", str(src), "-o", str(obj)]
+            cmd = [nvcc, *NVCC_FLAGS, *extra, _abi_flag(), "-I", str(CSRC), "-c", str(src), "-o", str(obj)]
             if verbose:
                 cmd.insert(1, "-Xptxas=-v")
             jobs.append(cmd)

@@ -7,6 +7,7 @@
 #include <cuda_runtime.h>
 #include <cuda_bf16.h>
 #include <stdint.h>
+#include "entries.h"
 
 #define TPLR_API extern "C" __attribute__((visibility("default")))
 

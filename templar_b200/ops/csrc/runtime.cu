@@ -8,6 +8,9 @@
 #include "common.cuh"
 #include <string.h>
 
+// The number of the entry declarations that this library was built from (see entries.h).
+TPLR_API int tplr_abi() { return TPLR_ABI; }
+
 TPLR_API int tplr_heap_alloc(unsigned long long bytes, void** out) {
   TPLR_ENTER();
   void* p = nullptr;

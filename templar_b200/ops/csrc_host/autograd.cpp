@@ -13,6 +13,8 @@
 
 #include <atomic>
 
+#include "../csrc/entries.h"
+
 namespace {
 
 using torch::Tensor;
@@ -25,21 +27,20 @@ std::atomic<ll> g_launches{0};
 
 // C entry points of the kernel library
 struct Entries {
-  int (*add_rmsnorm_fwd)(const void*, const void*, const void*, void*, void*, float*, ll, int, float, void*);
-  int (*add_rmsnorm_bwd)(const void*, const void*, const void*, const float*, const void*, void*, float*, ll, int, unsigned*, void*);
-  int (*gemm)(const void*, const void*, void*, int, int, int, ll, ll, ll, int, int, int, unsigned*, int, void*);
-  int (*acc_splits)(int, int, int);
-  int (*acc_split)(const void*, const void*, float*, float*, int, int, int, ll, ll, ll, int, int, unsigned*, void*);
-  int (*out_splits)(int, int, int);
-  int (*gemm_split)(const void*, const void*, void*, float*, int, int, int, ll, ll, ll, int, int, unsigned*, void*);
-  int (*swiglu)(const void*, const void*, void*, void*, int, int, int, ll, ll, ll, ll, unsigned*, void*);
-  int (*swiglu_bwd)(const void*, const void*, const void*, void*, int, int, int, ll, ll, ll, ll, unsigned*, void*);
-  int (*gemm_rope)(const void*, const void*, void*, int, int, int, ll, ll, ll, const float*, const float*, int, int, int, unsigned*, void*);
-  int (*attention_fwd)(const void*, void*, float*, int, int, int, int, int, ll, ll, float, unsigned*, void*);
-  int (*attn_dout)(const void*, const void*, const void*, void*, float*, int, int, int, int, int, ll, ll, ll, ll, unsigned*, void*);
-  int (*bwd_scratch_cols)(int, int, int, int, int);
-  int (*attention_bwd)(const void*, const void*, const void*, const float*, float*, float*, void*, int, int, int, int, int, ll, ll,
-                       float, const float*, const float*, unsigned*, void*);
+  decltype(&tplr_add_rmsnorm_fwd) add_rmsnorm_fwd;
+  decltype(&tplr_add_rmsnorm_bwd_v2) add_rmsnorm_bwd;
+  decltype(&tplr_gemm2_bf16) gemm;
+  decltype(&tplr_gemm2_acc_splits) acc_splits;
+  decltype(&tplr_gemm2_acc_split) acc_split;
+  decltype(&tplr_gemm2_out_splits) out_splits;
+  decltype(&tplr_gemm2_bf16_split) gemm_split;
+  decltype(&tplr_gemm2_swiglu) swiglu;
+  decltype(&tplr_gemm2_swiglu_bwd) swiglu_bwd;
+  decltype(&tplr_gemm2_rope) gemm_rope;
+  decltype(&tplr_attention_fwd) attention_fwd;
+  decltype(&tplr_gemm2_attn_dout) attn_dout;
+  decltype(&tplr_attention_bwd_scratch_cols) bwd_scratch_cols;
+  decltype(&tplr_attention_bwd_unrope_delta) attention_bwd;
 } E;
 
 void bind(const std::string& path) {
@@ -50,6 +51,9 @@ void bind(const std::string& path) {
     TORCH_CHECK(p, name, " is missing in ", path);
     fn = reinterpret_cast<std::decay_t<decltype(fn)>>(p);
   };
+  decltype(&tplr_abi) abi;
+  get(abi, "tplr_abi");
+  TORCH_CHECK(abi() == TPLR_ABI, path, " was built from other entry declarations than the autograd nodes; build both again");
   get(E.add_rmsnorm_fwd, "tplr_add_rmsnorm_fwd");
   get(E.add_rmsnorm_bwd, "tplr_add_rmsnorm_bwd_v2");
   get(E.gemm, "tplr_gemm2_bf16");

@@ -27,6 +27,7 @@ def tree(monkeypatch, tmp_path):
     for d in ("csrc", "csrc_host", "_lib"):
         (tmp_path / d).mkdir()
     (tmp_path / "csrc" / "a.cu").write_text("")
+    (tmp_path / "csrc" / "entries.h").write_text("")
     (tmp_path / "csrc_host" / "b.cpp").write_text("")
     for name in ("nvcc", "cxx"):
         f = tmp_path / name
@@ -99,3 +100,30 @@ def test_missing_host_sources_are_named(tree):
     with pytest.raises(RuntimeError, match="no sources of the autograd nodes"):
         B.build()
     assert calls() == ["nvcc", "nvcc"]                         # the library is built all the same
+
+
+def test_changed_declarations_rebuild_both(tree):
+    root, calls = tree
+    B.build()
+    calls()
+    (root / "csrc" / "entries.h").write_text("int changed();")
+    os.utime(root / "csrc" / "entries.h", (B.lib_path().stat().st_mtime + 10,) * 2)
+    B.build()
+    assert calls() == ["cxx", "nvcc", "nvcc"]
+
+
+@pytest.mark.parametrize("entry", ["int tplr_abi() { return -1; }", "int other() { return 0; }"])
+def test_nodes_refuse_a_library_of_other_declarations(entry, tmp_path):
+    """Before any of its entries is taken: a changed argument list would hand shifted arguments to a kernel."""
+    import shutil
+    import subprocess
+
+    from templar_b200.ops import native
+
+    if shutil.which("gcc") is None:
+        pytest.skip("no C compiler for the stand-in library")
+    (tmp_path / "l.c").write_text(entry)
+    subprocess.run(["gcc", "-shared", "-fPIC", "-o", str(tmp_path / "l.so"), str(tmp_path / "l.c")], check=True)
+    with pytest.raises(RuntimeError, match="entry declarations|tplr_abi is missing"):
+        native.host().bind(str(tmp_path / "l.so"))
+    native.host().bind(str(B.lib_path()))
