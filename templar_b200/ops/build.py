@@ -115,7 +115,7 @@ def build_host(force: bool = False) -> Path:
 
     LIBDIR.mkdir(exist_ok=True)
     inc = [x for p in [*include_paths("cuda"), sysconfig.get_paths()["include"]] for x in ("-isystem", p)]
-    tmp = out.with_suffix(".so.tmp")
+    tmp = out.with_suffix(f".{os.getpid()}.tmp")       # ranks that start together may all build
     _run([os.environ.get("CXX", "g++"), *HOST_FLAGS, _abi_flag(), *inc, *map(str, srcs), "-o", str(tmp),
           "-L" + str(Path(torch.__file__).parent / "lib"), "-lc10", "-ltorch_cpu", "-ltorch", "-ltorch_python", "-lc10_cuda"])
     os.replace(tmp, out)
@@ -145,7 +145,7 @@ def build_library(verbose: bool = False, force: bool = False) -> Path:
     lib = lib_path()
     # an object may be newer than the library without having been compiled here: a build that failed later leaves it
     if not lib.exists() or any(o.stat().st_mtime > lib.stat().st_mtime for o in objs):
-        tmp = lib.with_suffix(".so.tmp")          # link beside the target, then rename: readers never see a partial file
+        tmp = lib.with_suffix(f".{os.getpid()}.tmp")          # link beside the target, then rename: readers never see a partial file
         _run([nvcc, "-shared", "-o", str(tmp), *map(str, objs), "-lcudart"])
         os.replace(tmp, lib)
     return lib

@@ -22,7 +22,7 @@ from . import build as _build
 
 _lock = threading.Lock()
 _lib = None
-_host = None
+_host = None              # the module, or False once it proved unavailable
 _launches = 0             # kernel-launching native calls made through check(); see launch_count below
 
 
@@ -54,25 +54,40 @@ def lib() -> ctypes.CDLL:
 
 
 def host():
-    """The extension module with the autograd nodes of the block's operators (``csrc_host/autograd.cpp``)."""
+    """The extension module with the autograd nodes of the block's operators (``csrc_host/autograd.cpp``), or None where it
+    can neither be loaded nor built: said once, after which the operators keep their Python nodes, which launch the same
+    kernels.  An error under ``TPLR_STRICT_NATIVE=1``."""
     global _host
     if _host is not None:
-        return _host
+        return _host or None
     lib()
     with _lock:
         if _host is None:
-            import importlib.machinery
-            import importlib.util
+            try:
+                _host = _load_host()
+            except (RuntimeError, OSError, ImportError) as e:
+                import os
+                import warnings
 
-            path = _build.host_path()
-            if not _build.host_usable():
-                _build.build_host()
-            loader = importlib.machinery.ExtensionFileLoader("tplr_host", str(path))
-            mod = importlib.util.module_from_spec(importlib.util.spec_from_loader("tplr_host", loader))
-            loader.exec_module(mod)
-            mod.bind(str(_build.lib_path()))
-            _host = mod
-    return _host
+                if os.environ.get("TPLR_STRICT_NATIVE") == "1":
+                    raise
+                _host = False
+                warnings.warn(f"the autograd nodes in C++ are not available ({str(e)[:500]}); using the Python nodes (same "
+                              f"kernels, more host time)", RuntimeWarning, stacklevel=3)
+    return _host or None
+
+
+def _load_host():
+    import importlib.machinery
+    import importlib.util
+
+    if not _build.host_usable():
+        _build.build_host()
+    loader = importlib.machinery.ExtensionFileLoader("tplr_host", str(_build.host_path()))
+    mod = importlib.util.module_from_spec(importlib.util.spec_from_loader("tplr_host", loader))
+    loader.exec_module(mod)
+    mod.bind(str(_build.lib_path()))
+    return mod
 
 
 def _declare(L: ctypes.CDLL) -> None:
@@ -160,12 +175,12 @@ class _Module(types.ModuleType):
     @property
     def launch_count(self) -> int:
         """Kernel-launching native calls made by this process, from here and from the autograd nodes in C++."""
-        return _launches + (_host.launches() if _host is not None else 0)
+        return _launches + (_host.launches() if _host else 0)
 
     @launch_count.setter
     def launch_count(self, n: int) -> None:
         global _launches
-        _launches = n - (_host.launches() if _host is not None else 0)
+        _launches = n - (_host.launches() if _host else 0)
 
 
 sys.modules[__name__].__class__ = _Module

@@ -127,3 +127,28 @@ def test_nodes_refuse_a_library_of_other_declarations(entry, tmp_path):
     with pytest.raises(RuntimeError, match="entry declarations|tplr_abi is missing"):
         native.host().bind(str(tmp_path / "l.so"))
     native.host().bind(str(B.lib_path()))
+
+
+def test_operators_keep_their_python_nodes_without_the_extension_module(monkeypatch):
+    """Said once; an error where nothing but the native path is wanted."""
+    from templar_b200.ops import native
+
+    def broken(*a):
+        raise RuntimeError("compiler failed: no such thing")
+
+    monkeypatch.setattr(native, "_host", None)
+    monkeypatch.setattr(B, "host_usable", lambda: False)
+    monkeypatch.setattr(B, "build_host", broken)
+    monkeypatch.setenv("TPLR_STRICT_NATIVE", "1")
+    with pytest.raises(RuntimeError, match="compiler failed"):
+        native.host()
+    monkeypatch.delenv("TPLR_STRICT_NATIVE")
+    with pytest.warns(RuntimeWarning, match="using the Python nodes"):
+        assert native.host() is None
+    import warnings
+
+    with warnings.catch_warnings():
+        warnings.simplefilter("error")
+        assert native.host() is None
+    native.launch_count = 5
+    assert native.launch_count == 5
