@@ -679,3 +679,56 @@ def test_norms_refuse_rows_of_no_elements():
         OF.add_rmsnorm(x, x, w)
     with pytest.raises(RuntimeError):
         native.host().rmsnorm(x, w, None, 1e-5, 0)
+
+
+def _node_case(op, T, with_buffers):
+    """(function of the operator on fresh leaves, incoming gradients) for a node test; one key block, so that dQ has one addend."""
+    g = torch.Generator(device=DEV).manual_seed(T)
+    bf = lambda *s: torch.randn(*s, generator=g, device=DEV).to(torch.bfloat16)      # noqa: E731
+    D, Fd, H, KV, hd = 256, 384, 4, 2, 64
+    cos, sin = OF.rope_tables(T, hd, 10000.0, DEV)
+    make = {
+        "rmsnorm": lambda: ([bf(T, D), bf(D)], lambda x, w, *m: (OF.rmsnorm(x, w, 1e-5, *m),), [1]),
+        "add_rmsnorm": lambda: ([bf(T, D), bf(T, D), bf(D)], lambda a, b, w, *m: OF.add_rmsnorm(a, b, w, 1e-5, *m), [2]),
+        "linear": lambda: ([bf(2, T, D), bf(Fd, D)], lambda x, w, *m: (OF.linear(x, w, *m),), [1]),
+        "feed_forward": lambda: ([bf(T, D), bf(2 * Fd, D), bf(D, Fd)], lambda x, a, b, *m: (OF.feed_forward(x, a, b, *m),), [1, 2]),
+        "attention_block": lambda: ([bf(2, T, D), bf((H + 2 * KV) * hd, D), bf(D, H * hd)],
+                                    lambda x, a, b, *m: (OF.attention_block(x, a, b, cos, sin, H, KV, hd, *m),), [1, 2]),
+    }[op]
+    leaves, fn, weights = make()
+    buffers = [torch.randn(leaves[i].shape, generator=g, device=DEV) for i in weights] if with_buffers else []
+    grads = None
+
+    def run():
+        nonlocal grads
+        ls = [t.clone().requires_grad_() for t in leaves]
+        bs = [b.clone() for b in buffers]
+        out = fn(*ls, *bs)
+        if grads is None:
+            grads = [bf(*o.shape) for o in out]
+        name = type(out[0].grad_fn).__name__
+        got = torch.autograd.grad(out, ls, grads, allow_unused=True)
+        return name, [o.detach() for o in out], list(got), bs
+
+    return run
+
+
+@pytest.mark.parametrize("with_buffers", [False, True])
+@pytest.mark.parametrize("T", [7, 128])
+@pytest.mark.parametrize("op", ["rmsnorm", "add_rmsnorm", "linear", "feed_forward", "attention_block"])
+def test_nodes_in_python_and_cpp_give_the_same_bits(op, T, with_buffers, monkeypatch):
+    """The same operands through both nodes of an operator: outputs, input gradients and weight gradients, returned or added
+    into a buffer."""
+    run = _node_case(op, T, with_buffers)
+    name, out, got, buf = run()
+    assert name == "CppFunction"
+    monkeypatch.setattr(native, "host", lambda: None)
+    name_p, out_p, got_p, buf_p = run()
+    assert name_p != "CppFunction"
+    for a, b in zip(out + got + buf, out_p + got_p + buf_p):
+        assert (a is None) == (b is None)
+        if a is not None and "norm" in op and a.dim() == 1:
+            # a norm's weight gradient is added over blocks with atomics: T products below 30 in fp32, then bf16
+            assert torch.allclose(a.float(), b.float(), atol=30 * T * 2 ** -23, rtol=2 ** -7 if a.dtype == torch.bfloat16 else 0)
+        elif a is not None:
+            assert torch.equal(a, b)
