@@ -75,7 +75,8 @@ void check(int err, const char* what) {
   TORCH_CHECK(err == 0, what, " failed with CUDA error ", err);
 }
 void* stream() { return c10::cuda::getCurrentCUDAStream().stream(); }
-unsigned* word(int64_t status) { return reinterpret_cast<unsigned*>(status); }
+// the device's status word, as the kernels take it; the nodes keep the tensor and no pointer into it
+unsigned* word(const Tensor& status) { return reinterpret_cast<unsigned*>(status.data_ptr()); }
 
 // A gradient as the kernels read it: dense, on a 16-byte boundary.
 Tensor dense(const Tensor& t) {
@@ -96,7 +97,7 @@ void keep(AutogradContext* ctx, const char* key, const Aside& a) {
 }
 
 // out = op(a) op(b)^T as functional.gemm; epi 0: store bf16, 1: add into fp32
-void gemm(const Tensor& a, const Tensor& b, const Tensor& out, bool a_mn, bool b_mn, int epi, int64_t status) {
+void gemm(const Tensor& a, const Tensor& b, const Tensor& out, bool a_mn, bool b_mn, int epi, const Tensor& status) {
   const ll M = a_mn ? a.size(1) : a.size(0), K = a_mn ? a.size(0) : a.size(1), N = b_mn ? b.size(1) : b.size(0);
   const ll plane = (M + 31) / 32 * 32 * N;             // workspace of one part of K, where K is cut
   if (epi == 0) {
@@ -121,7 +122,7 @@ void gemm(const Tensor& a, const Tensor& b, const Tensor& out, bool a_mn, bool b
         "tplr_gemm_bf16");
 }
 // dW of y = x W^T: added into the gradient buffer when there is one, else returned when wanted
-Tensor weight_grad(const Tensor& buffer, const Tensor& dy2, const Tensor& x2, const Tensor& w, bool wanted, int64_t status) {
+Tensor weight_grad(const Tensor& buffer, const Tensor& dy2, const Tensor& x2, const Tensor& w, bool wanted, const Tensor& status) {
   if (buffer.defined()) {
     gemm(dy2, x2, buffer, true, true, 1, status);
     return Tensor();
@@ -142,7 +143,7 @@ ll count_rows(const Tensor& t, ll D) {
 // inputs: x (or res, delta), w, buffer, eps, status
 variable_list norm_backward(AutogradContext* ctx, const Tensor& dh, const Tensor& dy_in, const Tensor& h, const Tensor& w,
                             const Tensor& rstd, int w_index) {
-  const int64_t status = ctx->saved_data["status"].toInt();
+  const Tensor status = aside(ctx, "status");
   const Tensor buffer = aside(ctx, "buffer");
   const ll D = h.size(-1), T = count_rows(h, D);
   const Tensor dy = dy_in.defined() ? dense(dy_in) : at::zeros_like(h);
@@ -156,7 +157,7 @@ variable_list norm_backward(AutogradContext* ctx, const Tensor& dh, const Tensor
 }
 
 struct RMSNorm : Function<RMSNorm> {
-  static Tensor forward(AutogradContext* ctx, const Tensor& x, const Tensor& w, Aside buffer, double eps, int64_t status) {
+  static Tensor forward(AutogradContext* ctx, const Tensor& x, const Tensor& w, Aside buffer, double eps, Aside status) {
     const ll D = x.size(-1), T = count_rows(x, D);
     Tensor y = at::empty_like(x), rstd = f32({T}, x);
     check(E.add_rmsnorm_fwd(x.data_ptr(), nullptr, w.data_ptr(), nullptr, y.data_ptr(), rstd.data_ptr<float>(), T, (int)D, (float)eps,
@@ -164,7 +165,7 @@ struct RMSNorm : Function<RMSNorm> {
           "rmsnorm_fwd");
     ctx->save_for_backward({x, w, rstd});
     keep(ctx, "buffer", buffer);
-    ctx->saved_data["status"] = status;
+    keep(ctx, "status", status);
     return y;
   }
   static variable_list backward(AutogradContext* ctx, variable_list g) {
@@ -176,7 +177,7 @@ struct RMSNorm : Function<RMSNorm> {
 
 struct AddRMSNorm : Function<AddRMSNorm> {
   static variable_list forward(AutogradContext* ctx, const Tensor& res, const Tensor& delta, const Tensor& w, Aside buffer, double eps,
-                               int64_t status) {
+                               Aside status) {
     const ll D = res.size(-1), T = count_rows(res, D);
     Tensor h = at::empty_like(res), y = at::empty_like(res), rstd = f32({T}, res);
     check(E.add_rmsnorm_fwd(res.data_ptr(), delta.data_ptr(), w.data_ptr(), h.data_ptr(), y.data_ptr(), rstd.data_ptr<float>(), T,
@@ -184,7 +185,7 @@ struct AddRMSNorm : Function<AddRMSNorm> {
           "add_rmsnorm_fwd");
     ctx->save_for_backward({h, w, rstd});
     keep(ctx, "buffer", buffer);
-    ctx->saved_data["status"] = status;
+    keep(ctx, "status", status);
     return {h, y};
   }
   static variable_list backward(AutogradContext* ctx, variable_list g) {
@@ -196,19 +197,19 @@ struct AddRMSNorm : Function<AddRMSNorm> {
 
 // ------------------------------------------------------------------------------------------ projections
 struct Linear : Function<Linear> {
-  static Tensor forward(AutogradContext* ctx, const Tensor& x, const Tensor& w, Aside buffer, int64_t status) {
+  static Tensor forward(AutogradContext* ctx, const Tensor& x, const Tensor& w, Aside buffer, Aside status) {
     auto shape = x.sizes().vec();
     shape.back() = w.size(0);
     Tensor y = bf16(shape, x);
-    gemm(rows(x), w, y.view({-1, w.size(0)}), false, false, 0, status);
+    gemm(rows(x), w, y.view({-1, w.size(0)}), false, false, 0, status.t);
     ctx->save_for_backward({x, w});
     keep(ctx, "buffer", buffer);
-    ctx->saved_data["status"] = status;
+    keep(ctx, "status", status);
     return y;
   }
   static variable_list backward(AutogradContext* ctx, variable_list g) {
     auto s = ctx->get_saved_variables();
-    const int64_t status = ctx->saved_data["status"].toInt();
+    const Tensor status = aside(ctx, "status");
     const Tensor dy2 = dense(rows(g[0])), x2 = rows(s[0]);
     Tensor dx;
     if (ctx->needs_input_grad(0)) {
@@ -221,27 +222,27 @@ struct Linear : Function<Linear> {
 
 struct FeedForward : Function<FeedForward> {
   static Tensor forward(AutogradContext* ctx, const Tensor& x, const Tensor& w13, const Tensor& w2, Aside buffer13, Aside buffer2,
-                        int64_t status) {
+                        Aside status) {
     const Tensor x2 = rows(x);
     const ll T = x2.size(0), F2 = w13.size(0), F = F2 / 2;
     Tensor gu = bf16({T, F2}, x), h = bf16({T, F}, x);
     check(E.swiglu(x2.data_ptr(), w13.data_ptr(), gu.data_ptr(), h.data_ptr(), (int)T, (int)F, (int)x2.size(1), x2.stride(0),
-                   w13.stride(0), F2, F, word(status), stream()),
+                   w13.stride(0), F2, F, word(status.t), stream()),
           "gemm2_swiglu");
     auto shape = x.sizes().vec();
     shape.back() = w2.size(0);
     Tensor y = bf16(shape, x);
-    gemm(h, w2, y.view({-1, w2.size(0)}), false, false, 0, status);
+    gemm(h, w2, y.view({-1, w2.size(0)}), false, false, 0, status.t);
     ctx->save_for_backward({x, w13, w2, gu, h});
     keep(ctx, "buffer13", buffer13);
     keep(ctx, "buffer2", buffer2);
-    ctx->saved_data["status"] = status;
+    keep(ctx, "status", status);
     return y;
   }
   static variable_list backward(AutogradContext* ctx, variable_list g) {
     auto s = ctx->get_saved_variables();
     const Tensor &x = s[0], &w13 = s[1], &w2 = s[2], &gu = s[3], &h = s[4];
-    const int64_t status = ctx->saved_data["status"].toInt();
+    const Tensor status = aside(ctx, "status");
     const Tensor dy2 = dense(rows(g[0])), x2 = rows(x);
     const ll T = gu.size(0), F = gu.size(1) / 2;
     Tensor dgu = at::empty_like(gu);
@@ -261,31 +262,33 @@ struct FeedForward : Function<FeedForward> {
 
 struct AttentionBlock : Function<AttentionBlock> {
   static Tensor forward(AutogradContext* ctx, const Tensor& x, const Tensor& wqkv, const Tensor& wo, Aside buffer_qkv, Aside buffer_o,
-                        Aside cos, Aside sin, int64_t heads, int64_t kv, int64_t hd, int64_t status) {
+                        Aside cos, Aside sin, int64_t heads, int64_t kv, int64_t hd, Aside status) {
     const ll B = x.size(0), S = x.size(1), C = wqkv.size(0), N = heads * hd;
     const Tensor x2 = rows(x);
     Tensor qkv = bf16({B, S, C}, x);
     check(E.gemm_rope(x2.data_ptr(), wqkv.data_ptr(), qkv.data_ptr(), (int)x2.size(0), (int)C, (int)x2.size(1), x2.stride(0),
                       wqkv.stride(0), C, cos.t.data_ptr<float>(), sin.t.data_ptr<float>(), (int)S, (int)((heads + kv) * hd), (int)hd,
-                      word(status), stream()),
+                      word(status.t), stream()),
           "gemm2_rope");
     Tensor out = bf16({B, S, N}, x), lse = f32({B, heads, S}, x);
     check(E.attention_fwd(qkv.data_ptr(), out.data_ptr(), lse.data_ptr<float>(), (int)B, (int)S, (int)heads, (int)kv, (int)hd, C, N,
-                          (float)std::pow((double)hd, -0.5), word(status), stream()),
+                          (float)std::pow((double)hd, -0.5), word(status.t), stream()),
           "attention_fwd");
     Tensor y = bf16({B, S, wo.size(0)}, x);
-    gemm(out.view({-1, N}), wo, y.view({-1, wo.size(0)}), false, false, 0, status);
+    gemm(out.view({-1, N}), wo, y.view({-1, wo.size(0)}), false, false, 0, status.t);
     ctx->save_for_backward({x, wqkv, wo, qkv, out, lse, cos.t, sin.t});
     keep(ctx, "buffer_qkv", buffer_qkv);
     keep(ctx, "buffer_o", buffer_o);
-    ctx->saved_data["dims"] = std::vector<int64_t>{heads, kv, hd, status};
+    keep(ctx, "status", status);
+    ctx->saved_data["dims"] = std::vector<int64_t>{heads, kv, hd};
     return y;
   }
   static variable_list backward(AutogradContext* ctx, variable_list g) {
     auto s = ctx->get_saved_variables();
     const Tensor &x = s[0], &wqkv = s[1], &wo = s[2], &qkv = s[3], &out = s[4], &lse = s[5], &cos = s[6], &sin = s[7];
     const auto dims = ctx->saved_data["dims"].toIntVector();
-    const int64_t heads = dims[0], kv = dims[1], hd = dims[2], status = dims[3];
+    const int64_t heads = dims[0], kv = dims[1], hd = dims[2];
+    const Tensor status = aside(ctx, "status");
     const ll B = qkv.size(0), S = qkv.size(1), C = qkv.size(2), T = B * S, N = heads * hd;
     const Tensor dy2 = dense(rows(g[0])), out2 = out.view({T, N});
     Tensor dO = bf16({T, N}, qkv), delta = f32({B, heads, S}, qkv);
@@ -322,24 +325,24 @@ PYBIND11_MODULE(tplr_host, m) {
   typedef py::call_guard<py::gil_scoped_release> nogil;
   m.def("bind", &bind);
   m.def("launches", [] { return g_launches.load(std::memory_order_relaxed); });
-  m.def("rmsnorm", [](const Tensor& x, const Tensor& w, const std::optional<Tensor>& buffer, double eps, int64_t status) {
-    return RMSNorm::apply(x, w, opt(buffer), eps, status);
+  m.def("rmsnorm", [](const Tensor& x, const Tensor& w, const std::optional<Tensor>& buffer, double eps, const Tensor& status) {
+    return RMSNorm::apply(x, w, opt(buffer), eps, Aside{status});
   }, nogil());
   m.def("add_rmsnorm", [](const Tensor& res, const Tensor& delta, const Tensor& w, const std::optional<Tensor>& buffer, double eps,
-                          int64_t status) {
-    auto r = AddRMSNorm::apply(res, delta, w, opt(buffer), eps, status);
+                          const Tensor& status) {
+    auto r = AddRMSNorm::apply(res, delta, w, opt(buffer), eps, Aside{status});
     return std::make_tuple(r[0], r[1]);
   }, nogil());
-  m.def("linear", [](const Tensor& x, const Tensor& w, const std::optional<Tensor>& buffer, int64_t status) {
-    return Linear::apply(x, w, opt(buffer), status);
+  m.def("linear", [](const Tensor& x, const Tensor& w, const std::optional<Tensor>& buffer, const Tensor& status) {
+    return Linear::apply(x, w, opt(buffer), Aside{status});
   }, nogil());
   m.def("feed_forward", [](const Tensor& x, const Tensor& w13, const Tensor& w2, const std::optional<Tensor>& b13,
-                           const std::optional<Tensor>& b2, int64_t status) {
-    return FeedForward::apply(x, w13, w2, opt(b13), opt(b2), status);
+                           const std::optional<Tensor>& b2, const Tensor& status) {
+    return FeedForward::apply(x, w13, w2, opt(b13), opt(b2), Aside{status});
   }, nogil());
   m.def("attention_block", [](const Tensor& x, const Tensor& wqkv, const Tensor& wo, const std::optional<Tensor>& bq,
                               const std::optional<Tensor>& bo, const Tensor& cos, const Tensor& sin, int64_t heads, int64_t kv,
-                              int64_t hd, int64_t status) {
-    return AttentionBlock::apply(x, wqkv, wo, opt(bq), opt(bo), Aside{cos}, Aside{sin}, heads, kv, hd, status);
+                              int64_t hd, const Tensor& status) {
+    return AttentionBlock::apply(x, wqkv, wo, opt(bq), opt(bo), Aside{cos}, Aside{sin}, heads, kv, hd, Aside{status});
   }, nogil());
 }

@@ -205,7 +205,7 @@ def linear(x: torch.Tensor, w: torch.Tensor, main_grad: torch.Tensor | None = No
     if (_GEMM_BACKEND == "tcgen05_2sm" and _native_ok(x, w) and x.is_contiguous() and w.is_contiguous() and w.shape[0] % 8 == 0
             and w.shape[1] % 8 == 0 and x.shape[-1] == w.shape[1] and _buffers_ok((main_grad, w)) and _aligned(x, w)
             and (host := native.host())):
-        return host.linear(x, w, main_grad, status_word(x.device).data_ptr())
+        return host.linear(x, w, main_grad, status_word(x.device))
     return _Linear.apply(x, w, main_grad)
 
 
@@ -282,7 +282,7 @@ def rmsnorm(x, w, eps: float = 1e-5, main_grad=None):
     D = x.shape[-1]
     if (_norm_native(D, w, x) and D > 0 and x.is_contiguous() and w.is_contiguous() and _buffers_ok((main_grad, w)) and _aligned(x, w)
             and (host := native.host())):
-        return host.rmsnorm(x, w, main_grad, eps, status_word(x.device).data_ptr())
+        return host.rmsnorm(x, w, main_grad, eps, status_word(x.device))
     return _RMSNorm.apply(x, w, eps, main_grad)
 
 
@@ -356,7 +356,7 @@ def add_rmsnorm(res, delta, w, eps: float = 1e-5, main_grad=None):
     if (_norm_native(D, w, res, delta) and D > 0 and res.shape == delta.shape and res.is_contiguous() and delta.is_contiguous()
             and w.is_contiguous() and _buffers_ok((main_grad, w)) and _aligned(res, delta, w)
             and (host := native.host())):
-        return host.add_rmsnorm(res, delta, w, main_grad, eps, status_word(res.device).data_ptr())
+        return host.add_rmsnorm(res, delta, w, main_grad, eps, status_word(res.device))
     return _AddRMSNorm.apply(res, delta, w, eps, main_grad)
 
 
@@ -565,7 +565,7 @@ def feed_forward(x, w13, w2, main_grad13=None, main_grad2=None):
             gemm(h, w2, out=y.view(-1, w2.shape[0]))
             return y
         if _buffers_ok((main_grad13, w13), (main_grad2, w2)) and (host := native.host()):
-            return host.feed_forward(x, w13, w2, main_grad13, main_grad2, status_word(x.device).data_ptr())
+            return host.feed_forward(x, w13, w2, main_grad13, main_grad2, status_word(x.device))
         return _FeedForward.apply(x, w13, w2, main_grad13, main_grad2)
     return _Linear.apply(linear_swiglu(x, w13, main_grad13), w2, main_grad2)
 
@@ -967,7 +967,7 @@ def attention_block(x, wqkv, wo, cos, sin, n_heads: int, n_kv: int, hd: int, mai
             and _rope_tables_ok(cos, sin, S, hd)):
         if _buffers_ok((main_grad_qkv, wqkv), (main_grad_wo, wo)) and (host := native.host()):
             return host.attention_block(x, wqkv, wo, main_grad_qkv, main_grad_wo, cos, sin, n_heads, n_kv, hd,
-                                        status_word(x.device).data_ptr())
+                                        status_word(x.device))
         return _AttentionBlock.apply(x, wqkv, wo, main_grad_qkv, main_grad_wo, cos, sin, n_heads, n_kv, hd)
     return _Linear.apply(rope_attention_projection(x, wqkv, cos, sin, n_heads, n_kv, hd, main_grad_qkv), wo, main_grad_wo)
 

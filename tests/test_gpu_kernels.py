@@ -678,7 +678,7 @@ def test_norms_refuse_rows_of_no_elements():
     with pytest.raises(ZeroDivisionError):
         OF.add_rmsnorm(x, x, w)
     with pytest.raises(RuntimeError):
-        native.host().rmsnorm(x, w, None, 1e-5, 0)
+        native.host().rmsnorm(x, w, None, 1e-5, OF.status_word(x.device))
 
 
 def _node_case(op, T, with_buffers):
