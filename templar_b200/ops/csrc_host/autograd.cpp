@@ -7,9 +7,11 @@
 //
 // functional.py decides which calls come here (operand types, strides and alignment) and keeps its nodes for all others.
 // Tensors are saved as saved variables only; the gradient buffers of the flat store are held by reference as there.
+#include <ATen/ATen.h>
 #include <c10/cuda/CUDAStream.h>
 #include <dlfcn.h>
-#include <torch/extension.h>
+#include <torch/csrc/autograd/custom_function.h>
+#include <torch/csrc/utils/pybind.h>
 
 #include <atomic>
 
@@ -17,7 +19,7 @@
 
 namespace {
 
-using torch::Tensor;
+using at::Tensor;
 using torch::autograd::AutogradContext;
 using torch::autograd::Function;
 using torch::autograd::variable_list;
