@@ -771,7 +771,7 @@ def attention(q, k, v):
     return o.transpose(1, 2)
 
 
-OWN_HEAD_DIMS = (64, 128)      # head dimensions of the own flash-attention kernels (any sequence length)
+OWN_HEAD_DIMS = (64, 128)      # head dimensions of the own flash-attention kernels (any sequence length, see _own_attention_faster)
 _ATTN_BACKEND = "tcgen05"      # "tcgen05": own flash-attention kernels; "sdpa": torch SDPA (library)
 
 
@@ -947,6 +947,27 @@ def _own_heads(width: int, n_heads: int, n_kv: int, hd: int) -> bool:
     return hd in OWN_HEAD_DIMS and n_heads % n_kv == 0 and width == (n_heads + 2 * n_kv) * hd
 
 
+def _own_attention_faster(B: int, S: int, n_heads: int, n_kv: int, hd: int, grad: bool, fused: bool) -> bool:
+    """Whether the own attention kernels are the faster path for these sizes; ``fused``: together with the projection (one node,
+    rotation in the epilogue), else on a packed projection alone.
+
+    Heads of 128 with sequences of whole tiles stay here.  For heads of 64 and odd lengths the library kernel does more
+    products a second, but pays for a copy of q, k and v, of their gradients, and for its launches: which weighs more depends on
+    the sequence length alone, once the device is the bound.  Measured at 16384 tokens, library against own, microseconds:
+    forward and backward, 12 heads of 64, S 3072 975 and 844, 4096 1097 and 1040, 8192 1468 and 1682; 32 on 8 heads of 64, S 2048
+    1971 and 1868, 3072 2119 and 2163; 16 heads of 128, S 6000 2468 and 2382, 8000 3597 and 3676; 32 on 8 heads of 128, S 4000
+    5683 and 5632, 6000 4878 and 5053.  Forward alone, fused, 32 on 8 heads of 64, S 1024 418 and 415, 2048 491 and 510; 16 heads of
+    128, S 1000 535 and 521, 3000 591 and 620.  Forward alone on a packed projection nothing is copied: 12 heads of 64, S 512 81
+    and 71 (launches), 2048 99 and 118; only calls bound by their launches are faster here (1 x 2048, 12 heads of 64: 82 and 35)."""
+    if hd == 128 and S % 128 == 0:
+        return True
+    group = n_heads // n_kv
+    if grad:
+        return S <= ((4096 if group == 1 else 2560) if hd == 64 else (6656 if group == 1 else 4608))
+    small = B * S * n_heads * hd <= 1 << 22
+    return small or S <= (1536 if hd == 64 else 2048) if fused else small and S <= 2048
+
+
 def _rope_tables_ok(cos, sin, S: int, hd: int) -> bool:
     return all(t.is_cuda and t.dtype == torch.float32 and t.is_contiguous() and t.dim() == 2 and t.shape[0] >= S
                and t.shape[1] == hd // 2 and t.data_ptr() % 16 == 0 for t in (cos, sin))
@@ -964,7 +985,7 @@ def attention_block(x, wqkv, wo, cos, sin, n_heads: int, n_kv: int, hd: int, mai
             and x.dtype == torch.bfloat16 and _own_heads(wqkv.shape[0], n_heads, n_kv, hd) and x.is_contiguous()
             and wqkv.stride(1) == 1 and wo.stride(1) == 1 and wqkv.stride(0) % 8 == 0 and wo.stride(0) % 8 == 0 and K % 8 == 0
             and wqkv.shape[1] == K and wo.shape[0] % 8 == 0 and wo.shape[1] == n_heads * hd and _aligned(x, wqkv, wo)
-            and _rope_tables_ok(cos, sin, S, hd)):
+            and _rope_tables_ok(cos, sin, S, hd) and _own_attention_faster(B, S, n_heads, n_kv, hd, torch.is_grad_enabled(), True)):
         if _buffers_ok((main_grad_qkv, wqkv), (main_grad_wo, wo)) and (host := native.host()):
             return host.attention_block(x, wqkv, wo, main_grad_qkv, main_grad_wo, cos, sin, n_heads, n_kv, hd,
                                         status_word(x.device))
@@ -981,7 +1002,8 @@ def rope_attention_projection(x, w, cos, sin, n_heads: int, n_kv: int, hd: int, 
     B, S, K = x.shape
     if (FUSED_PROJECTIONS and _ATTN_BACKEND == "tcgen05" and _GEMM_BACKEND == "tcgen05_2sm" and _native_ok(x, w) and x.dtype == torch.bfloat16
             and _own_heads(w.shape[0], n_heads, n_kv, hd) and x.is_contiguous() and w.stride(1) == 1 and w.stride(0) % 8 == 0
-            and K % 8 == 0 and w.shape[1] == K and _aligned(x, w) and _rope_tables_ok(cos, sin, S, hd)):
+            and K % 8 == 0 and w.shape[1] == K and _aligned(x, w) and _rope_tables_ok(cos, sin, S, hd)
+            and _own_attention_faster(B, S, n_heads, n_kv, hd, torch.is_grad_enabled(), True)):
         return _QKVRopeAttention.apply(x, w, main_grad, cos, sin, n_heads, n_kv, hd)
     qkv = rope(_Linear.apply(x, w, main_grad), cos, sin, n_heads + n_kv, hd)
     return attention_packed(qkv, n_heads, n_kv, hd)
@@ -995,7 +1017,7 @@ def attention_packed(qkv, n_heads: int, n_kv: int, hd: int):
     B, S, C = qkv.shape
     if (_ATTN_BACKEND == "tcgen05" and qkv.is_cuda and qkv.dtype == torch.bfloat16 and _own_heads(C, n_heads, n_kv, hd)
             and qkv.stride(2) == 1 and qkv.stride(0) == S * qkv.stride(1) and qkv.stride(1) >= C and qkv.stride(1) % 8 == 0
-            and qkv.data_ptr() % 16 == 0):
+            and qkv.data_ptr() % 16 == 0 and _own_attention_faster(B, S, n_heads, n_kv, hd, torch.is_grad_enabled(), False)):
         return _AttentionPacked.apply(qkv, n_heads, n_kv, hd)
     if _ATTN_BACKEND == "tcgen05" and qkv.is_cuda and (hd, qkv.dtype) not in _attn_fallback_seen:
         # said once per shape class: a GPU run that silently uses the library kernel would misreport what ran
@@ -1003,7 +1025,8 @@ def attention_packed(qkv, n_heads: int, n_kv: int, hd: int):
         import warnings
 
         warnings.warn(f"attention_packed: head_dim {hd}, sequence {S}, dtype {qkv.dtype} is outside the own flash-attention "
-                      f"kernels (bf16, head_dim 64 or 128, rows of whole heads); using torch SDPA for it", stacklevel=2)
+                      f"kernels (bf16, head_dim 64 or 128, rows of whole heads, sizes at which they are the faster path); using "
+                      f"torch SDPA for it", stacklevel=2)
     q, k, v = _split_qkv(qkv, n_heads, n_kv, hd)
     return attention(q, k, v).reshape(B, S, n_heads * hd)
 

@@ -84,3 +84,19 @@ def test_attention_block_equals_projection_rotation_attention_projection():
     o2 = OF.linear(OF.attention_packed(OF.rope(OF.linear(x, w), cos, sin, H + KV, hd), H, KV, hd), wo)
     g2 = _grads(o2, x, w, wo)
     assert torch.equal(o, o2) and all(torch.equal(a, b) for a, b in zip(g, g2))
+
+
+def test_attention_route_by_size():
+    """Which attention kernel a call takes: heads of 128 on whole tiles always the own one; others by sequence length, by whether
+    a backward pass follows and by whether the launches are the bound."""
+    own = OF._own_attention_faster
+    assert all(own(B, S, 16, 16, 128, g, f) for B in (1, 64) for S in (128, 2048, 65536) for g in (True, False) for f in (True, False))
+    # with a backward pass: the last length of each kind and the next
+    for H, KV, hd, last in ((12, 12, 64, 4096), (32, 8, 64, 2560), (16, 16, 128, 6655), (32, 8, 128, 4607)):
+        assert own(4, last, H, KV, hd, True, True) and own(4, last, H, KV, hd, True, False)
+        assert not own(4, last + 2, H, KV, hd, True, True) and not own(1, 2 * last + 1, H, KV, hd, True, False)
+    # forward alone
+    assert own(64, 1536, 12, 12, 64, False, True) and not own(64, 1537, 12, 12, 64, False, True)
+    assert own(64, 2047, 16, 16, 128, False, True) and not own(64, 2049, 16, 16, 128, False, True)
+    assert not own(64, 256, 12, 12, 64, False, False) and own(1, 2048, 12, 12, 64, False, False)
+    assert own(1, 4100, 12, 12, 64, False, True) and not own(1, 4100, 12, 12, 64, False, False)

@@ -287,3 +287,29 @@ def test_attention_refuses_widths_that_do_not_fit_the_heads(S, hd):
         OF.attention_block(bf(1, S, D), bf(C, D - 8), bf(D, H * hd), cos, sin, H, KV, hd)
     with pytest.raises(ValueError):
         OF.rope_attention_projection(bf(1, S, D), bf(C, D + 8), cos, sin, H, KV, hd)
+
+
+@pytest.mark.parametrize("B,S,H,KV,hd,grad", [(1, 4104, 2, 2, 64, True), (1, 2568, 4, 2, 64, True), (1, 4616, 2, 1, 128, True),
+                                              (4, 1544, 12, 12, 64, False), (16, 1544, 12, 4, 64, False), (9, 2056, 2, 2, 128, False)])
+def test_attention_routes_agree_beyond_their_limits(B, S, H, KV, hd, grad, monkeypatch):
+    """Sizes just past those that stay with the own kernels: the general path and the own kernels give the same attention block."""
+    torch.manual_seed(S)
+    D = H * hd
+    x = torch.randn(B, S, D, device=DEV).to(torch.bfloat16)
+    wqkv = (torch.randn((H + 2 * KV) * hd, D, device=DEV) / D ** 0.5).to(torch.bfloat16)
+    wo = (torch.randn(D, D, device=DEV) / D ** 0.5).to(torch.bfloat16)
+    cos, sin = OF.rope_tables(S, hd, 10000.0, DEV)
+    dy = torch.randn(B, S, D, device=DEV).to(torch.bfloat16)
+
+    def run():
+        leaves = [t.clone().requires_grad_(grad) for t in (x, wqkv, wo)]
+        with torch.set_grad_enabled(grad):
+            y = OF.attention_block(*leaves, cos, sin, H, KV, hd)
+        return [y, *(torch.autograd.grad(y, leaves, dy) if grad else ())]
+
+    if grad or B * S * H * hd > 1 << 22:
+        assert not OF._own_attention_faster(B, S, H, KV, hd, grad, True)
+    general = run()
+    monkeypatch.setattr(OF, "_own_attention_faster", lambda *a: True)
+    for got, want in zip(run(), general):
+        assert ((got.float() - want.float()).norm() / want.float().norm()).item() < 2e-2      # five roundings to bf16 on the way, 2^-9 each
