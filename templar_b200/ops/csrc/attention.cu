@@ -113,9 +113,10 @@ __device__ __forceinline__ uint32_t idesc_mn(int n, bool a_mn, bool b_mn) {
 
 // Softmax over one row of S (128 fp32 columns in tensor memory, lane = query row).  DIAG = the block on the diagonal
 // (columns above the row are masked); the other blocks run the variant without the per-element compare and select.
-// The row is read from tensor memory once: two passes of four loads, each with its own wait, made the softmax the longer
-// part of a step.  B 8, S 2048: neutral at
-// 16 heads of 128 (193 us), 125 -> 118 us at 12 heads of 64, where it lets the next S be computed ahead.
+// At heads of 64 the row is read from tensor memory once and stays in registers, which lets the next S be computed ahead
+// (B 8, S 2048, 12 heads: 125 us with two reads, 118 us).  At 128, where P lies over S, it is read twice, 32 columns at a time, for
+// the maximum and for the exponentials: holding it spills and gains nothing there (16 heads, B 8, S 2048 189 us with two
+// reads and 193 with one; B 2 56 and 65).
 // packed fp32 pairs (sm_100): one instruction for two lanes of fma / add, and the three-input max
 __device__ __forceinline__ unsigned long long pack_f32x2(uint32_t lo, uint32_t hi) {
   unsigned long long r;
@@ -182,6 +183,23 @@ __device__ __forceinline__ float attn_row_max(uint32_t (&v)[128], int r) {
   }
   return fmaxf(mx, mx2);
 }
+template <bool DIAG>
+__device__ __forceinline__ float attn_row_max(uint32_t ts_lane, int r) {
+  float mx = -INFINITY;
+#pragma unroll 1
+  for (int c = 0; c < 4; ++c) {
+    uint32_t v[32];
+    tmem_ld32(ts_lane + c * 32, v);
+    if (DIAG) {
+#pragma unroll
+      for (int e = 0; e < 32; ++e) mx = fmaxf(mx, (c * 32 + e > r) ? -INFINITY : __uint_as_float(v[e]));
+    } else {
+#pragma unroll
+      for (int e = 0; e < 16; ++e) mx = max3(mx, __uint_as_float(v[2 * e]), __uint_as_float(v[2 * e + 1]));
+    }
+  }
+  return mx;
+}
 // P = exp2(S * scale - m) written as packed bf16 to 64 columns; returns the row sum of P.
 __device__ __forceinline__ float attn_row_exp(const uint32_t (&v)[128], uint32_t tp_lane, float sl2, float m_used) {
   const unsigned long long sl2x2 = pack_f32x2(__float_as_uint(sl2), __float_as_uint(sl2));
@@ -200,6 +218,36 @@ __device__ __forceinline__ float attn_row_exp(const uint32_t (&v)[128], uint32_t
       pk[e] = *reinterpret_cast<uint32_t*>(&hh);
     }
     tmem_st16(tp_lane + c * 16, pk);
+  }
+  float s0, s1;
+  unpack_f32x2(sum, s0, s1);
+  return s0 + s1;
+}
+
+// the same over the first 64 columns of S
+template <bool DIAG>
+__device__ __forceinline__ float attn_row_exp(uint32_t ts_lane, int r, float sl2, float m_used) {
+  const unsigned long long sl2x2 = pack_f32x2(__float_as_uint(sl2), __float_as_uint(sl2));
+  const unsigned long long negm = pack_f32x2(__float_as_uint(-m_used), __float_as_uint(-m_used));
+  unsigned long long sum = 0ull;                         // (0.f, 0.f)
+#pragma unroll 1
+  for (int c = 0; c < 4; ++c) {
+    uint32_t v[32], pk[16];
+    tmem_ld32(ts_lane + c * 32, v);
+#pragma unroll
+    for (int e = 0; e < 16; ++e) {
+      float a0, a1;
+      unpack_f32x2(fma_f32x2(pack_f32x2(v[2 * e], v[2 * e + 1]), sl2x2, negm), a0, a1);
+      float p0 = exp2f(a0), p1 = exp2f(a1);
+      if (DIAG) {
+        if (c * 32 + 2 * e > r) p0 = 0.f;
+        if (c * 32 + 2 * e + 1 > r) p1 = 0.f;
+      }
+      sum = add_f32x2(sum, pack_f32x2(__float_as_uint(p0), __float_as_uint(p1)));
+      __nv_bfloat162 hh = __floats2bfloat162_rn(p0, p1);
+      pk[e] = *reinterpret_cast<uint32_t*>(&hh);
+    }
+    tmem_st16(ts_lane + c * 16, pk);
   }
   float s0, s1;
   unpack_f32x2(sum, s0, s1);
@@ -323,15 +371,17 @@ attn_fwd_kernel(const __grid_constant__ AttnFwdParams p) {
       if (!ok) break;
       tcgen05_fence_after();
       const bool diag = j == qi;
-      // the row is loaded once and stays in registers: maximum, then exponentials
-      uint32_t sv[128];
-      tmem_ld128(tS + lane_off, sv);
-      if (AHEAD) {
+      uint32_t sv[AHEAD ? 128 : 1];                        // AHEAD: the row, loaded once
+      float mx;
+      if constexpr (AHEAD) {
+        tmem_ld128(tS + lane_off, sv);
         tcgen05_fence_before();
         __syncwarp();
         if (lane == 0) mbar_arrive(smem_u32(&bar_s_read));
+        mx = diag ? attn_row_max<true>(sv, r) : attn_row_max<false>(sv, r);
+      } else {
+        mx = diag ? attn_row_max<true>(tS + lane_off, r) : attn_row_max<false>(tS + lane_off, r);
       }
-      const float mx = diag ? attn_row_max<true>(sv, r) : attn_row_max<false>(sv, r);
       if (AHEAD && j > 0) {                // O and the P columns: the product of block j-1 has finished with them
         ok = mbar_wait(smem_u32(&bar_v_empty), (uint32_t)((j - 1) & 1), abort_flag);
         ok = __all_sync(0xffffffffu, ok);
@@ -355,7 +405,8 @@ attn_fwd_kernel(const __grid_constant__ AttnFwdParams p) {
           }
         }
       }
-      l += attn_row_exp(sv, tP + lane_off, p.scale_log2, m_used);
+      if constexpr (AHEAD) l += attn_row_exp(sv, tP + lane_off, p.scale_log2, m_used);
+      else l += diag ? attn_row_exp<true>(tS + lane_off, r, p.scale_log2, m_used) : attn_row_exp<false>(tS + lane_off, r, p.scale_log2, m_used);
       tmem_wait_st();
       tcgen05_fence_before();
       __syncwarp();
