@@ -6,6 +6,9 @@
 // its own 128 rows of B (so every shared-memory byte feeds two SMs' tensor cores), the even CTA
 // issues tcgen05.mma.cta_group::2, and each CTA drains its 128 x 256 half of the accumulator
 // from its own tensor memory.  6 smem stages of 32 KB per CTA, two accumulator buffers.
+// The producer and the issuer are warp-uniform loops with one elected lane behind the issuing statements (see elect_one):
+// 505 cycles a k block of 64, which is the tensor pipe's 512 within the clock readings, for every operand layout; under
+// `lane == 0` 620 to 625.  2048 x 18944 x 2048 (8 tiles a pair): 113 -> 102 us K-major, 123 -> 102 us MN-major.
 //
 // Fused collectives (one process per GPU, peers mapped through the symmetric heap):
 //   gather  (all-gather -> GEMM): trailing "comm" CTAs of the same launch pull the peers' row
@@ -648,7 +651,7 @@ gemm2_kernel(const __grid_constant__ Gemm2Params p) {
   __shared__ __align__(8) uint64_t bar_gu[EPI == 5 ? 8 : 1];      // EPI 5: two per epilogue warp
   __shared__ uint32_t s_ready[32];   // gather: bit c set once chunk c was seen ready (1024 chunks)
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = warp_index(), lane = threadIdx.x & 31;
   const uint32_t cr = cluster_ctarank();
   const int pair = blockIdx.x >> 1, n_pairs = gridDim.x >> 1;
   const bool is_compute = pair < p.n_compute_pairs;
@@ -686,7 +689,8 @@ gemm2_kernel(const __grid_constant__ Gemm2Params p) {
   if (is_compute) {
     if (warp == 0) {
       // ----------------------------- TMA producer (both CTAs of the pair) ------------
-      if (lane == 0) {
+      {
+        const bool leader = elect_one();
         const int chunks_per_rank = p.ag_operand ? p.ag_rows_per_rank / CHUNK_ROWS : 1;
         // bounded wait until rows [r0, r0 + nrows) of the gathered operand are in local memory
         auto rows_ready = [&](int r0, int nrows) -> bool {
@@ -700,7 +704,10 @@ gemm2_kernel(const __grid_constant__ Gemm2Params p) {
           }
           return true;
         };
-        uint32_t it = 0;
+        // the lane that issues the loads waits for the rows; every lane gets the answer
+        auto rows_ready_warp = [&](int r0, int nrows) -> bool { return __all_sync(0xffffffffu, !leader || rows_ready(r0, nrows)); };
+        uint32_t it = 0, s = 0, ph = 0;                  // ring position of `it` (no division in the loop)
+        const uint32_t full0 = smem_u32(&bar_full[0]), empty0 = smem_u32(&bar_empty[0]), fullp0 = mapa(full0, 0);
         bool ok = true;
         Work w;
         work_init(p, w, pair);
@@ -711,40 +718,40 @@ gemm2_kernel(const __grid_constant__ Gemm2Params p) {
           const int k_blocks = w.nkb;
           const int m0 = tm * TILE_M + (int)cr * CTA_M;
           const int n0 = EPI == 3 ? tn * CTA_N + (int)cr * p.swiglu_f : tn * TILE_N + (int)cr * CTA_N;
-          if (p.ag_operand == 1 && !A_MN) ok = rows_ready(m0, CTA_M);
-          if (p.ag_operand == 2 && !B_MN) ok = ok && rows_ready(n0, CTA_N);
+          if (p.ag_operand == 1 && !A_MN) ok = rows_ready_warp(m0, CTA_M);
+          if (p.ag_operand == 2 && !B_MN) ok = ok && rows_ready_warp(n0, CTA_N);
           for (int kb = 0; kb < k_blocks && ok; ++kb, ++it) {
             // k order rotated so that the rows of the local shard come first when k is the gathered dimension
             int kbr = kb0 + kb;
             if ((p.ag_operand == 1 && A_MN) || (p.ag_operand == 2 && B_MN)) {
               kbr = kb + p.rank * (p.ag_rows_per_rank / BK);       // gathered k: never split (host side)
               if (kbr >= k_blocks) kbr -= k_blocks;
-              if (!(ok = rows_ready(kbr * BK, BK))) break;
+              if (!(ok = rows_ready_warp(kbr * BK, BK))) break;
             }
-            const int s = it % STAGES;
-            const uint32_t ph = (it / STAGES) & 1;
-            if (!(ok = mbar_wait(smem_u32(&bar_empty[s]), ph ^ 1, abort_flag))) break;
-            const uint32_t fb_local = smem_u32(&bar_full[s]);
-            const uint32_t fb = mapa(fb_local, 0);
-            if (cr == 0) mbar_expect_tx(fb_local, 2 * STAGE_BYTES);
-            const uint32_t a_dst = sA + s * A_STAGE, b_dst = sB + s * B_STAGE;
-            const int k0 = kbr * BK;
-            if (!A_MN) {
-              tma_load_2d_pair(a_dst, &p.tmA, fb, k0, m0);
-            } else {
+            if (!(ok = __all_sync(0xffffffffu, mbar_wait(empty0 + 8u * s, ph ^ 1u, abort_flag)))) break;
+            if (leader) {
+              if (cr == 0) mbar_expect_tx(full0 + 8u * s, 2 * STAGE_BYTES);
+              const uint32_t fb = fullp0 + 8u * s;
+              const uint32_t a_dst = sA + s * A_STAGE, b_dst = sB + s * B_STAGE;
+              const int k0 = kbr * BK;
+              if (!A_MN) {
+                tma_load_2d_pair(a_dst, &p.tmA, fb, k0, m0);
+              } else {
 #pragma unroll
-              for (int j = 0; j < CTA_M / 64; ++j) tma_load_2d_pair(a_dst + j * (BK * 128), &p.tmA, fb, m0 + 64 * j, k0);
-            }
-            if (!B_MN) {
-              tma_load_2d_pair(b_dst, &p.tmB, fb, k0, n0);
-            } else {
+                for (int j = 0; j < CTA_M / 64; ++j) tma_load_2d_pair(a_dst + j * (BK * 128), &p.tmA, fb, m0 + 64 * j, k0);
+              }
+              if (!B_MN) {
+                tma_load_2d_pair(b_dst, &p.tmB, fb, k0, n0);
+              } else {
 #pragma unroll
-              for (int j = 0; j < CTA_N / 64; ++j) tma_load_2d_pair(b_dst + j * (BK * 128), &p.tmB, fb, n0 + 64 * j, k0);
+                for (int j = 0; j < CTA_N / 64; ++j) tma_load_2d_pair(b_dst + j * (BK * 128), &p.tmB, fb, n0 + 64 * j, k0);
+              }
             }
+            if (++s == STAGES) { s = 0; ph ^= 1u; }
           }
         }
-        // drain (leader): every armed stage has landed in both CTAs before the pair may retire
-        if (cr == 0) {
+        // drain (even CTA): every armed stage has landed in both CTAs before the pair may retire
+        if (leader && cr == 0) {
           Drain drain;
           for (uint32_t back = 0; back < STAGES && back < it; ++back) {
             const uint32_t j = it - 1 - back;
@@ -754,7 +761,8 @@ gemm2_kernel(const __grid_constant__ Gemm2Params p) {
       }
     } else if (warp == 1) {
       // ----------------------------- MMA issuer (even CTA only) ----------------------
-      if (lane == 0 && cr == 0) {
+      if (cr == 0) {
+        const bool leader = elect_one();
         const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((A_MN ? 1u : 0u) << 15) |
                                ((B_MN ? 1u : 0u) << 16) | ((uint32_t)(TILE_N >> 3) << 17) | ((uint32_t)(TILE_M >> 4) << 24);
         uint32_t it = 0, tile_i = 0;
@@ -763,7 +771,6 @@ gemm2_kernel(const __grid_constant__ Gemm2Params p) {
         work_init(p, w, pair);
         // descriptors of stage 0, built once: a stage or a k step only moves the start address (bytes >> 4 in the low
         // word; the whole ring lies below 256 KB, so the additions never carry out of the 14-bit address field).
-        // The issuing thread is one lane: every instruction it does not execute per MMA is tensor-pipe time.
         const DescBase dA0 = A_MN ? desc_base(sA, BK * 128, 1024) : desc_base(sA, 16, 1024);
         const DescBase dB0 = B_MN ? desc_base(sB, BK * 128, 1024) : desc_base(sB, 16, 1024);
         constexpr uint32_t A_KSTEP = (A_MN ? UMMA_K * 128 : UMMA_K * 2) >> 4, B_KSTEP = (B_MN ? UMMA_K * 128 : UMMA_K * 2) >> 4;
@@ -778,14 +785,16 @@ gemm2_kernel(const __grid_constant__ Gemm2Params p) {
             if (!(ok = mbar_wait(smem_u32(&bar_full[s]), ph, abort_flag))) break;
             tcgen05_fence_after();
             const uint32_t a_lo = dA0.lo + s * (A_STAGE >> 4), b_lo = dB0.lo + s * (B_STAGE >> 4);
+            if (leader) {
 #pragma unroll
-            for (int kk = 0; kk < BK / UMMA_K; ++kk)
-              umma_bf16_pair_lohi(d_tmem, a_lo + kk * A_KSTEP, dA0.hi, b_lo + kk * B_KSTEP, dB0.hi, idesc,
-                                  (kb > 0 || kk > 0) ? 1u : 0u);
-            umma_commit_pair(smem_u32(&bar_empty[s]));
+              for (int kk = 0; kk < BK / UMMA_K; ++kk)
+                umma_bf16_pair_lohi(d_tmem, a_lo + kk * A_KSTEP, dA0.hi, b_lo + kk * B_KSTEP, dB0.hi, idesc,
+                                    (kb > 0 || kk > 0) ? 1u : 0u);
+              umma_commit_pair(smem_u32(&bar_empty[s]));
+            }
             if (++s == STAGES) { s = 0; ph ^= 1u; }
           }
-          if (ok) umma_commit_pair(smem_u32(&bar_tfull[acc]));
+          if (ok && leader) umma_commit_pair(smem_u32(&bar_tfull[acc]));
         }
       }
     } else {

@@ -58,6 +58,17 @@ struct Drain {
   __device__ __forceinline__ void wait(uint32_t bar, uint32_t parity) { (void)mbar_wait(bar, parity, &gave_up); }
 };
 
+// True in one lane of a converged warp.  The loops that issue tcgen05.mma and TMA are run by the whole warp and only the
+// issuing statements are behind this: under `if (lane == 0)` the loop's addresses and descriptors live in per-lane registers and
+// are moved into the uniform ones that these instructions take, one by one: 155 cycles for each MMA whatever its size, where
+// a 256 x 256 x 16 one of a CTA pair takes 125.  `warp` has to come from warp_index() for the same reason.
+__device__ __forceinline__ bool elect_one() {
+  uint32_t p;
+  asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(p));
+  return p != 0;
+}
+__device__ __forceinline__ int warp_index() { return __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0); }
+
 __device__ __forceinline__ void tma_load_2d(uint32_t dst, const CUtensorMap* map, uint32_t bar, int x, int y) {
   asm volatile(
       "cp.async.bulk.tensor.2d.shared::cta.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];"
