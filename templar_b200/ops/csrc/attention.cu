@@ -264,7 +264,7 @@ attn_fwd_kernel(const __grid_constant__ AttnFwdParams p) {
   __shared__ uint32_t s_tmem_base;
   __shared__ int s_abort;
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = warp_index(), lane = threadIdx.x & 31;
   const int nQ = (p.S + BQ - 1) / BQ;
   // heavy (late) query blocks first
   const int hb = p.H * p.B;
@@ -301,42 +301,54 @@ attn_fwd_kernel(const __grid_constant__ AttnFwdParams p) {
   const uint32_t sQ = smem_u32(smem), sK = sQ + TILE_BYTES, sV = sK + TILE_BYTES;
 
   if (warp == 0) {
-    if (lane == 0) {
-      mbar_expect_tx(smem_u32(&bar_q), TILE_BYTES);
-      load_tile<DH>(sQ, &p.tmQKV, smem_u32(&bar_q), qcol, row0, b);
+    {
+      const bool leader = elect_one();
+      if (leader) {
+        mbar_expect_tx(smem_u32(&bar_q), TILE_BYTES);
+        load_tile<DH>(sQ, &p.tmQKV, smem_u32(&bar_q), qcol, row0, b);
+      }
       bool ok = true;
       int n_k = 0, n_v = 0;                                // tiles asked for
       for (int j = 0; j < nb && ok; ++j) {
         const uint32_t ph = j & 1;
         const int krow = j * BKV;
         if (!(ok = mbar_wait(smem_u32(&bar_k_empty), ph ^ 1, abort_flag))) break;
-        mbar_expect_tx(smem_u32(&bar_k_full), TILE_BYTES);
-        load_tile<DH>(sK, &p.tmQKV, smem_u32(&bar_k_full), kcol, krow, b);
+        if (leader) {
+          mbar_expect_tx(smem_u32(&bar_k_full), TILE_BYTES);
+          load_tile<DH>(sK, &p.tmQKV, smem_u32(&bar_k_full), kcol, krow, b);
+        }
         ++n_k;
         if (!(ok = mbar_wait(smem_u32(&bar_v_empty), ph ^ 1, abort_flag))) break;
-        mbar_expect_tx(smem_u32(&bar_v_full), TILE_BYTES);
-        load_tile<DH>(sV, &p.tmQKV, smem_u32(&bar_v_full), vcol, krow, b);
+        if (leader) {
+          mbar_expect_tx(smem_u32(&bar_v_full), TILE_BYTES);
+          load_tile<DH>(sV, &p.tmQKV, smem_u32(&bar_v_full), vcol, krow, b);
+        }
         ++n_v;
       }
-      Drain drain;                                         // no load may land after the CTA has retired: a role may have given up
-      drain.wait(smem_u32(&bar_q), 0);
-      if (n_k) drain.wait(smem_u32(&bar_k_full), (uint32_t)((n_k - 1) & 1));
-      if (n_v) drain.wait(smem_u32(&bar_v_full), (uint32_t)((n_v - 1) & 1));
+      if (leader) {
+        Drain drain;                                         // no load may land after the CTA has retired: a role may have given up
+        drain.wait(smem_u32(&bar_q), 0);
+        if (n_k) drain.wait(smem_u32(&bar_k_full), (uint32_t)((n_k - 1) & 1));
+        if (n_v) drain.wait(smem_u32(&bar_v_full), (uint32_t)((n_v - 1) & 1));
+      }
     }
   } else if (warp == 1) {
-    if (lane == 0) {
+    {
+      const bool leader = elect_one();
       const uint32_t id_qk = idesc_mn(128, false, false), id_pv = idesc_mn(DH, false, true);
       const DescBase bQ = desc_base(sQ, 16, 1024), bK = desc_base(sK, 16, 1024), bV = desc_base(sV, 128 * 128, 1024);
       auto issue_s = [&](int j) -> bool {                  // S(j) = Q K(j)^T
         if (!mbar_wait(smem_u32(&bar_k_full), (uint32_t)(j & 1), abort_flag)) return false;
         tcgen05_fence_after();
+        if (leader) {
 #pragma unroll
-        for (int kk = 0; kk < DH / 16; ++kk) {
-          const uint32_t off = (uint32_t)(kk >> 2) * (128u * 128u / 16u) + (uint32_t)(kk & 3) * 2u;    // 16-byte units
-          umma_bf16_b(tS, bQ, off, bK, off, id_qk, kk > 0 ? 1u : 0u);
+          for (int kk = 0; kk < DH / 16; ++kk) {
+            const uint32_t off = (uint32_t)(kk >> 2) * (128u * 128u / 16u) + (uint32_t)(kk & 3) * 2u;    // 16-byte units
+            umma_bf16_b(tS, bQ, off, bK, off, id_qk, kk > 0 ? 1u : 0u);
+          }
+          umma_commit(smem_u32(&bar_s_full));
+          umma_commit(smem_u32(&bar_k_empty));
         }
-        umma_commit(smem_u32(&bar_s_full));
-        umma_commit(smem_u32(&bar_k_empty));
         return true;
       };
       bool ok = mbar_wait(smem_u32(&bar_q), 0, abort_flag);
@@ -352,11 +364,13 @@ attn_fwd_kernel(const __grid_constant__ AttnFwdParams p) {
         if (!(ok = mbar_wait(smem_u32(&bar_p_full), ph, abort_flag))) break;
         if (!(ok = mbar_wait(smem_u32(&bar_v_full), ph, abort_flag))) break;
         tcgen05_fence_after();
+        if (leader) {
 #pragma unroll
-        for (int kk = 0; kk < BKV / 16; ++kk)
-          umma_ts_bf16_b(tO, tP + 8 * kk, bV, (uint32_t)kk * 128u, id_pv, (j > 0 || kk > 0) ? 1u : 0u);
-        umma_commit(smem_u32(&bar_v_empty));
-        if (j == nb - 1) umma_commit(smem_u32(&bar_o_full));
+          for (int kk = 0; kk < BKV / 16; ++kk)
+            umma_ts_bf16_b(tO, tP + 8 * kk, bV, (uint32_t)kk * 128u, id_pv, (j > 0 || kk > 0) ? 1u : 0u);
+          umma_commit(smem_u32(&bar_v_empty));
+          if (j == nb - 1) umma_commit(smem_u32(&bar_o_full));
+        }
       }
     }
   } else {
@@ -508,7 +522,9 @@ TPLR_API int tplr_attention_fwd(const void* qkv, void* out, float* lse, int B, i
 // is split where P is ready.  S of the next step is issued as soon as every warp has read this one's (Q has two buffers
 // for it) and runs, with dV, while the warps form dS; dP of the next step runs while they exponentiate its S.
 // B 8, S 2048, 16 heads of 128: 692 us with the parts of a step one after the other, 620 us here; the
-// shared-memory traffic of the five products and of P, dS and dQ would allow about 350.
+// shared-memory traffic of the five products and of P, dS and dQ would allow about 350.  Issuing the products from a
+// warp-uniform loop (elect_one) instead of under `lane == 0`: 2 to 10 %, the most at heads of 64 (119 -> 112 us at 8 x 1024 x 12),
+// whose products are the shortest; forward 182 -> 170 us at 8 x 2048 x 16 of 128, 104 -> 89 at 8 x 2048 x 12 of 64.
 // ------------------------------------------------------------------------------------------ //
 namespace {
 
@@ -553,7 +569,7 @@ attn_bwd_kernel(const __grid_constant__ AttnBwdParams p) {
   __shared__ uint32_t s_tmem_base;
   __shared__ int s_abort;
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = warp_index(), lane = threadIdx.x & 31;
   const int nQ = (p.S + BQ - 1) / BQ;
   const int gb = p.KV * p.B * p.split;
   const int j = (int)(blockIdx.x / gb);                    // kv block; small j (long walks) first
@@ -591,10 +607,13 @@ attn_bwd_kernel(const __grid_constant__ AttnBwdParams p) {
                  sP = sdO + TILE_BYTES, sdS = sP + PT_BYTES;
 
   if (warp == 0) {
-    if (lane == 0) {
-      mbar_expect_tx(smem_u32(&bar_kv), 2 * TILE_BYTES);
-      load_tile<DH>(sK, &p.tmQKV, smem_u32(&bar_kv), kcol, kvrow0, b);
-      load_tile<DH>(sV, &p.tmQKV, smem_u32(&bar_kv), vcol, kvrow0, b);
+    {
+      const bool leader = elect_one();
+      if (leader) {
+        mbar_expect_tx(smem_u32(&bar_kv), 2 * TILE_BYTES);
+        load_tile<DH>(sK, &p.tmQKV, smem_u32(&bar_kv), kcol, kvrow0, b);
+        load_tile<DH>(sV, &p.tmQKV, smem_u32(&bar_kv), vcol, kvrow0, b);
+      }
       bool ok = true;
       int n_q = 0, n_do = 0;                                 // tiles asked for
       for (int t = 0; t < n_it && ok; ++t) {
@@ -602,22 +621,29 @@ attn_bwd_kernel(const __grid_constant__ AttnBwdParams p) {
         const int qrow0 = i * BQ, qcol = h * DH, s = t & 1;
         if (!(ok = mbar_wait(smem_u32(&bar_q_empty[s]), (uint32_t)(((t >> 1) & 1) ^ 1), abort_flag))) break;
         const uint32_t fq = smem_u32(&bar_q_full[s]);
-        mbar_expect_tx(fq, TILE_BYTES);
-        load_tile<DH>(sQ + s * TILE_BYTES, &p.tmQKV, fq, qcol, qrow0, b);
+        if (leader) {
+          mbar_expect_tx(fq, TILE_BYTES);
+          load_tile<DH>(sQ + s * TILE_BYTES, &p.tmQKV, fq, qcol, qrow0, b);
+        }
         ++n_q;
         if (!(ok = mbar_wait(smem_u32(&bar_do_empty), (uint32_t)((t & 1) ^ 1), abort_flag))) break;
         const uint32_t fd = smem_u32(&bar_do_full);
-        mbar_expect_tx(fd, TILE_BYTES);
-        load_tile<DH>(sdO, &p.tmDO, fd, qcol, qrow0, b);
+        if (leader) {
+          mbar_expect_tx(fd, TILE_BYTES);
+          load_tile<DH>(sdO, &p.tmDO, fd, qcol, qrow0, b);
+        }
         ++n_do;
       }
-      Drain drain;                                           // no load may land after the CTA has retired: a role may have given up
-      drain.wait(smem_u32(&bar_kv), 0);
-      for (int t = n_q > 2 ? n_q - 2 : 0; t < n_q; ++t) drain.wait(smem_u32(&bar_q_full[t & 1]), (uint32_t)((t >> 1) & 1));
-      if (n_do) drain.wait(smem_u32(&bar_do_full), (uint32_t)((n_do - 1) & 1));
+      if (leader) {
+        Drain drain;                                           // no load may land after the CTA has retired: a role may have given up
+        drain.wait(smem_u32(&bar_kv), 0);
+        for (int t = n_q > 2 ? n_q - 2 : 0; t < n_q; ++t) drain.wait(smem_u32(&bar_q_full[t & 1]), (uint32_t)((t >> 1) & 1));
+        if (n_do) drain.wait(smem_u32(&bar_do_full), (uint32_t)((n_do - 1) & 1));
+      }
     }
   } else if (warp == 1) {
-    if (lane == 0) {
+    {
+      const bool leader = elect_one();
       const uint32_t id_kk = idesc_mn(128, false, false), id_mm = idesc_mn(DH, true, true), id_km = idesc_mn(DH, false, true);
       // descriptor bases: "k" = contraction along the 128-byte rows, "m" = contraction along the tile rows
       // (every operand is made of 128-row blocks of 64 columns, 16 KB apart)
@@ -630,12 +656,14 @@ attn_bwd_kernel(const __grid_constant__ AttnBwdParams p) {
 #define TPLR_MOFF(kk) ((uint32_t)(kk) * 128u)
       auto issue_s = [&](int t) {
         const uint32_t q = (uint32_t)(t & 1) * (TILE_BYTES / 16);
+        if (!leader) return;
 #pragma unroll
         for (int kk = 0; kk < DH / 16; ++kk)
           umma_bf16_b(tS, kQ, q + TPLR_KOFF(kk), kK, TPLR_KOFF(kk), id_kk, kk > 0 ? 1u : 0u);
         umma_commit(smem_u32(&bar_s_full));
       };
       auto issue_dp = [&] {
+        if (!leader) return;
 #pragma unroll
         for (int kk = 0; kk < DH / 16; ++kk) umma_bf16_b(tdP, kdO, TPLR_KOFF(kk), kV, TPLR_KOFF(kk), id_kk, kk > 0 ? 1u : 0u);
         umma_commit(smem_u32(&bar_dp_full));
@@ -654,20 +682,24 @@ attn_bwd_kernel(const __grid_constant__ AttnBwdParams p) {
           tcgen05_fence_after();
           issue_s(t + 1);
         }
+        if (leader) {
 #pragma unroll
-        for (int kk = 0; kk < 8; ++kk)      // dV[kv, d] += P^T[kv, q] dO[q, d]
-          umma_bf16_b(tdV, mP, TPLR_MOFF(kk), mdO, TPLR_MOFF(kk), id_mm, (t > 0 || kk > 0) ? 1u : 0u);
-        umma_commit(smem_u32(&bar_do_empty));
+          for (int kk = 0; kk < 8; ++kk)    // dV[kv, d] += P^T[kv, q] dO[q, d]
+            umma_bf16_b(tdV, mP, TPLR_MOFF(kk), mdO, TPLR_MOFF(kk), id_mm, (t > 0 || kk > 0) ? 1u : 0u);
+          umma_commit(smem_u32(&bar_do_empty));
+        }
         if (!(ok = mbar_wait(smem_u32(&bar_ds_ready), ph, abort_flag))) break;     // dS stored, dP read by every warp
         tcgen05_fence_after();
+        if (leader) {
 #pragma unroll
-        for (int kk = 0; kk < 8; ++kk)      // dK[kv, d] += dS^T[kv, q] Q[q, d]
-          umma_bf16_b(tdK, mdS, TPLR_MOFF(kk), mQ, ph * (TILE_BYTES / 16) + TPLR_MOFF(kk), id_mm, (t > 0 || kk > 0) ? 1u : 0u);
-        umma_commit(smem_u32(&bar_q_empty[ph]));
+          for (int kk = 0; kk < 8; ++kk)    // dK[kv, d] += dS^T[kv, q] Q[q, d]
+            umma_bf16_b(tdK, mdS, TPLR_MOFF(kk), mQ, ph * (TILE_BYTES / 16) + TPLR_MOFF(kk), id_mm, (t > 0 || kk > 0) ? 1u : 0u);
+          umma_commit(smem_u32(&bar_q_empty[ph]));
 #pragma unroll
-        for (int kk = 0; kk < 8; ++kk)      // dQ[q, d] = dS[q, kv] K[kv, d], over dP; its commit covers every product before it
-          umma_bf16_b(tdP, kdS, TPLR_KOFF(kk), mK, TPLR_MOFF(kk), id_km, kk > 0 ? 1u : 0u);
-        umma_commit(smem_u32(&bar_dq_full));
+          for (int kk = 0; kk < 8; ++kk)    // dQ[q, d] = dS[q, kv] K[kv, d], over dP; its commit covers every product before it
+            umma_bf16_b(tdP, kdS, TPLR_KOFF(kk), mK, TPLR_MOFF(kk), id_km, kk > 0 ? 1u : 0u);
+          umma_commit(smem_u32(&bar_dq_full));
+        }
         if (t + 1 < n_it) {
           if (!(ok = mbar_wait(smem_u32(&bar_do_full), ph ^ 1u, abort_flag))) break;
           if (!(ok = mbar_wait(smem_u32(&bar_dq_free), ph, abort_flag))) break;    // dQ read by every warp
@@ -1012,7 +1044,7 @@ attn_bwd2_kernel(const __grid_constant__ AttnBwd2Params p) {
   __shared__ uint32_t s_tmem_base;
   __shared__ int s_abort;
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = warp_index(), lane = threadIdx.x & 31;
   const int nQ = p.S / B2_BQ;
   const int gb = p.KV * p.B;
   const int j = (int)(blockIdx.x / gb);
@@ -1049,12 +1081,15 @@ attn_bwd2_kernel(const __grid_constant__ AttnBwd2Params p) {
   const float* stat = reinterpret_cast<const float*>(smem + (sStat - sK));     // [2][lse 64 | delta 64]
 
   if (warp == 0) {
-    if (lane == 0) {
-      mbar_expect_tx(smem_u32(&bar_kv), 2 * TILE_BYTES);
-      tma_load_2d(sK, &p.tmKV, smem_u32(&bar_kv), kcol, kvrow0);
-      tma_load_2d(sK + TILE_BYTES / 2, &p.tmKV, smem_u32(&bar_kv), kcol + 64, kvrow0);
-      tma_load_2d(sV, &p.tmKV, smem_u32(&bar_kv), vcol, kvrow0);
-      tma_load_2d(sV + TILE_BYTES / 2, &p.tmKV, smem_u32(&bar_kv), vcol + 64, kvrow0);
+    {
+      const bool leader = elect_one();
+      if (leader) {
+        mbar_expect_tx(smem_u32(&bar_kv), 2 * TILE_BYTES);
+        tma_load_2d(sK, &p.tmKV, smem_u32(&bar_kv), kcol, kvrow0);
+        tma_load_2d(sK + TILE_BYTES / 2, &p.tmKV, smem_u32(&bar_kv), kcol + 64, kvrow0);
+        tma_load_2d(sV, &p.tmKV, smem_u32(&bar_kv), vcol, kvrow0);
+        tma_load_2d(sV + TILE_BYTES / 2, &p.tmKV, smem_u32(&bar_kv), vcol + 64, kvrow0);
+      }
       bool ok = true;
       int n_q = 0;                                           // steps asked for
       for (int t = 0; t < n_it && ok; ++t) {
@@ -1063,23 +1098,28 @@ attn_bwd2_kernel(const __grid_constant__ AttnBwd2Params p) {
         const int qrow0 = b * p.S + iq * B2_BQ, qcol = h * DH;
         if (!(ok = mbar_wait(smem_u32(&bar_q_empty[s]), (uint32_t)((k & 1) ^ 1), abort_flag))) break;
         const uint32_t fb = smem_u32(&bar_q_full[s]);
-        mbar_expect_tx(fb, 2 * B2_QTILE + 512);
-        const uint32_t q_dst = sQ0 + s * B2_QTILE, do_dst = sdO0 + s * B2_QTILE;
-        tma_load_2d(q_dst, &p.tmQ, fb, qcol, qrow0);
-        tma_load_2d(q_dst + 8192, &p.tmQ, fb, qcol + 64, qrow0);
-        tma_load_2d(do_dst, &p.tmDO, fb, qcol, qrow0);
-        tma_load_2d(do_dst + 8192, &p.tmDO, fb, qcol + 64, qrow0);
-        const long long so = ((long long)b * p.H + h) * p.S + (long long)iq * B2_BQ;
-        bulk_load_1d(sStat + s * 512, p.lse + so, 256, fb);
-        bulk_load_1d(sStat + s * 512 + 256, p.delta + so, 256, fb);
+        if (leader) {
+          mbar_expect_tx(fb, 2 * B2_QTILE + 512);
+          const uint32_t q_dst = sQ0 + s * B2_QTILE, do_dst = sdO0 + s * B2_QTILE;
+          tma_load_2d(q_dst, &p.tmQ, fb, qcol, qrow0);
+          tma_load_2d(q_dst + 8192, &p.tmQ, fb, qcol + 64, qrow0);
+          tma_load_2d(do_dst, &p.tmDO, fb, qcol, qrow0);
+          tma_load_2d(do_dst + 8192, &p.tmDO, fb, qcol + 64, qrow0);
+          const long long so = ((long long)b * p.H + h) * p.S + (long long)iq * B2_BQ;
+          bulk_load_1d(sStat + s * 512, p.lse + so, 256, fb);
+          bulk_load_1d(sStat + s * 512 + 256, p.delta + so, 256, fb);
+        }
         ++n_q;
       }
-      Drain drain;                                           // as in the kernel above
-      drain.wait(smem_u32(&bar_kv), 0);
-      for (int t = n_q > 2 ? n_q - 2 : 0; t < n_q; ++t) drain.wait(smem_u32(&bar_q_full[t & 1]), (uint32_t)((t >> 1) & 1));
+      if (leader) {
+        Drain drain;                                         // as in the kernel above
+        drain.wait(smem_u32(&bar_kv), 0);
+        for (int t = n_q > 2 ? n_q - 2 : 0; t < n_q; ++t) drain.wait(smem_u32(&bar_q_full[t & 1]), (uint32_t)((t >> 1) & 1));
+      }
     }
   } else if (warp == 1) {
-    if (lane == 0) {
+    {
+      const bool leader = elect_one();
       const uint32_t id_st = idesc_mn(64, false, false);     // S^T, dP^T : K-major A and B, N = 64
       const uint32_t id_dv = idesc_mn(128, false, true);     // dV, dK   : A from TMEM, B N-contiguous, N = 128
       const uint32_t id_dq = idesc_mn(64, true, true);       // dQ^T     : A M-contiguous (K^T), B N-contiguous
@@ -1096,12 +1136,14 @@ attn_bwd2_kernel(const __grid_constant__ AttnBwd2Params p) {
 #define TPLR_K64(kk) ((uint32_t)((kk) >> 2) * 512u + (uint32_t)((kk) & 3) * 2u)                /* 64-row tile */
 #define TPLR_M(kk) ((uint32_t)(kk) * 128u)
       auto issue_st = [&](int t) {                            // S^T(t) = K Q^T into S buffer t & 1
+        if (!leader) return;
 #pragma unroll
         for (int kk = 0; kk < 8; ++kk)
           umma_bf16_b(tS0 + (t & 1) * 64, kK, TPLR_K128(kk), kQ[t & 1], TPLR_K64(kk), id_st, kk > 0 ? 1u : 0u);
         umma_commit(smem_u32(&bar_s_full[t & 1]));
       };
       auto issue_dp = [&](int t) {                            // dP^T(t) = V dO^T
+        if (!leader) return;
 #pragma unroll
         for (int kk = 0; kk < 8; ++kk) umma_bf16_b(tdP, kV, TPLR_K128(kk), kdO[t & 1], TPLR_K64(kk), id_st, kk > 0 ? 1u : 0u);
         umma_commit(smem_u32(&bar_dp_full));
@@ -1122,21 +1164,26 @@ attn_bwd2_kernel(const __grid_constant__ AttnBwd2Params p) {
         const uint32_t ph = t & 1;
         if (!(ok = mbar_wait(smem_u32(&bar_p_ready), ph, abort_flag))) break;
         tcgen05_fence_after();
+        if (leader)
 #pragma unroll
         for (int kk = 0; kk < 4; ++kk)          // dV += P^T dO ; P^T packed at columns 0-15 and 32-47 of the S buffer
           umma_ts_bf16_b(tdV, tS0 + s * 64 + (kk >> 1) * 32 + (kk & 1) * 8, mdO[s], TPLR_M(kk), id_dv, (t > 0 || kk > 0) ? 1u : 0u);
         if (!(ok = mbar_wait(smem_u32(&bar_ds_ready), ph, abort_flag))) break;
         tcgen05_fence_after();
+        if (leader)
 #pragma unroll
         for (int kk = 0; kk < 4; ++kk)          // dK += dS^T Q
           umma_ts_bf16_b(tdK, tdP + (kk >> 1) * 32 + (kk & 1) * 8, mQ[s], TPLR_M(kk), id_dv, (t > 0 || kk > 0) ? 1u : 0u);
         if (t > 0 && !(ok = mbar_wait(smem_u32(&bar_dq_free), (uint32_t)((t - 1) & 1), abort_flag))) break;
         tcgen05_fence_after();
+        if (leader)
 #pragma unroll
         for (int kk = 0; kk < 8; ++kk)          // dQ^T = K^T dS^T
           umma_bf16_b(tdQ, mK, TPLR_M(kk), mdS[s], TPLR_M(kk), id_dq, kk > 0 ? 1u : 0u);
-        umma_commit(smem_u32(&bar_dq_full));
-        umma_commit(smem_u32(&bar_q_empty[s]));
+        if (leader) {
+          umma_commit(smem_u32(&bar_dq_full));
+          umma_commit(smem_u32(&bar_q_empty[s]));
+        }
         if (t + 1 < n_it) issue_dp(t + 1);
         if (t + 2 < n_it) {
           if (!(ok = mbar_wait(smem_u32(&bar_q_full[s]), (uint32_t)(((t + 2) >> 1) & 1), abort_flag))) break;
