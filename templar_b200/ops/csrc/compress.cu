@@ -679,21 +679,20 @@ __device__ __forceinline__ void load_basis_split(const float* __restrict__ g, ui
 // D[128 x 64] = A B with the six significant products of the 3-term splits.  a_mn: A tile holds K rows of
 // 128 bytes of M (two 64-wide M blocks 8 KB apart); otherwise A tile holds 128 M rows of 128 bytes of K.
 // b_mn: the basis tile is read with its rows as K (B = F); otherwise with its rows as N (B = F^T).
+// Called by an elected lane of a warp-uniform branch: 24 products of 128 x 64 x 16 are short, and under `tid == 0` each took 155
+// cycles to issue.  compress_1b layout (402 M parameters, k = 32) 4114 -> 3749 us a call, the same bits; eight peers' outer step 1576 -> 1506.
 __device__ __forceinline__ void issue_split_gemm(uint32_t tD, uint32_t sA, uint32_t sB, bool a_mn, bool b_mn) {
   const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((a_mn ? 1u : 0u) << 15) | ((b_mn ? 1u : 0u) << 16) |
                          ((uint32_t)(64 >> 3) << 17) | ((uint32_t)(128 >> 4) << 24);
   const int ta[6] = {0, 0, 1, 0, 1, 2}, tb[6] = {0, 1, 0, 2, 1, 0};
-  uint32_t first = 1;
+  const DescBase dA = a_mn ? desc_base(sA, 8192, 1024) : desc_base(sA, 16, 1024), dB = b_mn ? desc_base(sB, 8192, 1024) : desc_base(sB, 16, 1024);
+  const uint32_t sa = a_mn ? 2048u / 16u : 32u / 16u, sb = b_mn ? 2048u / 16u : 32u / 16u;
 #pragma unroll
   for (int kk = 0; kk < 4; ++kk) {
 #pragma unroll
-    for (int t = 0; t < 6; ++t) {
-      const uint32_t a0 = sA + (uint32_t)ta[t] * TC_A_TILE, b0 = sB + (uint32_t)tb[t] * TC_B_TILE;
-      const uint64_t da = a_mn ? make_desc(a0 + kk * 2048u, 8192, 1024) : make_desc(a0 + kk * 32u, 16, 1024);
-      const uint64_t db = b_mn ? make_desc(b0 + kk * 2048u, 8192, 1024) : make_desc(b0 + kk * 32u, 16, 1024);
-      umma_bf16(tD, da, db, idesc, first ? 0u : 1u);
-      first = 0;
-    }
+    for (int t = 0; t < 6; ++t)
+      umma_bf16_b(tD, dA, (uint32_t)ta[t] * (TC_A_TILE / 16) + kk * sa, dB, (uint32_t)tb[t] * (TC_B_TILE / 16) + kk * sb, idesc,
+                  kk > 0 || t > 0 ? 1u : 0u);
   }
 }
 
@@ -711,7 +710,7 @@ __global__ void __launch_bounds__(NT, 3) aggregate_tc_kernel(const AggArgs a) {
   const unsigned short* Cnt16 = reinterpret_cast<const unsigned short*>(Cnt);
   const uint32_t sA = smem_u32(smem), sB = sA + TC_ACC_BYTES;
 
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int tid = threadIdx.x, warp = warp_index(), lane = tid & 31;
   const int qd = warp & 3, hf = warp >> 2;                         // TMEM lane quadrant, column half
   const int ch = qd >> 1, rin = (qd & 1) * 32 + lane;              // chunk of the pair, row inside the chunk
   const int trow = ch * 64 + rin;                                  // row of the stacked 128-row tiles
@@ -864,7 +863,7 @@ __global__ void __launch_bounds__(NT, 3) aggregate_tc_kernel(const AggArgs a) {
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     tcgen05_fence_before();
     __syncthreads();
-    if (tid == 0) {
+    if (warp == 0 && elect_one()) {
       tcgen05_fence_after();
       issue_split_gemm(tZ, sA, sB, /*a_mn=*/false, /*b_mn=*/true);      // Z = S^T F
       umma_commit(smem_u32(&bar_mma));
@@ -889,7 +888,7 @@ __global__ void __launch_bounds__(NT, 3) aggregate_tc_kernel(const AggArgs a) {
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     tcgen05_fence_before();
     __syncthreads();
-    if (tid == 0) {
+    if (warp == 0 && elect_one()) {
       tcgen05_fence_after();
       issue_split_gemm(tG, sA, sB, /*a_mn=*/true, /*b_mn=*/true);       // g = Z^T F
       umma_commit(smem_u32(&bar_mma));
@@ -1001,7 +1000,7 @@ __global__ void __launch_bounds__(NT, 3) compress_tc_kernel(const CompressArgs a
   __shared__ float s_sel_val[2][TPLR_TILE];
   const uint32_t sA = smem_u32(smem), sB = sA + 3 * TC_A_TILE;
 
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int tid = threadIdx.x, warp = warp_index(), lane = tid & 31;
   const int qd = warp & 3, hf = warp >> 2;
   const int ch = qd >> 1, rin = (qd & 1) * 32 + lane;
   const int trow = ch * 64 + rin;
@@ -1033,7 +1032,7 @@ __global__ void __launch_bounds__(NT, 3) compress_tc_kernel(const CompressArgs a
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     tcgen05_fence_before();
     __syncthreads();
-    if (tid == 0) {
+    if (warp == 0 && elect_one()) {
       tcgen05_fence_after();
       issue_split_gemm(tD, sA, sB, a_mn, b_mn);
       umma_commit(smem_u32(&bar_mma));
