@@ -38,6 +38,7 @@ constexpr int STAGE_BYTES = A_STAGE + B_STAGE;     // 32 KB
 constexpr int EPI_STAGE_BYTES = 4 * 2 * 4096;      // 4 epilogue warps x 2 buffers x (32 rows x 128 B)
 constexpr int SMEM_BYTES = STAGES * STAGE_BYTES + EPI_STAGE_BYTES + 1024;
 constexpr int EPI5_STAGES = STAGES - 1;            // the SwiGLU backward has a second pair of staging buffers per warp instead
+constexpr int MAX_STAGES = 8;                      // narrower tiles have smaller stages, so more of them fit the ring
 static_assert(4 * 8192 <= STAGE_BYTES, "the freed stage holds four warps' second pair");
 constexpr int NUM_THREADS = 192;
 constexpr int MAX_RANKS = 8;
@@ -52,6 +53,7 @@ struct Gemm2Params {
   long long ldc;
   int M, N, K;
   unsigned int* status;
+  int tile_n;                        // columns of a pair's tile: 256, 192 or 128 (see plan_cost); each CTA stages half of them
   int n_compute_pairs;               // CTA pairs [0, n_compute_pairs) compute, the rest are comm CTAs
   int group_m;                       // tile order: bands of group_m tile rows, tile row fastest inside a band
   int m_rot;                         // rotation of the tile-row order (in 256-row tiles)
@@ -230,7 +232,7 @@ template <int EPI>
 __device__ __forceinline__ void epilogue_direct(const Gemm2Params& p, uint32_t tmem_acc, int quad, int lane, int m0, int n0) {
   const int row = m0 + quad * 32 + lane;
 #pragma unroll 1
-  for (int c = 0; c < TILE_N / 32; ++c) {
+  for (int c = 0; c < p.tile_n / 32; ++c) {
     uint32_t r[32];
     tmem_ld32(tmem_acc + c * 32 + ((uint32_t)(quad * 32) << 16), r);
     const int col0 = n0 + c * 32;
@@ -309,7 +311,7 @@ __device__ __forceinline__ void epilogue_tma(const Gemm2Params& p, uint32_t tmem
     y = row0 - p.rs_bound[owner];
   }
 #pragma unroll 1
-  for (int c = 0; c < TILE_N / COLS; ++c) {
+  for (int c = 0; c < p.tile_n / COLS; ++c) {
     const int col0 = n0 + c * COLS;
     if (row0 >= p.M || col0 >= p.N) break;          // warp-uniform: nothing of this box is inside C
     const uint32_t buf = stage_base + (n_boxes & 1u) * 4096u;
@@ -416,7 +418,7 @@ __device__ __forceinline__ void epilogue_rope(const Gemm2Params& p, uint32_t tme
   RopeRow<DH> rr;
   if (n0 < p.rope_cols) rr.load(p, min(row0 + lane, p.M - 1));
 #pragma unroll 1
-  for (int h = 0; h < TILE_N / DH; ++h) {
+  for (int h = 0; h < p.tile_n / DH; ++h) {
     if (n0 + h * DH >= p.N) break;
     const bool rot = n0 + h * DH < p.rope_cols;      // whole heads (rope_cols is a multiple of DH)
 #pragma unroll
@@ -444,9 +446,9 @@ __device__ __forceinline__ void epilogue_rope(const Gemm2Params& p, uint32_t tme
   }
 }
 
-// Epilogue of the fused [w1; w3] projection (EPI 3): accumulator columns 0..127 of a row are the gate values g of features
-// [128 tn, 128 tn + 128), columns 128..255 the up values u of the same features.  Per 64 features: g and u go to C (bf16,
-// columns 128 tn + .. and swiglu_f + 128 tn + ..: what the backward pass reads) and h = silu(g) * u, computed from the fp32
+// Epilogue of the fused [w1; w3] projection (EPI 3): the first half of a row's accumulator columns are the gate values g of
+// features [h tn, h tn + h) with h = tile_n / 2, the second half the up values u of the same features.  Per 64 features: g and
+// u go to C (bf16, columns h tn + .. and swiglu_f + h tn + ..: what the backward pass reads) and h = silu(g) * u, computed from the fp32
 // accumulators, goes to the [M, swiglu_f] tensor behind tmCr[0].  Replaces a separate pass that re-reads g and u
 // (the reference's F.silu(w1(x)) * w3(x), torchtitan models/llama3/model/model.py FeedForward.forward).
 // The accumulators are read twice (once for the g / u boxes, once for h): tensor-memory loads are cheap and 32 values
@@ -456,9 +458,10 @@ __device__ __forceinline__ void epilogue_swiglu(const Gemm2Params& p, uint32_t t
   const int row0 = m0 + quad * 32;
   if (row0 >= p.M) return;                           // warp-uniform
   const uint32_t lane_sel = (uint32_t)(quad * 32) << 16;
+  const int half = p.tile_n / 2;                     // features of a tile
 #pragma unroll 1
-  for (int c = 0; c < 2; ++c) {
-    const int f0 = tn * CTA_N + c * 64;              // first feature of this box
+  for (int c = 0; c < half / 64; ++c) {
+    const int f0 = tn * half + c * 64;               // first feature of this box
     if (f0 >= p.swiglu_f) break;
 #pragma unroll 1
     for (int part = p.C ? 0 : 2; part < 2; ++part) { // 0: g box, 1: u box; a caller without a backward pass has no C
@@ -467,7 +470,7 @@ __device__ __forceinline__ void epilogue_swiglu(const Gemm2Params& p, uint32_t t
       for (int hh = 0; hh < 2; ++hh) {
         uint32_t r[32];
         float v[32];
-        tmem_ld32(tmem_acc + part * CTA_N + c * 64 + hh * 32 + lane_sel, r);
+        tmem_ld32(tmem_acc + part * half + c * 64 + hh * 32 + lane_sel, r);
 #pragma unroll
         for (int e = 0; e < 32; ++e) v[e] = __uint_as_float(r[e]);
         box_half(buf, lane, hh, v);
@@ -480,7 +483,7 @@ __device__ __forceinline__ void epilogue_swiglu(const Gemm2Params& p, uint32_t t
       uint32_t rg[32], ru[32];
       float v[32];
       tmem_ld32(tmem_acc + c * 64 + hh * 32 + lane_sel, rg);
-      tmem_ld32(tmem_acc + CTA_N + c * 64 + hh * 32 + lane_sel, ru);
+      tmem_ld32(tmem_acc + half + c * 64 + hh * 32 + lane_sel, ru);
 #pragma unroll
       for (int e = 0; e < 32; ++e) {
         const float g = __uint_as_float(rg[e]);
@@ -523,10 +526,10 @@ __device__ __forceinline__ bool epilogue_swiglu_bwd(const Gemm2Params& p, uint32
   const uint32_t lane_sel = (uint32_t)(quad * 32) << 16;
   const uint32_t sw = (uint32_t)(lane & 7);
 #pragma unroll 1
-  for (int c = 0; c < TILE_N / 64; ++c) {
+  for (int c = 0; c < p.tile_n / 64; ++c) {
     const int f0 = n0 + c * 64;
     if (f0 >= p.swiglu_f) break;                     // warp-uniform (swiglu_f is a multiple of 64)
-    if (c + 1 < TILE_N / 64 && f0 + 64 < p.swiglu_f) gu_issue(p, L, lane, f0 + 64, row0);
+    if (c + 1 < p.tile_n / 64 && f0 + 64 < p.swiglu_f) gu_issue(p, L, lane, f0 + 64, row0);
     const uint32_t s = L.used & 1u;
     const bool ok = mbar_wait(L.bar + 8u * s, (L.used >> 1) & 1u, abort_flag);
     if (!__all_sync(0xffffffffu, ok)) return false;
@@ -599,12 +602,13 @@ __device__ __forceinline__ void epilogue_attn_dout(const Gemm2Params& p, uint32_
   };
   fetch(0, oq);
   float acc = 0.f;
-#pragma unroll
-  for (int step = 0; step < TILE_N / 32; ++step) {
+  const int steps = p.tile_n / 32;
+#pragma unroll 2
+  for (int step = 0; step < steps; ++step) {
     const int c = step >> 1, hh = step & 1;
     const int f0 = n0 + c * 64;
     if (f0 >= p.N) break;                            // warp-uniform (N is a multiple of 64)
-    if (step + 1 < TILE_N / 32) fetch(step + 1, on);
+    if (step + 1 < steps) fetch(step + 1, on);
     uint32_t buf = 0;
     if (hh == 0) buf = box_begin(lane, stage_base, n_boxes); else buf = stage_base + (n_boxes & 1u) * 4096u;
     uint32_t r[32];
@@ -642,10 +646,10 @@ __device__ __forceinline__ void epilogue_attn_dout(const Gemm2Params& p, uint32_
 template <bool A_MN, bool B_MN, int EPI>
 __global__ void __launch_bounds__(NUM_THREADS, 1)
 gemm2_kernel(const __grid_constant__ Gemm2Params p) {
-  constexpr int STAGES = EPI == 5 ? EPI5_STAGES : ::STAGES;
+  constexpr int RING_BYTES = (EPI == 5 ? EPI5_STAGES : STAGES) * STAGE_BYTES;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
-  __shared__ __align__(8) uint64_t bar_full[STAGES], bar_empty[STAGES], bar_tfull[2], bar_tempty[2];
+  __shared__ __align__(8) uint64_t bar_full[MAX_STAGES], bar_empty[MAX_STAGES], bar_tfull[2], bar_tempty[2];
   __shared__ uint32_t s_tmem_base;
   __shared__ int s_abort;
   __shared__ __align__(8) uint64_t bar_gu[EPI == 5 ? 8 : 1];      // EPI 5: two per epilogue warp
@@ -655,7 +659,10 @@ gemm2_kernel(const __grid_constant__ Gemm2Params p) {
   const uint32_t cr = cluster_ctarank();
   const int pair = blockIdx.x >> 1, n_pairs = gridDim.x >> 1;
   const bool is_compute = pair < p.n_compute_pairs;
-  const int tiles_m = (p.M + TILE_M - 1) / TILE_M, tiles_n = (p.N + TILE_N - 1) / TILE_N;
+  const int tile_n = p.tile_n, cta_n = tile_n / 2;                  // cta_n: columns of B that each CTA stages
+  const uint32_t b_stage = B_MN ? (uint32_t)((cta_n + 63) / 64) * (BK * 128) : (uint32_t)cta_n * 128u;
+  const int n_stages = min(MAX_STAGES, (int)(RING_BYTES / (A_STAGE + b_stage)));
+  const int tiles_m = (p.M + TILE_M - 1) / TILE_M, tiles_n = (p.N + tile_n - 1) / tile_n;
   const int k_blocks_all = (p.K + BK - 1) / BK;
   const int k_per = (k_blocks_all + p.k_splits - 1) / p.k_splits;   // k blocks per work unit (static mode)
   const int num_tiles = p.tri ? tiles_m * (tiles_m + 1) / 2 : tiles_m * tiles_n;
@@ -663,7 +670,7 @@ gemm2_kernel(const __grid_constant__ Gemm2Params p) {
 
   if (threadIdx.x == 0) {
     s_abort = 0;
-    for (int s = 0; s < STAGES; ++s) {
+    for (int s = 0; s < MAX_STAGES; ++s) {
       mbar_init(smem_u32(&bar_full[s]), 1);
       mbar_init(smem_u32(&bar_empty[s]), 1);
     }
@@ -684,7 +691,7 @@ gemm2_kernel(const __grid_constant__ Gemm2Params p) {
   tcgen05_fence_after();
   const uint32_t tmem_base = s_tmem_base;
   const uint32_t sbase = smem_u32(smem);
-  const uint32_t sA = sbase, sB = sbase + STAGES * A_STAGE, sEpi = sbase + STAGES * STAGE_BYTES;
+  const uint32_t sA = sbase, sB = sbase + n_stages * A_STAGE, sEpi = sbase + RING_BYTES;
 
   if (is_compute) {
     if (warp == 0) {
@@ -717,9 +724,9 @@ gemm2_kernel(const __grid_constant__ Gemm2Params p) {
           const int kb0 = w.kb0;
           const int k_blocks = w.nkb;
           const int m0 = tm * TILE_M + (int)cr * CTA_M;
-          const int n0 = EPI == 3 ? tn * CTA_N + (int)cr * p.swiglu_f : tn * TILE_N + (int)cr * CTA_N;
+          const int n0 = EPI == 3 ? tn * cta_n + (int)cr * p.swiglu_f : tn * tile_n + (int)cr * cta_n;
           if (p.ag_operand == 1 && !A_MN) ok = rows_ready_warp(m0, CTA_M);
-          if (p.ag_operand == 2 && !B_MN) ok = ok && rows_ready_warp(n0, CTA_N);
+          if (p.ag_operand == 2 && !B_MN) ok = ok && rows_ready_warp(n0, cta_n);
           for (int kb = 0; kb < k_blocks && ok; ++kb, ++it) {
             // k order rotated so that the rows of the local shard come first when k is the gathered dimension
             int kbr = kb0 + kb;
@@ -728,11 +735,13 @@ gemm2_kernel(const __grid_constant__ Gemm2Params p) {
               if (kbr >= k_blocks) kbr -= k_blocks;
               if (!(ok = rows_ready_warp(kbr * BK, BK))) break;
             }
-            if (!(ok = __all_sync(0xffffffffu, mbar_wait(empty0 + 8u * s, ph ^ 1u, abort_flag)))) break;
+            ok = mbar_wait(empty0 + 8u * s, ph ^ 1u, abort_flag);
+            if (p.ag_operand) ok = __all_sync(0xffffffffu, ok);        // the votes above need every lane
+            if (!ok) break;
             if (leader) {
-              if (cr == 0) mbar_expect_tx(full0 + 8u * s, 2 * STAGE_BYTES);
+              if (cr == 0) mbar_expect_tx(full0 + 8u * s, 2 * (A_STAGE + b_stage));
               const uint32_t fb = fullp0 + 8u * s;
-              const uint32_t a_dst = sA + s * A_STAGE, b_dst = sB + s * B_STAGE;
+              const uint32_t a_dst = sA + s * A_STAGE, b_dst = sB + s * b_stage;
               const int k0 = kbr * BK;
               if (!A_MN) {
                 tma_load_2d_pair(a_dst, &p.tmA, fb, k0, m0);
@@ -743,19 +752,18 @@ gemm2_kernel(const __grid_constant__ Gemm2Params p) {
               if (!B_MN) {
                 tma_load_2d_pair(b_dst, &p.tmB, fb, k0, n0);
               } else {
-#pragma unroll
-                for (int j = 0; j < CTA_N / 64; ++j) tma_load_2d_pair(b_dst + j * (BK * 128), &p.tmB, fb, n0 + 64 * j, k0);
+                for (int j = 0; j < cta_n; j += 64) tma_load_2d_pair(b_dst + j * 128, &p.tmB, fb, n0 + j, k0);
               }
             }
-            if (++s == STAGES) { s = 0; ph ^= 1u; }
+            if (++s == (uint32_t)n_stages) { s = 0; ph ^= 1u; }
           }
         }
         // drain (even CTA): every armed stage has landed in both CTAs before the pair may retire
         if (leader && cr == 0) {
           Drain drain;
-          for (uint32_t back = 0; back < STAGES && back < it; ++back) {
+          for (uint32_t back = 0; back < (uint32_t)n_stages && back < it; ++back) {
             const uint32_t j = it - 1 - back;
-            drain.wait(smem_u32(&bar_full[j % STAGES]), (j / STAGES) & 1);
+            drain.wait(smem_u32(&bar_full[j % n_stages]), (j / n_stages) & 1);
           }
         }
       }
@@ -764,8 +772,8 @@ gemm2_kernel(const __grid_constant__ Gemm2Params p) {
       if (cr == 0) {
         const bool leader = elect_one();
         const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((A_MN ? 1u : 0u) << 15) |
-                               ((B_MN ? 1u : 0u) << 16) | ((uint32_t)(TILE_N >> 3) << 17) | ((uint32_t)(TILE_M >> 4) << 24);
-        uint32_t it = 0, tile_i = 0;
+                               ((B_MN ? 1u : 0u) << 16) | ((uint32_t)(tile_n >> 3) << 17) | ((uint32_t)(TILE_M >> 4) << 24);
+        uint32_t tile_i = 0;
         bool ok = true;
         Work w;
         work_init(p, w, pair);
@@ -774,25 +782,26 @@ gemm2_kernel(const __grid_constant__ Gemm2Params p) {
         const DescBase dA0 = A_MN ? desc_base(sA, BK * 128, 1024) : desc_base(sA, 16, 1024);
         const DescBase dB0 = B_MN ? desc_base(sB, BK * 128, 1024) : desc_base(sB, 16, 1024);
         constexpr uint32_t A_KSTEP = (A_MN ? UMMA_K * 128 : UMMA_K * 2) >> 4, B_KSTEP = (B_MN ? UMMA_K * 128 : UMMA_K * 2) >> 4;
-        uint32_t s = 0, ph = 0;                          // ring position of `it` (no division in the loop)
+        uint32_t s = 0, ph = 0;                          // ring position (no division in the loop)
+        const uint32_t full0 = smem_u32(&bar_full[0]), empty0 = smem_u32(&bar_empty[0]);
         for (; ok && work_get(p, w, num_tiles, k_blocks_all, k_per); work_next(p, w), ++tile_i) {
           const int k_blocks = w.nkb;
           const uint32_t acc = tile_i & 1, acc_ph = (tile_i >> 1) & 1;
           if (!(ok = mbar_wait(smem_u32(&bar_tempty[acc]), acc_ph ^ 1, abort_flag))) break;
           tcgen05_fence_after();
           const uint32_t d_tmem = tmem_base + acc * TILE_N;
-          for (int kb = 0; kb < k_blocks; ++kb, ++it) {
-            if (!(ok = mbar_wait(smem_u32(&bar_full[s]), ph, abort_flag))) break;
+          for (int kb = 0; kb < k_blocks; ++kb) {
+            if (!(ok = mbar_wait(full0 + 8u * s, ph, abort_flag))) break;
             tcgen05_fence_after();
-            const uint32_t a_lo = dA0.lo + s * (A_STAGE >> 4), b_lo = dB0.lo + s * (B_STAGE >> 4);
+            const uint32_t a_lo = dA0.lo + s * (A_STAGE >> 4), b_lo = dB0.lo + s * (b_stage >> 4);
             if (leader) {
 #pragma unroll
               for (int kk = 0; kk < BK / UMMA_K; ++kk)
                 umma_bf16_pair_lohi(d_tmem, a_lo + kk * A_KSTEP, dA0.hi, b_lo + kk * B_KSTEP, dB0.hi, idesc,
                                     (kb > 0 || kk > 0) ? 1u : 0u);
-              umma_commit_pair(smem_u32(&bar_empty[s]));
+              umma_commit_pair(empty0 + 8u * s);
             }
-            if (++s == STAGES) { s = 0; ph ^= 1u; }
+            if (++s == (uint32_t)n_stages) { s = 0; ph ^= 1u; }
           }
           if (ok && leader) umma_commit_pair(smem_u32(&bar_tfull[acc]));
         }
@@ -809,7 +818,7 @@ gemm2_kernel(const __grid_constant__ Gemm2Params p) {
       for (; ok && work_get(p, w, num_tiles, k_blocks_all, k_per); work_next(p, w), ++tile_i) {
         int tm, tn;
         tile_coords(p, w.tile, tiles_m, tiles_n, tm, tn);
-        const int m0 = tm * TILE_M + (int)cr * CTA_M, n0 = tn * TILE_N;
+        const int m0 = tm * TILE_M + (int)cr * CTA_M, n0 = tn * tile_n;
         const uint32_t acc = tile_i & 1, acc_ph = (tile_i >> 1) & 1;
         if (EPI == 5 && m0 + quad * 32 < p.M && n0 < p.swiglu_f) gu_issue(p, gl, lane, n0, m0 + quad * 32);   // while the main loop runs
         ok = mbar_wait(smem_u32(&bar_tfull[acc]), acc_ph, abort_flag);
@@ -934,7 +943,7 @@ int launch2(Gemm2Params& p, int n_comm_pairs, int max_pairs, cudaStream_t st) {
   if (max_pairs > 0 && pairs > max_pairs) pairs = max_pairs;
   if (n_comm_pairs >= pairs) return -106;
   const int tiles_m_h = (p.M + TILE_M - 1) / TILE_M;
-  const int tiles = p.tri ? tiles_m_h * (tiles_m_h + 1) / 2 : tiles_m_h * ((p.N + TILE_N - 1) / TILE_N);
+  const int tiles = p.tri ? tiles_m_h * (tiles_m_h + 1) / 2 : tiles_m_h * ((p.N + p.tile_n - 1) / p.tile_n);
   int compute = pairs - n_comm_pairs;
   if (compute > tiles * p.k_splits) compute = tiles * p.k_splits;
   p.n_compute_pairs = compute;
@@ -959,28 +968,67 @@ int forced_splits() {                                     // tuning override
   return forced;
 }
 
-// Parts of K of an accumulating GEMM (C += ...): where its tiles fill the chip's CTA pairs badly, a tile's K range is cut into
-// several work units that run on different pairs.  Part 0 adds into C, the others store fp32 planes, and a second kernel adds
-// those to C in order: the same bits on every run, which parts added into C as they arrive do not give.  The number with the
-// fewest k block times (0.37 us each) wins, fitted on 33 weight-gradient shapes from 768 x 768 to 32000 x 2048, K 333 to
-// 16384: waves of units, 8 k blocks per unit for its pipeline fill and its reduction, and for the planes 6 for the launch and
-// 2 + 1.2 * parts per million elements of C.  A cut has to win 5 %.  One part against the chosen number: 768 x 768 x 8192
-// (9 tiles on 74 pairs) 53.0 -> 17.7 us with 8, 2304 x 768 x 8192 53.2 -> 35.1 with 2, 1536 x 1536 x 4096 31.5 -> 25.1 with 2;
-// beyond that the planes cost what the fuller waves win: 768 x 3072 x 2048 19.4 in one part and 19.3 in two,
-// 1536 x 4096 x 4096 65.4 and 66.6, and where the waves are full already a cut loses (8192 x 1536 x 4096 87.5 and 116.9).
-int pick_acc_splits(int M, int N, int K) {
-  const long long kb = (K + BK - 1) / BK, tiles = (long long)((M + TILE_M - 1) / TILE_M) * ((N + TILE_N - 1) / TILE_N);
-  if (N % 8) return 1;
-  if (forced_splits() > 0) return kb / forced_splits() >= 1 ? forced_splits() : 1;
+// Width of the tiles and parts of K of a product.
+//
+// A 256 x 256 tile takes 500 cycles for a k block of 64, which is the tensor pipe's own time.  A narrower one moves more bytes
+// for each product: 400 cycles at 192, 345 at 128 while one wave of tiles covers the product and 400 to 440 with several (what
+// the SMs can take from L2), 440 and 560 where an operand is M- or N-contiguous (twice the loads).  So narrow tiles pay where
+// 256-wide ones leave CTA pairs idle or start a wave for a few of them: 2048 x 768 x 3072 (24 tiles on 74 pairs, 48 of 128)
+// 22.6 -> 16.5 us, 8192 x 768 x 3072 (96 tiles in two waves, 128 of 192 in two shorter ones) 43.2 -> 34.0, 1024 x 6144 x 4096 47.2
+// -> 39.0, 1111 x 8192 x 1536 30.7 -> 26.8, weight gradient 2304 x 768 x 2048 18.6 -> 16.5; at 16384 x 2048 x 2048 (512 tiles)
+// 92.9 us with 256, 99.9 with 192, 112 with 128.  192 only with K-major B (whole 64-column blocks for each CTA otherwise).
+//
+// K is cut where even so most pairs would idle over a long K: every part stores fp32 (an accumulating product's part 0 adds into C)
+// and a second kernel adds the planes in order, the same bits on every run, which parts added as they arrive would not give.
+// It costs a launch (4000 cycles) and the planes' bytes, 5000 a cycle while they stay in L2 and 2700 beyond.  768 x 768 x 8192
+// accumulating (9 tiles) 45.2 us whole, 18.8 in eight parts; 2304 x 768 x 8192 45.2 whole, 35.0 in two; 2048 x 768 x 6144 bf16 35.0
+// whole, 24.0 in three; 8192 x 768 x 32000 341 and 294 in three.  A cut has to win 10 %, a narrower tile 3 %.
+//
+// The costs (cycles) were fitted on 70 shapes of 300 to 16384 rows, K 300 to 32000, each with every width and 1 to 8 parts.
+double plan_cost(int M, int N, int K, bool a_mn, bool b_mn, int epi, int tile_n, int parts) {
+  const long long kb = (K + BK - 1) / BK, per = (kb + parts - 1) / parts;
+  const long long tiles = (long long)((M + TILE_M - 1) / TILE_M) * ((N + tile_n - 1) / tile_n);
   const int pairs = tplr_sm_count() / 2;
+  const long long waves = (tiles * parts + pairs - 1) / pairs;
+  const double block = tile_n == 256 ? 500 : tile_n == 192 ? 400 : (a_mn || b_mn) ? (waves > 1 ? 560 : 440) : (waves > 1 ? 400 : 345);
+  double cost = (double)waves * ((double)per * block + 900.0) + (epi == 1 || epi == 2 || parts > 1 ? 20.0 : 10.0) * tile_n;
+  if (parts > 1) {
+    const double bytes = (double)M * N * (epi == 1 ? 8.0 * parts : 8.0 * parts + 2.0);
+    cost += 4000.0 + bytes / (bytes < 6e7 ? 5000.0 : 2700.0);
+  }
+  return cost;
+}
+// The widths that a layout takes; col_unit: what a tile's columns must be a multiple of (64-column boxes, whole heads).
+int pick_tile(int M, int N, int K, bool a_mn, bool b_mn, int epi, int parts = 1, int col_unit = 64) {
+  int best = TILE_N;
+  double best_cost = plan_cost(M, N, K, a_mn, b_mn, epi, TILE_N, parts);
+  for (const int tn : {192, 128}) {
+    if (tn % col_unit || (tn == 192 && b_mn)) continue;
+    const double cost = plan_cost(M, N, K, a_mn, b_mn, epi, tn, parts);
+    if (cost < 0.97 * best_cost) { best = tn; best_cost = cost; }
+  }
+  return best;
+}
+// Parts of K: epi 1 an accumulating product, 0 one with a bf16 result (K of 4096 or more and 64 tiles at most: others do not ask).
+// The callers lay their workspace out by this number, so it does not depend on the operands' layout (the M-contiguous figures).
+int pick_parts(int M, int N, int K, int epi) {
+  const long long kb = (K + BK - 1) / BK, tiles = (long long)((M + TILE_M - 1) / TILE_M) * ((N + TILE_N - 1) / TILE_N);
+  const int pairs = tplr_sm_count() / 2;
+  if (N % 8) return 1;
+  if (epi == 0 && (K < 4096 || tiles > 64)) return 1;
+  if (epi == 1 && forced_splits() > 0) return kb / forced_splits() >= 1 ? forced_splits() : 1;
+  if (kb < 32) return 1;
+  auto cost = [&](int parts) {
+    const double wide = plan_cost(M, N, K, true, true, epi, 256, parts), narrow = plan_cost(M, N, K, true, true, epi, 128, parts);
+    return wide < narrow ? wide : narrow;
+  };
   int best = 1;
-  double best_cost = 0.0;
-  for (int ks = 1; ks <= 8 && ks <= kb; ks *= 2) {
-    const long long per = (kb + ks - 1) / ks;
-    if ((ks - 1) * per >= kb) break;                      // every unit has work
-    const double planes = ks == 1 ? 0.0 : 6.0 + (double)M * N * 1e-6 * (2.0 + 1.2 * ks);
-    const double cost = (double)((tiles * ks + pairs - 1) / pairs) * (double)(per + 8) + planes;
-    if (ks == 1 || cost < 0.95 * best_cost) { best = ks; best_cost = cost; }
+  double best_cost = 0.90 * cost(1);
+  for (int parts = 2; parts <= 8 && parts <= kb; ++parts) {
+    const long long per = (kb + parts - 1) / parts;
+    if ((parts - 1) * per >= kb || tiles * parts > 4 * pairs) continue;      // every unit has work
+    const double c = cost(parts);
+    if (c < best_cost) { best = parts; best_cost = c; }
   }
   return best;
 }
@@ -1005,28 +1053,6 @@ int pick_scatter_splits(int M, int N, int K) {
   if ((K + BK - 1) / BK < 128) return 1;
   auto eff = [&](long long units) { return (double)units / (double)(((units + pairs - 1) / pairs) * pairs); };
   return eff(2 * tiles) > eff(tiles) + 0.10 ? 2 : 1;
-}
-
-// Parts of a product with a bf16 result: for long K on few tiles, where most CTA pairs would idle, each part of K stores an
-// fp32 plane of its own and one kernel adds the planes in order and rounds once (the same bits on every run, which
-// reductions into one plane would not give).  In k block times (a third of a microsecond each): 10 for the second launch and
-// M * N * (8 * parts + 2) bytes for what moves, and the cut has to win 15 %.  One pass against the chosen number of parts:
-// 2048 x 768 x 6144 (24 tiles on 74 pairs) 39 -> 25 us, 777 x 1024 x 32000 (16 tiles) 166 -> 56 us.
-int pick_out_splits(int M, int N, int K) {
-  const int pairs = tplr_sm_count() / 2;
-  const long long tiles = (long long)((M + TILE_M - 1) / TILE_M) * ((N + TILE_N - 1) / TILE_N), kb = (K + BK - 1) / BK;
-  if (2 * tiles > pairs || kb < 64 || (N % 8)) return 1;      // a short K: not worth another launch
-  const double whole = (double)(kb + 8);
-  int best = 1;
-  double best_cost = 0.85 * whole;
-  for (int ks = 2; ks <= 8 && ks <= kb; ++ks) {
-    const long long per = (kb + ks - 1) / ks;
-    if ((ks - 1) * per >= kb) continue;                   // every unit has work
-    const double cost = (double)((tiles * ks + pairs - 1) / pairs) * (double)(per + 8) + 10.0 +
-                        (double)M * N * (8 * ks + 2) / 5e12 / 0.33e-6;
-    if (cost < best_cost) { best = ks; best_cost = cost; }
-  }
-  return best;
 }
 
 // C += the planes ([n_planes][plane] fp32, rows of N elements), in order; C: rows of ldc elements, all multiples of 4 and 16-byte
@@ -1068,10 +1094,11 @@ __global__ void __launch_bounds__(256) round_rows_kernel(const float* __restrict
 
 // Fills the operand maps and the plain fields; returns 0 or a negative argument error.
 int fill_common(Gemm2Params& p, const void* A, const void* B, void* C, int M, int N, int K, long long lda,
-                long long ldb, long long ldc, int a_mn, int b_mn, int epi, unsigned int* status) {
+                long long ldb, long long ldc, int a_mn, int b_mn, int epi, unsigned int* status, int tile_n = TILE_N) {
   if ((lda % 8) || (ldb % 8) || ((uintptr_t)A & 15) || ((uintptr_t)B & 15)) return -101;
   if (!(a_mn ? make_map(&p.tmA, A, M, K, lda, 64, BK) : make_map(&p.tmA, A, K, M, lda, BK, CTA_M))) return -102;
-  if (!(b_mn ? make_map(&p.tmB, B, N, K, ldb, 64, BK) : make_map(&p.tmB, B, K, N, ldb, BK, CTA_N))) return -103;
+  if (!(b_mn ? make_map(&p.tmB, B, N, K, ldb, 64, BK) : make_map(&p.tmB, B, K, N, ldb, BK, tile_n / 2))) return -103;
+  p.tile_n = tile_n;
   p.C = C; p.ldc = ldc; p.M = M; p.N = N; p.K = K; p.status = status;
   static const int group_m = [] { const char* e = getenv("TPLR_GEMM_GROUP_M"); const int v = e ? atoi(e) : 0; return v > 0 ? v : 8; }();
   p.world = 1; p.rank = 0; p.epoch = 0; p.group_m = group_m; p.m_rot = 0; p.n_rot = 0; p.m_inter = 1; p.k_splits = 1;
@@ -1124,12 +1151,13 @@ TPLR_API int tplr_gemm2_bf16(const void* A, const void* B, void* C, int M, int N
   TPLR_ENTER();
   if (M <= 0 || N <= 0 || K <= 0) return 0;
   Gemm2Params p = {};
-  if (int r = fill_common(p, A, B, C, M, N, K, lda, ldb, ldc, a_mn, b_mn, epi, status)) return r;
+  if (int r = fill_common(p, A, B, C, M, N, K, lda, ldb, ldc, a_mn, b_mn, epi, status,
+                          pick_tile(M, N, K, a_mn, b_mn, epi))) return r;
   return dispatch2(p, a_mn, b_mn, epi, 0, max_pairs, (cudaStream_t)stream);
 }
 
 // Parts that tplr_gemm2_acc_split cuts K into for this size; 1: no workspace, call tplr_gemm2_bf16 with epi 1.
-TPLR_API int tplr_gemm2_acc_splits(int M, int N, int K) { return pick_acc_splits(M, N, K); }
+TPLR_API int tplr_gemm2_acc_splits(int M, int N, int K) { return pick_parts(M, N, K, 1); }
 
 // tplr_gemm2_bf16 with epi 1 (C fp32, C += ...) with K cut into parts: the workspace `ws` holds (parts - 1) * (M rounded up to
 // 32) * N fp32 elements (contents irrelevant).  C and ws 16-byte aligned, ldc a multiple of 4, N a multiple of 8.
@@ -1139,8 +1167,9 @@ TPLR_API int tplr_gemm2_acc_split(const void* A, const void* B, float* C, float*
   if (M <= 0 || N <= 0 || K <= 0) return 0;
   if ((N % 8) || (ldc % 4) || (((uintptr_t)C | (uintptr_t)ws) & 15)) return -101;
   Gemm2Params p = {};
-  if (int r = fill_common(p, A, B, C, M, N, K, lda, ldb, ldc, a_mn, b_mn, 1, status)) return r;
-  p.k_splits = pick_acc_splits(M, N, K);
+  const int parts = pick_parts(M, N, K, 1);
+  if (int r = fill_common(p, A, B, C, M, N, K, lda, ldb, ldc, a_mn, b_mn, 1, status, pick_tile(M, N, K, a_mn, b_mn, 1, parts))) return r;
+  p.k_splits = parts;
   p.plane_rows = (M + 31) / 32 * 32;                    // a warp's box of 32 rows stays inside its plane
   const int n_planes = p.k_splits - 1;
   if (n_planes && !make_map(&p.tmCr[0], ws, N, (long long)n_planes * p.plane_rows, N, 32, 32, CU_TENSOR_MAP_SWIZZLE_128B, true)) return -110;
@@ -1154,7 +1183,7 @@ TPLR_API int tplr_gemm2_acc_split(const void* A, const void* B, float* C, float*
 }
 
 // Parts that tplr_gemm2_bf16_split would cut K into for a bf16 result of this size; 1: no workspace, call tplr_gemm2_bf16.
-TPLR_API int tplr_gemm2_out_splits(int M, int N, int K) { return pick_out_splits(M, N, K); }
+TPLR_API int tplr_gemm2_out_splits(int M, int N, int K) { return pick_parts(M, N, K, 0); }
 
 // tplr_gemm2_bf16 with a bf16 result (epi 0) through an fp32 workspace `ws` of parts * (M rounded up to 32) * N elements
 // (16-byte aligned, contents irrelevant); C 16-byte aligned with ldc a multiple of 8, N a multiple of 8.
@@ -1164,8 +1193,9 @@ TPLR_API int tplr_gemm2_bf16_split(const void* A, const void* B, void* C, float*
   if (M <= 0 || N <= 0 || K <= 0) return 0;
   if ((N % 8) || (ldc % 8) || (((uintptr_t)C | (uintptr_t)ws) & 15)) return -101;
   Gemm2Params p = {};
-  if (int r = fill_common(p, A, B, ws, M, N, K, lda, ldb, N, a_mn, b_mn, 2, status)) return r;
-  p.k_splits = pick_out_splits(M, N, K);
+  const int parts = pick_parts(M, N, K, 0);
+  if (int r = fill_common(p, A, B, ws, M, N, K, lda, ldb, N, a_mn, b_mn, 2, status, pick_tile(M, N, K, a_mn, b_mn, 0, parts))) return r;
+  p.k_splits = parts;
   p.plane_rows = (M + 31) / 32 * 32;                    // a warp's box of 32 rows stays inside its plane
   if (!make_map(&p.tmC, ws, N, (long long)p.k_splits * p.plane_rows, N, 32, 32, CU_TENSOR_MAP_SWIZZLE_128B, true)) return -110;
   if (int r = dispatch2(p, a_mn, b_mn, 2, 0, 0, (cudaStream_t)stream)) return r;
@@ -1187,7 +1217,7 @@ TPLR_API int tplr_gemm2_swiglu(const void* X, const void* W, void* GU, void* H, 
   if (M <= 0 || F <= 0 || K <= 0) return 0;
   if (F % CTA_N || ((uintptr_t)GU & 15) || ((uintptr_t)H & 15) || (ldgu % 8) || (ldh % 8)) return -111;
   Gemm2Params p = {};
-  if (int r = fill_common(p, X, W, GU, M, 2 * F, K, ldx, ldw, ldgu, 0, 0, 0, status)) return r;
+  if (int r = fill_common(p, X, W, GU, M, 2 * F, K, ldx, ldw, ldgu, 0, 0, 0, status, pick_tile(M, 2 * F, K, false, false, 3, 1, 128))) return r;
   if (!p.c_tma) return -111;
   if (!make_map(&p.tmCr[0], H, F, M, ldh, 64, 32, CU_TENSOR_MAP_SWIZZLE_128B, false)) return -110;
   p.swiglu_f = F;
@@ -1206,7 +1236,7 @@ TPLR_API int tplr_gemm2_swiglu_bwd(const void* dY, const void* W2, const void* G
   if (F % 64 || ((uintptr_t)GU & 15) || ((uintptr_t)dGU & 15) || (ldgu % 8) || (lddgu % 8)) return -111;
   Gemm2Params p = {};
   // operands and tile grid of the [M, F] product; the output map then covers the [M, 2F] packed gradient
-  if (int r = fill_common(p, dY, W2, dGU, M, F, K, lddy, ldw2, lddgu, 0, 1, 0, status)) return r;
+  if (int r = fill_common(p, dY, W2, dGU, M, F, K, lddy, ldw2, lddgu, 0, 1, 0, status, pick_tile(M, F, K, false, true, 5))) return r;
   if (!p.c_tma) return -111;
   if (!make_map(&p.tmC, dGU, 2LL * F, M, lddgu, 64, 32, CU_TENSOR_MAP_SWIZZLE_128B, false)) return -110;
   if (!make_map(&p.tmGU, GU, 2LL * F, M, ldgu, 64, 32, CU_TENSOR_MAP_SWIZZLE_128B, false)) return -110;
@@ -1224,7 +1254,7 @@ TPLR_API int tplr_gemm2_attn_dout(const void* dY, const void* Wo, const void* O,
   if (M <= 0 || N <= 0 || K <= 0) return 0;
   if ((head_dim != 128 && head_dim != 64) || N % head_dim || S <= 0 || M % S || ((uintptr_t)O & 15) || ((uintptr_t)dO & 15) || (ldo % 8) || (lddo % 8) || !delta) return -111;
   Gemm2Params p = {};
-  if (int r = fill_common(p, dY, Wo, dO, M, N, K, lddy, ldwo, lddo, 0, 1, 0, status)) return r;
+  if (int r = fill_common(p, dY, Wo, dO, M, N, K, lddy, ldwo, lddo, 0, 1, 0, status, pick_tile(M, N, K, false, true, 6, 1, head_dim))) return r;
   if (!p.c_tma) return -111;
   p.gu = (const __nv_bfloat16*)O; p.ld_gu = ldo;
   p.attn_delta = delta; p.attn_s = S; p.attn_heads = N / head_dim; p.attn_dh = head_dim;
@@ -1242,7 +1272,7 @@ TPLR_API int tplr_gemm2_rope(const void* X, const void* W, void* QKV, int M, int
   if (M <= 0 || N <= 0 || K <= 0) return 0;
   if (S <= 0 || head_dim % 32 || rope_cols % 32 || rope_cols > N || ((uintptr_t)cosb & 15) || ((uintptr_t)sinb & 15)) return -111;
   Gemm2Params p = {};
-  if (int r = fill_common(p, X, W, QKV, M, N, K, ldx, ldw, ldc, 0, 0, 0, status)) return r;
+  if (int r = fill_common(p, X, W, QKV, M, N, K, ldx, ldw, ldc, 0, 0, 0, status, head_dim == 64 || head_dim == 128 ? pick_tile(M, N, K, false, false, 4, 1, head_dim) : TILE_N)) return r;
   if (!p.c_tma) return -111;
   p.rope_cos = cosb; p.rope_sin = sinb; p.rope_s = S; p.rope_cols = rope_cols; p.rope_dh = head_dim;
   return dispatch2(p, 0, 0, 4, 0, 0, (cudaStream_t)stream);

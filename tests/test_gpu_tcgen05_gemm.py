@@ -281,3 +281,13 @@ def test_feed_forward_refuses_weights_of_other_widths(grad, backend):
         for a, b in ((bf(512, 248), w2), (bf(512, 264), w2), (w13, bf(256, 264)), (w13, bf(256, 248))):
             with pytest.raises(ValueError):
                 OF.feed_forward(x, a, b)
+
+
+@pytest.mark.parametrize("b_mn", [False, True])
+@pytest.mark.parametrize("M,N,K,epi", [(1111, 1536, 1536, "bf16"), (300, 760, 200, "bf16"), (300, 1160, 72, "bf16"),     # 128 wide, remainders
+                                       (2100, 3656, 776, "bf16"), (8192, 776, 768, "bf16"), (300, 5640, 64, "bf16"),     # 192 wide (K-major)
+                                       (520, 1032, 136, "f32"), (2304, 776, 2000, "acc"), (520, 136, 4104, "acc"),       # fp32 tiles, parts of K
+                                       (260, 1160, 8200, "bf16")])
+def test_narrow_tiles(M, N, K, epi, b_mn):
+    """Products whose 256-wide tiles would leave SMs idle: last tiles of 8 to 184 columns, with and without parts of K."""
+    _check(M, N, K, epi == "acc", b_mn, epi)
