@@ -602,7 +602,8 @@ attn_bwd_kernel(const __grid_constant__ AttnBwdParams p) {
   __syncthreads();
   tcgen05_fence_after();
   const uint32_t tmem_base = s_tmem_base;
-  const uint32_t tS = tmem_base, tdP = tmem_base + 128, tdV = tmem_base + 256, tdK = tmem_base + 256 + DH;
+  // dQ of a step lies over its dP at DH = 128; at 64 it has columns of its own
+  const uint32_t tS = tmem_base, tdP = tmem_base + 128, tdV = tmem_base + 256, tdK = tmem_base + 256 + DH, tdQ = DH == 64 ? tmem_base + 384 : tdP;
   const uint32_t sK = smem_u32(smem), sV = sK + TILE_BYTES, sQ = sV + TILE_BYTES, sdO = sQ + 2 * TILE_BYTES,
                  sP = sdO + TILE_BYTES, sdS = sP + PT_BYTES;
 
@@ -696,13 +697,14 @@ attn_bwd_kernel(const __grid_constant__ AttnBwdParams p) {
             umma_bf16_b(tdK, mdS, TPLR_MOFF(kk), mQ, ph * (TILE_BYTES / 16) + TPLR_MOFF(kk), id_mm, (t > 0 || kk > 0) ? 1u : 0u);
           umma_commit(smem_u32(&bar_q_empty[ph]));
 #pragma unroll
-          for (int kk = 0; kk < 8; ++kk)    // dQ[q, d] = dS[q, kv] K[kv, d], over dP; its commit covers every product before it
-            umma_bf16_b(tdP, kdS, TPLR_KOFF(kk), mK, TPLR_MOFF(kk), id_km, kk > 0 ? 1u : 0u);
+          for (int kk = 0; kk < 8; ++kk)    // dQ[q, d] = dS[q, kv] K[kv, d]; its commit covers every product before it
+            umma_bf16_b(tdQ, kdS, TPLR_KOFF(kk), mK, TPLR_MOFF(kk), id_km, kk > 0 ? 1u : 0u);
           umma_commit(smem_u32(&bar_dq_full));
         }
         if (t + 1 < n_it) {
           if (!(ok = mbar_wait(smem_u32(&bar_do_full), ph ^ 1u, abort_flag))) break;
-          if (!(ok = mbar_wait(smem_u32(&bar_dq_free), ph, abort_flag))) break;    // dQ read by every warp
+          // dP(t + 1) over dQ(t): read by every warp.  At 64, dS(t) has read dP(t), and dQ(t - 1) was read before P(t) was stored
+          if (DH == 128 && !(ok = mbar_wait(smem_u32(&bar_dq_free), ph, abort_flag))) break;
           tcgen05_fence_after();
           issue_dp();
         }
@@ -716,7 +718,7 @@ attn_bwd_kernel(const __grid_constant__ AttnBwdParams p) {
     const uint32_t sw = (uint32_t)(lane & 7);
     // two private 4 KB staging buffers: the bytes of this warp's own rows and column half in the P and dS tiles.  Free from
     // the step's last commit on (it covers the products that read them); the reduce-adds have read them before the warp
-    // writes its next P.
+    // writes its next P and dS.
     const uint32_t stg0 = sP + (uint32_t)ch * (PT_BYTES / 2) + (uint32_t)quad * 4096u;
     const uint32_t stg1 = sdS + (uint32_t)ch * (PT_BYTES / 2) + (uint32_t)quad * 4096u;
     const uint32_t prow = sP + (uint32_t)ch * (PT_BYTES / 2) + (uint32_t)r * 128u;
@@ -729,11 +731,40 @@ attn_bwd_kernel(const __grid_constant__ AttnBwdParams p) {
       lse2 = live ? p.lse[at] : INFINITY;
       dl = live ? p.delta[at] : 0.f;
     };
+    // dQ of step tt (fp32 in tensor memory) into the global fp32 dQ with TMA reduce-add: one group of copies for each box
+    auto drain = [&](int tt) -> bool {
+      const bool o = mbar_wait(smem_u32(&bar_dq_full), tt & 1, abort_flag);
+      if (!__all_sync(0xffffffffu, o)) return false;
+      tcgen05_fence_after();
+      uint32_t dq[DH / 64][32];
+#pragma unroll
+      for (int cc = 0; cc < DH / 64; ++cc) tmem_ld32(tdQ + (DH / 64 * ch + cc) * 32 + lane_off, dq[cc]);
+      tcgen05_fence_before();
+      __syncwarp();
+      if (DH == 128 && lane == 0) mbar_arrive(smem_u32(&bar_dq_free));
+      const int h = h0 + tt / n_i, qrow0 = (j + tt % n_i) * BQ + quad * 32;
+#pragma unroll
+      for (int cc = 0; cc < DH / 64; ++cc) {
+        const uint32_t stg = DH == 128 && cc == 0 ? stg0 : stg1;
+        const uint32_t rowaddr = stg + (uint32_t)lane * 128u;
+#pragma unroll
+        for (int q8 = 0; q8 < 8; ++q8)
+          asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(rowaddr + (((uint32_t)q8 ^ sw) << 4)), "r"(dq[cc][4 * q8]),
+                       "r"(dq[cc][4 * q8 + 1]), "r"(dq[cc][4 * q8 + 2]), "r"(dq[cc][4 * q8 + 3]) : "memory");
+        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+        __syncwarp();
+        if (lane == 0) {
+          if (qrow0 < p.S) tma_reduce_add_3d(&p.tmDQ, stg, h * DH + (DH / 64 * ch + cc) * 32, qrow0, b);
+          asm volatile("cp.async.bulk.commit_group;" ::: "memory");
+        }
+      }
+      return true;
+    };
     float lse_n, dl_n;
     stats(0, lse_n, dl_n);
     bool ok = true;
     for (int t = 0; t < n_it && ok; ++t) {
-      const int h = h0 + t / n_i, i = j + t % n_i;
+      const int i = j + t % n_i;
       const float lse2 = lse_n * 1.4426950408889634f, dls = dl_n * p.scale;
       if (t + 1 < n_it) stats(t + 1, lse_n, dl_n);           // in flight during this step
       ok = mbar_wait(smem_u32(&bar_s_full), t & 1, abort_flag);
@@ -742,7 +773,7 @@ attn_bwd_kernel(const __grid_constant__ AttnBwdParams p) {
       tcgen05_fence_after();
       // P of this warp's 64 columns, kept in fp32 for dS; the diagonal block runs the variant with the causal mask
       float pv[64];
-      auto p_part = [&](auto DIAG) {
+      auto exp_part = [&](auto DIAG) {
         constexpr bool kDiag = decltype(DIAG)::value;
 #pragma unroll
         for (int cc = 0; cc < 2; ++cc) {
@@ -754,24 +785,29 @@ attn_bwd_kernel(const __grid_constant__ AttnBwdParams p) {
             if (kDiag && ch * 64 + cc * 32 + e > r) x = 0.f;
             pv[cc * 32 + e] = x;
           }
-          if (cc == 0 && t > 0) {                            // the staged dQ of the previous step has left these bytes
-            if (lane == 0) asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
-            __syncwarp();
-          }
-#pragma unroll
-          for (int q4 = 0; q4 < 4; ++q4) {
-            uint32_t pw[4];
-#pragma unroll
-            for (int e = 0; e < 4; ++e) {
-              __nv_bfloat162 hp = __floats2bfloat162_rn(pv[cc * 32 + q4 * 8 + 2 * e], pv[cc * 32 + q4 * 8 + 2 * e + 1]);
-              pw[e] = *reinterpret_cast<uint32_t*>(&hp);
-            }
-            asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(prow + ((((uint32_t)(cc * 4 + q4)) ^ sw) << 4)),
-                         "r"(pw[0]), "r"(pw[1]), "r"(pw[2]), "r"(pw[3]) : "memory");
-          }
         }
       };
-      if (i == j) p_part(cuda::std::true_type{}); else p_part(cuda::std::false_type{});
+      if (i == j) exp_part(cuda::std::true_type{}); else exp_part(cuda::std::false_type{});
+      // dQ of the step before: its products ran while this step's exponentials were taken.  Its last commit covers every
+      // product that reads the P and dS tiles, so from here on they may be written.
+      if (t > 0) {
+        if (!(ok = drain(t - 1))) break;
+        if (DH == 128) {                                     // the box staged in this warp's bytes of the P tile has left them
+          if (lane == 0) asm volatile("cp.async.bulk.wait_group.read 1;" ::: "memory");
+          __syncwarp();
+        }
+      }
+#pragma unroll
+      for (int q8 = 0; q8 < 8; ++q8) {
+        uint32_t pw[4];
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          __nv_bfloat162 hp = __floats2bfloat162_rn(pv[q8 * 8 + 2 * e], pv[q8 * 8 + 2 * e + 1]);
+          pw[e] = *reinterpret_cast<uint32_t*>(&hp);
+        }
+        asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(prow + (((uint32_t)q8 ^ sw) << 4)), "r"(pw[0]), "r"(pw[1]),
+                     "r"(pw[2]), "r"(pw[3]) : "memory");
+      }
       asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
       tcgen05_fence_before();
       __syncwarp();
@@ -785,6 +821,10 @@ attn_bwd_kernel(const __grid_constant__ AttnBwdParams p) {
       for (int cc = 0; cc < 2; ++cc) {
         uint32_t dv[32];
         tmem_ld32(tdP + ch * 64 + cc * 32 + lane_off, dv);
+        if (cc == 0 && t > 0) {                              // the box staged in this warp's bytes of the dS tile has left them
+          if (lane == 0) asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
+          __syncwarp();
+        }
 #pragma unroll
         for (int q4 = 0; q4 < 4; ++q4) {
           uint32_t dw[4];
@@ -804,35 +844,8 @@ attn_bwd_kernel(const __grid_constant__ AttnBwdParams p) {
       tcgen05_fence_before();
       __syncwarp();
       if (lane == 0) mbar_arrive(smem_u32(&bar_ds_ready));
-      // drain dQ_partial (fp32, in the dP columns) into the global fp32 dQ with TMA reduce-add
-      ok = mbar_wait(smem_u32(&bar_dq_full), t & 1, abort_flag);
-      ok = __all_sync(0xffffffffu, ok);
-      if (!ok) break;
-      tcgen05_fence_after();
-      uint32_t dq[DH / 64][32];
-#pragma unroll
-      for (int cc = 0; cc < DH / 64; ++cc) tmem_ld32(tdP + (DH / 64 * ch + cc) * 32 + lane_off, dq[cc]);
-      tcgen05_fence_before();
-      __syncwarp();
-      if (lane == 0) mbar_arrive(smem_u32(&bar_dq_free));
-      const int qrow0 = i * BQ + quad * 32;
-#pragma unroll
-      for (int cc = 0; cc < DH / 64; ++cc) {
-        const uint32_t rowaddr = (cc ? stg1 : stg0) + (uint32_t)lane * 128u;
-#pragma unroll
-        for (int q8 = 0; q8 < 8; ++q8)
-          asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(rowaddr + (((uint32_t)q8 ^ sw) << 4)), "r"(dq[cc][4 * q8]),
-                       "r"(dq[cc][4 * q8 + 1]), "r"(dq[cc][4 * q8 + 2]), "r"(dq[cc][4 * q8 + 3]) : "memory");
-      }
-      asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-      __syncwarp();
-      if (lane == 0 && qrow0 < p.S) {
-#pragma unroll
-        for (int cc = 0; cc < DH / 64; ++cc)
-          tma_reduce_add_3d(&p.tmDQ, cc ? stg1 : stg0, h * DH + (DH / 64 * ch + cc) * 32, qrow0, b);
-        asm volatile("cp.async.bulk.commit_group;" ::: "memory");
-      }
     }
+    if (ok && n_it > 0) ok = drain(n_it - 1);
     // dV and dK of this kv block.  Whole group in this CTA: TMEM -> bf16 -> staging -> TMA store into the packed gradient;
     // a part of it: stored in fp32 in columns of its own; the pass that rotates dQ back and rounds it adds the parts in order.
     if (ok) {
