@@ -312,13 +312,13 @@ attn_fwd_kernel(const __grid_constant__ AttnFwdParams p) {
       for (int j = 0; j < nb && ok; ++j) {
         const uint32_t ph = j & 1;
         const int krow = j * BKV;
-        if (!(ok = mbar_wait(smem_u32(&bar_k_empty), ph ^ 1, abort_flag))) break;
+        if (!(ok = mbar_wait_warp(smem_u32(&bar_k_empty), ph ^ 1, abort_flag))) break;
         if (leader) {
           mbar_expect_tx(smem_u32(&bar_k_full), TILE_BYTES);
           load_tile<DH>(sK, &p.tmQKV, smem_u32(&bar_k_full), kcol, krow, b);
         }
         ++n_k;
-        if (!(ok = mbar_wait(smem_u32(&bar_v_empty), ph ^ 1, abort_flag))) break;
+        if (!(ok = mbar_wait_warp(smem_u32(&bar_v_empty), ph ^ 1, abort_flag))) break;
         if (leader) {
           mbar_expect_tx(smem_u32(&bar_v_full), TILE_BYTES);
           load_tile<DH>(sV, &p.tmQKV, smem_u32(&bar_v_full), vcol, krow, b);
@@ -338,7 +338,7 @@ attn_fwd_kernel(const __grid_constant__ AttnFwdParams p) {
       const uint32_t id_qk = idesc_mn(128, false, false), id_pv = idesc_mn(DH, false, true);
       const DescBase bQ = desc_base(sQ, 16, 1024), bK = desc_base(sK, 16, 1024), bV = desc_base(sV, 128 * 128, 1024);
       auto issue_s = [&](int j) -> bool {                  // S(j) = Q K(j)^T
-        if (!mbar_wait(smem_u32(&bar_k_full), (uint32_t)(j & 1), abort_flag)) return false;
+        if (!mbar_wait_warp(smem_u32(&bar_k_full), (uint32_t)(j & 1), abort_flag)) return false;
         tcgen05_fence_after();
         if (leader) {
 #pragma unroll
@@ -351,18 +351,18 @@ attn_fwd_kernel(const __grid_constant__ AttnFwdParams p) {
         }
         return true;
       };
-      bool ok = mbar_wait(smem_u32(&bar_q), 0, abort_flag);
+      bool ok = mbar_wait_warp(smem_u32(&bar_q), 0, abort_flag);
       if (AHEAD && ok) ok = issue_s(0);
       for (int j = 0; j < nb && ok; ++j) {
         const uint32_t ph = j & 1;
         if (!AHEAD) {
           if (!(ok = issue_s(j))) break;
         } else if (j + 1 < nb) {
-          if (!(ok = mbar_wait(smem_u32(&bar_s_read), ph, abort_flag))) break;
+          if (!(ok = mbar_wait_warp(smem_u32(&bar_s_read), ph, abort_flag))) break;
           if (!(ok = issue_s(j + 1))) break;
         }
-        if (!(ok = mbar_wait(smem_u32(&bar_p_full), ph, abort_flag))) break;
-        if (!(ok = mbar_wait(smem_u32(&bar_v_full), ph, abort_flag))) break;
+        if (!(ok = mbar_wait_warp(smem_u32(&bar_p_full), ph, abort_flag))) break;
+        if (!(ok = mbar_wait_warp(smem_u32(&bar_v_full), ph, abort_flag))) break;
         tcgen05_fence_after();
         if (leader) {
 #pragma unroll
@@ -620,14 +620,14 @@ attn_bwd_kernel(const __grid_constant__ AttnBwdParams p) {
       for (int t = 0; t < n_it && ok; ++t) {
         const int h = h0 + t / n_i, i = j + t % n_i;
         const int qrow0 = i * BQ, qcol = h * DH, s = t & 1;
-        if (!(ok = mbar_wait(smem_u32(&bar_q_empty[s]), (uint32_t)(((t >> 1) & 1) ^ 1), abort_flag))) break;
+        if (!(ok = mbar_wait_warp(smem_u32(&bar_q_empty[s]), (uint32_t)(((t >> 1) & 1) ^ 1), abort_flag))) break;
         const uint32_t fq = smem_u32(&bar_q_full[s]);
         if (leader) {
           mbar_expect_tx(fq, TILE_BYTES);
           load_tile<DH>(sQ + s * TILE_BYTES, &p.tmQKV, fq, qcol, qrow0, b);
         }
         ++n_q;
-        if (!(ok = mbar_wait(smem_u32(&bar_do_empty), (uint32_t)((t & 1) ^ 1), abort_flag))) break;
+        if (!(ok = mbar_wait_warp(smem_u32(&bar_do_empty), (uint32_t)((t & 1) ^ 1), abort_flag))) break;
         const uint32_t fd = smem_u32(&bar_do_full);
         if (leader) {
           mbar_expect_tx(fd, TILE_BYTES);
@@ -669,17 +669,17 @@ attn_bwd_kernel(const __grid_constant__ AttnBwdParams p) {
         for (int kk = 0; kk < DH / 16; ++kk) umma_bf16_b(tdP, kdO, TPLR_KOFF(kk), kV, TPLR_KOFF(kk), id_kk, kk > 0 ? 1u : 0u);
         umma_commit(smem_u32(&bar_dp_full));
       };
-      bool ok = mbar_wait(smem_u32(&bar_kv), 0, abort_flag);
-      if (ok) ok = mbar_wait(smem_u32(&bar_q_full[0]), 0, abort_flag);
+      bool ok = mbar_wait_warp(smem_u32(&bar_kv), 0, abort_flag);
+      if (ok) ok = mbar_wait_warp(smem_u32(&bar_q_full[0]), 0, abort_flag);
       if (ok) { tcgen05_fence_after(); issue_s(0); }
-      if (ok) ok = mbar_wait(smem_u32(&bar_do_full), 0, abort_flag);
+      if (ok) ok = mbar_wait_warp(smem_u32(&bar_do_full), 0, abort_flag);
       if (ok) { tcgen05_fence_after(); issue_dp(); }
       for (int t = 0; t < n_it && ok; ++t) {
         const uint32_t ph = t & 1;
-        if (!(ok = mbar_wait(smem_u32(&bar_p_ready), ph, abort_flag))) break;      // P stored, S read by every warp
+        if (!(ok = mbar_wait_warp(smem_u32(&bar_p_ready), ph, abort_flag))) break;      // P stored, S read by every warp
         tcgen05_fence_after();
         if (t + 1 < n_it) {
-          if (!(ok = mbar_wait(smem_u32(&bar_q_full[(t + 1) & 1]), (uint32_t)(((t + 1) >> 1) & 1), abort_flag))) break;
+          if (!(ok = mbar_wait_warp(smem_u32(&bar_q_full[(t + 1) & 1]), (uint32_t)(((t + 1) >> 1) & 1), abort_flag))) break;
           tcgen05_fence_after();
           issue_s(t + 1);
         }
@@ -689,7 +689,7 @@ attn_bwd_kernel(const __grid_constant__ AttnBwdParams p) {
             umma_bf16_b(tdV, mP, TPLR_MOFF(kk), mdO, TPLR_MOFF(kk), id_mm, (t > 0 || kk > 0) ? 1u : 0u);
           umma_commit(smem_u32(&bar_do_empty));
         }
-        if (!(ok = mbar_wait(smem_u32(&bar_ds_ready), ph, abort_flag))) break;     // dS stored, dP read by every warp
+        if (!(ok = mbar_wait_warp(smem_u32(&bar_ds_ready), ph, abort_flag))) break;     // dS stored, dP read by every warp
         tcgen05_fence_after();
         if (leader) {
 #pragma unroll
@@ -702,9 +702,9 @@ attn_bwd_kernel(const __grid_constant__ AttnBwdParams p) {
           umma_commit(smem_u32(&bar_dq_full));
         }
         if (t + 1 < n_it) {
-          if (!(ok = mbar_wait(smem_u32(&bar_do_full), ph ^ 1u, abort_flag))) break;
+          if (!(ok = mbar_wait_warp(smem_u32(&bar_do_full), ph ^ 1u, abort_flag))) break;
           // dP(t + 1) over dQ(t): read by every warp.  At 64, dS(t) has read dP(t), and dQ(t - 1) was read before P(t) was stored
-          if (DH == 128 && !(ok = mbar_wait(smem_u32(&bar_dq_free), ph, abort_flag))) break;
+          if (DH == 128 && !(ok = mbar_wait_warp(smem_u32(&bar_dq_free), ph, abort_flag))) break;
           tcgen05_fence_after();
           issue_dp();
         }
@@ -1109,7 +1109,7 @@ attn_bwd2_kernel(const __grid_constant__ AttnBwd2Params p) {
         const int s = t & 1, k = t >> 1;
         const int h = g * group + t / n_i, iq = iq0 + t % n_i;
         const int qrow0 = b * p.S + iq * B2_BQ, qcol = h * DH;
-        if (!(ok = mbar_wait(smem_u32(&bar_q_empty[s]), (uint32_t)((k & 1) ^ 1), abort_flag))) break;
+        if (!(ok = mbar_wait_warp(smem_u32(&bar_q_empty[s]), (uint32_t)((k & 1) ^ 1), abort_flag))) break;
         const uint32_t fb = smem_u32(&bar_q_full[s]);
         if (leader) {
           mbar_expect_tx(fb, 2 * B2_QTILE + 512);
@@ -1161,33 +1161,33 @@ attn_bwd2_kernel(const __grid_constant__ AttnBwd2Params p) {
         for (int kk = 0; kk < 8; ++kk) umma_bf16_b(tdP, kV, TPLR_K128(kk), kdO[t & 1], TPLR_K64(kk), id_st, kk > 0 ? 1u : 0u);
         umma_commit(smem_u32(&bar_dp_full));
       };
-      bool ok = mbar_wait(smem_u32(&bar_kv), 0, abort_flag);
-      if (ok) ok = mbar_wait(smem_u32(&bar_q_full[0]), 0, abort_flag);
+      bool ok = mbar_wait_warp(smem_u32(&bar_kv), 0, abort_flag);
+      if (ok) ok = mbar_wait_warp(smem_u32(&bar_q_full[0]), 0, abort_flag);
       if (ok) {
         tcgen05_fence_after();
         issue_st(0);
         issue_dp(0);
       }
       if (ok && n_it > 1) {
-        ok = mbar_wait(smem_u32(&bar_q_full[1]), 0, abort_flag);
+        ok = mbar_wait_warp(smem_u32(&bar_q_full[1]), 0, abort_flag);
         if (ok) { tcgen05_fence_after(); issue_st(1); }
       }
       for (int t = 0; t < n_it && ok; ++t) {
         const int s = t & 1;
         const uint32_t ph = t & 1;
-        if (!(ok = mbar_wait(smem_u32(&bar_p_ready), ph, abort_flag))) break;
+        if (!(ok = mbar_wait_warp(smem_u32(&bar_p_ready), ph, abort_flag))) break;
         tcgen05_fence_after();
         if (leader)
 #pragma unroll
         for (int kk = 0; kk < 4; ++kk)          // dV += P^T dO ; P^T packed at columns 0-15 and 32-47 of the S buffer
           umma_ts_bf16_b(tdV, tS0 + s * 64 + (kk >> 1) * 32 + (kk & 1) * 8, mdO[s], TPLR_M(kk), id_dv, (t > 0 || kk > 0) ? 1u : 0u);
-        if (!(ok = mbar_wait(smem_u32(&bar_ds_ready), ph, abort_flag))) break;
+        if (!(ok = mbar_wait_warp(smem_u32(&bar_ds_ready), ph, abort_flag))) break;
         tcgen05_fence_after();
         if (leader)
 #pragma unroll
         for (int kk = 0; kk < 4; ++kk)          // dK += dS^T Q
           umma_ts_bf16_b(tdK, tdP + (kk >> 1) * 32 + (kk & 1) * 8, mQ[s], TPLR_M(kk), id_dv, (t > 0 || kk > 0) ? 1u : 0u);
-        if (t > 0 && !(ok = mbar_wait(smem_u32(&bar_dq_free), (uint32_t)((t - 1) & 1), abort_flag))) break;
+        if (t > 0 && !(ok = mbar_wait_warp(smem_u32(&bar_dq_free), (uint32_t)((t - 1) & 1), abort_flag))) break;
         tcgen05_fence_after();
         if (leader)
 #pragma unroll
@@ -1199,7 +1199,7 @@ attn_bwd2_kernel(const __grid_constant__ AttnBwd2Params p) {
         }
         if (t + 1 < n_it) issue_dp(t + 1);
         if (t + 2 < n_it) {
-          if (!(ok = mbar_wait(smem_u32(&bar_q_full[s]), (uint32_t)(((t + 2) >> 1) & 1), abort_flag))) break;
+          if (!(ok = mbar_wait_warp(smem_u32(&bar_q_full[s]), (uint32_t)(((t + 2) >> 1) & 1), abort_flag))) break;
           tcgen05_fence_after();
           issue_st(t + 2);
         }

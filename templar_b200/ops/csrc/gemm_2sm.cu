@@ -735,9 +735,7 @@ gemm2_kernel(const __grid_constant__ Gemm2Params p) {
               if (kbr >= k_blocks) kbr -= k_blocks;
               if (!(ok = rows_ready_warp(kbr * BK, BK))) break;
             }
-            ok = mbar_wait(empty0 + 8u * s, ph ^ 1u, abort_flag);
-            if (p.ag_operand) ok = __all_sync(0xffffffffu, ok);        // the votes above need every lane
-            if (!ok) break;
+            if (!(ok = mbar_wait_warp(empty0 + 8u * s, ph ^ 1u, abort_flag))) break;
             if (leader) {
               if (cr == 0) mbar_expect_tx(full0 + 8u * s, 2 * (A_STAGE + b_stage));
               const uint32_t fb = fullp0 + 8u * s;
@@ -787,11 +785,11 @@ gemm2_kernel(const __grid_constant__ Gemm2Params p) {
         for (; ok && work_get(p, w, num_tiles, k_blocks_all, k_per); work_next(p, w), ++tile_i) {
           const int k_blocks = w.nkb;
           const uint32_t acc = tile_i & 1, acc_ph = (tile_i >> 1) & 1;
-          if (!(ok = mbar_wait(smem_u32(&bar_tempty[acc]), acc_ph ^ 1, abort_flag))) break;
+          if (!(ok = mbar_wait_warp(smem_u32(&bar_tempty[acc]), acc_ph ^ 1, abort_flag))) break;
           tcgen05_fence_after();
           const uint32_t d_tmem = tmem_base + acc * TILE_N;
           for (int kb = 0; kb < k_blocks; ++kb) {
-            if (!(ok = mbar_wait(full0 + 8u * s, ph, abort_flag))) break;
+            if (!(ok = mbar_wait_warp(full0 + 8u * s, ph, abort_flag))) break;
             tcgen05_fence_after();
             const uint32_t a_lo = dA0.lo + s * (A_STAGE >> 4), b_lo = dB0.lo + s * (b_stage >> 4);
             if (leader) {

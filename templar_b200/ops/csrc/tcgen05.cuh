@@ -50,6 +50,12 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatil
   return false;
 }
 
+// The same by a whole warp, which leaves together and with one answer.  A role whose loop is run by all its lanes (see elect_one)
+// waits this way: a lane that fell behind its warp by more than a phase would look for a parity that has passed.
+__device__ __forceinline__ bool mbar_wait_warp(uint32_t bar, uint32_t parity, volatile int* abort_flag) {
+  return __all_sync(0xffffffffu, mbar_wait(bar, parity, abort_flag));
+}
+
 // Waits for copies in flight before a role returns.  A role also gets there when another one has given up, and mbar_wait
 // returns at once then, because the CTA's flag is up: a drain has a flag of its own, so that only its own time limit (one for
 // all its waits) ends it.
