@@ -528,8 +528,12 @@ TPLR_API int tplr_attention_fwd(const void* qkv, void* out, float* lse, int B, i
 // ------------------------------------------------------------------------------------------ //
 namespace {
 
-template <int DH> constexpr int bwd_smem() { return 5 * tile_bytes<DH>() + 2 * PT_BYTES + 1024; }   // K, V, two Q, dO; P, dS
-constexpr int BWD_THREADS = 320;                        // TMA warp, MMA warp, 8 softmax warps (2 per TMEM lane quadrant)
+// K, V, two Q, dO; P, dS; at 64 the staging of dQ
+template <int DH> constexpr int bwd_smem() { return 5 * tile_bytes<DH>() + 2 * PT_BYTES + (DH == 64 ? 4 * 8192 : 0) + 1024; }
+// TMA warp, MMA warp, 8 softmax warps (2 per TMEM lane quadrant); at 64 four more that drain dQ.  At 128 the softmax warps drain
+// it: there is no shared memory left for a staging of its own, and warps that stage it in the dS tile hold back the next dS
+// (8 x 2048 x 16 heads 655 us, 690 with them; at 64, 8 x 2048 x 12 279 -> 263, 2 x 8192 x 12 814 -> 743).
+template <int DH> constexpr int bwd_threads() { return DH == 64 ? 448 : 320; }
 
 struct AttnBwdParams {
   CUtensorMap tmQKV;    // [B, S, C] bf16, box 64 x 128 x 1
@@ -559,7 +563,7 @@ __device__ __forceinline__ void tma_reduce_add_3d(const CUtensorMap* map, uint32
 }
 
 template <int DH>
-__global__ void __launch_bounds__(BWD_THREADS, 1)
+__global__ void __launch_bounds__(bwd_threads<DH>(), 1)
 attn_bwd_kernel(const __grid_constant__ AttnBwdParams p) {
   constexpr int TILE_BYTES = tile_bytes<DH>();
   extern __shared__ uint8_t smem_raw[];
@@ -590,7 +594,7 @@ attn_bwd_kernel(const __grid_constant__ AttnBwdParams p) {
     mbar_init(smem_u32(&bar_do_full), 1); mbar_init(smem_u32(&bar_do_empty), 1);
     mbar_init(smem_u32(&bar_s_full), 1); mbar_init(smem_u32(&bar_dp_full), 1);
     mbar_init(smem_u32(&bar_p_ready), 8); mbar_init(smem_u32(&bar_ds_ready), 8);
-    mbar_init(smem_u32(&bar_dq_full), 1); mbar_init(smem_u32(&bar_dq_free), 8);
+    mbar_init(smem_u32(&bar_dq_full), 1); mbar_init(smem_u32(&bar_dq_free), DH == 64 ? 4 : 8);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
   }
@@ -690,6 +694,7 @@ attn_bwd_kernel(const __grid_constant__ AttnBwdParams p) {
           umma_commit(smem_u32(&bar_do_empty));
         }
         if (!(ok = mbar_wait_warp(smem_u32(&bar_ds_ready), ph, abort_flag))) break;     // dS stored, dP read by every warp
+        if (DH == 64 && t > 0 && !(ok = mbar_wait_warp(smem_u32(&bar_dq_free), ph ^ 1u, abort_flag))) break;      // dQ(t - 1) read
         tcgen05_fence_after();
         if (leader) {
 #pragma unroll
@@ -703,13 +708,53 @@ attn_bwd_kernel(const __grid_constant__ AttnBwdParams p) {
         }
         if (t + 1 < n_it) {
           if (!(ok = mbar_wait_warp(smem_u32(&bar_do_full), ph ^ 1u, abort_flag))) break;
-          // dP(t + 1) over dQ(t): read by every warp.  At 64, dS(t) has read dP(t), and dQ(t - 1) was read before P(t) was stored
+          // dP(t + 1) lies over dQ(t) at 128; at 64 over dP(t), which dS(t) has read
           if (DH == 128 && !(ok = mbar_wait_warp(smem_u32(&bar_dq_free), ph, abort_flag))) break;
           tcgen05_fence_after();
           issue_dp();
         }
       }
     }
+  } else if (DH == 64 && warp >= 10) {
+    // dQ of every step (fp32 in tensor memory) into the global fp32 dQ: two 32-column boxes through shared memory, TMA reduce-add.
+    // Warps of their own, so that the softmax warps go on meanwhile.
+    const int quad = warp & 3;
+    const uint32_t lane_off = (uint32_t)(quad * 32) << 16, sw = (uint32_t)(lane & 7);
+    const uint32_t stg = sdS + PT_BYTES + (uint32_t)quad * 8192u;
+    const bool leader = elect_one();
+    bool ok = true;
+    for (int t = 0; t < n_it && ok; ++t) {
+      if (!(ok = mbar_wait_warp(smem_u32(&bar_dq_full), t & 1, abort_flag))) break;
+      tcgen05_fence_after();
+      uint32_t dq[2][32];
+#pragma unroll
+      for (int cc = 0; cc < 2; ++cc) tmem_ld32(tdQ + cc * 32 + lane_off, dq[cc]);
+      tcgen05_fence_before();
+      __syncwarp();
+      if (leader) {
+        mbar_arrive(smem_u32(&bar_dq_free));
+        asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");                  // the boxes of the step before have left
+      }
+      __syncwarp();
+#pragma unroll
+      for (int cc = 0; cc < 2; ++cc) {
+        const uint32_t rowaddr = stg + (uint32_t)cc * 4096u + (uint32_t)lane * 128u;
+#pragma unroll
+        for (int q8 = 0; q8 < 8; ++q8)
+          asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(rowaddr + (((uint32_t)q8 ^ sw) << 4)), "r"(dq[cc][4 * q8]),
+                       "r"(dq[cc][4 * q8 + 1]), "r"(dq[cc][4 * q8 + 2]), "r"(dq[cc][4 * q8 + 3]) : "memory");
+      }
+      asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+      __syncwarp();
+      const int h = h0 + t / n_i, qrow0 = (j + t % n_i) * BQ + quad * 32;
+      if (leader && qrow0 < p.S) {
+#pragma unroll
+        for (int cc = 0; cc < 2; ++cc) tma_reduce_add_3d(&p.tmDQ, stg + cc * 4096, h * DH + cc * 32, qrow0, b);
+        asm volatile("cp.async.bulk.commit_group;" ::: "memory");
+      }
+      __syncwarp();
+    }
+    if (leader) asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
   } else {
     const int quad = warp & 3;                 // TMEM lane quadrant this warp may access
     const int ch = (warp - 2) >> 2;            // column half (64 columns) this warp works on
@@ -731,7 +776,7 @@ attn_bwd_kernel(const __grid_constant__ AttnBwdParams p) {
       lse2 = live ? p.lse[at] : INFINITY;
       dl = live ? p.delta[at] : 0.f;
     };
-    // dQ of step tt (fp32 in tensor memory) into the global fp32 dQ with TMA reduce-add: one group of copies for each box
+    // DH = 128: dQ of step tt (fp32 in tensor memory) into the global fp32 dQ with TMA reduce-add: one group of copies for each box
     auto drain = [&](int tt) -> bool {
       const bool o = mbar_wait(smem_u32(&bar_dq_full), tt & 1, abort_flag);
       if (!__all_sync(0xffffffffu, o)) return false;
@@ -741,11 +786,11 @@ attn_bwd_kernel(const __grid_constant__ AttnBwdParams p) {
       for (int cc = 0; cc < DH / 64; ++cc) tmem_ld32(tdQ + (DH / 64 * ch + cc) * 32 + lane_off, dq[cc]);
       tcgen05_fence_before();
       __syncwarp();
-      if (DH == 128 && lane == 0) mbar_arrive(smem_u32(&bar_dq_free));
+      if (lane == 0) mbar_arrive(smem_u32(&bar_dq_free));
       const int h = h0 + tt / n_i, qrow0 = (j + tt % n_i) * BQ + quad * 32;
 #pragma unroll
       for (int cc = 0; cc < DH / 64; ++cc) {
-        const uint32_t stg = DH == 128 && cc == 0 ? stg0 : stg1;
+        const uint32_t stg = cc == 0 ? stg0 : stg1;
         const uint32_t rowaddr = stg + (uint32_t)lane * 128u;
 #pragma unroll
         for (int q8 = 0; q8 < 8; ++q8)
@@ -788,13 +833,15 @@ attn_bwd_kernel(const __grid_constant__ AttnBwdParams p) {
         }
       };
       if (i == j) exp_part(cuda::std::true_type{}); else exp_part(cuda::std::false_type{});
-      // dQ of the step before: its products ran while this step's exponentials were taken.  Its last commit covers every
-      // product that reads the P and dS tiles, so from here on they may be written.
       if (t > 0) {
-        if (!(ok = drain(t - 1))) break;
-        if (DH == 128) {                                     // the box staged in this warp's bytes of the P tile has left them
-          if (lane == 0) asm volatile("cp.async.bulk.wait_group.read 1;" ::: "memory");
+        if constexpr (DH == 128) {
+          // dQ of the step before: its products ran while this step's exponentials were taken.  Its last commit covers every
+          // product that reads the P and dS tiles, so from here on they may be written.
+          if (!(ok = drain(t - 1))) break;
+          if (lane == 0) asm volatile("cp.async.bulk.wait_group.read 1;" ::: "memory");    // the box in this warp's bytes of the P tile has left
           __syncwarp();
+        } else if (!(ok = mbar_wait_warp(smem_u32(&bar_do_empty), (t - 1) & 1, abort_flag))) {      // dV has read the P tile
+          break;
         }
       }
 #pragma unroll
@@ -812,16 +859,15 @@ attn_bwd_kernel(const __grid_constant__ AttnBwdParams p) {
       tcgen05_fence_before();
       __syncwarp();
       if (lane == 0) mbar_arrive(smem_u32(&bar_p_ready));
-      ok = mbar_wait(smem_u32(&bar_dp_full), t & 1, abort_flag);
-      ok = __all_sync(0xffffffffu, ok);
-      if (!ok) break;
+      if (DH == 64 && t > 0 && !(ok = mbar_wait_warp(smem_u32(&bar_dq_full), (t - 1) & 1, abort_flag))) break;    // dS tile: dK, dQ done
+      if (!(ok = mbar_wait_warp(smem_u32(&bar_dp_full), t & 1, abort_flag))) break;
       tcgen05_fence_after();
       // dS carries the softmax scale: d = p * (dp - delta) * scale = p * fma(dp, scale, -delta * scale)
 #pragma unroll
       for (int cc = 0; cc < 2; ++cc) {
         uint32_t dv[32];
         tmem_ld32(tdP + ch * 64 + cc * 32 + lane_off, dv);
-        if (cc == 0 && t > 0) {                              // the box staged in this warp's bytes of the dS tile has left them
+        if (DH == 128 && cc == 0 && t > 0) {                 // the box staged in this warp's bytes of the dS tile has left them
           if (lane == 0) asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
           __syncwarp();
         }
@@ -845,7 +891,10 @@ attn_bwd_kernel(const __grid_constant__ AttnBwdParams p) {
       __syncwarp();
       if (lane == 0) mbar_arrive(smem_u32(&bar_ds_ready));
     }
-    if (ok && n_it > 0) ok = drain(n_it - 1);
+    if (ok && n_it > 0) {                                    // every product done
+      if constexpr (DH == 128) ok = drain(n_it - 1);
+      else ok = mbar_wait_warp(smem_u32(&bar_dq_full), (n_it - 1) & 1, abort_flag);
+    }
     // dV and dK of this kv block.  Whole group in this CTA: TMEM -> bf16 -> staging -> TMA store into the packed gradient;
     // a part of it: stored in fp32 in columns of its own; the pass that rotates dQ back and rounds it adds the parts in order.
     if (ok) {
@@ -1426,7 +1475,7 @@ int launch_bwd(const void* qkv, const void* out, const void* dout, const float* 
   p.rope_cos = cosb; p.rope_sin = sinb;
   cudaError_t e = cudaFuncSetAttribute(attn_bwd_kernel<HD>, cudaFuncAttributeMaxDynamicSharedMemorySize, bwd_smem<HD>());
   if (e != cudaSuccess) return (int)e;
-  attn_bwd_kernel<HD><<<(unsigned)(((S + BKV - 1) / BKV) * KV * B * p.split), BWD_THREADS, bwd_smem<HD>(), st>>>(p);
+  attn_bwd_kernel<HD><<<(unsigned)(((S + BKV - 1) / BKV) * KV * B * p.split), bwd_threads<HD>(), bwd_smem<HD>(), st>>>(p);
   auto cast = kv_cols ? attn_dq_cast_kernel<HD, true> : attn_dq_cast_kernel<HD, false>;
   cast<<<tplr_sm_count() * 8, 256, 0, st>>>(dq32, part, p.split, (__nv_bfloat16*)dqkv, tokens, H * HD, kv_cols, (H + KV) * HD, ld_qkv,
                                             cosb, sinb, S);
