@@ -993,6 +993,7 @@ __global__ void __launch_bounds__(NT, 3) compress_tc_kernel(const CompressArgs a
   // writes to them (both behind a barrier)
   int (*s_hist)[256] = reinterpret_cast<int (*)[256]>(smem);
   __shared__ unsigned int s_thr[8];                      // per warp
+  __shared__ unsigned int s_took[2][TC_NCAND / 32];      // a bit for each candidate that is taken
   __shared__ long long s_gbase[2];                       // element offset of each chunk of the pair, -1: none
   __shared__ int s_cols[2];
   __shared__ TplrParamDesc s_d[2];                       // the chunks' table entries (20 registers a thread otherwise)
@@ -1131,25 +1132,28 @@ __global__ void __launch_bounds__(NT, 3) compress_tc_kernel(const CompressArgs a
     // Result: prefix = the k-th largest key, krem = how many keys equal to it belong to the selection.
     // Fast path: every warp finds the ceil(k / 4)-th largest of its 32 per-thread maxima; the smallest of the four
     // is a lower bound of the k-th largest key (k distinct keys are at least that large), so only the keys at or
-    // above it (a few dozen for k = 32) are candidates (the k-th of all 128 maxima is a little closer, for 350
-    // instructions a thread more and a barrier); they are compacted into shared memory and the exact threshold is found by counting
-    // among them.  No shared-memory atomics: the histogram of the radix select below serialises on the
-    // few exponent values that the keys share.  More candidates than fit (many equal keys) or
-    // k > 128 take the radix select.
+    // above it (a few dozen for k = 32) are candidates.  They are listed in shared memory in the order of the selection, and
+    // all that follows works on the list: a candidate is taken when fewer than k come before it.  402 M parameters, k = 32:
+    // 2800 us for the kernel with the threshold searched in the list and the 32 coefficients of every thread looked
+    // through again for their places, 2490 us here.  No shared-memory atomics: the histogram of the radix select below
+    // serialises on the few exponent values that the keys share.  More candidates than fit (many equal keys) or k > 128 take
+    // the radix select, a chunk of fewer than k non-zero coefficients the search of the threshold; those place the selection by
+    // a second look at the coefficients.
     unsigned int prefix = 0u, mask = 0u;
     int krem = k;
-    bool radix = true;
+    bool radix = true, listed = false;                   // listed: the selection was made from the candidates
     if (k <= 128 && (a.variant & 1)) {
-      unsigned int m = 0u;
+      float mf = 0.f;                                    // of the numbers: a NaN is a candidate whatever the bound
 #pragma unroll
-      for (int i = 0; i < 32; ++i) m = max(m, __float_as_uint(v[i]) & 0x7fffffffu);
-      int rank = 0;
-#pragma unroll
-      for (int j = 0; j < 32; ++j) {
-        const unsigned int o = __shfl_sync(0xffffffffu, m, j);
-        rank += (o > m) || (o == m && j < lane);
+      for (int i = 0; i < 32; ++i) mf = fmaxf(mf, fabsf(v[i]));
+      unsigned int m = __float_as_uint(mf), bound = 0u;
+      for (int need = (k + 3) / 4; need > 0;) {          // the maxima in order, equal ones together
+        bound = __reduce_max_sync(0xffffffffu, m);
+        if (bound == 0u) break;
+        need -= __popc(__ballot_sync(0xffffffffu, m == bound));
+        if (m == bound) m = 0u;
       }
-      if (rank == (k + 3) / 4 - 1) s_thr[warp] = m;
+      if (lane == 0) s_thr[warp] = bound;
       __syncthreads();
       // warps of chunk ch: 2ch, 2ch+1, 2ch+4, 2ch+5
       const unsigned int low = min(min(s_thr[2 * ch], s_thr[2 * ch + 1]), min(s_thr[2 * ch + 4], s_thr[2 * ch + 5]));
@@ -1157,9 +1161,11 @@ __global__ void __launch_bounds__(NT, 3) compress_tc_kernel(const CompressArgs a
       // no token touched, a null round) is resolved without any search: all non-zero keys and the first k - n_cand
       // zeros in order
       const unsigned int t0 = low ? low : 1u;
-      int cnt = 0;
+      const float t0f = __uint_as_float(t0);
+      unsigned int own = 0u;                             // bit i: v[i] is a candidate
 #pragma unroll
-      for (int i = 0; i < 32; ++i) cnt += (__float_as_uint(v[i]) & 0x7fffffffu) >= t0;
+      for (int i = 0; i < 32; ++i) own |= !(fabsf(v[i]) < t0f) ? 1u << i : 0u;
+      const int cnt = __popc(own);
       int incl = cnt;
 #pragma unroll
       for (int o = 1; o < 32; o <<= 1) {
@@ -1176,28 +1182,78 @@ __global__ void __launch_bounds__(NT, 3) compress_tc_kernel(const CompressArgs a
       // both chunks of the pair take the same path (the radix select synchronises the whole CTA)
       const int n_other = s_wsum[2 * (ch ^ 1)] + s_wsum[2 * (ch ^ 1) + 1] + s_wsum[2 * (ch ^ 1) + 4] + s_wsum[2 * (ch ^ 1) + 5];
       radix = n_cand > TC_NCAND || n_other > TC_NCAND;
+      listed = !radix && n_cand >= k && n_other >= s_d[ch ^ 1].k;
       if (!radix) {
+        // key and (sign, row-major index of Y[32*hf + i][rin]) of every candidate, in the order of the selection
         unsigned int* cand = reinterpret_cast<unsigned int*>(s_hist[ch]);
+        unsigned short* cidx = reinterpret_cast<unsigned short*>(smem + 2 * 256 * 4) + ch * TC_NCAND;
 #pragma unroll
         for (int i = 0; i < 32; ++i) {
-          const unsigned int key = __float_as_uint(v[i]) & 0x7fffffffu;
-          if (key >= t0) cand[off++] = key;
-        }
-        __syncthreads();
-        for (int j = lt; j < n_cand; j += 128) {
-          const unsigned int cj = cand[j];
-          int gt = 0, ge = 0;
-          for (int i = 0; i < n_cand; ++i) {
-            const unsigned int x = cand[i];
-            gt += x > cj; ge += x >= cj;
+          if (own & (1u << i)) {
+            const unsigned int x = __float_as_uint(v[i]);
+            cand[off] = x & 0x7fffffffu;
+            cidx[off++] = (unsigned short)(((hf * 32 + i) * 64 + rin) | ((x >> 31) << 15));
           }
-          if (gt < k && k <= ge) { s_bin[ch] = (int)cj; s_krem[ch] = k - gt; }   // ties write the same pair
         }
+        if (lt < 4 && n_cand + lt < TC_NCAND) cand[n_cand + lt] = 0u;       // the counts go four at a time
         __syncthreads();
-        if (n_cand < k) { prefix = 0u; krem = k - n_cand; }      // sparse chunk (only possible with t0 == 1)
-        else { prefix = (unsigned int)s_bin[ch]; krem = s_krem[ch]; }
+        if (listed) {
+          // A candidate is taken when fewer than k come before it: larger ones, and equal ones of a lower place.  Its slot is
+          // the number of taken ones before it in the list.
+          const int n4 = (n_cand + 3) & ~3;
+          bool take[TC_NCAND / 128];
+#pragma unroll
+          for (int rep = 0; rep < TC_NCAND / 128; ++rep) {
+            const int jb = rep * 128 + (lt & ~31), j = jb + lane;
+            take[rep] = false;
+            if (jb >= n_cand) continue;                  // the whole warp
+            const unsigned int cj = j < n_cand ? cand[j] : 0xffffffffu;
+            int before = 0;
+            auto count = [&](int from, int to, unsigned int over) {          // keys above `over`
+              for (int i = from; i < to; i += 4) {
+                const uint4 x = *reinterpret_cast<const uint4*>(cand + i);
+                before += (x.x > over) + (x.y > over) + (x.z > over) + (x.w > over);
+              }
+            };
+            count(0, jb, cj - 1u);                       // keys are at least 1
+            const int je = min(jb + 32, n4);
+            for (int i = jb; i < je; ++i) before += cand[i] > cj - (i < j ? 1u : 0u);
+            count(je, n4, cj);
+            take[rep] = j < n_cand && before < k;
+          }
+#pragma unroll
+          for (int rep = 0; rep < TC_NCAND / 128; ++rep) {
+            const unsigned int b = __ballot_sync(0xffffffffu, take[rep]);
+            if (lane == 0) s_took[ch][rep * 4 + (lt >> 5)] = b;
+          }
+          __syncthreads();
+#pragma unroll
+          for (int rep = 0; rep < TC_NCAND / 128; ++rep) {
+            if (take[rep]) {
+              const int word = rep * 4 + (lt >> 5), j = rep * 128 + lt;
+              int pos = __popc(s_took[ch][word] & ((1u << lane) - 1u));
+              for (int w = 0; w < word; ++w) pos += __popc(s_took[ch][w]);
+              const unsigned int ci = cidx[j];
+              s_sel_idx[ch][pos] = (int)(ci & 0xfffu);
+              s_sel_val[ch][pos] = __uint_as_float(cand[j] | ((ci & 0x8000u) << 16));
+            }
+          }
+        } else {
+          for (int j = lt; j < n_cand; j += 128) {
+            const unsigned int cj = cand[j];
+            int gt = 0, ge = 0;
+            for (int i = 0; i < n_cand; ++i) {
+              const unsigned int x = cand[i];
+              gt += x > cj; ge += x >= cj;
+            }
+            if (gt < k && k <= ge) { s_bin[ch] = (int)cj; s_krem[ch] = k - gt; }   // ties write the same pair
+          }
+          __syncthreads();
+          if (n_cand < k) { prefix = 0u; krem = k - n_cand; }      // sparse chunk (only possible with t0 == 1)
+          else { prefix = (unsigned int)s_bin[ch]; krem = s_krem[ch]; }
+        }
       }
-      __syncthreads();            // s_hist, s_wsum, s_bin and s_krem are reused below
+      __syncthreads();            // s_hist, s_wsum, s_bin and s_krem are reused below; a list's selection is complete
     }
 #pragma unroll 1
     for (int pass = 0; radix && pass < 4; ++pass) {
@@ -1243,42 +1299,44 @@ __global__ void __launch_bounds__(NT, 3) compress_tc_kernel(const CompressArgs a
       __syncthreads();
     }
     // ---- ordered compaction inside each chunk's four warps -----------------------------------
-    int gcnt = 0, qcnt = 0;
+    if (!listed) {
+      int gcnt = 0, qcnt = 0;
 #pragma unroll
-    for (int i = 0; i < 32; ++i) {
-      const unsigned int key = __float_as_uint(v[i]) & 0x7fffffffu;
-      gcnt += key > prefix; qcnt += key == prefix;
-    }
-    const int packed = gcnt | (qcnt << 16);
-    int incl = packed;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-      int t = __shfl_up_sync(0xffffffffu, incl, o);
-      if (lane >= o) incl += t;
-    }
-    if (lane == 31) s_wsum[warp] = incl;
-    __syncthreads();
-    int woff = 0;
-    {
-      // warps of chunk ch in order: 2ch, 2ch+1, 2ch+4, 2ch+5
-      const int order[4] = {2 * ch, 2 * ch + 1, 2 * ch + 4, 2 * ch + 5};
-#pragma unroll
-      for (int jj = 0; jj < 4; ++jj) if (order[jj] != warp && ((order[jj] < warp && (order[jj] >> 2) == (warp >> 2)) || (order[jj] >> 2) < (warp >> 2))) woff += s_wsum[order[jj]];
-    }
-    const int excl = incl - packed + woff;
-    int gb = excl & 0xffff, qb = excl >> 16;
-#pragma unroll
-    for (int i = 0; i < 32; ++i) {
-      const unsigned int key = __float_as_uint(v[i]) & 0x7fffffffu;
-      int pos = -1;
-      if (key > prefix) { pos = gb + min(qb, krem); ++gb; }
-      else if (key == prefix) { if (qb < krem) pos = gb + qb; ++qb; }
-      if (pos >= 0 && pos < TPLR_TILE) {
-        s_sel_idx[ch][pos] = (hf * 32 + i) * 64 + rin;     // row-major index of Y[32*hf + i][rin]
-        s_sel_val[ch][pos] = v[i];
+      for (int i = 0; i < 32; ++i) {
+        const unsigned int key = __float_as_uint(v[i]) & 0x7fffffffu;
+        gcnt += key > prefix; qcnt += key == prefix;
       }
+      const int packed = gcnt | (qcnt << 16);
+      int incl = packed;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        int t = __shfl_up_sync(0xffffffffu, incl, o);
+        if (lane >= o) incl += t;
+      }
+      if (lane == 31) s_wsum[warp] = incl;
+      __syncthreads();
+      int woff = 0;
+      {
+        // warps of chunk ch in order: 2ch, 2ch+1, 2ch+4, 2ch+5
+        const int order[4] = {2 * ch, 2 * ch + 1, 2 * ch + 4, 2 * ch + 5};
+#pragma unroll
+        for (int jj = 0; jj < 4; ++jj) if (order[jj] != warp && ((order[jj] < warp && (order[jj] >> 2) == (warp >> 2)) || (order[jj] >> 2) < (warp >> 2))) woff += s_wsum[order[jj]];
+      }
+      const int excl = incl - packed + woff;
+      int gb = excl & 0xffff, qb = excl >> 16;
+#pragma unroll
+      for (int i = 0; i < 32; ++i) {
+        const unsigned int key = __float_as_uint(v[i]) & 0x7fffffffu;
+        int pos = -1;
+        if (key > prefix) { pos = gb + min(qb, krem); ++gb; }
+        else if (key == prefix) { if (qb < krem) pos = gb + qb; ++qb; }
+        if (pos >= 0 && pos < TPLR_TILE) {
+          s_sel_idx[ch][pos] = (hf * 32 + i) * 64 + rin;     // row-major index of Y[32*hf + i][rin]
+          s_sel_val[ch][pos] = v[i];
+        }
+      }
+      __syncthreads();
     }
-    __syncthreads();
     // ---- payload ------------------------------------------------------------------------------
     if (active) {
       const int cl = c - d.chunk_begin;

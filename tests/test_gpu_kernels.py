@@ -732,3 +732,40 @@ def test_nodes_in_python_and_cpp_give_the_same_bits(op, T, with_buffers, monkeyp
             assert torch.allclose(a.float(), b.float(), atol=30 * T * 2 ** -23, rtol=2 ** -7 if a.dtype == torch.bfloat16 else 0)
         elif a is not None:
             assert torch.equal(a, b)
+
+
+@pytest.mark.parametrize("topk", [2, 32, 64])
+def test_selection_from_the_candidate_list_is_the_radix_selection(topk):
+    """The listed selection against the radix select of the same kernel, bit for bit: chunks of zeros beside full ones, single
+    coefficients, equal magnitudes (a place and its mirror), few non-zero values, infinities and NaN."""
+    from templar_b200.ops import native
+
+    def run(variant):
+        eng = WindowEngine(_Bag([(256, 320), (192, 64)]).to(DEV), EngineConfig(topk=topk), device=DEV)
+        eng.snapshot()
+        g = torch.Generator(device=DEV).manual_seed(3)
+        x = torch.randn(eng.ef.numel(), device=DEV, generator=g) * 1e-2
+        c = x[: 256 * 320].view(4, 64, 5, 64).transpose(1, 2)               # [chunk row, chunk column, 64, 64]
+        c[0, 0] = 0                                                         # nothing beside a full chunk
+        c[0, 2] = 1.0                                                       # one coefficient, the rest rounding
+        c[1, 0] = c[1, 0] + c[1, 0].t()                                     # equal pairs
+        c[1, 1] = 0
+        c[1, 1, 5, 7] = 1.0
+        c[1, 2] = torch.sign(c[1, 2])
+        c[1, 3] = 0
+        c[1, 3, 0] = 1.0                                                    # 64 non-zero coefficients
+        c[2, 0] *= 1e-38                                                    # subnormal coefficients
+        c[2, 1, 3, 3] = float("inf")
+        c[2, 2, 3, 3] = float("nan")
+        c[2, 3] *= 1e30
+        eng.ef.copy_(x)
+        old = native.lib().tplr_compress_set_variant(variant)
+        try:
+            eng.compress()
+            torch.cuda.synchronize()
+        finally:
+            native.lib().tplr_compress_set_variant(old)
+        return eng.own_idx, eng.own_val.view(torch.int32), eng.ef.view(torch.int32)
+
+    for a, b in zip(run(7), run(6)):
+        assert torch.equal(a, b)
