@@ -293,6 +293,8 @@ attn_fwd_kernel(const __grid_constant__ AttnFwdParams p) {
   tcgen05_fence_before();
   __syncthreads();
   tcgen05_fence_after();
+  grid_wait();
+  grid_release();
   const uint32_t tmem_base = s_tmem_base;
   // S columns 0..127, O from column 128.  P lies over S at DH = 128; at 64 it has the 64 columns that O leaves, so that the
   // next block's S is computed as soon as the softmax warps hold this one's in registers (AHEAD).
@@ -490,8 +492,7 @@ int launch_fwd(const void* qkv, void* out, float* lse, int B, int S, int H, int 
   cudaError_t e = cudaFuncSetAttribute(attn_fwd_kernel<DH>, cudaFuncAttributeMaxDynamicSharedMemorySize, fwd_smem<DH>());
   if (e != cudaSuccess) return (int)e;
   const unsigned grid = (unsigned)(((S + BQ - 1) / BQ) * H * B);
-  attn_fwd_kernel<DH><<<grid, FWD_THREADS, fwd_smem<DH>(), st>>>(p);
-  return (int)cudaGetLastError();
+  return (int)launch_pdl(attn_fwd_kernel<DH>, grid, FWD_THREADS, fwd_smem<DH>(), st, p);
 }
 }  // namespace
 
@@ -605,6 +606,8 @@ attn_bwd_kernel(const __grid_constant__ AttnBwdParams p) {
   tcgen05_fence_before();
   __syncthreads();
   tcgen05_fence_after();
+  grid_wait();
+  grid_release();
   const uint32_t tmem_base = s_tmem_base;
   // dQ of a step lies over its dP at DH = 128; at 64 it has columns of its own
   const uint32_t tS = tmem_base, tdP = tmem_base + 128, tdV = tmem_base + 256, tdK = tmem_base + 256 + DH, tdQ = DH == 64 ? tmem_base + 384 : tdP;
@@ -1020,6 +1023,9 @@ __global__ void __launch_bounds__(256) attn_dq_cast_kernel(const float* __restri
                                                            __nv_bfloat16* __restrict__ dqkv, long long tokens, int q_cols, int kv_cols,
                                                            int rot_cols, long long ld, const float* __restrict__ cosb,
                                                            const float* __restrict__ sinb, int S) {
+  grid_wait();
+  grid_release();
+  behind_grid_wait(dq32); behind_grid_wait(part); behind_grid_wait(cosb); behind_grid_wait(sinb);
   const unsigned w8 = (unsigned)(PARTS ? q_cols + kv_cols : q_cols) / 8;
   const long long n8 = tokens * w8;                     // below 2^32: the scratch would be 137 GB there
   for (long long v = (long long)blockIdx.x * blockDim.x + threadIdx.x; v < n8; v += (long long)gridDim.x * blockDim.x) {
@@ -1136,6 +1142,8 @@ attn_bwd2_kernel(const __grid_constant__ AttnBwd2Params p) {
   tcgen05_fence_before();
   __syncthreads();
   tcgen05_fence_after();
+  grid_wait();
+  grid_release();
   const uint32_t tmem_base = s_tmem_base;
   const uint32_t tS0 = tmem_base, tdP = tmem_base + 128, tdQ = tmem_base + 192, tdV = tmem_base + 256, tdK = tmem_base + 384;
   const uint32_t sK = smem_u32(smem), sV = sK + TILE_BYTES, sQ0 = sV + TILE_BYTES, sdO0 = sQ0 + 2 * B2_QTILE,
@@ -1475,11 +1483,10 @@ int launch_bwd(const void* qkv, const void* out, const void* dout, const float* 
   p.rope_cos = cosb; p.rope_sin = sinb;
   cudaError_t e = cudaFuncSetAttribute(attn_bwd_kernel<HD>, cudaFuncAttributeMaxDynamicSharedMemorySize, bwd_smem<HD>());
   if (e != cudaSuccess) return (int)e;
-  attn_bwd_kernel<HD><<<(unsigned)(((S + BKV - 1) / BKV) * KV * B * p.split), bwd_threads<HD>(), bwd_smem<HD>(), st>>>(p);
+  e = launch_pdl(attn_bwd_kernel<HD>, (unsigned)(((S + BKV - 1) / BKV) * KV * B * p.split), bwd_threads<HD>(), bwd_smem<HD>(), st, p);
+  if (e != cudaSuccess) return (int)e;
   auto cast = kv_cols ? attn_dq_cast_kernel<HD, true> : attn_dq_cast_kernel<HD, false>;
-  cast<<<tplr_sm_count() * 8, 256, 0, st>>>(dq32, part, p.split, (__nv_bfloat16*)dqkv, tokens, H * HD, kv_cols, (H + KV) * HD, ld_qkv,
-                                            cosb, sinb, S);
-  return (int)cudaGetLastError();
+  return (int)launch_pdl(cast, tplr_sm_count() * 8, 256, 0, st, dq32, part, p.split, (__nv_bfloat16*)dqkv, tokens, H * HD, kv_cols, (H + KV) * HD, ld_qkv, cosb, sinb, S);
 }
 }  // namespace
 

@@ -86,6 +86,31 @@ static __device__ __forceinline__ float block_max(float v, float* red) {
   return red[0];
 }
 
+// Programmatic dependent launch: a kernel launched with pdl_attr may start while the one before it on the stream still runs, and
+// sets up its barriers and tensor memory meanwhile; nothing before grid_wait reads or writes global memory.  grid_release lets the
+// next one be launched; it is called behind grid_wait, so a kernel never runs beside the one before the last.  A chain of
+// GEMMs gains 2.5 us a kernel (2048 x 768 x 768 12.4 -> 9.9 us): launch latency, barriers, tensor memory, tensor maps.
+static __device__ __forceinline__ void grid_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+static __device__ __forceinline__ void grid_release() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+// A pointer whose loads may be taken for loads of constants (const, __restrict__): taken anew behind grid_wait, so that none of
+// them can be moved before it.
+template <class T> static __device__ __forceinline__ void behind_grid_wait(T* __restrict__& p) { asm volatile("" : "+l"(p) :: "memory"); }
+
+static inline cudaLaunchAttribute pdl_attr(bool on = true) {
+  cudaLaunchAttribute a = {};
+  a.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  a.val.programmaticStreamSerializationAllowed = on ? 1 : 0;
+  return a;
+}
+template <class... P, class... A>
+static inline cudaError_t launch_pdl(void (*kern)(P...), dim3 grid, unsigned block, size_t smem, cudaStream_t st, A&&... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid; cfg.blockDim = dim3(block); cfg.dynamicSmemBytes = smem; cfg.stream = st;
+  cudaLaunchAttribute attr = pdl_attr();
+  cfg.attrs = &attr; cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, kern, static_cast<P>(args)...);
+}
+
 static inline int tplr_sm_count() {
   static int sms = 0;
   if (!sms) {

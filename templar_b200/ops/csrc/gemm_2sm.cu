@@ -680,6 +680,7 @@ gemm2_kernel(const __grid_constant__ Gemm2Params p) {
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
   }
+  if (threadIdx.x == 32) { prefetch_map(&p.tmA); prefetch_map(&p.tmB); }
   if (threadIdx.x < 32) s_ready[threadIdx.x] = 0;
   if (warp == 1 && is_compute) {
     asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], 512;" ::"r"(smem_u32(&s_tmem_base)) : "memory");
@@ -689,6 +690,8 @@ gemm2_kernel(const __grid_constant__ Gemm2Params p) {
   __syncthreads();
   cluster_sync_all();   // the peer's barriers are initialised before any remote arrive or TMA completion
   tcgen05_fence_after();
+  grid_wait();          // everything up to here ran beside the kernel before
+  grid_release();
   const uint32_t tmem_base = s_tmem_base;
   const uint32_t sbase = smem_u32(smem);
   const uint32_t sA = sbase, sB = sbase + n_stages * A_STAGE, sEpi = sbase + RING_BYTES;
@@ -919,13 +922,15 @@ int launch2(Gemm2Params& p, int n_comm_pairs, int max_pairs, cudaStream_t st) {
   cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES);
   if (e != cudaSuccess) return (int)e;
   cudaLaunchConfig_t cfg = {};
-  cudaLaunchAttribute attr[1];
+  cudaLaunchAttribute attr[2];
   attr[0].id = cudaLaunchAttributeClusterDimension;
   attr[0].val.clusterDim.x = 2; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
   cfg.blockDim = dim3(NUM_THREADS);
   cfg.dynamicSmemBytes = SMEM_BYTES;
   cfg.stream = st;
-  cfg.attrs = attr; cfg.numAttrs = 1;
+  // not for the fused collectives: their CTAs wait for other ranks' kernels and start as one
+  attr[1] = pdl_attr(p.world == 1);
+  cfg.attrs = attr; cfg.numAttrs = 2;
   // all CTAs must be resident at once: compute CTAs wait for comm CTAs of the same launch
   static int max_clusters[2][2][7] = {};
   int& mc = max_clusters[A_MN][B_MN][EPI];
@@ -1057,6 +1062,9 @@ int pick_scatter_splits(int M, int N, int K) {
 // aligned.
 __global__ void __launch_bounds__(256) add_planes_kernel(const float* __restrict__ x, float* __restrict__ c, long long M, int n4, long long ldc,
                                                          int n_planes, long long plane) {
+  grid_wait();
+  grid_release();
+  behind_grid_wait(x);
   const long long total = M * n4;
   for (long long i = blockIdx.x * 256LL + threadIdx.x; i < total; i += gridDim.x * 256LL) {
     const long long row = i / n4;
@@ -1074,6 +1082,9 @@ __global__ void __launch_bounds__(256) add_planes_kernel(const float* __restrict
 // multiples of 8, 16-byte aligned.
 __global__ void __launch_bounds__(256) round_rows_kernel(const float* __restrict__ x, __nv_bfloat16* __restrict__ y, long long M, int n8,
                                                          long long ldc, int parts, long long plane) {
+  grid_wait();
+  grid_release();
+  behind_grid_wait(x);
   const long long total = M * n8;
   for (long long i = blockIdx.x * 256LL + threadIdx.x; i < total; i += gridDim.x * 256LL) {
     float4 a = reinterpret_cast<const float4*>(x)[2 * i], b = reinterpret_cast<const float4*>(x)[2 * i + 1];
@@ -1175,7 +1186,7 @@ TPLR_API int tplr_gemm2_acc_split(const void* A, const void* B, float* C, float*
   if (n_planes) {
     const long long n = ((long long)M * (N / 4) + 255) / 256;
     const unsigned grid = (unsigned)(n < 8LL * tplr_sm_count() ? n : 8LL * tplr_sm_count());
-    add_planes_kernel<<<grid, 256, 0, (cudaStream_t)stream>>>(ws, C, M, N / 4, ldc, n_planes, (long long)p.plane_rows * N);
+    return (int)launch_pdl(add_planes_kernel, grid, 256, 0, (cudaStream_t)stream, ws, C, M, N / 4, ldc, n_planes, (long long)p.plane_rows * N);
   }
   return (int)cudaGetLastError();
 }
@@ -1199,9 +1210,8 @@ TPLR_API int tplr_gemm2_bf16_split(const void* A, const void* B, void* C, float*
   if (int r = dispatch2(p, a_mn, b_mn, 2, 0, 0, (cudaStream_t)stream)) return r;
   const long long n = (long long)M * (N / 8);
   const unsigned grid = (unsigned)((n + 255) / 256 < 8LL * tplr_sm_count() ? (n + 255) / 256 : 8LL * tplr_sm_count());
-  round_rows_kernel<<<grid, 256, 0, (cudaStream_t)stream>>>(ws, (__nv_bfloat16*)C, M, N / 8, ldc, p.k_splits,
-                                                            (long long)p.plane_rows * N);
-  return (int)cudaGetLastError();
+  return (int)launch_pdl(round_rows_kernel, grid, 256, 0, (cudaStream_t)stream, ws, (__nv_bfloat16*)C, M, N / 8, ldc, p.k_splits,
+                         (long long)p.plane_rows * N);
 }
 
 // GU[M, 2F] = X W^T for the packed weight W = [w1; w3] ([2F, K] bf16, K-major) and H[M, F] = silu(GU[:, :F]) * GU[:, F:]

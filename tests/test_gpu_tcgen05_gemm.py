@@ -291,3 +291,32 @@ def test_feed_forward_refuses_weights_of_other_widths(grad, backend):
 def test_narrow_tiles(M, N, K, epi, b_mn):
     """Products whose 256-wide tiles would leave SMs idle: last tiles of 8 to 184 columns, with and without parts of K."""
     _check(M, N, K, epi == "acc", b_mn, epi)
+
+
+def test_chain_of_dependent_launches(backend):
+    """Kernels that may start while the one before them runs: a chain in which each reads what the one before wrote (products, parts
+    of K added by a second kernel, attention both ways, a torch kernel between), against the same chain with a wait behind every call."""
+    torch.manual_seed(0)
+    bf = lambda *s, std=1.0: (torch.randn(*s, device=DEV) * std).to(torch.bfloat16)      # noqa: E731
+    x, w, up, wide = bf(512, 384), bf(384, 384, std=0.05), bf(8192, 384, std=0.05), bf(384, 8192, std=0.01)
+    mg = torch.zeros(384, 384, device=DEV)
+
+    def chain(wait):
+        h, grad = x, mg.clone()
+        for _ in range(4):
+            h = OF.gemm(h, w)
+            wait()
+            h = OF.gemm(OF.gemm(h, up), wide)                  # K = 8192: parts
+            wait()
+            q = OF.attention_packed(OF.gemm(h, w).view(2, 256, 384), 2, 2, 64)
+            wait()
+            h = OF.gemm(torch.cat([q.reshape(512, 128)] * 3, dim=1), w) + x
+            wait()
+            OF.gemm(h, h, a_mn=True, b_mn=True, out=grad, accumulate=True)
+            wait()
+        return h, grad
+
+    want = chain(torch.cuda.synchronize)
+    for _ in range(20):
+        assert all(torch.equal(a, b) for a, b in zip(chain(lambda: None), want))
+    assert int(OF.status_word(DEV).item()) == 0
