@@ -769,3 +769,32 @@ def test_selection_from_the_candidate_list_is_the_radix_selection(topk):
 
     for a, b in zip(run(7), run(6)):
         assert torch.equal(a, b)
+
+
+@pytest.mark.parametrize("V,ld", [(4088, 4096), (4096, 4096), (4104, 4112), (32000, 32000), (36864, 36872), (36872, 36872), (32004, 32008)])
+def test_cross_entropy_rows_in_shared_memory_and_beyond(V, ld):
+    """Row lengths on both sides of the limits of the kernel that keeps a row in shared memory, with a pitch: loss and gradient against
+    64 bits, ignored rows, masked logits (-inf), a row of equal ones, and nothing written between the rows."""
+    from templar_b200.ops import native
+
+    torch.manual_seed(V)
+    T = 37
+    wide = torch.full((T, ld), 3.0, device=DEV, dtype=torch.bfloat16)
+    z = wide[:, :V]
+    z.copy_(torch.randn(T, V, device=DEV) * 4)
+    z[3, : V // 2] = float("-inf")
+    z[4] = 1.5
+    labels = torch.randint(0, V, (T,), device=DEV)
+    labels[3], labels[5], labels[6], labels[7] = V - 1, -100, 0, V - 1
+    zr = z.double().requires_grad_()
+    want = torch.nn.functional.cross_entropy(zr, labels, ignore_index=-100)
+    want.backward()
+    losses, loss, n = torch.empty(T, device=DEV), torch.empty(1, device=DEV), torch.empty(1, device=DEV, dtype=torch.int32)
+    st = torch.zeros(1, device=DEV, dtype=torch.int32)
+    native.check(native.lib().tplr_cross_entropy(wide.data_ptr(), labels.data_ptr(), losses.data_ptr(), n.data_ptr(), loss.data_ptr(), 1.0, T, V,
+                                                 ld, -100, 1, st.data_ptr(), native.stream_ptr()), "cross_entropy")
+    assert int(st) == 0
+    assert abs(float(loss) - float(want)) < 1e-5 * float(want)
+    got, g = wide[:, :V].double(), zr.grad
+    assert ((got - g).abs() <= g.abs() * 2 ** -8 + 1e-9).all()          # one rounding to bf16, and the exponential's own error
+    assert (wide[:, V:] == 3).all()
