@@ -954,11 +954,13 @@ def _own_attention_faster(B: int, S: int, n_heads: int, n_kv: int, hd: int, grad
     Heads of 128 with sequences of whole tiles stay here.  For heads of 64 and odd lengths the library kernel does more
     products a second, but pays for a copy of q, k and v, of their gradients, and for its launches: which weighs more depends on
     the sequence length alone, once the device is the bound.  Measured at 16384 tokens, library against own, microseconds:
-    forward and backward, 12 heads of 64, S 3072 975 and 844, 4096 1097 and 1040, 8192 1468 and 1682; 32 on 8 heads of 64, S 2048
-    1971 and 1868, 3072 2119 and 2163; 16 heads of 128, S 6000 2468 and 2382, 8000 3597 and 3676; 32 on 8 heads of 128, S 4000
-    5683 and 5632, 6000 4878 and 5053.  Forward alone, fused, 32 on 8 heads of 64, S 1024 418 and 415, 2048 491 and 510; 16 heads of
-    128, S 1000 535 and 521, 3000 591 and 620.  Forward alone on a packed projection nothing is copied: 12 heads of 64, S 512 81
-    and 71 (launches), 2048 99 and 118; only calls bound by their launches are faster here (1 x 2048, 12 heads of 64: 82 and 35)."""
+    forward and backward, 12 heads of 64, S 3072 771 and 602, 4096 907 and 742, 8192 1285 and 1172, 16384 2050 and 2158; 32 on 8 heads of
+    64, S 2048 1587 and 1274, 4096 2088 and 1982, 8192 3094 and 3334; 16 heads of 128, S 6000 2137 and 2106, 8000 3181 and 3387; 32 on 8
+    heads of 128, S 3000 3724 and 3676, 4000 4335 and 4415 (the limits lie where they lay before the own backward of heads of 64 became
+    faster, on the safe side there).  Forward alone, fused, 32 on 8 heads of 64, S 1024 299 and 278, 2048 374 and 361, 3072 405 and 410;
+    12 heads of 64, S 2048 150 and 148; 16 heads of 128, S 1000 402 and 382, 3000 464 and 469.  Forward alone on a packed projection
+    nothing is copied: 12 heads of 64, S 1024 55 and 62, 2048 82 and 92; only calls bound by their launches are faster here (1 x 2048,
+    12 heads of 64: 38 and 27)."""
     if hd == 128 and S % 128 == 0:
         return True
     group = n_heads // n_kv
