@@ -515,17 +515,18 @@ TPLR_API int tplr_attention_fwd(const void* qkv, void* out, float* lse, int B, i
 //   P = exp2(S*scale - lse), dS = P * (dP - delta) * scale   (softmax warps, one query row per thread;
 //                                      P and dS go to shared memory as bf16 in 128-byte-swizzled tiles)
 //   dV += P^T dO, dK += dS^T Q        (accumulated in TMEM over the whole walk)
-//   dQ_partial = dS K                 (into the dP columns, then TMA reduce-add into the fp32 dQ buffer)
+//   dQ_partial = dS K                 (at DH = 128 into the dP columns, then TMA reduce-add into the fp32 dQ buffer)
 // The same swizzled tile serves as a K-major operand of one MMA and an MN-major operand of another,
 // so Q, dO, P and dS are each stored once.  K and V stay resident in shared memory.
 //
 // What bounds it is the chain of a step, not the tensor pipe (five products of 512 cycles each at DH = 128): so the step
 // is split where P is ready.  S of the next step is issued as soon as every warp has read this one's (Q has two buffers
-// for it) and runs, with dV, while the warps form dS; dP of the next step runs while they exponentiate its S.
-// B 8, S 2048, 16 heads of 128: 692 us with the parts of a step one after the other, 620 us here; the
-// shared-memory traffic of the five products and of P, dS and dQ would allow about 350.  Issuing the products from a
-// warp-uniform loop (elect_one) instead of under `lane == 0`: 2 to 10 %, the most at heads of 64 (119 -> 112 us at 8 x 1024 x 12),
-// whose products are the shortest; forward 182 -> 170 us at 8 x 2048 x 16 of 128, 104 -> 89 at 8 x 2048 x 12 of 64.
+// for it) and runs, with dV, while the warps form dS; dK and dQ run while they take the next step's exponentials, and dQ is
+// drained behind those (at 64 by warps of its own).  A step of 128 x 128 took 6400 to 7900 cycles at DH = 128 and 5200 at 64 with
+// dQ drained at its own end, 5250 to 6300 and 3950 behind the exponentials; the shared-memory traffic of the products, P, dS and dQ
+// would allow 4600 and 2900.  With the delta and rounding passes, B 8, S 2048: 16 heads of 128 728 us with the products issued
+// under `lane == 0`, 718 from a warp-uniform loop (elect_one), 655 with the late drain; 12 heads of 64 349, 320 and 279, with warps of
+// their own 263.  Forward, issued from a warp-uniform loop: 182 -> 170 us and 104 -> 89.
 // ------------------------------------------------------------------------------------------ //
 namespace {
 

@@ -691,7 +691,7 @@ gemm2_kernel(const __grid_constant__ Gemm2Params p) {
   cluster_sync_all();   // the peer's barriers are initialised before any remote arrive or TMA completion
   tcgen05_fence_after();
   grid_wait();          // everything up to here ran beside the kernel before
-  grid_release();
+  if (p.world == 1) grid_release();      // a fused collective has its SMs to itself until it ends
   const uint32_t tmem_base = s_tmem_base;
   const uint32_t sbase = smem_u32(smem);
   const uint32_t sA = sbase, sB = sbase + n_stages * A_STAGE, sEpi = sbase + RING_BYTES;
