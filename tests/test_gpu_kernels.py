@@ -798,3 +798,22 @@ def test_cross_entropy_rows_in_shared_memory_and_beyond(V, ld):
     got, g = wide[:, :V].double(), zr.grad
     assert ((got - g).abs() <= g.abs() * 2 ** -8 + 1e-9).all()          # one rounding to bf16, and the exponential's own error
     assert (wide[:, V:] == 3).all()
+
+
+@pytest.mark.parametrize("T,D", [(5, 520), (33, 768), (2400, 776), (2400, 1024), (33, 1032), (9, 1536), (17, 1544)])
+def test_norm_backward_by_vectors_per_lane(T, D):
+    """Widths at the edges of the register forms (3, 4 and 6 vectors a lane), fewer and more rows than resident warps."""
+    from templar_b200.ops import native
+
+    torch.manual_seed(D)
+    bf = lambda *s: torch.randn(*s, device=DEV).to(torch.bfloat16)      # noqa: E731
+    dy, x, w, dres = bf(T, D), bf(T, D), bf(D), bf(T, D)
+    xd, wd = x.double().requires_grad_(), w.double().requires_grad_()
+    rstd = torch.rsqrt(xd.square().mean(-1, keepdim=True) + 1e-5)
+    (xd * rstd * wd).backward(dy.double())
+    dx, dw = torch.empty_like(x), torch.zeros(D, device=DEV)
+    native.check(native.lib().tplr_add_rmsnorm_bwd(dy.data_ptr(), x.data_ptr(), w.data_ptr(), rstd.detach().float().contiguous().data_ptr(),
+                                                   dres.data_ptr(), dx.data_ptr(), dw.data_ptr(), T, D, native.stream_ptr()), "rmsnorm_bwd")
+    want = xd.grad + dres.double()
+    assert ((dx.double() - want).abs() <= want.abs() * 2 ** -8 + 1e-4).all()          # one rounding to bf16
+    assert ((dw.double() - wd.grad).norm() / wd.grad.norm()).item() < 1e-5            # fp32 sums
