@@ -1149,13 +1149,13 @@ __global__ void __launch_bounds__(NT, 3) compress_tc_kernel(const CompressArgs a
     // all that follows works on the list: a candidate is taken when fewer than k come before it.  402 M parameters, k = 32:
     // 2800 us for the kernel with the threshold searched in the list and the 32 coefficients of every thread looked
     // through again for their places, 2490 us here.  No shared-memory atomics: the histogram of the radix select below
-    // serialises on the few exponent values that the keys share.  More candidates than fit (many equal keys) or k > 128 take
+    // serialises on the few exponent values that the keys share.  More candidates than fit (many equal keys) take
     // the radix select, a chunk of fewer than k non-zero coefficients the search of the threshold; those place the selection by
     // a second look at the coefficients.
     unsigned int prefix = 0u, mask = 0u;
     int krem = k;
     bool radix = true, listed = false;                   // listed: the selection was made from the candidates
-    if (k <= 128 && (a.variant & 1)) {
+    if (k <= TPLR_TILE && (a.variant & 1)) {             // s_sel_idx and s_sel_val hold no more
       float mf = 0.f;                                    // of the numbers: a NaN is a candidate whatever the bound
 #pragma unroll
       for (int i = 0; i < 32; ++i) mf = fmaxf(mf, fabsf(v[i]));

@@ -109,6 +109,7 @@ class WindowEngine:
                                     n_buffers=cfg.gather_buffers, group=group, heap=heap, status=self.status,
                                     materialize=materialize)
         L = self.layout = self.store.layout
+        self._largest_k = max((s.topk(cfg.topk) for s in L.specs), default=0)
         n_shard = self.store.n_shard
         z = lambda n, dt=torch.float32: torch.zeros(n, dtype=dt, device=self.device)
         self.exp_avg, self.exp_avg_sq = z(n_shard), z(n_shard)
@@ -653,6 +654,8 @@ class WindowEngine:
         self._own_merged = False
         if not self.cuda:
             return self._compress_torch(null_round)
+        # the kernels hold a chunk's selection in arrays of this size (TPLR_TILE) and cannot check k on the host
+        native.require(self._largest_k <= 64, f"compression kernels select at most 64 values a chunk, not {self._largest_k}")
         idx_ptr, val_ptr = own_slot_ptrs or (self.own_idx.data_ptr(), self.own_val.data_ptr())
         if self.world_size > 1 and own_slot_ptrs is None:
             self.own_idx.zero_()                    # only this rank's chunks are written: the rest must read as

@@ -1,9 +1,14 @@
 """CPU checks of engine-level helpers that have a GPU fast path elsewhere."""
 
+import re
+from pathlib import Path
+
+import pytest
 import torch
 
 from templar_b200 import compress as C
 from templar_b200.models.llama import ModelArgs, build_model
+from templar_b200.ops import native
 from templar_b200.parallel.tensor_parallel import TensorParallel
 from templar_b200.parallel.window_engine import EngineConfig, WindowEngine
 
@@ -135,3 +140,33 @@ def quantised_window_identity(device):
 
 def test_quantised_window_identity_cpu():
     quantised_window_identity("cpu")
+
+
+@pytest.mark.parametrize("topk,refused", [(64, False), (66, True), (128, True), (4096, True)])
+def test_more_values_than_the_kernels_hold_are_refused(topk, refused, monkeypatch):
+    """The compression kernels keep a chunk's selection in arrays of 64: a larger ``topk`` is an error before anything is
+    launched, while the torch path takes it."""
+    args = ModelArgs(dim=128, n_layers=1, n_heads=2, vocab_size=256, intermediate_size=256, max_seq_len=32)
+    eng = WindowEngine(build_model(args, device="cpu", dtype=torch.float32, seed=2), EngineConfig(topk=topk), device="cpu")
+    eng.snapshot()
+    eng.compress()
+
+    class Reached(Exception):
+        pass
+
+    def lib():
+        raise Reached
+
+    monkeypatch.setattr(native, "lib", lib)
+    eng.cuda = True
+    with pytest.raises(ValueError if refused else Reached):
+        eng.compress()
+
+
+def test_list_selection_stays_inside_its_arrays():
+    """The selection from the candidate list writes a place for every value taken, k of them, without a bound of its own: the
+    kernel enters it only for k that its arrays hold."""
+    text = (Path(native.__file__).parent / "csrc" / "compress.cu").read_text()
+    kernel = text[text.index("compress_tc_kernel(const CompressArgs a)"):]
+    size = re.search(r"__shared__ int s_sel_idx\[2\]\[(\w+)\]", kernel).group(1)
+    assert re.search(r"if \(k <= (\w+) && \(a\.variant & 1\)\)", kernel).group(1) == size
