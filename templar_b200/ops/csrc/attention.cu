@@ -1026,7 +1026,7 @@ __global__ void __launch_bounds__(256) attn_dq_cast_kernel(const float* __restri
                                                            const float* __restrict__ sinb, int S) {
   grid_wait();
   grid_release();
-  behind_grid_wait(dq32); behind_grid_wait(part); behind_grid_wait(cosb); behind_grid_wait(sinb);
+  behind_grid_wait(dq32); behind_grid_wait(part); behind_grid_wait(dqkv); behind_grid_wait(cosb); behind_grid_wait(sinb);
   const unsigned w8 = (unsigned)(PARTS ? q_cols + kv_cols : q_cols) / 8;
   const long long n8 = tokens * w8;                     // below 2^32: the scratch would be 137 GB there
   for (long long v = (long long)blockIdx.x * blockDim.x + threadIdx.x; v < n8; v += (long long)gridDim.x * blockDim.x) {

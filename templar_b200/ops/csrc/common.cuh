@@ -92,8 +92,9 @@ static __device__ __forceinline__ float block_max(float v, float* red) {
 // GEMMs gains 2.5 us a kernel (2048 x 768 x 768 12.4 -> 9.9 us): launch latency, barriers, tensor memory, tensor maps.
 static __device__ __forceinline__ void grid_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 static __device__ __forceinline__ void grid_release() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
-// A pointer whose loads may be taken for loads of constants (const, __restrict__): taken anew behind grid_wait, so that none of
-// them can be moved before it.
+// A __restrict__ pointer is taken anew behind grid_wait: its accesses may otherwise be moved before it.  Loads through a const one may
+// be taken for loads of constants, and no statement that does not get the pointer, the wait among them, counts as touching what
+// any other one points to.
 template <class T> static __device__ __forceinline__ void behind_grid_wait(T* __restrict__& p) { asm volatile("" : "+l"(p) :: "memory"); }
 
 static inline cudaLaunchAttribute pdl_attr(bool on = true) {

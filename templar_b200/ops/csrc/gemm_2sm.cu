@@ -1064,7 +1064,7 @@ __global__ void __launch_bounds__(256) add_planes_kernel(const float* __restrict
                                                          int n_planes, long long plane) {
   grid_wait();
   grid_release();
-  behind_grid_wait(x);
+  behind_grid_wait(x); behind_grid_wait(c);
   const long long total = M * n4;
   for (long long i = blockIdx.x * 256LL + threadIdx.x; i < total; i += gridDim.x * 256LL) {
     const long long row = i / n4;
@@ -1084,7 +1084,7 @@ __global__ void __launch_bounds__(256) round_rows_kernel(const float* __restrict
                                                          long long ldc, int parts, long long plane) {
   grid_wait();
   grid_release();
-  behind_grid_wait(x);
+  behind_grid_wait(x); behind_grid_wait(y);
   const long long total = M * n8;
   for (long long i = blockIdx.x * 256LL + threadIdx.x; i < total; i += gridDim.x * 256LL) {
     float4 a = reinterpret_cast<const float4*>(x)[2 * i], b = reinterpret_cast<const float4*>(x)[2 * i + 1];

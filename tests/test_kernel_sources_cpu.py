@@ -28,3 +28,29 @@ def test_every_kernel_that_asks_for_copies_drains_them(src):
     assert arming
     for k in arming:
         assert "Drain drain" in k, k[:200]
+
+
+def _kernels(src):
+    """(name, parameter list, body) of every kernel of a source file."""
+    text = re.sub(r"//[^\n]*", "", (CSRC / src).read_text())
+    for m in re.finditer(r"__global__[^;{]*?(\w+)\s*\(([^(){}]*)\)\s*\{", text):
+        depth, i = 1, m.end()
+        while depth:
+            depth += {"{": 1, "}": -1}.get(text[i], 0)
+            i += 1
+        yield m.group(1), m.group(2), text[m.end():i]
+
+
+@pytest.mark.parametrize("src", sorted(p.name for p in CSRC.glob("*.cu") if "grid_wait();" in p.read_text()))
+def test_restrict_pointers_are_taken_anew_behind_the_grid_wait(src):
+    """A kernel that may start while the one before it runs touches no memory before ``grid_wait``.  The compiler may move an
+    access through a ``__restrict__`` pointer across the wait unless the pointer goes through ``behind_grid_wait`` there, those
+    that are written and read as well as the constant ones."""
+    waiting = [k for k in _kernels(src) if "grid_wait();" in k[2]]
+    assert waiting
+    for name, params, body in waiting:
+        pointers = re.findall(r"__restrict__\s+(\w+)", params)
+        before, behind = body.split("grid_wait();", 1)
+        taken = set(re.findall(r"behind_grid_wait\((\w+)\)", behind))
+        assert set(pointers) <= taken, (name, set(pointers) - taken)
+        assert not any(re.search(rf"\b{p}\b", before) for p in pointers), name
