@@ -8,7 +8,7 @@
 // CE of the torchtitan LLaMA (models/llama3/model/model.py:69-95, :236-237, :276-277;
 // components/loss.py:18-22) and torch.optim.AdamW(fused=True) + clip_grad_norm_
 // (neurons/trainer.py:280-298, :940).
-#include "tcgen05.cuh"
+#include "common.cuh"
 #include "no_alloc.h"
 #include <atomic>
 
@@ -399,12 +399,14 @@ __global__ void __launch_bounds__(512) ce_kernel(bf16* __restrict__ logits, cons
   }
 }
 
-// The same with the row in shared memory: it comes and goes as one bulk copy, and the three looks at it (maximum, sum, gradient) do
-// not go through L2 again, which bounded the kernel above (2.1 GB moved for 1.05 GB of logits).  Three CTAs share an SM, so one row
-// loads while others are computed; the maximum is taken on packed bf16 pairs, the rest on packed fp32 ones.  What bounds it
-// now are the two exponentials of a logit (16 a cycle and SM) and DRAM.  8192 rows of 32000: 296 us with the kernel above, 193 here
-// (5.4 TB/s); of 36864 330 and 210, of 8064 113 and 93, of 4096 (16384 rows) 144 and 142, of 2048 56 and 58; 256 rows of 32000 23 and 21.
-constexpr int CE_ROW_MAX = 36864, CE_ROW_MIN = 4096;     // logits of a row: three rows of 72 KB in an SM; short rows do not pay the copies
+// The same with the row in shared memory: the three looks at it (maximum, sum, gradient) do not go through L2 again, which bounded
+// the kernel above (2.1 GB moved for 1.05 GB of logits).  It comes by 16-byte asynchronous copies, whose wait cannot run out: a
+// row whose loss is not written has no way to be told from one whose is (sum_rows_kernel adds whatever the array holds).
+// Three CTAs share an SM, so one row loads while others are computed; the maximum is taken on packed bf16 pairs, the rest on
+// packed fp32 ones.  What bounds it now are the two exponentials of a logit (16 a cycle and SM) and DRAM.  8192 rows of 32000:
+// 290 us with the kernel above, 175 here (6.0 TB/s; 186 with the row coming and going as one bulk copy); of 36864 324 and 196, of
+// 8064 109 and 82, of 4096 (16384 rows) 139 and 124, of 2048 56 and 58 (bulk copies); 256 rows of 32000 20 and 17, loss alone 159 and 104.
+constexpr int CE_ROW_MAX = 36864, CE_ROW_MIN = 4096;     // logits of a row: three rows of 72 KB in an SM; short rows do not gain
 static __device__ __forceinline__ unsigned long long ce_pack(float a, float b) {
   unsigned long long v;
   asm("mov.b64 %0, {%1, %2};" : "=l"(v) : "f"(a), "f"(b));
@@ -424,12 +426,9 @@ static __device__ __forceinline__ void ce_exp2(uint32_t w, unsigned long long ne
 __global__ void __launch_bounds__(512, 3) ce_row_kernel(bf16* __restrict__ logits, const long long* __restrict__ labels,
                                                         float* __restrict__ losses, const int* __restrict__ n_valid,
                                                         float grad_scale, int V, long long ld, long long ignore_index,
-                                                        int write_grad, unsigned int* __restrict__ status) {
-  using namespace tplr_tc;
-  extern __shared__ __align__(128) uint8_t ce_row[];
+                                                        int write_grad) {
+  extern __shared__ __align__(16) uint8_t ce_row[];
   __shared__ float red[32];
-  __shared__ __align__(8) uint64_t bar;
-  __shared__ int s_abort;
   const long long row = blockIdx.x;
   bf16* z = logits + row * ld;
   const long long label = labels[row];
@@ -440,25 +439,11 @@ __global__ void __launch_bounds__(512, 3) ce_row_kernel(bf16* __restrict__ logit
       for (int i = threadIdx.x; i < nv; i += 512) reinterpret_cast<uint4*>(z)[i] = make_uint4(0, 0, 0, 0);
     return;
   }
-  const uint32_t buf = smem_u32(ce_row), b = smem_u32(&bar);
-  if (threadIdx.x == 0) {
-    s_abort = 0;
-    mbar_init(b, 1);
-    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-    mbar_expect_tx(b, (uint32_t)V * 2u);
-    asm volatile("cp.async.bulk.shared::cta.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
-                 ::"r"(buf), "l"(z), "r"((uint32_t)V * 2u), "r"(b) : "memory");
-  }
-  __syncthreads();
-  if (!__syncthreads_and(mbar_wait(b, 0, &s_abort))) {
-    if (threadIdx.x == 0) {
-      Drain drain;
-      drain.wait(b, 0);
-      if (status) atomicOr(status, TPLR_ST_WAIT_TIMEOUT);
-    }
-    return;
-  }
-  uint4* zs = reinterpret_cast<uint4*>(ce_row);
+  const uint32_t buf = (uint32_t)__cvta_generic_to_shared(ce_row);
+  for (int i = threadIdx.x; i < nv; i += 512)
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(buf + 16u * (uint32_t)i), "l"(z + 8 * i) : "memory");
+  asm volatile("cp.async.wait_all;" ::: "memory");         // this thread's; it looks at no others until the label's logit
+  const uint4* zs = reinterpret_cast<const uint4*>(ce_row);
   __nv_bfloat162 m2 = __halves2bfloat162(__ushort_as_bfloat16(0xff80), __ushort_as_bfloat16(0xff80));       // -inf
   for (int i = threadIdx.x; i < nv; i += 512) {
     const uint4 q = zs[i];
@@ -487,7 +472,6 @@ __global__ void __launch_bounds__(512, 3) ce_row_kernel(bf16* __restrict__ logit
   const float sc = grad_scale / (float)max(n_valid[0], 1);
   const unsigned long long inv = ce_pack(sc / s, sc / s);
   const int lv = (int)(label / 8), le = (int)(label % 8);
-  __syncthreads();                                       // the label's logit has been read
   for (int i = threadIdx.x; i < nv; i += 512) {
     const uint4 q = zs[i];
     const uint32_t w[4] = {q.x, q.y, q.z, q.w};
@@ -503,23 +487,16 @@ __global__ void __launch_bounds__(512, 3) ce_row_kernel(bf16* __restrict__ logit
       const __nv_bfloat162 h = __floats2bfloat162_rn(a, c);
       o[e] = *reinterpret_cast<const uint32_t*>(&h);
     }
-    zs[i] = make_uint4(o[0], o[1], o[2], o[3]);
-  }
-  asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    asm volatile("cp.async.bulk.global.shared::cta.bulk_group [%0], [%1], %2;" ::"l"(z), "r"(buf), "r"((uint32_t)V * 2u) : "memory");
-    asm volatile("cp.async.bulk.commit_group;" ::: "memory");
-    asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
+    reinterpret_cast<uint4*>(z)[i] = make_uint4(o[0], o[1], o[2], o[3]);
   }
 }
 // rows: see ce_kernel
 static cudaError_t launch_ce(bf16* logits, const long long* labels, float* losses, const int* n_valid, float grad_scale, long long T, int V,
-                             long long ld, long long ignore_index, int write_grad, unsigned int* status, cudaStream_t st) {
+                             long long ld, long long ignore_index, int write_grad, cudaStream_t st) {
   if (V % 8 == 0 && V >= CE_ROW_MIN && V <= CE_ROW_MAX) {
     const cudaError_t e = cudaFuncSetAttribute(ce_row_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, CE_ROW_MAX * 2);
     if (e != cudaSuccess) return e;
-    ce_row_kernel<<<(unsigned)T, 512, (size_t)V * 2, st>>>(logits, labels, losses, n_valid, grad_scale, V, ld, ignore_index, write_grad, status);
+    ce_row_kernel<<<(unsigned)T, 512, (size_t)V * 2, st>>>(logits, labels, losses, n_valid, grad_scale, V, ld, ignore_index, write_grad);
   } else {
     ce_kernel<<<(unsigned)T, 512, 0, st>>>(logits, labels, losses, n_valid, grad_scale, V, ld, ignore_index, write_grad);
   }
@@ -547,7 +524,7 @@ TPLR_API int tplr_cross_entropy(void* logits, const long long* labels, float* lo
   if ((ld % 8) || ld < V || V <= 0 || ((uintptr_t)logits & 15)) return (int)cudaErrorInvalidValue;
   cudaStream_t st = (cudaStream_t)stream;
   count_valid_kernel<<<1, 1024, 0, st>>>(labels, T, ignore_index, V, n_valid, status);
-  if (const cudaError_t e = launch_ce((bf16*)logits, labels, losses, n_valid, grad_scale, T, V, ld, ignore_index, write_grad, status, st)) return (int)e;
+  if (const cudaError_t e = launch_ce((bf16*)logits, labels, losses, n_valid, grad_scale, T, V, ld, ignore_index, write_grad, st)) return (int)e;
   sum_rows_kernel<<<1, 1024, 0, st>>>(losses, T, n_valid, 1.f, loss_out);
   return (int)cudaGetLastError();
 }
@@ -958,10 +935,10 @@ TPLR_API int tplr_cross_entropy_noalloc(void* logits, const long long* labels, f
   int* n_valid = reinterpret_cast<int*>(sc);
   float* losses = sc + CE_SCRATCH_HEADER;
   cudaStream_t st = (cudaStream_t)stream;
-  // count_valid_kernel overwrites n_valid and ce_kernel writes losses[0..rows) before
+  // count_valid_kernel overwrites n_valid and the loss kernel writes losses[0..rows) before
   // sum_rows_kernel reads them, so whatever an earlier call left in the array is never used.
   count_valid_kernel<<<1, 1024, 0, st>>>(labels, rows, ignore_index, vocab, n_valid, nullptr);
-  if (const cudaError_t e = launch_ce((bf16*)logits, labels, losses, n_valid, grad_scale, rows, vocab, ld, ignore_index, write_grad, nullptr, st)) return (int)e;
+  if (const cudaError_t e = launch_ce((bf16*)logits, labels, losses, n_valid, grad_scale, rows, vocab, ld, ignore_index, write_grad, st)) return (int)e;
   sum_rows_kernel<<<1, 1024, 0, st>>>(losses, rows, n_valid, 1.f, loss_out);
   return (int)cudaGetLastError();
 }

@@ -54,3 +54,14 @@ def test_restrict_pointers_are_taken_anew_behind_the_grid_wait(src):
         taken = set(re.findall(r"behind_grid_wait\((\w+)\)", behind))
         assert set(pointers) <= taken, (name, set(pointers) - taken)
         assert not any(re.search(rf"\b{p}\b", before) for p in pointers), name
+
+
+def test_every_exit_of_a_loss_kernel_has_written_its_row():
+    """The mean is taken over the rows' array whatever it holds, and the entry that must not allocate has no status word, so a
+    kernel that writes rows of losses has neither a wait that can run out nor a ``return`` in front of the row's loss."""
+    kernels = [k for k in _kernels("elementwise.cu") if re.search(r"\blosses\[\w+\] = ", k[2])]
+    assert len(kernels) == 2
+    for name, _, body in kernels:
+        assert "mbar_wait" not in body, name
+        for exit_at in re.finditer(r"\breturn;", body):
+            assert re.search(r"\blosses\[row\] = ", body[:exit_at.start()]), name
