@@ -10,6 +10,7 @@
 // (neurons/trainer.py:280-298, :940).
 #include "common.cuh"
 #include "no_alloc.h"
+#include <cuda/std/type_traits>
 #include <atomic>
 
 typedef __nv_bfloat16 bf16;
@@ -404,8 +405,10 @@ __global__ void __launch_bounds__(512) ce_kernel(bf16* __restrict__ logits, cons
 // row whose loss is not written has no way to be told from one whose is (sum_rows_kernel adds whatever the array holds).
 // Three CTAs share an SM, so one row loads while others are computed; the maximum is taken on packed bf16 pairs, the rest on
 // packed fp32 ones.  What bounds it now are the two exponentials of a logit (16 a cycle and SM) and DRAM.  8192 rows of 32000:
-// 290 us with the kernel above, 175 here (6.0 TB/s; 186 with the row coming and going as one bulk copy); of 36864 324 and 196, of
-// 8064 109 and 82, of 4096 (16384 rows) 139 and 124, of 2048 56 and 58 (bulk copies); 256 rows of 32000 20 and 17, loss alone 159 and 104.
+// 290 us with the kernel above, 178 here (5.9 TB/s; 186 with the row coming and going as one bulk copy); of 36864 324 and 199, of
+// 8064 109 and 85, of 4096 (16384 rows) 139 and 128, of 2048 56 and 58 (bulk copies); 256 rows of 32000 20 and 17, loss alone 159 and
+// 103.  Exponentials below the smallest normal number are kept, as in the kernel above, by the threads that find a logit so low
+// (the least is taken beside the largest): 193 us when every thread kept them, 175 without.
 constexpr int CE_ROW_MAX = 36864, CE_ROW_MIN = 4096;     // logits of a row: three rows of 72 KB in an SM; short rows do not gain
 static __device__ __forceinline__ unsigned long long ce_pack(float a, float b) {
   unsigned long long v;
@@ -413,15 +416,20 @@ static __device__ __forceinline__ unsigned long long ce_pack(float a, float b) {
   return v;
 }
 static __device__ __forceinline__ void ce_unpack(unsigned long long v, float& a, float& b) { asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v)); }
-// exp(x - m) of a packed bf16 pair
-static __device__ __forceinline__ void ce_exp2(uint32_t w, unsigned long long negm, float& a, float& b) {
+// exp(x - m) of a packed bf16 pair.  LOW keeps results below the smallest normal number, for three instructions more each.
+template <bool LOW> static __device__ __forceinline__ void ce_exp2(uint32_t w, unsigned long long negm, float& a, float& b) {
   unsigned long long d = ce_pack(__uint_as_float(w << 16), __uint_as_float(w & 0xffff0000u));
   const unsigned long long l2e = ce_pack(1.4426950408889634f, 1.4426950408889634f);
   asm("add.rn.f32x2 %0, %0, %1;" : "+l"(d) : "l"(negm));
   asm("mul.rn.f32x2 %0, %0, %1;" : "+l"(d) : "l"(l2e));
   ce_unpack(d, a, b);
-  asm("ex2.approx.ftz.f32 %0, %0;" : "+f"(a));
-  asm("ex2.approx.ftz.f32 %0, %0;" : "+f"(b));
+  if (LOW) {
+    asm("ex2.approx.f32 %0, %0;" : "+f"(a));
+    asm("ex2.approx.f32 %0, %0;" : "+f"(b));
+  } else {
+    asm("ex2.approx.ftz.f32 %0, %0;" : "+f"(a));
+    asm("ex2.approx.ftz.f32 %0, %0;" : "+f"(b));
+  }
 }
 __global__ void __launch_bounds__(512, 3) ce_row_kernel(bf16* __restrict__ logits, const long long* __restrict__ labels,
                                                         float* __restrict__ losses, const int* __restrict__ n_valid,
@@ -445,24 +453,31 @@ __global__ void __launch_bounds__(512, 3) ce_row_kernel(bf16* __restrict__ logit
   asm volatile("cp.async.wait_all;" ::: "memory");         // this thread's; it looks at no others until the label's logit
   const uint4* zs = reinterpret_cast<const uint4*>(ce_row);
   __nv_bfloat162 m2 = __halves2bfloat162(__ushort_as_bfloat16(0xff80), __ushort_as_bfloat16(0xff80));       // -inf
+  __nv_bfloat162 n2 = __halves2bfloat162(__ushort_as_bfloat16(0x7f80), __ushort_as_bfloat16(0x7f80));       // inf
   for (int i = threadIdx.x; i < nv; i += 512) {
     const uint4 q = zs[i];
     const __nv_bfloat162* h = reinterpret_cast<const __nv_bfloat162*>(&q);
     m2 = __hmax2(__hmax2(m2, __hmax2(h[0], h[1])), __hmax2(h[2], h[3]));
+    n2 = __hmin2(__hmin2(n2, __hmin2(h[0], h[1])), __hmin2(h[2], h[3]));
   }
   const float m = block_max(fmaxf(__low2float(m2), __high2float(m2)), red);
   const unsigned long long negm = ce_pack(-m, -m);
+  // of the logits that this thread looks at all three times; exp(-87) is still a normal number
+  const bool low = fminf(__low2float(n2), __high2float(n2)) - m < -87.f;
   unsigned long long s2 = 0ull;                          // (0.f, 0.f)
-  for (int i = threadIdx.x; i < nv; i += 512) {
-    const uint4 q = zs[i];
-    const uint32_t w[4] = {q.x, q.y, q.z, q.w};
+  auto sum_part = [&](auto LOW) {
+    for (int i = threadIdx.x; i < nv; i += 512) {
+      const uint4 q = zs[i];
+      const uint32_t w[4] = {q.x, q.y, q.z, q.w};
 #pragma unroll
-    for (int e = 0; e < 4; ++e) {
-      float a, c;
-      ce_exp2(w[e], negm, a, c);
-      asm("add.rn.f32x2 %0, %0, %1;" : "+l"(s2) : "l"(ce_pack(a, c)));
+      for (int e = 0; e < 4; ++e) {
+        float a, c;
+        ce_exp2<decltype(LOW)::value>(w[e], negm, a, c);
+        asm("add.rn.f32x2 %0, %0, %1;" : "+l"(s2) : "l"(ce_pack(a, c)));
+      }
     }
-  }
+  };
+  if (low) sum_part(cuda::std::true_type{}); else sum_part(cuda::std::false_type{});
   float s0, s1;
   ce_unpack(s2, s0, s1);
   const float s = block_sum(s0 + s1, red);
@@ -472,23 +487,26 @@ __global__ void __launch_bounds__(512, 3) ce_row_kernel(bf16* __restrict__ logit
   const float sc = grad_scale / (float)max(n_valid[0], 1);
   const unsigned long long inv = ce_pack(sc / s, sc / s);
   const int lv = (int)(label / 8), le = (int)(label % 8);
-  for (int i = threadIdx.x; i < nv; i += 512) {
-    const uint4 q = zs[i];
-    const uint32_t w[4] = {q.x, q.y, q.z, q.w};
-    uint32_t o[4];
+  auto grad_part = [&](auto LOW) {
+    for (int i = threadIdx.x; i < nv; i += 512) {
+      const uint4 q = zs[i];
+      const uint32_t w[4] = {q.x, q.y, q.z, q.w};
+      uint32_t o[4];
 #pragma unroll
-    for (int e = 0; e < 4; ++e) {
-      float a, c;
-      ce_exp2(w[e], negm, a, c);
-      unsigned long long g = ce_pack(a, c);
-      asm("mul.rn.f32x2 %0, %0, %1;" : "+l"(g) : "l"(inv));
-      ce_unpack(g, a, c);
-      if (i == lv && e == (le >> 1)) { if (le & 1) c -= sc; else a -= sc; }
-      const __nv_bfloat162 h = __floats2bfloat162_rn(a, c);
-      o[e] = *reinterpret_cast<const uint32_t*>(&h);
+      for (int e = 0; e < 4; ++e) {
+        float a, c;
+        ce_exp2<decltype(LOW)::value>(w[e], negm, a, c);
+        unsigned long long g = ce_pack(a, c);
+        asm("mul.rn.f32x2 %0, %0, %1;" : "+l"(g) : "l"(inv));
+        ce_unpack(g, a, c);
+        if (i == lv && e == (le >> 1)) { if (le & 1) c -= sc; else a -= sc; }
+        const __nv_bfloat162 h = __floats2bfloat162_rn(a, c);
+        o[e] = *reinterpret_cast<const uint32_t*>(&h);
+      }
+      reinterpret_cast<uint4*>(z)[i] = make_uint4(o[0], o[1], o[2], o[3]);
     }
-    reinterpret_cast<uint4*>(z)[i] = make_uint4(o[0], o[1], o[2], o[3]);
-  }
+  };
+  if (low) grad_part(cuda::std::true_type{}); else grad_part(cuda::std::false_type{});
 }
 // rows: see ce_kernel
 static cudaError_t launch_ce(bf16* logits, const long long* labels, float* losses, const int* n_valid, float grad_scale, long long T, int V,

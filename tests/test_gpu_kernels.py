@@ -817,3 +817,29 @@ def test_norm_backward_by_vectors_per_lane(T, D):
     want = xd.grad + dres.double()
     assert ((dx.double() - want).abs() <= want.abs() * 2 ** -8 + 1e-4).all()          # one rounding to bf16
     assert ((dw.double() - wd.grad).norm() / wd.grad.norm()).item() < 1e-5            # fp32 sums
+
+
+@pytest.mark.parametrize("V", [4088, 4096, 32000])
+def test_cross_entropy_keeps_exponentials_below_the_smallest_normal_number(V):
+    """Logits 88 to 103 below the row's largest: their exponentials are subnormal in fp32, and a large scale of the gradient shows
+    them.  Against 64 bits: one rounding to bf16, and two of the 2^-149 that such an exponential is a multiple of."""
+    from templar_b200.ops import native
+
+    T, scale = 4, 2.0 ** 40
+    gap = torch.arange(V, device=DEV) % 31 * 0.5 + 88
+    z = (3 - gap).to(torch.bfloat16).repeat(T, 1)
+    z[:, 1] = 3.0
+    z[1, V // 2:] = 3.0                                                     # parts of a row without small ones
+    z[2, V // 2:] = float("-inf")
+    labels = torch.tensor([0, 1, 2, V - 1], device=DEV)
+    p = torch.softmax(z.double(), dim=-1)
+    sums = torch.exp(z.double() - 3).sum(dim=-1, keepdim=True)
+    want = p.clone()
+    want[torch.arange(T), labels] -= 1
+    want *= scale / T
+    losses, loss, n = torch.empty(T, device=DEV), torch.empty(1, device=DEV), torch.empty(1, device=DEV, dtype=torch.int32)
+    st = torch.zeros(1, device=DEV, dtype=torch.int32)
+    native.check(native.lib().tplr_cross_entropy(z.data_ptr(), labels.data_ptr(), losses.data_ptr(), n.data_ptr(), loss.data_ptr(), scale, T, V,
+                                                 V, -100, 1, st.data_ptr(), native.stream_ptr()), "cross_entropy")
+    assert int(st) == 0
+    assert ((z.double() - want).abs() <= want.abs() * 2 ** -8 + 2 * 2.0 ** -149 * scale / T / sums).all()
