@@ -985,7 +985,9 @@ int forced_splits() {                                     // tuning override
 // and a second kernel adds the planes in order, the same bits on every run, which parts added as they arrive would not give.
 // It costs a launch (4000 cycles) and the planes' bytes, 5000 a cycle while they stay in L2 and 2700 beyond.  768 x 768 x 8192
 // accumulating (9 tiles) 45.2 us whole, 18.8 in eight parts; 2304 x 768 x 8192 45.2 whole, 35.0 in two; 2048 x 768 x 6144 bf16 35.0
-// whole, 24.0 in three; 8192 x 768 x 32000 341 and 294 in three.  A cut has to win 10 %, a narrower tile 3 %.
+// whole, 24.0 in three; 8192 x 768 x 32000 341 and 294 in three.  A cut has to win 10 %, a narrower tile 3 %.  Where the result is
+// stored in fp32, what bounds a short K is the store, so a narrower tile must not take more waves there: 472 x 9168 x 64 8.0 us
+// in one wave of 256, 8.4 in two of 128; 712 x 5960 x 248 9.3 and 9.9; with K of 1000 the two are even.
 //
 // The costs (cycles) were fitted on 70 shapes of 300 to 16384 rows, K 300 to 32000, each with every width and 1 to 8 parts.
 double plan_cost(int M, int N, int K, bool a_mn, bool b_mn, int epi, int tile_n, int parts) {
@@ -1005,8 +1007,11 @@ double plan_cost(int M, int N, int K, bool a_mn, bool b_mn, int epi, int tile_n,
 int pick_tile(int M, int N, int K, bool a_mn, bool b_mn, int epi, int parts = 1, int col_unit = 64) {
   int best = TILE_N;
   double best_cost = plan_cost(M, N, K, a_mn, b_mn, epi, TILE_N, parts);
+  const int pairs = tplr_sm_count() / 2;
+  auto waves = [&](int tn) { return ((long long)((M + TILE_M - 1) / TILE_M) * ((N + tn - 1) / tn) + pairs - 1) / pairs; };
   for (const int tn : {192, 128}) {
     if (tn % col_unit || (tn == 192 && b_mn)) continue;
+    if (epi == 2 && waves(tn) > waves(TILE_N)) continue;
     const double cost = plan_cost(M, N, K, a_mn, b_mn, epi, tn, parts);
     if (cost < 0.97 * best_cost) { best = tn; best_cost = cost; }
   }
