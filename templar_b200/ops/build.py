@@ -35,7 +35,7 @@ HOST_FLAGS = ["-O2", "-std=c++17", "-fPIC", "-shared", "-fvisibility=hidden"]
 # Approximate intrinsics and flush-to-zero only where the arithmetic is a softmax in base 2 (the flash
 # attention kernels).  The loss, the norms, the optimizer, the quantiser and the compression kernels are
 # compiled with IEEE division / square root and keep denormals; where they want a fast exponential they
-# call __expf explicitly.
+# call __expf or its instruction explicitly.
 FAST_MATH_SOURCES = {"attention.cu"}
 
 

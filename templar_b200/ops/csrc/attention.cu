@@ -1422,8 +1422,9 @@ __global__ void __launch_bounds__(256) attn_dq_transpose_kernel(const float* __r
 
 }  // namespace
 
-// Backward variant: 1 = one 128-row query block per step, P / dS through shared memory (default: measured
-// 0.72 ms against 0.76 ms for B8 S2048 H16 KV8); 2 = pipelined transposed form, 64 query rows per step.
+// Backward variant: 1 = one 128-row query block per step, P / dS through shared memory (default: with the delta and rounding
+// passes 0.57 ms against 0.65 to 0.70 at B 8, S 2048, 16 on 8 heads, 0.66 against 0.81 at 16 on 16, 0.09 against 0.15 at B 1, S 1024,
+// 32 on 8); 2 = pipelined transposed form, 64 query rows per step, slower at every size tried.
 static int g_bwd_variant = [] { const char* e = getenv("TPLR_ATTN_BWD"); return (e && atoi(e) == 2) ? 2 : 1; }();
 TPLR_API int tplr_attention_set_bwd_variant(int v) {
   if (v != 1 && v != 2) return -1;

@@ -86,7 +86,8 @@ __global__ void __launch_bounds__(256) add_rmsnorm_fwd_warp_kernel(const bf16* _
 }
 
 // Two CTAs an SM up to four vectors a lane: at 157 registers one was resident and the launch, made for two, ran in two waves.
-// 16384 x 1024: 59 -> 39 us; 16384 x 768, with three vectors instead of four, 49 -> 32; 2048 x 1536 with six instead of eight 14.4 -> 12.4.
+// 16384 x 1024: 57 -> 37 us; 16384 x 768, with three vectors instead of four, 42 -> 24, 4096 x 768 11.4 -> 8.4.  Rows of more than 1024
+// elements come here when they are fewer than 64 or off their 16-byte boundary: 63 x 1536 with six vectors instead of eight 7.7 -> 7.0.
 template <int VPL>
 __global__ void __launch_bounds__(256, VPL <= 4 ? 2 : 1) add_rmsnorm_bwd_warp_kernel(const bf16* __restrict__ dy, const bf16* __restrict__ x,
                                                                    const bf16* __restrict__ w, const float* __restrict__ rstd,

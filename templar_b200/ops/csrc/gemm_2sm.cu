@@ -2,12 +2,12 @@
 //
 //   C[M,N] (+)= op(A) * op(B)     same operand layouts as tplr_gemm_bf16 (K-major or MN-major)
 //
-// A cluster of two CTAs computes one 256 x 256 tile: each CTA stages its own 128 rows of A and
-// its own 128 rows of B (so every shared-memory byte feeds two SMs' tensor cores), the even CTA
-// issues tcgen05.mma.cta_group::2, and each CTA drains its 128 x 256 half of the accumulator
-// from its own tensor memory.  6 smem stages of 32 KB per CTA, two accumulator buffers.
+// A cluster of two CTAs computes one tile of 256 rows and 256, 192 or 128 columns (see plan_cost): each CTA stages its own
+// 128 rows of A and its own half of the tile's rows of B (so every shared-memory byte feeds two SMs' tensor cores), the even
+// CTA issues tcgen05.mma.cta_group::2, and each CTA drains its 128 rows of the accumulator from its own tensor memory.  A ring
+// of 192 KB per CTA (6 stages at 256 and 192 columns, 8 at 128), two accumulator buffers.
 // The producer and the issuer are warp-uniform loops with one elected lane behind the issuing statements (see elect_one):
-// 505 cycles a k block of 64, which is the tensor pipe's 512 within the clock readings, for every operand layout; under
+// 505 cycles a k block of 64 at 256 columns, which is the tensor pipe's 512 within the clock readings, for every operand layout; under
 // `lane == 0` 620 to 625.  2048 x 18944 x 2048 (8 tiles a pair): 113 -> 102 us K-major, 123 -> 102 us MN-major.
 //
 // Fused collectives (one process per GPU, peers mapped through the symmetric heap):

@@ -11,7 +11,8 @@
 //
 // CTA = 6 warps: warp 0 TMA producer, warp 1 MMA issuer + TMEM owner, warps 2-5 epilogue
 // (one per TMEM lane quadrant). Tile 128 x 256 x 64, 4 smem stages (192 KB), persistent
-// over tiles. No cluster multicast is used anywhere. Every mbarrier wait is bounded; on
+// over tiles. The issuing loops are run by one lane, as those of the CTA-pair kernel were before elect_one: what a
+// comparison of the two shows is that as well as the pairing. No cluster multicast is used anywhere. Every mbarrier wait is bounded; on
 // expiry the CTA records TPLR_ST_WAIT_TIMEOUT in *status, all roles leave their loops, TMEM
 // is freed and the kernel returns.
 //

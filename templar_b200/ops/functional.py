@@ -953,13 +953,14 @@ def _own_attention_faster(B: int, S: int, n_heads: int, n_kv: int, hd: int, grad
 
     Heads of 128 with sequences of whole tiles stay here.  For heads of 64 and odd lengths the library kernel does more
     products a second, but pays for a copy of q, k and v, of their gradients, and for its launches: which weighs more depends on
-    the sequence length alone, once the device is the bound.  Measured at 16384 tokens, library against own, microseconds:
-    forward and backward, 12 heads of 64, S 3072 771 and 602, 4096 907 and 742, 8192 1285 and 1172, 16384 2050 and 2158; 32 on 8 heads of
-    64, S 2048 1587 and 1274, 4096 2088 and 1982, 8192 3094 and 3334; 16 heads of 128, S 6000 2137 and 2106, 8000 3181 and 3387; 32 on 8
-    heads of 128, S 3000 3724 and 3676, 4000 4335 and 4415 (the limits lie where they lay before the own backward of heads of 64 became
-    faster, on the safe side there).  Forward alone, fused, 32 on 8 heads of 64, S 1024 299 and 278, 2048 374 and 361, 3072 405 and 410;
-    12 heads of 64, S 2048 150 and 148; 16 heads of 128, S 1000 402 and 382, 3000 464 and 469.  Forward alone on a packed projection
-    nothing is copied: 12 heads of 64, S 1024 55 and 62, 2048 82 and 92; only calls bound by their launches are faster here (1 x 2048,
+    the sequence length alone, once the device is the bound.  The limits were measured with earlier own kernels; with the present
+    ones the two are even further up at heads of 64, and near 3500 at grouped heads of 128.  At 16384 tokens, library against own, microseconds:
+    forward and backward, 12 heads of 64 (limit 4096), S 3072 771 and 602, 4096 907 and 742, 8192 1285 and 1172, 16384 2050 and 2158;
+    32 on 8 heads of 64 (2560), S 2048 1587 and 1274, 4096 2088 and 1982, 8192 3094 and 3334; 16 heads of 128 (6656), S 6000 2137 and
+    2106, 8000 3181 and 3387; 32 on 8 heads of 128 (4608), S 3000 3724 and 3676, 4000 4335 and 4415.
+    Forward alone, fused, 32 on 8 heads of 64 (1536), S 1024 299 and 278, 2048 374 and 361, 3072 405 and 410; 12 heads of 64, S 2048 150
+    and 148; 16 heads of 128 (2048), S 1000 402 and 382, 3000 464 and 469.  Forward alone on a packed projection nothing is copied: 12
+    heads of 64, S 1024 55 and 62, 2048 82 and 92; only calls bound by their launches are faster here (1 x 2048,
     12 heads of 64: 38 and 27)."""
     if hd == 128 and S % 128 == 0:
         return True
